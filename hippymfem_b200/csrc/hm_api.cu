@@ -46,6 +46,7 @@ extern "C" int hm_lattice_create(int nx, int ny, int nz, double Lx, double Ly, d
   if (nnz > INT32_MAX || L.ne * 729 > INT32_MAX || L.tz > 65535 || L.ty > 65535) return HM_ERR_UNSUPPORTED;
   hm_lattice* h = new (std::nothrow) hm_lattice;
   if (!h) return HM_ERR_NOMEM;
+  hm_plan_apply(&L);
   h->L = L;
   *out = h;
   return HM_OK;

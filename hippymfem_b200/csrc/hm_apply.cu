@@ -1,0 +1,623 @@
+// The matrix-free Jacobian apply y = A(D) x of the Q2 lattice in one pass (sm_100a), with
+// the smoothing steps of the multigrid cycle and the inner product of a CG step in its
+// epilogue.
+//
+// A CTA owns a tile of T1 x T2 element columns and marches T3 element layers up z, one
+// thread per column (the "cell" (cx, cy, cz) owns the nodes (2cx + {0,1}, 2cy + {0,1},
+// 2cz + {0,1}); the cells nx, ny, nz are virtual and own the last node only).  Node planes
+// arrive in a ring in shared memory by asynchronous copies, two layers ahead; D of the
+// next layer as one TMA box.  Per layer a thread interpolates its
+// two new node planes to the 3 x 3 in-plane Gauss points, the three planes to the 27
+// points, takes the derivatives *at the Gauss points* (three points carry a quadratic, so
+// a 1D derivative is the 3 x 3 matrix (-3 4 -1; -1 0 1; 1 -4 3) / (2 sqrt(0.15))), and goes
+// back the same way.  The upper plane's in-plane values, and its sums before they return
+// to nodes, stay in the thread for the next layer.  The ten results that other columns'
+// nodes need (the element's upper x and y faces on the two lower planes) go through a
+// double-buffered exchange, one block barrier a layer, and each thread writes its own 8
+// nodes.  A tile recomputes the columns (and the layer) below its first own ones.  Every
+// node is summed in one fixed order (the lower layer's sums first, then own column, left,
+// front, corner), whatever the tiling: results do not depend on the tile sizes or on how
+// a mesh is cut into slabs.
+//
+// Bound: FP64 arithmetic (~680 operations an element) and its latency.  At 64^3 that is
+// 10 us at the full FP64 rate; the 91 MB of traffic take 14 us at the measured copy rate.
+// Measured with the product's inner product (CG's A p): 41 us at 64^3, 20 at 48^3, 14 at
+// 32^3, 9 at 16^3, against 80, 37, 16 and 10 us for an element pass (three threads an
+// element, element results through memory) and a node gather.  A layer of two CTAs takes
+// ~4,800 cycles: ~2,000 the arithmetic (1,350 at the full rate), 1,000 the requests, 950
+// the epilogue; 12 warps per SM at 168 registers spill and are slower (81 us).  D as one
+// TMA box: row by row as bulk copies, or per thread by 8-byte copies, the issue alone
+// costs 1,500-2,500 cycles a layer.
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
+#include <atomic>
+
+#include "hm_async.cuh"
+#include "hm_common.cuh"
+#include "hm_internal.h"
+
+namespace hm {
+
+constexpr int kApplyThreads = 128;   // columns of a tile at most
+constexpr int kApplyBlocks = 2;      // CTAs per SM in FP64 (8 warps, up to 255 registers)
+constexpr int kApplyItems = 5;       // entries of a node plane per thread at most
+constexpr int kRing = 6;             // node planes: a layer's two upper ones, four arriving
+
+// what the input vector stands for: the vector itself (zero on the Dirichlet nodes), or the
+// vector with the Dirichlet nodes zeroed on the fly
+enum ApplyIn { IN_CLEAN = 0, IN_ESS = 1 };
+// what is written for a node's product: y = A x (x itself on the Dirichlet nodes); the
+// residual b - A x; the smoothing step x + (b - A x) idiag / theta
+enum ApplyOut { OUT_Y = 0, OUT_R = 1, OUT_STEP = 2 };
+
+template <typename src, typename vec, typename res>
+struct ApplyArgs {
+  const uint8_t* ess;
+  const src* x;            // the input vector
+  const double* b;         // the right-hand side (OUT_R, OUT_STEP)
+  const double* idiag;     // reciprocal of the Jacobi diagonal (OUT_STEP)
+  const double* cheb;      // theta = cheb[0] (OUT_STEP)
+  vec* y;                  // OUT_Y, OUT_R
+  res* z;                  // OUT_STEP
+  double* part;            // OUT_Y: partial sums of x . y, one per CTA (NULL: none)
+  double* sc;              // with part: the CG step's scalars (alpha from the last block)
+  unsigned* counter;
+  uint32_t* status;        // the library's status word (a bounded wait that gave up)
+  int tma, pitch;          // D by TMA; its row pitch
+};
+
+// ------------------------------------------------------------- 1D transforms
+// nodes (x0, x1, x2) -> values at the points: 6 operations
+template <typename T>
+__device__ __forceinline__ void to_points(T x0, T x1, T x2, T& v0, T& v1, T& v2) {
+  const T s = x0 + x2, d = x2 - x0;
+  const T e = fma(T(0.4), x1, T(0.3) * s);
+  v0 = fma(T(-kS), d, e);
+  v1 = x1;
+  v2 = fma(T(kS), d, e);
+}
+// values at the points -> derivatives there, times 2 sqrt(0.15): 5 operations
+template <typename T>
+__device__ __forceinline__ void derivs(T v0, T v1, T v2, T& g0, T& g1, T& g2) {
+  const T d = v2 - v0;
+  const T c = fma(T(-2), v1, v0 + v2);
+  g0 = fma(T(-2), c, d);
+  g1 = d;
+  g2 = fma(T(2), c, d);
+}
+// the transposes: points -> nodes
+template <typename T>
+__device__ __forceinline__ void from_points(T f0, T f1, T f2, T& y0, T& y1, T& y2) {
+  const T s = f0 + f2, m = f0 - f2;
+  const T t = T(0.3) * s;
+  y0 = fma(T(kS), m, t);
+  y1 = fma(T(0.4), s, f1);
+  y2 = fma(T(-kS), m, t);
+}
+// r += w (derivs transposed) f, with w4 = 4 w
+template <typename T>
+__device__ __forceinline__ void add_from_derivs(T f0, T f1, T f2, T w, T w4, T& r0, T& r1, T& r2) {
+  const T m = f0 - f2;
+  const T t = f1 + (f0 + f2);
+  r0 = fma(-w, fma(T(2), m, t), r0);
+  r1 = fma(w4, m, r1);
+  r2 = fma(w, fma(T(-2), m, t), r2);
+}
+
+// a node plane at the element to its 9 points: x its first node, rows rs apart
+template <typename T>
+__device__ __forceinline__ void plane_to_points(const T* x, int rs, T (&v)[9]) {
+  T r[9];
+#pragma unroll
+  for (int a2 = 0; a2 < 3; ++a2)
+    to_points(x[a2 * rs], x[a2 * rs + 1], x[a2 * rs + 2], r[3 * a2], r[3 * a2 + 1], r[3 * a2 + 2]);
+#pragma unroll
+  for (int q1 = 0; q1 < 3; ++q1)
+    to_points(r[q1], r[3 + q1], r[6 + q1], v[q1], v[3 + q1], v[6 + q1]);
+}
+template <typename T>
+__device__ __forceinline__ void plane_from_points(T (&v)[9]) {
+#pragma unroll
+  for (int q1 = 0; q1 < 3; ++q1) from_points(v[q1], v[3 + q1], v[6 + q1], v[q1], v[3 + q1], v[6 + q1]);
+#pragma unroll
+  for (int a2 = 0; a2 < 3; ++a2)
+    from_points(v[3 * a2], v[3 * a2 + 1], v[3 * a2 + 2], v[3 * a2], v[3 * a2 + 1], v[3 * a2 + 2]);
+}
+// One element at its 27 points: v0, v1, v2 the in-plane values of its three node planes,
+// D(q) the weights; on return the in-plane sums of the three planes
+template <typename T, typename LDD>
+__device__ __forceinline__ void element_points(T (&v0)[9], T (&v1)[9], T (&v2)[9], LDD D, T ry, T rz) {
+  T V[27], R[27];          // [q1 + 3 q2 + 9 q3]
+#pragma unroll
+  for (int i = 0; i < 9; ++i) to_points(v0[i], v1[i], v2[i], V[i], V[9 + i], V[18 + i]);
+#pragma unroll
+  for (int i = 0; i < 9; ++i) {          // z lines
+    T g0, g1, g2;
+    derivs(V[i], V[9 + i], V[18 + i], g0, g1, g2);
+    g0 *= D(i); g1 *= D(9 + i); g2 *= D(18 + i);
+    R[i] = R[9 + i] = R[18 + i] = T(0);
+    add_from_derivs(g0, g1, g2, rz, T(4) * rz, R[i], R[9 + i], R[18 + i]);
+  }
+#pragma unroll
+  for (int q3 = 0; q3 < 3; ++q3) {       // x and y lines of slice q3
+    T d[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) d[i] = D(9 * q3 + i);
+#pragma unroll
+    for (int q2 = 0; q2 < 3; ++q2) {
+      const int i = 9 * q3 + 3 * q2;
+      T g0, g1, g2;
+      derivs(V[i], V[i + 1], V[i + 2], g0, g1, g2);
+      add_from_derivs(g0 * d[3 * q2], g1 * d[3 * q2 + 1], g2 * d[3 * q2 + 2], T(1), T(4), R[i], R[i + 1], R[i + 2]);
+    }
+#pragma unroll
+    for (int q1 = 0; q1 < 3; ++q1) {
+      const int i = 9 * q3 + q1;
+      T g0, g1, g2;
+      derivs(V[i], V[i + 3], V[i + 6], g0, g1, g2);
+      add_from_derivs(g0 * d[q1], g1 * d[3 + q1], g2 * d[6 + q1], ry, T(4) * ry, R[i], R[i + 3], R[i + 6]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 9; ++i) from_points(R[i], R[9 + i], R[18 + i], v0[i], v1[i], v2[i]);
+}
+
+// Dynamic shared memory: D of two layers [q][row][column] (one TMA box from the 16-byte
+// boundary at or before the tile's first column), the ring of node planes, the exchange.
+template <typename real> HM_HD constexpr int row_align() { return 16 / (int)sizeof(real); }
+template <typename real>
+HM_HD int box_columns(int T1) {
+  constexpr int A = row_align<real>();
+  return (T1 + 2 * A - 2) / A * A;
+}
+template <typename real>
+struct ApplySmem {
+  int dbuf, ring, exch, bytes;       // bytes of one D buffer, offsets in bytes
+  HM_HD ApplySmem(const ApplyPlan& p) {
+    const int s = (int)sizeof(real);
+    dbuf = (27 * p.T2 * box_columns<real>(p.T1) * s + 127) / 128 * 128;
+    ring = 2 * dbuf;
+    exch = ring + kRing * (2 * p.T1 + 1) * (2 * p.T2 + 1) * s;
+    bytes = exch + 20 * p.threads * s;
+  }
+};
+
+template <typename real, typename src, typename vec, typename res, int IN, int OUT>
+__global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlocks : 4)
+    k_apply_tile(const __grid_constant__ CUtensorMap map, const Lattice L, const real* __restrict__ Dq,
+                 const ApplyArgs<src, vec, res> a) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ unsigned long long mbar[2];           // D of the even and the odd layers
+  const ApplySmem<real> at(L.ap);
+  constexpr int A = row_align<real>();
+  const int T1 = L.ap.T1, T2 = L.ap.T2, nt = blockDim.x;
+  real* const ring = reinterpret_cast<real*>(smem_raw + at.ring);
+  real* const exch = reinterpret_cast<real*>(smem_raw + at.exch);
+  const int RS = 2 * T1 + 1, P = RS * (2 * T2 + 1), TB = box_columns<real>(T1);
+  const int tid = threadIdx.x;
+  // this CTA's first cells (a later tile's first column, row and layer are the halo)
+  const int bt = blockIdx.x;
+  const int i1 = bt % L.ap.t1, i2 = (bt / L.ap.t1) % L.ap.t2, i3 = bt / (L.ap.t1 * L.ap.t2);
+  const int c1 = i1 * (T1 - 1), c2 = i2 * (T2 - 1), c3 = i3 * (L.ap.T3 - 1);
+  const int layers = min(L.ap.T3, L.nz + 1 - c3);
+  const unsigned nsy = (unsigned)L.Nx, nsz = (unsigned)L.Nx * (unsigned)L.Ny;
+
+  // ---- D of layer l (thread 0)
+  auto request_D = [&](int l) {
+    if (tid != 0 || !a.tma || l >= layers || c3 + l >= L.nz) return;
+    fence_proxy_async();                   // the buffer's readers are done (block barrier)
+    mbar_expect(&mbar[l & 1], 27u * (uint32_t)(T2 * TB) * (uint32_t)sizeof(real));
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(smem_raw + (l & 1) * at.dbuf)),
+        "l"(reinterpret_cast<uint64_t>(&map)), "r"(c1 & ~(A - 1)), "r"(c2), "r"(c3 + l), "r"(0),
+        "r"(smem_u32(&mbar[l & 1]))
+        : "memory");
+  };
+  if (tid == 0) {
+    mbar_init(&mbar[0], 1);
+    mbar_init(&mbar[1], 1);
+    fence_mbar_init();
+  }
+  request_D(0);
+  request_D(1);
+  // ---- node planes: plane j (relative to 2 c3) into ring slot j % kRing, entry i of a
+  // plane by thread i % nt, the same ones every time
+  constexpr bool kDirect = sizeof(src) == sizeof(real);        // copied as it is
+  unsigned off[kApplyItems];               // the entries' nodes in the mesh's plane (~0: none)
+  {
+    const int step_r = nt / RS, step_c = nt - step_r * RS;
+    int r = tid / RS, c = tid - r * RS;
+#pragma unroll
+    for (int k = 0; k < kApplyItems; ++k) {
+      const int gx = 2 * c1 + c, gy = 2 * c2 + r;
+      off[k] = tid + k * nt < P && gx < L.Nx && gy < L.Ny ? (unsigned)gx + nsy * (unsigned)gy : ~0u;
+      r += step_r;
+      c += step_c;
+      if (c >= RS) { c -= RS; ++r; }
+    }
+  }
+  auto request = [&](int j) {
+    if constexpr (kDirect) {
+      if (2 * c3 + j < L.Nz && j <= 2 * layers) {
+        real* const plane = ring + j % kRing * P + tid;
+        const real* const x = reinterpret_cast<const real*>(a.x) + (size_t)nsz * (2 * c3 + j);
+#pragma unroll
+        for (int k = 0; k < kApplyItems; ++k)
+          if (off[k] != ~0u) copy_async(plane + k * nt, x + off[k]);
+      }
+    }
+  };
+  // after the copies of plane j, by the same threads: the Dirichlet nodes zeroed, operands of
+  // another type than the arithmetic's converted
+  auto finish = [&](int j) {
+    if constexpr (kDirect && IN == IN_CLEAN) return;
+    if (2 * c3 + j >= L.Nz || j > 2 * layers) return;
+    real* const plane = ring + j % kRing * P + tid;
+    const size_t z0 = (size_t)nsz * (2 * c3 + j);
+    src v[kApplyItems];
+    bool zero[kApplyItems];
+#pragma unroll
+    for (int k = 0; k < kApplyItems; ++k) {
+      const bool on = off[k] != ~0u;
+      zero[k] = IN == IN_ESS && on && a.ess != nullptr && __ldg(a.ess + z0 + off[k]) != 0;
+      v[k] = !kDirect && on ? __ldg(a.x + z0 + off[k]) : src(0);
+    }
+#pragma unroll
+    for (int k = 0; k < kApplyItems; ++k)
+      if (off[k] != ~0u) {
+        if (zero[k]) plane[k * nt] = real(0);
+        else if constexpr (!kDirect) plane[k * nt] = (real)v[k];
+      }
+  };
+  // D is requested a layer ahead, node planes two layers, a group of copies each
+  for (int j = 0; j < 3; ++j) request(j);
+  copy_commit();
+  request(3);
+  request(4);
+  copy_commit();
+  const int ty = tid / T1, tx = tid - ty * T1;
+  const int cx = c1 + tx, cy = c2 + ty;
+  const bool column = ty < T2;
+  const bool element = column && cx < L.nx && cy < L.ny;
+  const bool own = column && cx <= L.nx && cy <= L.ny && (tx > 0 || i1 == 0) && (ty > 0 || i2 == 0);
+  double inv_theta = 0.0;
+  if constexpr (OUT == OUT_STEP) inv_theta = 1.0 / __ldg(a.cheb);
+  copy_wait<1>();
+  for (int j = 0; j < 3; ++j) finish(j);
+  __syncthreads();
+
+  // the derivatives carry 2 sqrt(0.15) each: 1 / (4 * 0.15) in the product
+  const real sx = (real)(1.0 / (0.6 * L.hx * L.hx));
+  const real ry = (real)((L.hx * L.hx) / (L.hy * L.hy)), rz = (real)((L.hx * L.hx) / (L.hz * L.hz));
+  const int base = 2 * ty * RS + 2 * tx;  // the element's first node in a plane
+  // in-plane values of the lower node plane, sums of the lower layer on it, the input at
+  // the own nodes there
+  real low[9], carry[9], xlow[4];
+#pragma unroll
+  for (int i = 0; i < 9; ++i) low[i] = carry[i] = real(0);
+  if (element) plane_to_points(ring + base, RS, low);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) xlow[k] = own ? ring[base + (k >> 1) * RS + (k & 1)] : real(0);
+  double dot = 0.0;
+#pragma unroll 1
+  for (int l = 0; l < layers; ++l) {
+    const int cz = c3 + l;
+    const real* const p1 = ring + (2 * l + 1) % kRing * P + base;
+    const real* const p2 = ring + (2 * l + 2) % kRing * P + base;
+    request(2 * l + 5);
+    request(2 * l + 6);
+    copy_commit();
+    if (l > 0) request_D(l + 1);
+    // The own nodes h = (x, y, z parity bits): which of them exist, their markers
+    // (requested here, used after the barrier)
+    const bool out = own && (l > 0 || i3 == 0);
+    const unsigned n0 = (unsigned)(2 * cx) + nsy * (unsigned)(2 * cy) + nsz * (unsigned)(2 * cz);
+    unsigned have = 0;
+    if (out) have = 0x55u | (cx < L.nx ? 0xaau : 0u);
+    if (cy >= L.ny) have &= 0x33u;
+    if (cz >= L.nz) have &= 0x0fu;
+    uint32_t mark[8];
+#pragma unroll
+    for (int h = 0; h < 8; ++h)
+      mark[h] = a.ess != nullptr && ((have >> h) & 1u)
+                    ? __ldg(a.ess + n0 + (h & 1) + ((h & 2) ? nsy : 0u) + ((h & 4) ? nsz : 0u))
+                    : 0u;
+    real y[18];                            // the element's sums on its two lower planes
+    const bool layer = cz < L.nz;          // not the virtual one
+    const bool ok = !a.tma || !layer || mbar_wait(&mbar[l & 1], (uint32_t)(l >> 1) & 1u);
+    if (element && layer) {
+      const int ds = T2 * TB;
+      real* const Dl = reinterpret_cast<real*>(smem_raw + (l & 1) * at.dbuf) + ty * TB + tx + (c1 & (A - 1));
+      if (!a.tma) {                        // storage without a 16-byte pitch: this thread's own
+        const real* const Dg = Dq + (size_t)cx + (size_t)a.pitch * ((size_t)cy + (size_t)L.ny * (size_t)cz);
+#pragma unroll 1
+        for (int q = 0; q < 27; ++q) Dl[q * ds] = __ldg(Dg + (size_t)q * a.pitch * L.ny * L.nz);
+      }
+      real v1[9], v2[9];
+      plane_to_points(p1, RS, v1);
+      plane_to_points(p2, RS, v2);
+      real up[9];
+#pragma unroll
+      for (int i = 0; i < 9; ++i) up[i] = v2[i];
+      element_points(low, v1, v2, [&](int q) { return Dl[q * ds]; }, ry, rz);
+#pragma unroll
+      for (int i = 0; i < 9; ++i) {
+        low[i] += carry[i];
+        carry[i] = v2[i];
+      }
+      plane_from_points(low);
+      plane_from_points(v1);
+#pragma unroll
+      for (int i = 0; i < 9; ++i) { y[i] = low[i]; y[9 + i] = v1[i]; low[i] = up[i]; }
+    } else {
+      plane_from_points(carry);
+#pragma unroll
+      for (int i = 0; i < 9; ++i) { y[i] = carry[i]; y[9 + i] = carry[i] = real(0); }
+    }
+    // (keeps the markers' first use here, after the arithmetic)
+#pragma unroll
+    for (int h = 0; h < 8; ++h) asm volatile("" : "+r"(mark[h]));
+    // the results other columns' nodes need: a1 = 2 (a2 = 0, 1, 2), a2 = 2 (a1 = 0, 1)
+    real* const ex = exch + (l & 1) * 10 * nt;
+#pragma unroll
+    for (int a3 = 0; a3 < 2; ++a3) {
+      real* const e = ex + a3 * 5 * nt + tid;
+      e[0] = y[9 * a3 + 2];
+      e[nt] = y[9 * a3 + 5];
+      e[2 * nt] = y[9 * a3 + 8];
+      e[3 * nt] = y[9 * a3 + 6];
+      e[4 * nt] = y[9 * a3 + 7];
+    }
+    // the input at the own nodes, the smoother's operands
+    real xc[8];
+    double bn[OUT == OUT_Y ? 1 : 8], gn[OUT == OUT_STEP ? 8 : 1];
+    unsigned fixed = 0;
+#pragma unroll
+    for (int h = 0; h < 8; ++h) {
+      const bool on = (have >> h) & 1u;
+      const unsigned node = n0 + (h & 1) + ((h & 2) ? nsy : 0u) + ((h & 4) ? nsz : 0u);
+      if constexpr (OUT != OUT_Y) bn[h] = on ? __ldg(a.b + node) : 0.0;
+      if constexpr (OUT == OUT_STEP) gn[h] = on ? __ldg(a.idiag + node) : 0.0;
+      const int o = ((h >> 1) & 1) * RS + (h & 1);
+      if (h < 4) {
+        xc[h] = xlow[h];
+        xlow[h] = own ? p2[o] : real(0);
+      } else {
+        xc[h] = own ? p1[o] : real(0);
+      }
+      fixed |= (unsigned)(mark[h] != 0u) << h;
+    }
+    copy_wait<1>();                        // the next layer's planes
+    finish(2 * l + 3);
+    finish(2 * l + 4);
+    if (__syncthreads_or(!ok)) {           // a copy never landed: flagged, nothing more written
+      if (tid == 0) {
+        if (a.status != nullptr) atomicOr(a.status, HM_STATUS_TIMEOUT);
+        // the other buffer's copy, before the CTA leaves
+        if (l + 1 < layers && cz + 1 < L.nz) (void)mbar_wait(&mbar[(l + 1) & 1], (uint32_t)((l + 1) >> 1) & 1u);
+      }
+      break;
+    }
+    if (have) {
+      const bool left = tx > 0, front = ty > 0;
+#pragma unroll
+      for (int a3 = 0; a3 < 2; ++a3) {
+        const real* const e = ex + a3 * 5 * nt + tid;
+        real n[4];                        // nodes (0,0), (1,0), (0,1), (1,1)
+        n[0] = y[9 * a3]; n[1] = y[9 * a3 + 1]; n[2] = y[9 * a3 + 3]; n[3] = y[9 * a3 + 4];
+        if (left) { n[0] += e[-1]; n[2] += e[nt - 1]; }
+        if (front) { n[0] += e[3 * nt - T1]; n[1] += e[4 * nt - T1]; }
+        if (left && front) n[0] += e[2 * nt - T1 - 1];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int h = 4 * a3 + k;
+          if (!((have >> h) & 1u)) continue;
+          const unsigned node = n0 + (k & 1) + ((k & 2) ? nsy : 0u) + (a3 ? nsz : 0u);
+          const bool fx = (fixed >> h) & 1u;
+          const double acc = (double)(sx * n[k]);
+          if constexpr (OUT == OUT_Y) {
+            // the ring's value is the input's own, but for zeroed or rounded entries
+            const double xv = (IN == IN_CLEAN && kDirect) ? (double)xc[h]
+                              : (fx || (a.part != nullptr && !kDirect)) ? (double)__ldg(a.x + node)
+                                                                        : (double)xc[h];
+            const double yv = fx ? xv : acc;
+            a.y[node] = (vec)yv;
+            dot = fma(xv, yv, dot);
+          } else if constexpr (OUT == OUT_R) {
+            a.y[node] = (vec)(bn[h] - (fx ? (double)xc[h] : acc));
+          } else {
+            // the update rounded on its own before the add, as the step-by-step smoother
+            const double xn = (double)xc[h];
+            a.z[node] = (res)(xn + __dmul_rn(inv_theta * (bn[h] - (fx ? xn : acc)), gn[h]));
+          }
+        }
+      }
+    }
+  }
+  copy_wait<0>();
+  if (OUT == OUT_Y && a.part != nullptr) {
+    __shared__ double sh[32];
+    const double t = block_sum(dot, sh);
+    if (tid == 0) a.part[blockIdx.x] = t;
+    // a CG step: the last block takes alpha from the partials
+    if (a.sc != nullptr && last_block(a.counter)) finish_alpha(a.part, gridDim.x, a.sc, a.counter, sh);
+  }
+}
+
+}  // namespace hm
+
+using namespace hm;
+
+// ------------------------------------------------------------------ host side
+// The tiling: t_d tiles of T_d cells along axis d (the first owns T_d cells, the others
+// T_d - 1 and the halo cell below), at most kApplyThreads columns.  Estimated time: a
+// layer of a warp takes its arithmetic's share of the SM (4 warps of the CTAs on an SM
+// progress together), or at least its own latency, with two CTAs resident per SM.
+constexpr double kWarpLayer = 0.31, kLayer = 2.2, kStart = 4.5;   // us, measured
+void hm_plan_apply(Lattice* L) {
+  const int n[3] = {L->nx, L->ny, L->nz};
+  double best = 0.0;
+  ApplyPlan p{};
+  int seen1 = 0;
+  for (int t1 = 1; t1 <= n[0]; ++t1) {
+    const int T1 = (n[0] + t1 - 1) / t1 + 1;
+    if (T1 == seen1) continue;
+    seen1 = T1;
+    int seen2 = 0;
+    for (int t2 = 1; t2 <= n[1]; ++t2) {
+      const int T2 = (n[1] + t2 - 1) / t2 + 1;
+      if (T2 == seen2) continue;
+      seen2 = T2;
+      const int warps = (T1 * T2 + 31) / 32;
+      if (T1 * T2 > kApplyThreads || (2 * T1 + 1) * (2 * T2 + 1) > kApplyItems * 32 * warps) continue;
+      int seen3 = 0;
+      for (int t3 = 1; t3 <= n[2]; ++t3) {
+        const int T3 = (n[2] + t3 - 1) / t3 + 1;
+        if (T3 == seen3) continue;
+        seen3 = T3;
+        const int a1 = (n[0] + T1 - 2) / (T1 - 1), a2 = (n[1] + T2 - 2) / (T2 - 1),
+                  a3 = (n[2] + T3 - 2) / (T3 - 1);
+        const int64_t ctas = (int64_t)a1 * a2 * a3;
+        const int64_t per_sm = (ctas + 147) / 148;
+        const int resident = per_sm < kApplyBlocks ? (int)per_sm : kApplyBlocks;
+        const double waves = (double)((per_sm + resident - 1) / resident);
+        const double layer = resident * warps * kWarpLayer;
+        const double cost = waves * (T3 * (layer > kLayer ? layer : kLayer) + kStart);
+        if (p.threads == 0 || cost < best) {
+          best = cost;
+          p.T1 = T1; p.T2 = T2; p.T3 = T3;
+          p.t1 = a1; p.t2 = a2; p.t3 = a3;
+          p.threads = 32 * warps;
+        }
+      }
+    }
+  }
+  L->ap = p;
+}
+
+// row pitch of the operator's D [q][ez][ey][ex]: a multiple of 16 bytes where the storage
+// (54 reals an element) holds it
+int hm_jac_pitch(const Lattice& L, int precision) {
+  const int A = precision == HM_FP32 ? 4 : 2, p = (L.nx + A - 1) / A * A;
+  return p <= 2 * L.nx ? p : L.nx;
+}
+
+namespace {
+template <typename real, typename src, typename vec, typename res, int IN, int OUT>
+int launch(const Lattice& L, const void* jac, ApplyArgs<src, vec, res> a, void* stream) {
+  auto kern = k_apply_tile<real, src, vec, res, IN, OUT>;
+  const size_t smem = (size_t)ApplySmem<real>(L.ap).bytes;
+  a.pitch = hm_jac_pitch(L, sizeof(real) == 8 ? HM_FP64 : HM_FP32);
+  CUtensorMap map{};
+  a.tma = (reinterpret_cast<uintptr_t>(jac) & 15u) == 0 && a.pitch * sizeof(real) % 16 == 0;
+  if (a.tma) {
+    auto encode = hm_tensor_map_encoder();
+    if (encode == nullptr) return HM_ERR_CUDA;
+    const cuuint64_t row = (cuuint64_t)a.pitch * sizeof(real);
+    const cuuint64_t dims[4] = {(cuuint64_t)L.nx, (cuuint64_t)L.ny, (cuuint64_t)L.nz, 27};
+    const cuuint64_t strides[3] = {row, row * L.ny, row * L.ny * L.nz};
+    const cuuint32_t box[4] = {(cuuint32_t)box_columns<real>(L.ap.T1), (cuuint32_t)L.ap.T2, 1, 27};
+    const cuuint32_t one[4] = {1, 1, 1, 1};
+    if (encode(&map, sizeof(real) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
+               const_cast<void*>(jac), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return HM_ERR_CUDA;
+  }
+  a.status = hm_status_word();
+  if (smem > 40 * 1024) {                     // with the static part above 48 KB
+    static std::atomic<uint64_t> done{0};     // devices on which the limit is raised
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return HM_ERR_CUDA;
+    if (dev < 0 || dev >= 64) return HM_ERR_UNSUPPORTED;
+    if (!((done.load() >> dev) & 1u)) {
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
+        return HM_ERR_CUDA;
+      done.fetch_or(1ull << dev);
+    }
+  }
+  kern<<<L.ap.t1 * L.ap.t2 * L.ap.t3, L.ap.threads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
+      map, L, static_cast<const real*>(jac), a);
+  return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
+}
+template <typename real, typename T>
+int apply_y(const Lattice& L, const void* jac, const uint8_t* ess, const T* x, T* y, bool clean,
+            double* part, double* sc, unsigned* counter, void* stream) {
+  ApplyArgs<T, T, T> a{};
+  a.ess = ess; a.x = x; a.y = y; a.part = part;
+  a.sc = part != nullptr ? sc : nullptr;
+  a.counter = counter;
+  if (clean) return launch<real, T, T, T, IN_CLEAN, OUT_Y>(L, jac, a, stream);
+  return launch<real, T, T, T, IN_ESS, OUT_Y>(L, jac, a, stream);
+}
+}  // namespace
+
+// number of partial sums of the fused inner product
+int64_t hm_apply_dot_parts(const Lattice& L) { return (int64_t)L.ap.t1 * L.ap.t2 * L.ap.t3; }
+
+int hm_launch_apply_A(const Lattice& L, void* jac, int precision, const uint8_t* ess,
+                      const double* x, double* y, void* stream) {
+  if (precision == HM_FP32) return apply_y<float>(L, jac, ess, x, y, false, nullptr, nullptr, nullptr, stream);
+  return apply_y<double>(L, jac, ess, x, y, false, nullptr, nullptr, nullptr, stream);
+}
+
+// with sc and counter the last block also takes the CG step's alpha; x must be zero on
+// the Dirichlet nodes (the solves keep every search direction so)
+int hm_launch_apply_A_dot(const Lattice& L, void* jac, int precision, const uint8_t* ess,
+                          const double* x, double* y, double* part, void* stream, double* sc,
+                          unsigned* counter) {
+  if (precision == HM_FP32) return apply_y<float>(L, jac, ess, x, y, true, part, sc, counter, stream);
+  return apply_y<double>(L, jac, ess, x, y, true, part, sc, counter, stream);
+}
+
+int hm_launch_apply_A_clean(const Lattice& L, void* jac, const uint8_t* ess, const double* x,
+                            double* y, void* stream) {
+  return apply_y<double>(L, jac, ess, x, y, true, nullptr, nullptr, nullptr, stream);
+}
+
+int hm_launch_apply_A32(const Lattice& L, void* jac32, const uint8_t* ess, const float* x,
+                        float* y, bool clean, void* stream) {
+  return apply_y<float>(L, jac32, ess, x, y, clean, nullptr, nullptr, nullptr, stream);
+}
+
+// the FP32 operator on FP32 vectors (the inner solves of the mixed-precision PCG), x zero
+// on the Dirichlet nodes
+int hm_launch_apply_A32_dot(const Lattice& L, void* jac32, const uint8_t* ess, const float* x,
+                            float* y, double* part, void* stream, double* sc, unsigned* counter) {
+  return apply_y<float>(L, jac32, ess, x, y, true, part, sc, counter, stream);
+}
+
+// The operator passes of a Chebyshev-Jacobi smoothing step of degree 1 (every vector zero
+// on the Dirichlet nodes; idiag the reciprocal of the Jacobi diagonal, theta = cheb[0]):
+//   r = b - A d                        (pre-smoothing from zero: d = b idiag / theta)
+//   z = x + (b - A x) idiag / theta    (post-smoothing; z != x)
+// the same arithmetic as the start / step / finish kernels of the multigrid smoother.  In
+// the FP32 cycle d, r and x are FP32; b, the update and z stay FP64.
+int hm_launch_residual(const Lattice& L, void* jac, const uint8_t* ess, const double* b,
+                       const double* d, double* r, void* stream) {
+  ApplyArgs<double, double, double> a{};
+  a.ess = ess; a.x = d; a.b = b; a.y = r;
+  return launch<double, double, double, double, IN_CLEAN, OUT_R>(L, jac, a, stream);
+}
+int hm_launch_residual32(const Lattice& L, void* jac32, const uint8_t* ess, const double* b,
+                         const float* d, float* r, void* stream) {
+  ApplyArgs<float, float, float> a{};
+  a.ess = ess; a.x = d; a.b = b; a.y = r;
+  return launch<float, float, float, float, IN_CLEAN, OUT_R>(L, jac32, a, stream);
+}
+int hm_launch_cheb1_step(const Lattice& L, void* jac, const uint8_t* ess, const double* b,
+                         const double* idiag, const double* cheb, const double* x, double* z,
+                         void* stream) {
+  ApplyArgs<double, double, double> a{};
+  a.ess = ess; a.x = x; a.b = b; a.idiag = idiag; a.cheb = cheb; a.z = z;
+  return launch<double, double, double, double, IN_CLEAN, OUT_STEP>(L, jac, a, stream);
+}
+int hm_launch_cheb1_step32(const Lattice& L, void* jac32, const uint8_t* ess, const double* b,
+                           const double* idiag, const double* cheb, const float* x, double* z,
+                           void* stream) {
+  ApplyArgs<float, float, double> a{};
+  a.ess = ess; a.x = x; a.b = b; a.idiag = idiag; a.cheb = cheb; a.z = z;
+  return launch<float, float, float, double, IN_CLEAN, OUT_STEP>(L, jac32, a, stream);
+}

@@ -87,12 +87,16 @@ HM_HD constexpr double vrow_coef(int tab, int r, int t) {
 }
 
 // ------------------------------------------------------------------ lattice
+// tiling of the matrix-free apply: t1 x t2 x t3 tiles of T1 x T2 x T3 cells (the halo
+// included), `threads` per CTA
+struct ApplyPlan { int T1, T2, T3, t1, t2, t3, threads; };
 struct Lattice {
   int nx, ny, nz;      // elements per axis
   int Nx, Ny, Nz;      // nodes per axis (2 n + 1)
   int tx, ty, tz;      // tiles per axis (ceil(N / 4))
   double hx, hy, hz;   // element sizes
   int64_t ne, ndof;
+  ApplyPlan ap;        // hm_plan_apply
 };
 
 // 1D stencil of node i on an axis of N nodes: [lo, lo + n)

@@ -11,6 +11,12 @@ struct Lattice;
 
 // the geometry behind a lattice handle
 const hm::Lattice* hm_lattice_geometry(const hm_lattice* h);
+// the device address of the library's status word (hm_device_status)
+uint32_t* hm_status_word();
+// row pitch of the matrix-free operator's D [q][ez][ey][ex]
+int hm_jac_pitch(const hm::Lattice& L, int precision);
+// the tiling of the matrix-free apply for the lattice's sizes
+void hm_plan_apply(hm::Lattice* L);
 
 int hm_launch_pattern(const hm::Lattice& L, int32_t* indptr, int32_t* indices, int32_t* slot,
                       void* stream);
@@ -43,24 +49,26 @@ int hm_launch_ess_take_b(const hm::Lattice& L, const uint8_t* ess, const double*
                          void* stream);
 // the right-hand side and solution buffers a solve plan was created with
 int hm_plan_buffers(const hm_pcg_plan* plan, double** b, double** x);
-// one Chebyshev-Jacobi step of degree 1 of the multigrid smoother on the lattice
-// operator, fused with the operator pass: from zero (x = b idiag / theta, r = b - A x)
-// or from x (x += (b - A x) idiag / theta); theta = cheb[0], idiag the reciprocal of the
-// Jacobi diagonal
-int hm_launch_cheb1_from_zero(const hm::Lattice& L, void* jac, const uint8_t* ess, const double* b,
-                              const double* idiag, const double* cheb, double* x, double* r,
-                              void* stream);
-int hm_launch_cheb1_from_x(const hm::Lattice& L, void* jac, const uint8_t* ess, const double* b,
-                           const double* idiag, const double* cheb, double* x, void* stream);
-// the FP32 operator (jac32: the points' D in FP32, then the FP32 element results) on
-// FP32 vectors; clean: x zero on the Dirichlet nodes
+// the FP32 operator (jac32: the points' D in FP32) on FP32 vectors; clean: x zero on the Dirichlet nodes
 int hm_launch_apply_A32(const hm::Lattice& L, void* jac32, const uint8_t* ess, const float* x,
                         float* y, bool clean, void* stream);
-// the two fused smoothing steps above with the FP32 operator: from zero, b FP64 in, x and
-// r FP32 out; from x (FP32), the result z = x + (b - A x) idiag / theta written in FP64
-int hm_launch_cheb1_from_zero32(const hm::Lattice& L, void* jac32, const uint8_t* ess,
-                                const double* b, const double* idiag, const double* cheb,
-                                float* x, float* r, void* stream);
-int hm_launch_cheb1_from_x32(const hm::Lattice& L, void* jac32, const uint8_t* ess, const double* b,
-                             const double* idiag, const double* cheb, const float* x, double* z,
-                             void* stream);
+// the operator passes of the multigrid smoother's steps of degree 1 (hm_apply.cu)
+int hm_launch_residual(const hm::Lattice& L, void* jac, const uint8_t* ess, const double* b,
+                       const double* d, double* r, void* stream);
+int hm_launch_residual32(const hm::Lattice& L, void* jac32, const uint8_t* ess, const double* b,
+                         const float* d, float* r, void* stream);
+int hm_launch_cheb1_step(const hm::Lattice& L, void* jac, const uint8_t* ess, const double* b,
+                         const double* idiag, const double* cheb, const double* x, double* z,
+                         void* stream);
+int hm_launch_cheb1_step32(const hm::Lattice& L, void* jac32, const uint8_t* ess, const double* b,
+                           const double* idiag, const double* cheb, const float* x, double* z,
+                           void* stream);
+// Inside the MG-PCG: where the level-0 smoother's first direction d = r idiag / theta is
+// wanted (d64 or d32; both null: nowhere), formed by the kernel that forms r
+struct HmFirstDir {
+  const double* idiag;
+  const double* cheb;
+  double* d64;
+  float* d32;
+};
+HmFirstDir hm_mg_first_dir(const hm_mg* mg);

@@ -3,7 +3,8 @@
 //   k_pattern_*     the CSR graph (diagonal first), the entry->slot map and the
 //                   transpose map of a Q2 x Q2 block, arithmetically
 //   k_quad          pointwise data D, E = D grad u, F = D grad p, W = D grad u.grad p
-//   k_elem_apply,   the matrix-free Jacobian apply
+//   k_extract_D     the matrix-free Jacobian's data (its apply is in hm_apply.cu)
+//   k_elem_vectors, the assembled vectors straight from the fields
 //   k_node_gather
 // (the fused assembly k_tile_assemble is in hm_tile.cu)
 #include <cstdio>
@@ -195,155 +196,25 @@ __global__ void __launch_bounds__(216) k_quad(Lattice L, const double* __restric
   if (!finite) atomicOr(status, HM_STATUS_NONFINITE);
 }
 
-// ====================================================== matrix-free Jacobian apply
-// y = A(D) x in two deterministic passes:
-//   k_elem_apply   three threads per element, thread t owning Gauss slice q3 = t:
-//                  x at the element's nodes -> gradients at the slice's 9 points (sum
-//                  factorisation in registers) -> flux D grad x / h^2 -> back to the
-//                  element's nodes; the three slices' contributions are combined with
-//                  warp shuffles and y_e written in SoA layout Ye[a][e]
-//   k_node_gather  one thread per node: the sum of its <= 8 element contributions in a
-//                  fixed order; y = x on Dirichlet nodes (the Jacobian's elimination,
-//                  x zeroed there on input)
-// D is kept in SoA layout Dq[q][e] (hm_lattice_jacobian_prepare), so both passes read
-// and write coalesced.
-
+// =============================================== data of the matrix-free Jacobian apply
+// D as Dq[q][ez][ey][ex] with rows `pitch` apart (hm_jac_pitch), which the apply
+// (hm_apply.cu) reads as TMA boxes
 template <typename src, typename real>
-__global__ void k_extract_D(Lattice L, const src* __restrict__ quad, real* __restrict__ Dq) {
+__global__ void k_extract_D(Lattice L, int pitch, const src* __restrict__ quad, real* __restrict__ Dq) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= L.ne * 27) return;
   const int64_t e = i / 27;
   const int q = (int)(i - e * 27);
-  Dq[(int64_t)q * L.ne + e] = (real)quad[e * 216 + q];
+  const int64_t row = e / L.nx;
+  Dq[((int64_t)q * L.ny * L.nz + row) * pitch + (e - row * L.nx)] = (real)quad[e * 216 + q];
 }
 
-// B(q, a) and B'(q, a) for a run-time point index q (a compile-time)
-template <typename real>
-__device__ __forceinline__ real bq_rt(int q, int a) {
-  return q == 0 ? (real)bq(0, a) : q == 1 ? (real)bq(1, a) : (real)bq(2, a);
-}
-template <typename real>
-__device__ __forceinline__ real dbq_rt(int q, int a) {
-  return q == 0 ? (real)dbq(0, a) : q == 1 ? (real)dbq(1, a) : (real)dbq(2, a);
-}
-
-// ESS: zero x on the Dirichlet nodes on the fly (callers whose x is already zero there
-// -- every vector inside the lattice solves -- skip the markers).  CHEB: the input is the
-// first Chebyshev direction d = b idiag / theta of a smoother started from zero, formed
-// on the fly from b (xin), the reciprocal Jacobi diagonal (cdiag) and theta = cheb[0].
-template <typename real, typename vec, bool ESS = true, bool CHEB = false>
-__global__ void __launch_bounds__(256, 2)
-    k_elem_apply(Lattice L, const real* __restrict__ Dq, const uint8_t* __restrict__ ess,
-                 const vec* __restrict__ xin, real* __restrict__ Ye,
-                 const double* __restrict__ cdiag = nullptr, const double* __restrict__ cheb = nullptr) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int k = lane / 3, t = lane - 3 * k;                 // element slot, Gauss slice
-  const int64_t e = warp * 10 + k;
-  const bool live = lane < 30 && e < L.ne;
-  // 32-bit decode (the lattice keeps every index below 2^31)
-  const unsigned ec = live ? (unsigned)e : 0u;
-  const unsigned exy = ec / (unsigned)L.nx;
-  const int ex = (int)(ec - exy * (unsigned)L.nx);
-  const int ez = (int)(exy / (unsigned)L.ny), ey = (int)(exy - (unsigned)ez * (unsigned)L.ny);
-  const unsigned n0 = (unsigned)(2 * ex) + (unsigned)L.Nx * ((unsigned)(2 * ey) + (unsigned)L.Ny * (unsigned)(2 * ez));
-  const unsigned nsy = (unsigned)L.Nx, nsz = (unsigned)L.Nx * (unsigned)L.Ny;
-  const double inv_theta = CHEB ? 1.0 / __ldg(cheb) : 0.0;
-  // z interpolation onto slice t, one node plane a3 at a time: Xb[a2][a1], Xd[a2][a1]
-  real Xb[9], Xd[9];
-#pragma unroll
-  for (int a3 = 0; a3 < 3; ++a3) {
-    const real b3 = bq_rt<real>(t, a3), d3 = dbq_rt<real>(t, a3);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      const unsigned n = n0 + (unsigned)(i % 3) + nsy * (unsigned)(i / 3) + nsz * (unsigned)a3;
-      real xv = (real)0;
-      if (live) {
-        if constexpr (CHEB) xv = (real)__dmul_rn(inv_theta * (double)__ldg(xin + n), __ldg(cdiag + n));
-        else xv = (real)__ldg(xin + n);
-      }
-      const bool fixed = ESS && ess != nullptr && live && __ldg(ess + n) != 0;
-      const real x = fixed ? (real)0 : xv;
-      Xb[i] = a3 == 0 ? b3 * x : fma(b3, x, Xb[i]);
-      Xd[i] = a3 == 0 ? d3 * x : fma(d3, x, Xd[i]);
-    }
-  }
-  const real sx = (real)(1.0 / (L.hx * L.hx)), sy = (real)(1.0 / (L.hy * L.hy)),
-             sz = (real)(1.0 / (L.hz * L.hz));
-  // gradients and fluxes at the slice's points, folded straight back along x:
-  // Z0[a1][q2] = sum_q1 B'(q1,a1) Fx,  Z1 = sum B Fy,  Z2 = sum B Fz
-  real Z0[9], Z1[9], Z2[9];
-#pragma unroll
-  for (int q2 = 0; q2 < 3; ++q2) {
-    real bb[3], db[3], bd[3];
-#pragma unroll
-    for (int a1 = 0; a1 < 3; ++a1) {
-      bb[a1] = (real)bq(q2, 0) * Xb[a1] + (real)bq(q2, 1) * Xb[a1 + 3] + (real)bq(q2, 2) * Xb[a1 + 6];
-      db[a1] = (real)dbq(q2, 0) * Xb[a1] + (real)dbq(q2, 1) * Xb[a1 + 3] + (real)dbq(q2, 2) * Xb[a1 + 6];
-      bd[a1] = (real)bq(q2, 0) * Xd[a1] + (real)bq(q2, 1) * Xd[a1 + 3] + (real)bq(q2, 2) * Xd[a1 + 6];
-    }
-#pragma unroll
-    for (int a1 = 0; a1 < 3; ++a1) { Z0[a1 * 3 + q2] = 0; Z1[a1 * 3 + q2] = 0; Z2[a1 * 3 + q2] = 0; }
-#pragma unroll
-    for (int q1 = 0; q1 < 3; ++q1) {
-      const real gx = (real)dbq(q1, 0) * bb[0] + (real)dbq(q1, 1) * bb[1] + (real)dbq(q1, 2) * bb[2];
-      const real gy = (real)bq(q1, 0) * db[0] + (real)bq(q1, 1) * db[1] + (real)bq(q1, 2) * db[2];
-      const real gz = (real)bq(q1, 0) * bd[0] + (real)bq(q1, 1) * bd[1] + (real)bq(q1, 2) * bd[2];
-      const real d = live ? Dq[(int64_t)(q1 + 3 * q2 + 9 * t) * L.ne + ec] : (real)0;  // coalesced in e
-      const real fx = d * gx * sx, fy = d * gy * sy, fz = d * gz * sz;
-#pragma unroll
-      for (int a1 = 0; a1 < 3; ++a1) {
-        Z0[a1 * 3 + q2] = fma((real)dbq(q1, a1), fx, Z0[a1 * 3 + q2]);
-        Z1[a1 * 3 + q2] = fma((real)bq(q1, a1), fy, Z1[a1 * 3 + q2]);
-        Z2[a1 * 3 + q2] = fma((real)bq(q1, a1), fz, Z2[a1 * 3 + q2]);
-      }
-    }
-  }
-  // back along y: UB[a2][a1] = sum_q2 B(q2,a2) Z0 + B'(q2,a2) Z1,  UD = sum_q2 B(q2,a2) Z2
-  real UB[9], UD[9];
-#pragma unroll
-  for (int a2 = 0; a2 < 3; ++a2)
-#pragma unroll
-    for (int a1 = 0; a1 < 3; ++a1) {
-      real ub = 0, ud = 0;
-#pragma unroll
-      for (int q2 = 0; q2 < 3; ++q2) {
-        ub = fma((real)bq(q2, a2), Z0[a1 * 3 + q2], ub);
-        ub = fma((real)dbq(q2, a2), Z1[a1 * 3 + q2], ub);
-        ud = fma((real)bq(q2, a2), Z2[a1 * 3 + q2], ud);
-      }
-      UB[a2 * 3 + a1] = ub;
-      UD[a2 * 3 + a1] = ud;
-    }
-  // back along z: thread t owns node plane a3 = t and sums the three slices' parts,
-  // slice order 0, 1, 2 (fixed)
-  real y[9];
-#pragma unroll
-  for (int i = 0; i < 9; ++i) y[i] = 0;
-  const int base = 3 * k;
-#pragma unroll
-  for (int src = 0; src < 3; ++src) {
-    const real cb = bq_rt<real>(src, 0) * (t == 0) + bq_rt<real>(src, 1) * (t == 1) + bq_rt<real>(src, 2) * (t == 2);
-    const real cd = dbq_rt<real>(src, 0) * (t == 0) + dbq_rt<real>(src, 1) * (t == 1) + dbq_rt<real>(src, 2) * (t == 2);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      const real ub = __shfl_sync(0xffffffffu, UB[i], base + src);
-      const real ud = __shfl_sync(0xffffffffu, UD[i], base + src);
-      y[i] = fma(cb, ub, fma(cd, ud, y[i]));
-    }
-  }
-  if (live) {
-#pragma unroll
-    for (int i = 0; i < 9; ++i) Ye[(int64_t)(i + 9 * t) * L.ne + e] = y[i];
-  }
-}
-
-// One thread per pair of x-neighbours (2m, 2m+1) of a node row (the row's last node,
-// 2n, alone), so that every lane of a warp runs the same loop: node 2m takes element
-// m-1 (local a1 = 2) and m (a1 = 0), node 2m+1 element m (a1 = 1); consecutive lanes
-// read consecutive elements of each Ye plane.  Per node the contributions are summed
-// over (z, y, x) element pairs with the lower element first, a fixed order.  With part
-// != nullptr each block also writes its partial sum of dotw . y (the p.q of a CG step).
+// Element vectors Ye[a][e] to nodes.  One thread per pair of x-neighbours (2m, 2m+1) of a
+// node row (the row's last node, 2n, alone), so that every lane of a warp runs the same
+// loop: node 2m takes element m-1 (local a1 = 2) and m (a1 = 0), node 2m+1 element m
+// (a1 = 1); consecutive lanes read consecutive elements of each Ye plane.  Per node the
+// contributions are summed over (z, y, x) element pairs with the lower element first, a
+// fixed order.
 __device__ __forceinline__ void axis_elems(int i, int nel, int& e0, int& a0, int& cnt) {
   if (i & 1) { e0 = i >> 1; a0 = 1; cnt = 1; }
   else if (i == 0) { e0 = 0; a0 = 0; cnt = 1; }
@@ -351,134 +222,51 @@ __device__ __forceinline__ void axis_elems(int i, int nel, int& e0, int& a0, int
   else { e0 = (i >> 1) - 1; a0 = 2; cnt = 2; }   // elements i/2-1 (a=2), i/2 (a=0)
 }
 
-// OUT selects what is written for each node's product y (FP64 only for OUT != 0), with
-// c.b the smoother's right-hand side, c.diag the reciprocal of the Jacobi diagonal,
-// theta = c.cheb[0]:
-//   0  yout = y
-//   1  the first smoothing step from zero (the input was d = b c.diag / theta):
-//      c.r = b - y, c.x = d
-//   2  one smoothing step from c.x (the input): c.x += (b - y) c.diag / theta, in place,
-//      or into c.z (FP64) when given (this pass reads no x but the Dirichlet nodes' own)
-//   3  as 1 with d already in c.x (the input): c.r = b - y
-// c.r and c.x are in the vector type V (the updates are formed in FP64 and rounded once)
-template <typename V>
-struct ChebOutT {
-  const double* b;
-  const double* diag;
-  const double* cheb;
-  V* r;
-  V* x;
-  double* z;
-};
-using ChebOut = ChebOutT<double>;
-template <typename real, typename vec, int OUT = 0>
 __global__ void __launch_bounds__(256)
-    k_node_gather(Lattice L, const real* __restrict__ Ye, const uint8_t* __restrict__ ess,
-                  const vec* __restrict__ xin, vec* __restrict__ yout,
-                  const vec* __restrict__ dotw, double* __restrict__ part,
-                  double* __restrict__ sc, unsigned* __restrict__ counter, ChebOutT<vec> c = {},
+    k_node_gather(Lattice L, const double* __restrict__ Ye, double* __restrict__ yout,
                   const uint32_t* __restrict__ skip = nullptr) {
   if (skip != nullptr && *skip != 0u) return;    // the whole launch stands down
   const unsigned per_row = (unsigned)L.nx + 1u;                  // pairs + the last node
   const unsigned rows = (unsigned)L.Ny * (unsigned)L.Nz;
   const unsigned task = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = task < rows * per_row;
-  const unsigned row = live ? task / per_row : 0u;
-  const unsigned m = live ? task - row * per_row : 0u;
+  if (task >= rows * per_row) return;
+  const unsigned row = task / per_row;
+  const unsigned m = task - row * per_row;
   const unsigned iz = row / (unsigned)L.Ny, iy = row - iz * (unsigned)L.Ny;
   const bool last = m == (unsigned)L.nx;                          // node 2n alone
   const unsigned n0 = row * (unsigned)L.Nx + 2u * m;              // node 2m
-  double dot = 0.0;
-  if (live) {
-    int ey0, ay0, cy, ez0, az0, cz;
-    axis_elems((int)iy, L.ny, ey0, ay0, cy);
-    axis_elems((int)iz, L.nz, ez0, az0, cz);
-    const unsigned ne = (unsigned)L.ne, nx = (unsigned)L.nx;
-    const bool f0 = ess != nullptr && ess[n0];
-    const bool f1 = !last && ess != nullptr && ess[n0 + 1];
-    // every contribution is loaded before any is added (all twelve loads in flight at
-    // once), then summed in the fixed order (z, y element pairs, lower element first)
-    real v[4][3];
+  int ey0, ay0, cy, ez0, az0, cz;
+  axis_elems((int)iy, L.ny, ey0, ay0, cy);
+  axis_elems((int)iz, L.nz, ez0, az0, cz);
+  const unsigned ne = (unsigned)L.ne, nx = (unsigned)L.nx;
+  // every contribution is loaded before any is added (all twelve loads in flight at
+  // once), then summed in the fixed order (z, y element pairs, lower element first)
+  double v[4][3];
 #pragma unroll
-    for (int c3 = 0; c3 < 2; ++c3)
+  for (int c3 = 0; c3 < 2; ++c3)
 #pragma unroll
-      for (int c2 = 0; c2 < 2; ++c2) {
-        const int c = 2 * c3 + c2;
-        const bool on = c3 < cz && c2 < cy;
-        const unsigned a23 = 3u * (unsigned)(c2 ? 0 : ay0) + 9u * (unsigned)(c3 ? 0 : az0);
-        const unsigned erow = nx * ((unsigned)(ey0 + c2) + (unsigned)L.ny * (unsigned)(ez0 + c3));
-        // node 2m: element m-1 (a1 = 2) then element m (a1 = 0); node 2m+1: element m
-        v[c][0] = (on && m > 0) ? Ye[(size_t)(2u + a23) * ne + erow + m - 1u] : (real)0;
-        v[c][1] = (on && !last) ? Ye[(size_t)a23 * ne + erow + m] : (real)0;
-        v[c][2] = (on && !last) ? Ye[(size_t)(1u + a23) * ne + erow + m] : (real)0;
-      }
-    real acc0 = 0, acc1 = 0;
+    for (int c2 = 0; c2 < 2; ++c2) {
+      const int c = 2 * c3 + c2;
+      const bool on = c3 < cz && c2 < cy;
+      const unsigned a23 = 3u * (unsigned)(c2 ? 0 : ay0) + 9u * (unsigned)(c3 ? 0 : az0);
+      const unsigned erow = nx * ((unsigned)(ey0 + c2) + (unsigned)L.ny * (unsigned)(ez0 + c3));
+      // node 2m: element m-1 (a1 = 2) then element m (a1 = 0); node 2m+1: element m
+      v[c][0] = (on && m > 0) ? Ye[(size_t)(2u + a23) * ne + erow + m - 1u] : 0.0;
+      v[c][1] = (on && !last) ? Ye[(size_t)a23 * ne + erow + m] : 0.0;
+      v[c][2] = (on && !last) ? Ye[(size_t)(1u + a23) * ne + erow + m] : 0.0;
+    }
+  double acc0 = 0, acc1 = 0;
 #pragma unroll
-    for (int c3 = 0; c3 < 2; ++c3)
-#pragma unroll
-      for (int c2 = 0; c2 < 2; ++c2) {
-        const int c = 2 * c3 + c2;
-        if (c3 < cz && c2 < cy) {
-          if (m > 0) acc0 += v[c][0];
-          if (!last) {
-            acc0 += v[c][1];
-            acc1 += v[c][2];
-          }
-        }
-      }
-    if constexpr (OUT == 0) {
-      const double y0 = f0 ? (double)xin[n0] : (double)acc0;
-      yout[n0] = (vec)y0;
-      if (dotw) dot = (double)dotw[n0] * y0;
+  for (int c = 0; c < 4; ++c)
+    if ((c >> 1) < cz && (c & 1) < cy) {
+      if (m > 0) acc0 += v[c][0];
       if (!last) {
-        const double y1 = f1 ? (double)xin[n0 + 1] : (double)acc1;
-        yout[n0 + 1] = (vec)y1;
-        if (dotw) dot = fma((double)dotw[n0 + 1], y1, dot);
-      }
-    } else {
-      const double inv_theta = 1.0 / c.cheb[0];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (h == 1 && last) break;
-        const unsigned nn = n0 + (unsigned)h;
-        const bool fx = h ? f1 : f0;
-        const double acc = (double)(h ? acc1 : acc0);
-        const double bn = c.b[nn];
-        if constexpr (OUT == 1) {
-          const double d = __dmul_rn(inv_theta * bn, c.diag[nn]);
-          const double y = fx ? (double)(vec)d : acc;
-          c.r[nn] = (vec)(bn - y);
-          c.x[nn] = (vec)d;
-        } else if constexpr (OUT == 3) {
-          const double y = fx ? (double)c.x[nn] : acc;
-          c.r[nn] = (vec)(bn - y);
-        } else {
-          const double xn = (double)c.x[nn];
-          const double y = fx ? xn : acc;
-          // the update rounded on its own before the add, as the step-by-step smoother
-          const double xnew = xn + __dmul_rn(inv_theta * (bn - y), c.diag[nn]);
-          if (c.z != nullptr) c.z[nn] = xnew;
-          else c.x[nn] = (vec)xnew;
-        }
+        acc0 += v[c][1];
+        acc1 += v[c][2];
       }
     }
-  }
-  if (part != nullptr) {
-    __shared__ double sh[32];
-    double v = dot;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      double t = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (threadIdx.x == 0) part[blockIdx.x] = t;
-    }
-    // a CG step: the last block takes alpha from the partials
-    if (sc != nullptr && last_block(counter)) finish_alpha(part, gridDim.x, sc, counter, sh);
-  }
+  yout[n0] = acc0;
+  if (!last) yout[n0 + 1] = acc1;
 }
 
 // diagonal of A(D): sum_g D(g) sum_d (d_d phi_n)^2, one thread per node
@@ -572,140 +360,13 @@ int hm_launch_jacobian_prepare(const Lattice& L, const void* quad, int quad_prec
   const int blocks = grid1(L.ne * 27, 256);
   cudaStream_t s = S_(stream);
   if (quad_precision == HM_FP32) {
-    if (precision == HM_FP32) k_extract_D<float, float><<<blocks, 256, 0, s>>>(L, (const float*)quad, (float*)jac);
-    else k_extract_D<float, double><<<blocks, 256, 0, s>>>(L, (const float*)quad, (double*)jac);
+    if (precision == HM_FP32) k_extract_D<float, float><<<blocks, 256, 0, s>>>(L, hm_jac_pitch(L, precision), (const float*)quad, (float*)jac);
+    else k_extract_D<float, double><<<blocks, 256, 0, s>>>(L, hm_jac_pitch(L, precision), (const float*)quad, (double*)jac);
   } else {
-    if (precision == HM_FP32) k_extract_D<double, float><<<blocks, 256, 0, s>>>(L, (const double*)quad, (float*)jac);
-    else k_extract_D<double, double><<<blocks, 256, 0, s>>>(L, (const double*)quad, (double*)jac);
+    if (precision == HM_FP32) k_extract_D<double, float><<<blocks, 256, 0, s>>>(L, hm_jac_pitch(L, precision), (const double*)quad, (float*)jac);
+    else k_extract_D<double, double><<<blocks, 256, 0, s>>>(L, hm_jac_pitch(L, precision), (const double*)quad, (double*)jac);
   }
   return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
-}
-
-template <typename real, typename vec>
-static int launch_apply_t(const Lattice& L, void* jac, const uint8_t* ess, const vec* x,
-                          vec* y, const vec* dotw, double* part, void* stream,
-                          double* sc = nullptr, unsigned* counter = nullptr,
-                          bool x_zero_on_ess = false) {
-  real* Dq = static_cast<real*>(jac);
-  real* Ye = Dq + L.ne * 27;
-  const int64_t warps = (L.ne + 9) / 10;
-  if (x_zero_on_ess)
-    k_elem_apply<real, vec, false><<<grid1(warps * 32, 256), 256, 0, S_(stream)>>>(L, Dq, ess, x, Ye);
-  else
-    k_elem_apply<real, vec, true><<<grid1(warps * 32, 256), 256, 0, S_(stream)>>>(L, Dq, ess, x, Ye);
-  k_node_gather<real, vec><<<gather_blocks(L), 256, 0, S_(stream)>>>(
-      L, Ye, ess, x, y, dotw, part, part != nullptr ? sc : nullptr, counter);
-  return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
-}
-
-// One Chebyshev-Jacobi smoothing step of degree 1 on the lattice operator (FP64, every
-// vector zero on the Dirichlet nodes), the operator pass and the vector update fused:
-//   from zero:  x = d = b idiag / theta,  r = b - A d          (pre-smoothing)
-//   from x:     x += (b - A x) idiag / theta                   (post-smoothing)
-// (idiag: the reciprocal of the Jacobi diagonal)
-// the same arithmetic as the start / step / finish kernels of the multigrid smoother.
-int hm_launch_cheb1_from_zero(const Lattice& L, void* jac, const uint8_t* ess, const double* b,
-                              const double* idiag, const double* cheb, double* x, double* r,
-                              void* stream) {
-  double* Dq = static_cast<double*>(jac);
-  double* Ye = Dq + L.ne * 27;
-  const int64_t warps = (L.ne + 9) / 10;
-  k_elem_apply<double, double, false, true><<<grid1(warps * 32, 256), 256, 0, S_(stream)>>>(
-      L, Dq, ess, b, Ye, idiag, cheb);
-  ChebOut c{b, idiag, cheb, r, x, nullptr};
-  k_node_gather<double, double, 1><<<gather_blocks(L), 256, 0, S_(stream)>>>(
-      L, Ye, ess, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, c);
-  return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
-}
-int hm_launch_cheb1_from_x(const Lattice& L, void* jac, const uint8_t* ess, const double* b,
-                           const double* idiag, const double* cheb, double* x, void* stream) {
-  double* Dq = static_cast<double*>(jac);
-  double* Ye = Dq + L.ne * 27;
-  const int64_t warps = (L.ne + 9) / 10;
-  k_elem_apply<double, double, false><<<grid1(warps * 32, 256), 256, 0, S_(stream)>>>(L, Dq, ess, x, Ye);
-  ChebOut c{b, idiag, cheb, nullptr, x, nullptr};
-  k_node_gather<double, double, 2><<<gather_blocks(L), 256, 0, S_(stream)>>>(
-      L, Ye, ess, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, c);
-  return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
-}
-
-// the same two steps with the FP32 operator and FP32 level vectors (the multigrid cycle in
-// single precision): the first direction d = b idiag / theta is formed in FP64 from the
-// FP64 right-hand side, once per node, and rounded to FP32 into x (k_cheb_first32); the
-// element pass and the gather then read it from there; the post-smoothing result goes
-// to the FP64 z
-// d = b idiag / theta rounded to FP32, one thread per node (the FP64 product the FP64
-// element pass forms on the fly)
-__global__ void k_cheb_first32(int64_t n, const double* __restrict__ b, const double* __restrict__ idiag,
-                               const double* __restrict__ cheb, float* __restrict__ d) {
-  const double inv_theta = 1.0 / cheb[0];
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    d[i] = (float)__dmul_rn(inv_theta * b[i], idiag[i]);
-}
-int hm_launch_cheb1_from_zero32(const Lattice& L, void* jac32, const uint8_t* ess, const double* b,
-                                const double* idiag, const double* cheb, float* x, float* r,
-                                void* stream) {
-  float* Dq = static_cast<float*>(jac32);
-  float* Ye = Dq + L.ne * 27;
-  const int64_t warps = (L.ne + 9) / 10;
-  k_cheb_first32<<<grid1(L.ndof, 256), 256, 0, S_(stream)>>>(L.ndof, b, idiag, cheb, x);
-  k_elem_apply<float, float, false><<<grid1(warps * 32, 256), 256, 0, S_(stream)>>>(L, Dq, ess, x, Ye);
-  ChebOutT<float> c{b, idiag, cheb, r, x, nullptr};
-  k_node_gather<float, float, 3><<<gather_blocks(L), 256, 0, S_(stream)>>>(
-      L, Ye, ess, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, c);
-  return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
-}
-int hm_launch_cheb1_from_x32(const Lattice& L, void* jac32, const uint8_t* ess, const double* b,
-                             const double* idiag, const double* cheb, const float* x, double* z,
-                             void* stream) {
-  float* Dq = static_cast<float*>(jac32);
-  float* Ye = Dq + L.ne * 27;
-  const int64_t warps = (L.ne + 9) / 10;
-  k_elem_apply<float, float, false><<<grid1(warps * 32, 256), 256, 0, S_(stream)>>>(L, Dq, ess, x, Ye);
-  ChebOutT<float> c{b, idiag, cheb, nullptr, const_cast<float*>(x), z};
-  k_node_gather<float, float, 2><<<gather_blocks(L), 256, 0, S_(stream)>>>(
-      L, Ye, ess, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, c);
-  return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
-}
-int hm_launch_apply_A32(const Lattice& L, void* jac32, const uint8_t* ess, const float* x,
-                        float* y, bool clean, void* stream) {
-  return launch_apply_t<float, float>(L, jac32, ess, x, y, nullptr, nullptr, stream, nullptr,
-                                      nullptr, clean);
-}
-
-// number of partial sums k_node_gather writes when asked for the fused dot product
-int64_t hm_apply_dot_parts(const Lattice& L) { return gather_blocks(L); }
-
-int hm_launch_apply_A(const Lattice& L, void* jac, int precision, const uint8_t* ess,
-                      const double* x, double* y, void* stream) {
-  if (precision == HM_FP32)
-    return launch_apply_t<float, double>(L, jac, ess, x, y, nullptr, nullptr, stream);
-  return launch_apply_t<double, double>(L, jac, ess, x, y, nullptr, nullptr, stream);
-}
-
-// with sc and counter the gather's last block also takes the CG step's alpha; x must be
-// zero on the Dirichlet nodes (the solves keep every search direction so)
-int hm_launch_apply_A_dot(const Lattice& L, void* jac, int precision, const uint8_t* ess,
-                          const double* x, double* y, double* part, void* stream, double* sc,
-                          unsigned* counter) {
-  if (precision == HM_FP32)
-    return launch_apply_t<float, double>(L, jac, ess, x, y, x, part, stream, sc, counter, true);
-  return launch_apply_t<double, double>(L, jac, ess, x, y, x, part, stream, sc, counter, true);
-}
-
-// y = A x for an x that is zero on the Dirichlet nodes (FP64 operator)
-int hm_launch_apply_A_clean(const Lattice& L, void* jac, const uint8_t* ess, const double* x,
-                            double* y, void* stream) {
-  return launch_apply_t<double, double>(L, jac, ess, x, y, nullptr, nullptr, stream, nullptr,
-                                        nullptr, true);
-}
-
-// the FP32 operator on FP32 vectors (the inner solves of the mixed-precision PCG), x zero
-// on the Dirichlet nodes
-int hm_launch_apply_A32_dot(const Lattice& L, void* jac32, const uint8_t* ess, const float* x,
-                            float* y, double* part, void* stream, double* sc, unsigned* counter) {
-  return launch_apply_t<float, float>(L, jac32, ess, x, y, part ? x : nullptr, part, stream, sc,
-                                      counter, true);
 }
 
 // x = b on the Dirichlet nodes (the identity rows of the eliminated operator): after it
@@ -1005,8 +666,7 @@ extern "C" int hm_lattice_vectors(const hm_lattice* h, const double* d_u, const 
   k_elem_vectors<<<grid, 216, 0, s>>>(L, d_u, d_m, d_p, d_mhat, f, o, d_status);
   for (int i = 0; i < 3; ++i) {
     if (!outs[i]) continue;
-    k_node_gather<double, double, 0><<<gather_blocks(L), 256, 0, s>>>(
-        L, o.ye[i], nullptr, nullptr, outs[i], nullptr, nullptr, nullptr, nullptr);
+    k_node_gather<<<gather_blocks(L), 256, 0, s>>>(L, o.ye[i], outs[i]);
     if (zero_ess_vectors && d_ess && i != 2)
       k_zero_marked<<<grid1(L.ndof, 256), 256, 0, s>>>(L.ndof, d_ess, outs[i]);
   }
@@ -1044,8 +704,7 @@ extern "C" int hm_lattice_vectors_at(const hm_lattice* h, const double* d_u, con
   k_elem_vectors<<<grid, 216, 0, s>>>(L, d_u, d_m, d_p, nullptr, f, o, d_status, d_same);
   for (int i = 0; i < 3; ++i) {
     if (!outs[i]) continue;
-    k_node_gather<double, double, 0><<<gather_blocks(L), 256, 0, s>>>(
-        L, o.ye[i], nullptr, nullptr, outs[i], nullptr, nullptr, nullptr, nullptr, ChebOut{}, d_same);
+    k_node_gather<<<gather_blocks(L), 256, 0, s>>>(L, o.ye[i], outs[i], d_same);
     k_copy_if_same<<<cgrid, 256, 0, s>>>(L.ndof, d_same, kept[i], outs[i]);
   }
   return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;

@@ -187,14 +187,16 @@ __global__ void k_q1_diag(MGLevel lv, double* __restrict__ diag) {
   diag[n] = c * kaa;
 }
 
-// level-1 coefficients: sum_q D(q) / |e| (D = w|J| e^m in the operator's SoA layout)
-__global__ void k_coef_from_q2(int64_t ne, const double* __restrict__ Dq, double inv_vol,
+// level-1 coefficients: sum_q D(q) / |e| (D = w|J| e^m in the operator's layout)
+__global__ void k_coef_from_q2(Lattice L, int pitch, const double* __restrict__ Dq, double inv_vol,
                                double* __restrict__ coef) {
   const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= ne) return;
+  if (e >= L.ne) return;
+  const int64_t row = e / L.nx, rows = (int64_t)L.ny * L.nz;
+  const double* const D = Dq + row * pitch + (e - row * L.nx);
   double s = 0.0;
 #pragma unroll
-  for (int q = 0; q < 27; ++q) s += Dq[(int64_t)q * ne + e];
+  for (int q = 0; q < 27; ++q) s += D[(int64_t)q * rows * pitch];
   coef[e] = s * inv_vol;
 }
 
@@ -626,11 +628,12 @@ int vcycle(hm_mg* mg, int l, const T* b, T* x, bool clean, cudaStream_t s, T** o
   constexpr bool kFP64 = std::is_same<T, double>::value;
   const bool fuse = mg->fused && mg->degree == 1 &&
                     (l == 0 ? kFP64 && clean : (b == lv.b && x == lv.x));
+  // level 0 fused: the first direction, formed with the right-hand side (hm_mg_first_dir),
+  // is lv.t, which holds the iterate until the post-smoothing step writes to x
+  T* const xl = fuse && l == 0 ? lv.t : x;
   if (fuse && l == 0) {
     if constexpr (kFP64) {
-      if ((rc = hm_launch_cheb1_from_zero(mg->L, mg->jac, mg->ess, b, lv.idiag, lv.cheb, x, lv.r,
-                                          (void*)s)))
-        return rc;
+      if ((rc = hm_launch_residual(mg->L, mg->jac, mg->ess, b, xl, lv.r, (void*)s))) return rc;
     }
   } else if (fuse) {
     k_q1_cheb1_from_zero<T><<<blocks_for(lv.nodes), 256, 0, s>>>(lv, b);
@@ -640,10 +643,10 @@ int vcycle(hm_mg* mg, int l, const T* b, T* x, bool clean, cudaStream_t s, T** o
   k_restrict<T><<<blocks_for(cv.nodes), 256, 0, s>>>(lv, cv, lv.r, cv.b);
   T* xc = nullptr;
   if ((rc = vcycle<T>(mg, l + 1, cv.b, cv.x, clean, s, &xc))) return rc;
-  k_prolong_add<T><<<blocks_for(lv.nodes), 256, 0, s>>>(lv, cv, xc, x);
+  k_prolong_add<T><<<blocks_for(lv.nodes), 256, 0, s>>>(lv, cv, xc, xl);
   if (fuse && l == 0) {
     if constexpr (kFP64)
-      return hm_launch_cheb1_from_x(mg->L, mg->jac, mg->ess, b, lv.idiag, lv.cheb, x, (void*)s);
+      return hm_launch_cheb1_step(mg->L, mg->jac, mg->ess, b, lv.idiag, lv.cheb, xl, x, (void*)s);
   }
   if (fuse) {
     k_q1_cheb1_from_x<T><<<blocks_for(lv.nodes), 256, 0, s>>>(lv, b, x, lv.t);
@@ -657,28 +660,37 @@ __global__ void k_to_float(int64_t n, const double* __restrict__ a, float* __res
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     b[i] = (float)a[i];
 }
+// rows of nx entries from one pitch to another
+__global__ void k_jac_to_float(int64_t rows, int nx, int pa, int pb, const double* __restrict__ a,
+                               float* __restrict__ b) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < rows * nx;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = i / nx, c = i - r * nx;
+    b[r * pb + c] = (float)a[r * pa + c];
+  }
+}
 __global__ void k_to_double(int64_t n, const float* __restrict__ a, double* __restrict__ b) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     b[i] = (double)a[i];
 }
 
 // z = V(r) with the cycle in FP32: r and z FP64.  With degree-1 fused smoothing inside
-// the solves (clean) the level-0 passes read r and write z themselves; otherwise r is
-// rounded to FP32 first and the result widened at the end.
+// the solves (clean) the first direction is already in level 0's x (hm_mg_first_dir) and
+// the level-0 passes read r and write z themselves; otherwise r is rounded to FP32 first
+// and the result widened at the end.
 int vcycle_single(hm_mg* mg, const double* r, double* z, bool clean, cudaStream_t s) {
   MGLevelT<float>* lv = mg->lv32;
   int rc;
   if (mg->fused && mg->degree == 1 && clean && mg->nlev > 1) {
     const MGLevel& l0 = mg->lv[0];
-    if ((rc = hm_launch_cheb1_from_zero32(mg->L, mg->jac32, mg->ess, r, l0.idiag, l0.cheb,
-                                          lv[0].x, lv[0].r, (void*)s)))
+    if ((rc = hm_launch_residual32(mg->L, mg->jac32, mg->ess, r, lv[0].x, lv[0].r, (void*)s)))
       return rc;
     k_restrict<float><<<blocks_for(lv[1].nodes), 256, 0, s>>>(lv[0], lv[1], lv[0].r, lv[1].b);
     float* xc = nullptr;
     if ((rc = vcycle<float>(mg, 1, lv[1].b, lv[1].x, clean, s, &xc))) return rc;
     k_prolong_add<float><<<blocks_for(lv[0].nodes), 256, 0, s>>>(lv[0], lv[1], xc, lv[0].x);
-    return hm_launch_cheb1_from_x32(mg->L, mg->jac32, mg->ess, r, l0.idiag, l0.cheb, lv[0].x, z,
-                                    (void*)s);
+    return hm_launch_cheb1_step32(mg->L, mg->jac32, mg->ess, r, l0.idiag, l0.cheb, lv[0].x, z,
+                                  (void*)s);
   }
   k_to_float<<<kMGBlocks, 256, 0, s>>>(lv[0].nodes, r, lv[0].b);
   float* out = nullptr;
@@ -768,7 +780,9 @@ int64_t layout_single(hm_mg* mg, float* work32) {
 // diagonals, the coarse inverse; the Chebyshev coefficients are shared)
 void refresh_single(hm_mg* mg, cudaStream_t s) {
   const Lattice& L = mg->L;
-  k_to_float<<<4 * kMGBlocks, 256, 0, s>>>(27 * L.ne, static_cast<const double*>(mg->jac), mg->jac32);
+  k_jac_to_float<<<4 * kMGBlocks, 256, 0, s>>>(27 * (int64_t)L.ny * L.nz, L.nx, hm_jac_pitch(L, HM_FP64),
+                                               hm_jac_pitch(L, HM_FP32),
+                                               static_cast<const double*>(mg->jac), mg->jac32);
   for (int l = 0; l < mg->nlev; ++l) {
     const MGLevel& d = mg->lv[l];
     MGLevelT<float>& f = mg->lv32[l];
@@ -798,6 +812,17 @@ int hm_mg_vcycle(hm_mg* mg, const double* r, double* z, void* stream) {
   if (mg->single) return vcycle_single(mg, r, z, true, S_(stream));
   double* out = nullptr;
   return vcycle<double>(mg, 0, r, z, true, S_(stream), &out);
+}
+// the buffer and operands of the level-0 smoother's first direction, where the cycle inside
+// the solves takes it ready made
+HmFirstDir hm_mg_first_dir(const hm_mg* mg) {
+  HmFirstDir f{};
+  if (!mg->fused || mg->degree != 1 || mg->nlev < 2) return f;
+  f.idiag = mg->lv[0].idiag;
+  f.cheb = mg->lv[0].cheb;
+  if (mg->single) f.d32 = mg->lv32[0].x;
+  else f.d64 = mg->lv[0].t;
+  return f;
 }
 bool hm_mg_flexible(const hm_mg* mg) { return mg->single != 0; }
 const double* hm_mg_level0_diag(const hm_mg* mg) { return mg->lv[0].diag; }
@@ -883,7 +908,8 @@ extern "C" int hm_mg_setup(hm_mg* mg, void* jac, const uint8_t* ess, const doubl
   // coefficients and diagonals of the Q1 levels
   if (mg->nlev > 1) {
     MGLevel& q = mg->lv[1];
-    k_coef_from_q2<<<blocks_for(L.ne), 256, 0, s>>>(L.ne, static_cast<const double*>(jac),
+    k_coef_from_q2<<<blocks_for(L.ne), 256, 0, s>>>(L, hm_jac_pitch(L, HM_FP64),
+                                                    static_cast<const double*>(jac),
                                                     1.0 / (L.hx * L.hy * L.hz), q.coef);
     for (int l = 2; l < mg->nlev; ++l)
       k_coef_coarsen<<<blocks_for(mg->lv[l].elems), 256, 0, s>>>(mg->lv[l - 1], mg->lv[l],

@@ -214,20 +214,29 @@ __global__ void k_pcg_pupdate(int64_t n, const double* __restrict__ sc, const T*
     p[i] = fma(beta, p[i], z[i]);
 }
 
-// x += alpha p, r -= alpha q; partials of r.r (for a preconditioner applied after it)
+// the multigrid smoother's first direction at a node (the product rounded on its own)
+__device__ __forceinline__ void put_first_dir(const HmFirstDir& f, double inv_theta, int64_t i, double r) {
+  if (f.d64 != nullptr) f.d64[i] = __dmul_rn(inv_theta * r, f.idiag[i]);
+  else if (f.d32 != nullptr) f.d32[i] = (float)__dmul_rn(inv_theta * r, f.idiag[i]);
+}
+
+// x += alpha p, r -= alpha q, and the smoother's first direction from r; partials of r.r
+// (for a preconditioner applied after it)
 // and, given the last preconditioned residual zold, of r.zold (slot 2: the flexible step)
 __global__ void __launch_bounds__(kReduceThreads)
     k_pcg_update_rr(int64_t n, const double* __restrict__ sc, double* __restrict__ x,
                     double* __restrict__ r, const double* __restrict__ p,
-                    const double* __restrict__ q, double* __restrict__ part,
+                    const double* __restrict__ q, double* __restrict__ part, HmFirstDir f,
                     const double* __restrict__ zold = nullptr) {
   __shared__ double sh[32];
   const double alpha = sc[SC_ALPHA];
+  const double inv_theta = f.cheb != nullptr ? 1.0 / f.cheb[0] : 0.0;
   double rr = 0.0, rzc = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     x[i] = fma(alpha, p[i], x[i]);
     const double ri = fma(-alpha, q[i], r[i]);
     r[i] = ri;
+    put_first_dir(f, inv_theta, i, ri);
     rr = fma(ri, ri, rr);
     if (zold != nullptr) rzc = fma(ri, zold[i], rzc);
   }
@@ -268,15 +277,17 @@ __global__ void __launch_bounds__(kReduceThreads)
   }
 }
 
-// r = b - q; partials of r.r and b.b (slots 1 and 2)
+// r = b - q and the smoother's first direction; partials of r.r and b.b (slots 1 and 2)
 __global__ void __launch_bounds__(kReduceThreads)
     k_pcg_mg_init(int64_t n, const double* __restrict__ b, const double* __restrict__ q,
-                  double* __restrict__ r, double* __restrict__ part) {
+                  double* __restrict__ r, double* __restrict__ part, HmFirstDir f) {
   __shared__ double sh[32];
+  const double inv_theta = f.cheb != nullptr ? 1.0 / f.cheb[0] : 0.0;
   double rr = 0.0, bb = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const double ri = b[i] - q[i];
     r[i] = ri;
+    put_first_dir(f, inv_theta, i, ri);
     rr = fma(ri, ri, rr);
     bb = fma(b[i], b[i], bb);
   }
@@ -643,7 +654,8 @@ int pcg_mg_run(hm_mg* mg, const double* b, double* x, double rtol, int maxiter, 
   int64_t np = 0;
   rc = op_apply(o, x, q, nullptr, &np, stream);
   if (rc) return rc;
-  k_pcg_mg_init<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, b, q, r, part);
+  const HmFirstDir fd = hm_mg_first_dir(mg);
+  k_pcg_mg_init<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, b, q, r, part, fd);
   if ((rc = hm_mg_vcycle(mg, r, z, stream))) return rc;
   k_dot_partial_t<double><<<kReduceBlocks, kReduceThreads, 0, s>>>(n, r, z, part);
   k_pcg_init_final<<<1, 1024, 0, s>>>(part, sc, rtol);
@@ -677,7 +689,7 @@ int pcg_mg_run(hm_mg* mg, const double* b, double* x, double rtol, int maxiter, 
         int e = op_apply(o, p, q, pq_part, &np, (void*)s, sc, cnt, &fused);
         if (e) return e;
         if (!fused) k_pcg_alpha<<<1, 1024, 0, s>>>(pq_part, np, sc);
-        k_pcg_update_rr<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, sc, x, r, p, q, part,
+        k_pcg_update_rr<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, sc, x, r, p, q, part, fd,
                                                                  flex ? z : nullptr);
         if ((e = hm_mg_vcycle(mg, r, z, (void*)s))) return e;
         k_pcg_rz_beta<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, r, z, part, cnt + 1, sc, flex);
@@ -977,7 +989,8 @@ int group_init(hm_pcg_plan* pl, double rtol, cudaStream_t s) {
   int64_t np = 0;
   if ((rc = op_apply(o, pl->x, B.q, nullptr, &np, (void*)s))) return rc;
   if (pl->mg != nullptr) {
-    k_pcg_mg_init<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, pl->b, B.q, B.r, B.part);
+    k_pcg_mg_init<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, pl->b, B.q, B.r, B.part,
+                                                           hm_mg_first_dir(pl->mg));
     if ((rc = hm_mg_vcycle(pl->mg, B.r, B.z, (void*)s))) return rc;
     k_dot_partial_t<double><<<kReduceBlocks, kReduceThreads, 0, s>>>(n, B.r, B.z, B.part);
     k_pcg_init_final<<<1, 1024, 0, s>>>(B.part, B.sc, rtol);
@@ -1007,6 +1020,7 @@ int group_batch(hm_pcg_plan* pl, int count, cudaStream_t s) {
     if (!fused) k_pcg_alpha<<<1, 1024, 0, s>>>(B.pq_part, np, B.sc);
     const int flex = hm_mg_flexible(pl->mg) ? 1 : 0;
     k_pcg_update_rr<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, B.sc, pl->x, B.r, B.p, B.q, B.part,
+                                                             hm_mg_first_dir(pl->mg),
                                                              flex ? B.z : nullptr);
     if ((e = hm_mg_vcycle(pl->mg, B.r, B.z, (void*)s))) return e;
     k_pcg_rz_beta<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, B.r, B.z, B.part, B.cnt + 1, B.sc, flex);

@@ -20,6 +20,7 @@
 
 #include <mutex>
 
+#include "hm_async.cuh"
 #include "hm_common.cuh"
 #include "hm_internal.h"
 
@@ -158,35 +159,7 @@ struct TileSmem {
 };
 static_assert(sizeof(TileSmem<double>) <= 113 * 1024, "two CTAs per SM");
 
-// ------------------------------------------------------------- TMA + mbarrier
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(unsigned long long* b, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void fence_mbar_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void fence_proxy_async() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// a bounded wait: false if the copy has not landed after ~2^20 polls
-__device__ __forceinline__ bool mbar_wait(unsigned long long* b, uint32_t parity) {
-  for (int i = 0; i < (1 << 20); ++i)
-    if (mbar_try_wait(b, parity)) return true;
-  return false;
-}
+// ------------------------------------------------------------- TMA
 // one thread: the phase's fields of the tile's 27 elements into a buffer
 template <typename real>
 __device__ __forceinline__ void issue_fields(const CUtensorMap* tmap, TileSmem<real>& S, int buf,
@@ -863,10 +836,8 @@ __global__ void __launch_bounds__(256, 2)
 }
 
 // ------------------------------------------------------------ host side
-namespace {
-inline cudaStream_t S_(void* s) { return reinterpret_cast<cudaStream_t>(s); }
-
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
+}  // namespace hm
+PFN_cuTensorMapEncodeTiled_v12000 hm_tensor_map_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   static std::once_flag once;
   std::call_once(once, [] {
@@ -879,10 +850,14 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
+namespace hm {
+namespace {
+inline cudaStream_t S_(void* s) { return reinterpret_cast<cudaStream_t>(s); }
+
 // the quadrature array as a 4D tensor (216 reals per element, ex, ey, ez)
 template <typename real>
 int make_quad_map(const Lattice& L, const void* quad, CUtensorMap* m) {
-  auto fn = encode_fn();
+  auto fn = hm_tensor_map_encoder();
   if (fn == nullptr) return HM_ERR_CUDA;
   if ((reinterpret_cast<uintptr_t>(quad) & 15u) != 0) return HM_ERR_ARG;
   const cuuint64_t es = sizeof(real);
@@ -941,6 +916,12 @@ int hm_launch_assemble(const Lattice& L, const void* quad, int precision, const 
     if ((reinterpret_cast<uintptr_t>(v) & 15u) != 0) return HM_ERR_ARG;
   if (precision == HM_FP32) return launch_assemble_t<float>(L, quad, indptr, ess, o, stream);
   return launch_assemble_t<double>(L, quad, indptr, ess, o, stream);
+}
+
+// the status word's address on the current device, for the other kernels' bounded waits
+uint32_t* hm_status_word() {
+  void* p = nullptr;
+  return cudaGetSymbolAddress(&p, g_device_status) == cudaSuccess ? static_cast<uint32_t*>(p) : nullptr;
 }
 
 extern "C" int hm_device_status(uint32_t* out, int clear) {
