@@ -300,6 +300,7 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlock
   if (element) plane_to_points(ring + base, RS, low);
 #pragma unroll
   for (int k = 0; k < 4; ++k) xlow[k] = own ? ring[base + (k >> 1) * RS + (k & 1)] : real(0);
+  __syncthreads();                        // plane 0's slot is plane 6's, requested next
   double dot = 0.0;
 #pragma unroll 1
   for (int l = 0; l < layers; ++l) {
