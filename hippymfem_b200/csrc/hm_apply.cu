@@ -47,22 +47,25 @@ constexpr int kRing = 6;             // node planes: a layer's two upper ones, f
 // what the input vector stands for: the vector itself (zero on the Dirichlet nodes), or the
 // vector with the Dirichlet nodes zeroed on the fly
 enum ApplyIn { IN_CLEAN = 0, IN_ESS = 1 };
-// what is written for a node's product: y = A x (x itself on the Dirichlet nodes); the
-// residual b - A x; the smoothing step x + (b - A x) idiag / theta
-enum ApplyOut { OUT_Y = 0, OUT_R = 1, OUT_STEP = 2 };
+// what is done with a node's product: y = A x (x itself on the Dirichlet nodes), or a pass
+// of the smoother (HmChebMode)
+enum ApplyOut { OUT_Y = 0, OUT_R = 1, OUT_STEP1 = 2, OUT_START = 3, OUT_NEXT = 4 };
 
-template <typename src, typename vec, typename res>
+// the constant of HmCheb's kChebMax (cheb[1 + k]: c1_k, cheb[1 + kChebMax + k]: c2_k)
+constexpr int kChebMax = 40;
+
+template <typename src, typename vec>
 struct ApplyArgs {
   const uint8_t* ess;
   const src* x;            // the input vector
-  const double* b;         // the right-hand side (OUT_R, OUT_STEP)
-  const double* idiag;     // reciprocal of the Jacobi diagonal (OUT_STEP)
-  const double* cheb;      // theta = cheb[0] (OUT_STEP)
-  vec* y;                  // OUT_Y, OUT_R
-  res* z;                  // OUT_STEP
-  double* part;            // OUT_Y: partial sums of x . y, one per CTA (NULL: none)
-  double* sc;              // with part: the CG step's scalars (alpha from the last block)
+  vec* y;                  // OUT_Y
+  HmCheb<vec> c;           // the smoother's operands
+  double* part;            // partial sums of x . y (OUT_Y) or b . z, one per CTA (NULL: none)
+  double* sc;              // with part: the CG step's scalars (alpha or beta from the last block)
   unsigned* counter;
+  const double* rr;        // beta: the partials of r.r
+  unsigned nrr;
+  int flex;
   uint32_t* status;        // the library's status word (a bounded wait that gave up)
   int tma, pitch;          // D by TMA; its row pitch
 };
@@ -183,10 +186,10 @@ struct ApplySmem {
   }
 };
 
-template <typename real, typename src, typename vec, typename res, int IN, int OUT>
+template <typename real, typename src, typename vec, int IN, int OUT>
 __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlocks : 4)
     k_apply_tile(const __grid_constant__ CUtensorMap map, const Lattice L, const real* __restrict__ Dq,
-                 const ApplyArgs<src, vec, res> a) {
+                 const ApplyArgs<src, vec> a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ unsigned long long mbar[2];           // D of the even and the odd layers
   const ApplySmem<real> at(L.ap);
@@ -283,7 +286,12 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlock
   const bool element = column && cx < L.nx && cy < L.ny;
   const bool own = column && cx <= L.nx && cy <= L.ny && (tx > 0 || i1 == 0) && (ty > 0 || i2 == 0);
   double inv_theta = 0.0;
-  if constexpr (OUT == OUT_STEP) inv_theta = 1.0 / __ldg(a.cheb);
+  if constexpr (OUT == OUT_STEP1 || OUT == OUT_START) inv_theta = 1.0 / __ldg(a.c.cheb);
+  double w1 = 0.0, w2 = 0.0;               // step k: dout = w1 in + w2 r idiag
+  if constexpr (OUT == OUT_NEXT) {
+    w1 = __ldg(a.c.cheb + 1 + a.c.k);
+    w2 = __ldg(a.c.cheb + 1 + kChebMax + a.c.k);
+  }
   copy_wait<1>();
   for (int j = 0; j < 3; ++j) finish(j);
   __syncthreads();
@@ -373,14 +381,19 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlock
     }
     // the input at the own nodes, the smoother's operands
     real xc[8];
-    double bn[OUT == OUT_Y ? 1 : 8], gn[OUT == OUT_STEP ? 8 : 1];
+    double bn[OUT == OUT_Y ? 1 : 8], gn[OUT == OUT_Y || OUT == OUT_R ? 1 : 8], xn[OUT == OUT_NEXT ? 8 : 1];
     unsigned fixed = 0;
 #pragma unroll
     for (int h = 0; h < 8; ++h) {
       const bool on = (have >> h) & 1u;
       const unsigned node = n0 + (h & 1) + ((h & 2) ? nsy : 0u) + ((h & 4) ? nsz : 0u);
-      if constexpr (OUT != OUT_Y) bn[h] = on ? __ldg(a.b + node) : 0.0;
-      if constexpr (OUT == OUT_STEP) gn[h] = on ? __ldg(a.idiag + node) : 0.0;
+      if constexpr (OUT == OUT_NEXT) {
+        bn[h] = !on ? 0.0 : a.c.first ? __ldg(a.c.b + node) : (double)a.c.r[node];
+        xn[h] = !on || a.c.first ? 0.0 : (double)a.c.x[node];
+      } else if constexpr (OUT != OUT_Y) {
+        bn[h] = on ? __ldg(a.c.b + node) : 0.0;
+      }
+      if constexpr (OUT != OUT_Y && OUT != OUT_R) gn[h] = on ? __ldg(a.c.idiag + node) : 0.0;
       const int o = ((h >> 1) & 1) * RS + (h & 1);
       if (h < 4) {
         xc[h] = xlow[h];
@@ -426,25 +439,74 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlock
             const double yv = fx ? xv : acc;
             a.y[node] = (vec)yv;
             dot = fma(xv, yv, dot);
-          } else if constexpr (OUT == OUT_R) {
-            a.y[node] = (vec)(bn[h] - (fx ? (double)xc[h] : acc));
           } else {
-            // the update rounded on its own before the add, as the step-by-step smoother
-            const double xn = (double)xc[h];
-            a.z[node] = (res)(xn + __dmul_rn(inv_theta * (bn[h] - (fx ? xn : acc)), gn[h]));
+            const double in = (double)xc[h];
+            const double ri = bn[h] - (fx ? in : acc);
+            if constexpr (OUT == OUT_R) {
+              a.c.r[node] = (vec)ri;
+            } else if constexpr (OUT == OUT_STEP1) {
+              // the update rounded on its own before the add, as the step-by-step smoother
+              const double z = in + __dmul_rn(inv_theta * ri, gn[h]);
+              a.c.z[node] = z;
+              dot = fma(bn[h], z, dot);
+            } else if constexpr (OUT == OUT_START) {
+              a.c.r[node] = (vec)ri;
+              a.c.dout[node] = (vec)(inv_theta * ri * gn[h]);
+            } else {
+              const double xi = a.c.first ? in : xn[h] + in;
+              const double dn = fma(w1, in, w2 * ri * gn[h]);
+              if (a.c.last == 2) {
+                const double z = xi + dn;
+                a.c.z[node] = z;
+                if (a.part != nullptr) dot = fma(__ldg(a.c.b + node), z, dot);
+              } else {
+                a.c.x[node] = (vec)xi;
+                a.c.r[node] = (vec)ri;
+                if (a.c.last == 0) a.c.dout[node] = (vec)dn;
+              }
+            }
           }
         }
       }
     }
   }
   copy_wait<0>();
-  if (OUT == OUT_Y && a.part != nullptr) {
+  if (OUT != OUT_R && OUT != OUT_START && a.part != nullptr) {
     __shared__ double sh[32];
     const double t = block_sum(dot, sh);
     if (tid == 0) a.part[blockIdx.x] = t;
-    // a CG step: the last block takes alpha from the partials
-    if (a.sc != nullptr && last_block(a.counter)) finish_alpha(a.part, gridDim.x, a.sc, a.counter, sh);
+    // a CG step: the last block takes alpha, or beta, from the partials
+    if (a.sc != nullptr && last_block(a.counter)) {
+      if constexpr (OUT == OUT_Y) finish_alpha(a.part, gridDim.x, a.sc, a.counter, sh);
+      else finish_beta(a.part, gridDim.x, a.rr, a.nrr, a.flex, a.sc, a.counter, sh);
+    }
   }
+}
+
+// b . z and the CG step's beta on their own, after a cycle that ends in another kernel: the
+// sum in k_apply_tile's order (a thread's own nodes layer by layer), so that a solve does
+// not depend on which of the two took it
+__global__ void __launch_bounds__(kApplyThreads)
+    k_tile_beta(const Lattice L, const double* __restrict__ b, const double* __restrict__ z, HmBeta be) {
+  __shared__ double sh[32];
+  const int T1 = L.ap.T1, T2 = L.ap.T2, bt = blockIdx.x;
+  const int i1 = bt % L.ap.t1, i2 = (bt / L.ap.t1) % L.ap.t2, i3 = bt / (L.ap.t1 * L.ap.t2);
+  const int ty = threadIdx.x / T1, tx = threadIdx.x - ty * T1;
+  const int cx = i1 * (T1 - 1) + tx, cy = i2 * (T2 - 1) + ty, c3 = i3 * (L.ap.T3 - 1);
+  const bool own = ty < T2 && cx <= L.nx && cy <= L.ny && (tx > 0 || i1 == 0) && (ty > 0 || i2 == 0);
+  const int layers = min(L.ap.T3, L.nz + 1 - c3);
+  double dot = 0.0;
+  if (own)
+    for (int l = i3 == 0 ? 0 : 1; l < layers; ++l)
+      for (int h = 0; h < 8; ++h) {
+        const int x = 2 * cx + (h & 1), y = 2 * cy + ((h >> 1) & 1), w = 2 * (c3 + l) + (h >> 2);
+        if (x >= L.Nx || y >= L.Ny || w >= L.Nz) continue;
+        const int64_t n = x + (int64_t)L.Nx * (y + (int64_t)L.Ny * w);
+        dot = fma(b[n], z[n], dot);
+      }
+  const double t = block_sum(dot, sh);
+  if (threadIdx.x == 0) be.rz[blockIdx.x] = t;
+  if (last_block(be.counter)) finish_beta(be.rz, gridDim.x, be.rr, be.n, be.flex, be.sc, be.counter, sh);
 }
 
 }  // namespace hm
@@ -506,9 +568,9 @@ int hm_jac_pitch(const Lattice& L, int precision) {
 }
 
 namespace {
-template <typename real, typename src, typename vec, typename res, int IN, int OUT>
-int launch(const Lattice& L, const void* jac, ApplyArgs<src, vec, res> a, void* stream) {
-  auto kern = k_apply_tile<real, src, vec, res, IN, OUT>;
+template <typename real, typename src, typename vec, int IN, int OUT>
+int launch(const Lattice& L, const void* jac, ApplyArgs<src, vec> a, void* stream) {
+  auto kern = k_apply_tile<real, src, vec, IN, OUT>;
   const size_t smem = (size_t)ApplySmem<real>(L.ap).bytes;
   a.pitch = hm_jac_pitch(L, sizeof(real) == 8 ? HM_FP64 : HM_FP32);
   CUtensorMap map{};
@@ -546,12 +608,12 @@ int launch(const Lattice& L, const void* jac, ApplyArgs<src, vec, res> a, void* 
 template <typename real, typename T>
 int apply_y(const Lattice& L, const void* jac, const uint8_t* ess, const T* x, T* y, bool clean,
             double* part, double* sc, unsigned* counter, void* stream) {
-  ApplyArgs<T, T, T> a{};
+  ApplyArgs<T, T> a{};
   a.ess = ess; a.x = x; a.y = y; a.part = part;
   a.sc = part != nullptr ? sc : nullptr;
   a.counter = counter;
-  if (clean) return launch<real, T, T, T, IN_CLEAN, OUT_Y>(L, jac, a, stream);
-  return launch<real, T, T, T, IN_ESS, OUT_Y>(L, jac, a, stream);
+  if (clean) return launch<real, T, T, IN_CLEAN, OUT_Y>(L, jac, a, stream);
+  return launch<real, T, T, IN_ESS, OUT_Y>(L, jac, a, stream);
 }
 }  // namespace
 
@@ -590,35 +652,28 @@ int hm_launch_apply_A32_dot(const Lattice& L, void* jac32, const uint8_t* ess, c
   return apply_y<float>(L, jac32, ess, x, y, true, part, sc, counter, stream);
 }
 
-// The operator passes of a Chebyshev-Jacobi smoothing step of degree 1 (every vector zero
-// on the Dirichlet nodes; idiag the reciprocal of the Jacobi diagonal, theta = cheb[0]):
-//   r = b - A d                        (pre-smoothing from zero: d = b idiag / theta)
-//   z = x + (b - A x) idiag / theta    (post-smoothing; z != x)
-// the same arithmetic as the start / step / finish kernels of the multigrid smoother.  In
-// the FP32 cycle d, r and x are FP32; b, the update and z stay FP64.
-int hm_launch_residual(const Lattice& L, void* jac, const uint8_t* ess, const double* b,
-                       const double* d, double* r, void* stream) {
-  ApplyArgs<double, double, double> a{};
-  a.ess = ess; a.x = d; a.b = b; a.y = r;
-  return launch<double, double, double, double, IN_CLEAN, OUT_R>(L, jac, a, stream);
+// A pass of the multigrid smoother: the arithmetic of its start / step / finish kernels.
+// In the FP32 cycle in, x, r and dout are FP32; b, the update and z stay FP64.
+template <typename T>
+int hm_launch_cheb(const Lattice& L, void* jac, const uint8_t* ess, const HmCheb<T>& c, void* stream) {
+  ApplyArgs<T, T> a{};
+  a.ess = ess; a.x = c.in; a.c = c;
+  a.c.beta = nullptr;                      // a host address
+  if (c.beta != nullptr && (c.mode == CH_STEP1 || (c.mode == CH_NEXT && c.last == 2))) {
+    a.part = c.beta->rz; a.sc = c.beta->sc; a.counter = c.beta->counter;
+    a.rr = c.beta->rr; a.nrr = c.beta->n; a.flex = c.beta->flex;
+    c.beta->done = 1;
+  }
+  switch (c.mode) {
+    case CH_RESIDUAL: return launch<T, T, T, IN_CLEAN, OUT_R>(L, jac, a, stream);
+    case CH_STEP1: return launch<T, T, T, IN_CLEAN, OUT_STEP1>(L, jac, a, stream);
+    case CH_START: return launch<T, T, T, IN_CLEAN, OUT_START>(L, jac, a, stream);
+    default: return launch<T, T, T, IN_CLEAN, OUT_NEXT>(L, jac, a, stream);
+  }
 }
-int hm_launch_residual32(const Lattice& L, void* jac32, const uint8_t* ess, const double* b,
-                         const float* d, float* r, void* stream) {
-  ApplyArgs<float, float, float> a{};
-  a.ess = ess; a.x = d; a.b = b; a.y = r;
-  return launch<float, float, float, float, IN_CLEAN, OUT_R>(L, jac32, a, stream);
-}
-int hm_launch_cheb1_step(const Lattice& L, void* jac, const uint8_t* ess, const double* b,
-                         const double* idiag, const double* cheb, const double* x, double* z,
-                         void* stream) {
-  ApplyArgs<double, double, double> a{};
-  a.ess = ess; a.x = x; a.b = b; a.idiag = idiag; a.cheb = cheb; a.z = z;
-  return launch<double, double, double, double, IN_CLEAN, OUT_STEP>(L, jac, a, stream);
-}
-int hm_launch_cheb1_step32(const Lattice& L, void* jac32, const uint8_t* ess, const double* b,
-                           const double* idiag, const double* cheb, const float* x, double* z,
-                           void* stream) {
-  ApplyArgs<float, float, double> a{};
-  a.ess = ess; a.x = x; a.b = b; a.idiag = idiag; a.cheb = cheb; a.z = z;
-  return launch<float, float, float, double, IN_CLEAN, OUT_STEP>(L, jac32, a, stream);
+template int hm_launch_cheb<double>(const Lattice&, void*, const uint8_t*, const HmCheb<double>&, void*);
+template int hm_launch_cheb<float>(const Lattice&, void*, const uint8_t*, const HmCheb<float>&, void*);
+int hm_launch_beta(const Lattice& L, const double* b, const double* z, const HmBeta& be, void* stream) {
+  k_tile_beta<<<L.ap.t1 * L.ap.t2 * L.ap.t3, L.ap.threads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(L, b, z, be);
+  return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
 }

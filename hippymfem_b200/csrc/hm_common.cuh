@@ -174,6 +174,43 @@ __device__ __forceinline__ void finish_alpha(const double* part, unsigned nparts
     *counter = 0u;
   }
 }
+// beta = ((r.z)_new - rzc) / (r.z)_old, the convergence test and the iteration count
+// (thread 0).  rzc = 0: Fletcher-Reeves; rzc = r_new . z_old: a Polak-Ribiere-type step
+// for a preconditioner that is symmetric only to rounding.  The textbook flexible step
+// (Golub and Ye 1999) takes z_new . r_old instead; for a symmetric preconditioner the
+// two cross terms are equal, and both vanish in exact arithmetic.  With the FP32 V-cycle
+// at high contrast the textbook step stalled on fields where this one converged.
+__device__ __forceinline__ void beta_step(double rz, double rr, double* sc, double rzc = 0.0) {
+  const bool was = sc[SC_CONV] >= 0.0;
+  if (!was) {
+    const double it = sc[SC_IT] + 1.0;
+    sc[SC_IT] = it;
+    sc[SC_RR] = rr;
+    if (rr <= sc[SC_TOL2] * sc[SC_BB]) sc[SC_CONV] = it;
+    const double beta = sc[SC_RZ] == 0.0 ? 0.0 : (rz - rzc) / sc[SC_RZ];
+    sc[SC_BETA] = isfinite(beta) ? beta : 0.0;
+    sc[SC_RZ] = rz;
+  }
+}
+
+// the step's beta from the partials of r.z (nz of them), r.r and, for the flexible step,
+// r.z_old (n each, rr and rr + n), by the last block
+__device__ __forceinline__ void finish_beta(const double* rz, unsigned nz, const double* rr, unsigned n,
+                                            int flex, double* sc, unsigned* counter, double* sh) {
+  double v0 = 0.0, v1 = 0.0, v2 = 0.0;
+  for (unsigned b = threadIdx.x; b < nz; b += blockDim.x) v0 += __ldcg(rz + b);
+  for (unsigned b = threadIdx.x; b < n; b += blockDim.x) {
+    v1 += __ldcg(rr + b);
+    if (flex) v2 += __ldcg(rr + n + b);
+  }
+  v0 = block_sum(v0, sh);
+  v1 = block_sum(v1, sh);
+  if (flex) v2 = block_sum(v2, sh);
+  if (threadIdx.x == 0) {
+    beta_step(v0, v1, sc, v2);
+    *counter = 0u;
+  }
+}
 #endif
 
 }  // namespace hm

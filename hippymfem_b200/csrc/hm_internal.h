@@ -52,17 +52,47 @@ int hm_plan_buffers(const hm_pcg_plan* plan, double** b, double** x);
 // the FP32 operator (jac32: the points' D in FP32) on FP32 vectors; clean: x zero on the Dirichlet nodes
 int hm_launch_apply_A32(const hm::Lattice& L, void* jac32, const uint8_t* ess, const float* x,
                         float* y, bool clean, void* stream);
-// the operator passes of the multigrid smoother's steps of degree 1 (hm_apply.cu)
-int hm_launch_residual(const hm::Lattice& L, void* jac, const uint8_t* ess, const double* b,
-                       const double* d, double* r, void* stream);
-int hm_launch_residual32(const hm::Lattice& L, void* jac32, const uint8_t* ess, const double* b,
-                         const float* d, float* r, void* stream);
-int hm_launch_cheb1_step(const hm::Lattice& L, void* jac, const uint8_t* ess, const double* b,
-                         const double* idiag, const double* cheb, const double* x, double* z,
-                         void* stream);
-int hm_launch_cheb1_step32(const hm::Lattice& L, void* jac32, const uint8_t* ess, const double* b,
-                           const double* idiag, const double* cheb, const float* x, double* z,
-                           void* stream);
+// Inside the MG-PCG: r.z and the step's beta, taken by the cycle's last operator pass
+// (done set) where it can: rz room for its partials, rr the n partials of r.r, then those of
+// r.z_old with flex
+struct HmBeta {
+  double* rz;
+  const double* rr;
+  unsigned n;
+  int flex;
+  double* sc;
+  unsigned* counter;
+  int done;
+};
+// the same on its own
+int hm_launch_beta(const hm::Lattice& L, const double* b, const double* z, const HmBeta& be, void* stream);
+int hm_mg_vcycle(hm_mg* mg, const double* r, double* z, void* stream, HmBeta* beta = nullptr);
+// One operator pass of the level-0 Chebyshev-Jacobi smoother (hm_apply.cu), every vector
+// zero on the Dirichlet nodes, T the cycle's precision:
+//   CH_RESIDUAL  r = b - A in                     (degree 1: in = x = the first direction)
+//   CH_STEP1     z = in + (b - A in) idiag / theta, z != in
+//   CH_START     r = b - A in, dout = r idiag / theta
+//   CH_NEXT      step k: r -= A in (first: r = b - A in), x += in (first: x = in),
+//                dout = c1_k in + c2_k r idiag; last = 1: no dout; last = 2: z = x + dout,
+//                nothing else stored
+// With beta (CH_STEP1, or CH_NEXT with last = 2) the pass also takes b.z and the CG
+// step's beta.
+enum HmChebMode { CH_RESIDUAL = 0, CH_STEP1 = 1, CH_START = 2, CH_NEXT = 3 };
+template <typename T>
+struct HmCheb {
+  int mode, k, first, last;
+  const double* b;
+  const double* idiag;
+  const double* cheb;
+  const T* in;
+  T* x;
+  T* r;
+  T* dout;
+  double* z;
+  HmBeta* beta;
+};
+template <typename T>
+int hm_launch_cheb(const hm::Lattice& L, void* jac, const uint8_t* ess, const HmCheb<T>& c, void* stream);
 // Inside the MG-PCG: where the level-0 smoother's first direction d = r idiag / theta is
 // wanted (d64 or d32; both null: nowhere), formed by the kernel that forms r
 struct HmFirstDir {

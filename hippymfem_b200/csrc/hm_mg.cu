@@ -19,6 +19,7 @@
 // written in FP64, the CG around it unchanged).  Deterministic, and free of host
 // synchronisation after set-up, so a CG iteration with its V-cycle can be captured as a
 // CUDA graph.
+#include <atomic>
 #include <cmath>
 #include <new>
 #include <type_traits>
@@ -60,8 +61,9 @@ struct hm_mg {
   int degree, coarse_degree;
   double* scratch;       // partial sums of the set-up's inner products, eigenvalue state
   const uint8_t* checked_ess;   // the markers last found to be the whole boundary
-  int tail_first;        // first level of the one-CTA tail (nlev: none)
-  int fused;             // degree-1 smoothing steps fused with their operator pass
+  int tail_first;        // first level of the one-launch tail (nlev: none)
+  int64_t tail_nodes;    // its levels' nodes at most
+  int fused;             // smoothing steps fused with their operator pass
   // the FP32 cycle (single != 0): every level's vectors, coefficients, reciprocal
   // diagonal and coarse inverse in single precision, refreshed from the FP64 set-up; the
   // level-0 operator data (the points' D, then the element results) in jac32
@@ -82,91 +84,148 @@ __device__ __forceinline__ bool on_boundary(int i, int j, int k, int Nx, int Ny,
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 
-// (A_l x)[n] for a Q1 level: node-centric, identity on the boundary, boundary values of
-// x taken as zero in the interior rows; x given by xv(node)
-template <typename T, typename XV>
-__device__ __forceinline__ T q1_apply_with(const MGLevelT<T>& lv, int64_t n, XV xv) {
-  const int i = (int)(n % lv.Nx);
-  const int64_t t = n / lv.Nx;
-  const int j = (int)(t % lv.Ny), k = (int)(t / lv.Ny);
-  if (on_boundary(i, j, k, lv.Nx, lv.Ny, lv.Nz)) return xv(n);
-  // 1D element matrices: k = [1 -1; -1 1] / h, m = [2 1; 1 2] h / 6
-  const T kx[2] = {T(1.0 / lv.hx), T(-1.0 / lv.hx)}, ky[2] = {T(1.0 / lv.hy), T(-1.0 / lv.hy)},
-          kz[2] = {T(1.0 / lv.hz), T(-1.0 / lv.hz)};
-  const T mx[2] = {T(lv.hx / 3.0), T(lv.hx / 6.0)}, my[2] = {T(lv.hy / 3.0), T(lv.hy / 6.0)},
-          mz[2] = {T(lv.hz / 3.0), T(lv.hz / 6.0)};
+// A node of a level by its number (32-bit: the lattice keeps every index below 2^31).
+struct MGNode { int i, j, k; };
+template <typename T>
+__device__ __forceinline__ MGNode node_at(const MGLevelT<T>& lv, unsigned n) {
+  const unsigned t = n / (unsigned)lv.Nx;
+  const unsigned k = t / (unsigned)lv.Ny;
+  return {(int)(n - t * (unsigned)lv.Nx), (int)(t - k * (unsigned)lv.Ny), (int)k};
+}
+template <typename T>
+__device__ __forceinline__ bool on_boundary(const MGLevelT<T>& lv, const MGNode& q) {
+  return on_boundary(q.i, q.j, q.k, lv.Nx, lv.Ny, lv.Nz);
+}
+
+// The eight entries of an element's matrix on unit coefficient, by the axes along which
+// its two nodes differ (bit 0: x, 1: y, 2: z): 1D k = [1 -1; -1 1] / h, m = [2 1; 1 2] h / 6.
+template <typename T>
+struct Q1Entries {
+  T k[8];
+  __host__ __device__ explicit Q1Entries(const T (&entries)[8]) {
+    for (int o = 0; o < 8; ++o) k[o] = entries[o];
+  }
+  template <typename Level>
+  __host__ __device__ explicit Q1Entries(const Level& lv) {
+    const T kx[2] = {T(1.0 / lv.hx), T(-1.0 / lv.hx)}, ky[2] = {T(1.0 / lv.hy), T(-1.0 / lv.hy)},
+            kz[2] = {T(1.0 / lv.hz), T(-1.0 / lv.hz)};
+    const T mx[2] = {T(lv.hx / 3.0), T(lv.hx / 6.0)}, my[2] = {T(lv.hy / 3.0), T(lv.hy / 6.0)},
+            mz[2] = {T(lv.hz / 3.0), T(lv.hz / 6.0)};
+    for (int o = 0; o < 8; ++o) {
+      const int x = o & 1, y = (o >> 1) & 1, z = o >> 2;
+      k[o] = kx[x] * my[y] * mz[z] + mx[x] * ky[y] * mz[z] + mx[x] * my[y] * kz[z];
+    }
+  }
+};
+
+// (A_l x) at an interior node of a Q1 level from the 8 elements' coefficients and the 27
+// nodes' values: the coefficients of the elements between the
+// node and each neighbour summed first (4 for a face neighbour, 2 for an edge, 1 for a
+// corner), the neighbours of one class then times that class's matrix entry.  x is zero on
+// the boundary (every vector of the coarse levels is).
+template <typename T>
+__device__ __forceinline__ T q1_stencil(const Q1Entries<T>& K, const T (&c)[2][2][2], const T (&xs)[3][3][3]) {
+  // edge sums (two elements), face sums (four), all eight
+  T zy[2][2], zx[2][2], yx[2][2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      zy[u][v] = c[u][v][0] + c[u][v][1];
+      zx[u][v] = c[u][0][v] + c[u][1][v];
+      yx[u][v] = c[0][u][v] + c[1][u][v];
+    }
+  const T fz[2] = {zy[0][0] + zy[0][1], zy[1][0] + zy[1][1]};
+  const T fy[2] = {zy[0][0] + zy[1][0], zy[0][1] + zy[1][1]};
+  const T fx[2] = {zx[0][0] + zx[1][0], zx[0][1] + zx[1][1]};
+  T acc = K.k[0] * ((fz[0] + fz[1]) * xs[1][1][1]);
+  acc = fma(K.k[1], fma(fx[0], xs[1][1][0], fx[1] * xs[1][1][2]), acc);
+  acc = fma(K.k[2], fma(fy[0], xs[1][0][1], fy[1] * xs[1][2][1]), acc);
+  acc = fma(K.k[4], fma(fz[0], xs[0][1][1], fz[1] * xs[2][1][1]), acc);
+  T s3 = T(0), s5 = T(0), s6 = T(0), s7 = T(0);
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      s3 = fma(yx[u][v], xs[1][2 * u][2 * v], s3);
+      s5 = fma(zx[u][v], xs[2 * u][1][2 * v], s5);
+      s6 = fma(zy[u][v], xs[2 * u][2 * v][1], s6);
+      s7 = fma(c[u][v][0], xs[2 * u][2 * v][0], s7);
+      s7 = fma(c[u][v][1], xs[2 * u][2 * v][2], s7);
+    }
+  acc = fma(K.k[3], s3, acc);
+  acc = fma(K.k[5], s5, acc);
+  acc = fma(K.k[6], s6, acc);
+  return fma(K.k[7], s7, acc);
+}
+template <typename T>
+__device__ __forceinline__ T q1_apply_at(const MGLevelT<T>& lv, const Q1Entries<T>& K, const T* x,
+                                         unsigned n, const MGNode& q) {
+  const unsigned sy = (unsigned)lv.Nx, sz = sy * (unsigned)lv.Ny;
+  const unsigned e0 = (unsigned)(q.i - 1) + (unsigned)lv.nx * ((unsigned)(q.j - 1) + (unsigned)lv.ny * (unsigned)(q.k - 1));
+  T c[2][2][2];
+#pragma unroll
+  for (int z = 0; z < 2; ++z)
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+      for (int w = 0; w < 2; ++w)
+        c[z][y][w] = lv.coef[e0 + w + (unsigned)lv.nx * (y + (unsigned)lv.ny * z)];
   T xs[3][3][3];
+  const T* const x0 = x + (n - 1u - sy - sz);
 #pragma unroll
-  for (int dk = 0; dk < 3; ++dk)
+  for (int z = 0; z < 3; ++z)
 #pragma unroll
-    for (int dj = 0; dj < 3; ++dj)
+    for (int y = 0; y < 3; ++y)
 #pragma unroll
-      for (int di = 0; di < 3; ++di) {
-        const int ii = i + di - 1, jj = j + dj - 1, kk = k + dk - 1;
-        xs[dk][dj][di] = on_boundary(ii, jj, kk, lv.Nx, lv.Ny, lv.Nz)
-                             ? T(0) : xv(ii + (int64_t)lv.Nx * (jj + (int64_t)lv.Ny * kk));
-      }
-  T acc = T(0);
-#pragma unroll
-  for (int e3 = 0; e3 < 2; ++e3)
-#pragma unroll
-    for (int e2 = 0; e2 < 2; ++e2)
-#pragma unroll
-      for (int e1 = 0; e1 < 2; ++e1) {
-        // element (i-1+e1, j-1+e2, k-1+e3); the node's local index is 1 - e
-        const T c = lv.coef[(i - 1 + e1) + (int64_t)lv.nx * ((j - 1 + e2) + (int64_t)lv.ny * (k - 1 + e3))];
-        T s = T(0);
-#pragma unroll
-        for (int b3 = 0; b3 < 2; ++b3)
-#pragma unroll
-          for (int b2 = 0; b2 < 2; ++b2)
-#pragma unroll
-            for (int b1 = 0; b1 < 2; ++b1) {
-              // K[a][b] with a = 1 - e, so |a - b| = |1 - e - b|: entry 0 on the diagonal
-              const int o1 = (1 - e1) != b1, o2 = (1 - e2) != b2, o3 = (1 - e3) != b3;
-              const T kab = kx[o1] * my[o2] * mz[o3] + mx[o1] * ky[o2] * mz[o3] +
-                            mx[o1] * my[o2] * kz[o3];
-              s = fma(kab, xs[e3 + b3][e2 + b2][e1 + b1], s);
-            }
-        acc = fma(c, s, acc);
-      }
-  return acc;
+      for (int w = 0; w < 3; ++w) xs[z][y][w] = x0[w + sy * y + sz * z];
+  return q1_stencil(K, c, xs);
 }
+// the same at any node (identity on the boundary)
 template <typename T>
-__device__ __forceinline__ T q1_apply_at(const MGLevelT<T>& lv, const T* __restrict__ x, int64_t n) {
-  return q1_apply_with(lv, n, [&](int64_t m) { return x[m]; });
+__device__ __forceinline__ T q1_row(const MGLevelT<T>& lv, const Q1Entries<T>& K, const T* x, unsigned n) {
+  const MGNode q = node_at(lv, n);
+  return on_boundary(lv, q) ? x[n] : q1_apply_at(lv, K, x, n, q);
 }
-// A Chebyshev-Jacobi step of degree 1 of a Q1 level with its operator pass (the same
-// arithmetic as k_cheb_start / k_cheb_step / k_cheb_finish around k_q1_apply):
-//   from zero (pre-smoothing):  x = d = b idiag / theta,  r = b - A d
-//   from xin (post-smoothing):  xout = xin + (b - A xin) idiag / theta   (xout != xin)
+
 template <typename T>
-__global__ void __launch_bounds__(256) k_q1_cheb1_from_zero(MGLevelT<T> lv, const T* __restrict__ b) {
-  const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (n >= lv.nodes) return;
-  const T inv_theta = T(1.0 / lv.cheb[0]);
-  const T* __restrict__ idiag = lv.idiag;
-  // the products rounded on their own (mul_rn), as the step-by-step kernels store them,
-  // so that no multiply-add contraction changes a bit
-  const T t = q1_apply_with(lv, n, [&](int64_t m) { return mul_rn(inv_theta * b[m], idiag[m]); });
-  lv.x[n] = mul_rn(inv_theta * b[n], idiag[n]);
-  lv.r[n] = b[n] - t;
-}
-template <typename T>
-__global__ void __launch_bounds__(256) k_q1_cheb1_from_x(MGLevelT<T> lv, const T* __restrict__ b,
-                                                         const T* __restrict__ xin,
-                                                         T* __restrict__ xout) {
-  const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (n >= lv.nodes) return;
-  const T inv_theta = T(1.0 / lv.cheb[0]);
-  const T t = q1_apply_at(lv, xin, n);
-  xout[n] = xin[n] + mul_rn(inv_theta * (b[n] - t), lv.idiag[n]);
-}
-template <typename T>
-__global__ void __launch_bounds__(256) k_q1_apply(MGLevelT<T> lv, const T* __restrict__ x,
+__global__ void __launch_bounds__(256) k_q1_apply(MGLevelT<T> lv, Q1Entries<T> K, const T* __restrict__ x,
                                                   T* __restrict__ y) {
-  const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (n < lv.nodes) y[n] = q1_apply_at(lv, x, n);
+  const unsigned n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n < (unsigned)lv.nodes) y[n] = q1_row(lv, K, x, n);
+}
+// The operator passes of a Chebyshev-Jacobi smoother of a Q1 level (the arithmetic of
+// k_cheb_start / k_cheb_step / k_cheb_finish around k_q1_apply; at degree 1 the products
+// rounded on their own, as those kernels store them, so that no contraction changes a bit);
+// the modes are HmChebMode's, z the result of the last step
+template <typename T, int MODE>
+__global__ void __launch_bounds__(256) k_q1_cheb(MGLevelT<T> lv, Q1Entries<T> K, const T* __restrict__ b,
+                                                 const T* __restrict__ in, T* x, T* r, T* __restrict__ dout,
+                                                 T* z, int k, int first, int last) {
+  const unsigned n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= (unsigned)lv.nodes) return;
+  const T t = q1_row(lv, K, in, n);
+  if constexpr (MODE == CH_RESIDUAL) {
+    r[n] = b[n] - t;
+  } else if constexpr (MODE == CH_STEP1) {
+    z[n] = in[n] + mul_rn(T(1.0 / lv.cheb[0]) * (b[n] - t), lv.idiag[n]);
+  } else if constexpr (MODE == CH_START) {
+    const T ri = b[n] - t;
+    r[n] = ri;
+    dout[n] = T(1.0 / lv.cheb[0]) * ri * lv.idiag[n];
+  } else {
+    const T di = in[n];
+    const T ri = (first ? b[n] : r[n]) - t;
+    const T xi = first ? di : x[n] + di;
+    const T dn = fma(T(lv.cheb[1 + k]), di, T(lv.cheb[1 + kChebMax + k]) * ri * lv.idiag[n]);
+    if (last == 2) {
+      z[n] = xi + dn;
+    } else {
+      x[n] = xi;
+      r[n] = ri;
+      if (last == 0) dout[n] = dn;
+    }
+  }
 }
 
 __global__ void k_q1_diag(MGLevel lv, double* __restrict__ diag) {
@@ -224,56 +283,84 @@ __global__ void k_coef_coarsen(MGLevel f, MGLevel c, const double* __restrict__ 
 // b_c = R r_f (full weighting, the transpose of trilinear interpolation); 0 on the
 // coarse boundary
 template <typename T>
-__device__ __forceinline__ T restrict_at(const MGLevelT<T>& f, const MGLevelT<T>& c,
-                                         const T* __restrict__ rf, int64_t n) {
-  const int i = (int)(n % c.Nx);
-  const int64_t t = n / c.Nx;
-  const int j = (int)(t % c.Ny), k = (int)(t / c.Ny);
-  if (on_boundary(i, j, k, c.Nx, c.Ny, c.Nz)) return T(0);
-  const T w[3] = {T(0.5), T(1.0), T(0.5)};
+__device__ __forceinline__ T restrict_at(const MGLevelT<T>& f, const MGLevelT<T>& c, const T* rf,
+                                         unsigned n) {
+  const MGNode q = node_at(c, n);
+  if (on_boundary(c, q)) return T(0);
+  const unsigned sy = (unsigned)f.Nx, sz = sy * (unsigned)f.Ny;
+  const T* const r0 = rf + ((unsigned)(2 * q.i - 1) + sy * (unsigned)(2 * q.j - 1) + sz * (unsigned)(2 * q.k - 1));
   T s = T(0);
 #pragma unroll
   for (int dk = 0; dk < 3; ++dk)
 #pragma unroll
     for (int dj = 0; dj < 3; ++dj) {
-      const T wjk = w[dj] * w[dk];
-      const int64_t row = (int64_t)f.Nx * ((2 * j + dj - 1) + (int64_t)f.Ny * (2 * k + dk - 1));
-#pragma unroll
-      for (int di = 0; di < 3; ++di) s = fma(wjk * w[di], rf[row + 2 * i + di - 1], s);
+      const T* const r = r0 + sy * dj + sz * dk;
+      const T w = T((dj == 1 ? 1.0 : 0.5) * (dk == 1 ? 1.0 : 0.5));
+      s = fma(w, fma(T(0.5), r[0] + r[2], r[1]), s);
     }
   return s;
 }
+// b_c = R r_f and, given d, the smoother's first direction d = b idiag / theta
 template <typename T>
-__global__ void k_restrict(MGLevelT<T> f, MGLevelT<T> c, const T* __restrict__ rf,
-                           T* __restrict__ bc) {
-  const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (n < c.nodes) bc[n] = restrict_at(f, c, rf, n);
+__global__ void __launch_bounds__(256) k_restrict(MGLevelT<T> f, MGLevelT<T> c, const T* __restrict__ rf,
+                                                  T* __restrict__ bc, T* __restrict__ d) {
+  const unsigned n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= (unsigned)c.nodes) return;
+  const T b = restrict_at(f, c, rf, n);
+  bc[n] = b;
+  if (d != nullptr) d[n] = mul_rn(T(1.0 / c.cheb[0]) * b, c.idiag[n]);
 }
 
-// x_f += P x_c (trilinear); fine boundary nodes untouched
+// P x_c (trilinear) at the fine nodes 2q, 2q + 1 along each axis of the coarse cell at q;
+// v[x + 2 y + 4 z]
 template <typename T>
-__device__ __forceinline__ void prolong_add_at(const MGLevelT<T>& f, const MGLevelT<T>& c,
-                                               const T* __restrict__ xc,
-                                               T* __restrict__ xf, int64_t n) {
-  const int i = (int)(n % f.Nx);
-  const int64_t t = n / f.Nx;
-  const int j = (int)(t % f.Ny), k = (int)(t / f.Ny);
-  if (on_boundary(i, j, k, f.Nx, f.Ny, f.Nz)) return;
-  const int ci0 = i >> 1, cj0 = j >> 1, ck0 = k >> 1;
-  const int ni = (i & 1) + 1, nj = (j & 1) + 1, nk = (k & 1) + 1;
-  const T wi = (i & 1) ? T(0.5) : T(1.0), wj = (j & 1) ? T(0.5) : T(1.0), wk = (k & 1) ? T(0.5) : T(1.0);
-  T s = T(0);
-  for (int dk = 0; dk < nk; ++dk)
-    for (int dj = 0; dj < nj; ++dj)
-      for (int di = 0; di < ni; ++di)
-        s += xc[(ci0 + di) + (int64_t)c.Nx * ((cj0 + dj) + (int64_t)c.Ny * (ck0 + dk))];
-  xf[n] += wi * wj * wk * s;
+__device__ __forceinline__ void prolong_cell(const MGLevelT<T>& c, const T* xc, unsigned nc, T (&v)[8]) {
+  const unsigned sy = (unsigned)c.Nx, sz = sy * (unsigned)c.Ny;
+  T e[2][2][2];
+#pragma unroll
+  for (int z = 0; z < 2; ++z)
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      const T a = xc[nc + sy * y + sz * z], b = xc[nc + 1u + sy * y + sz * z];
+      e[z][y][0] = a;
+      e[z][y][1] = T(0.5) * (a + b);
+    }
+#pragma unroll
+  for (int x = 0; x < 2; ++x) {
+    const T y0 = e[0][0][x], y1 = T(0.5) * (e[0][0][x] + e[0][1][x]);
+    const T z0 = e[1][0][x], z1 = T(0.5) * (e[1][0][x] + e[1][1][x]);
+    v[x] = y0;
+    v[2 + x] = y1;
+    v[4 + x] = T(0.5) * (y0 + z0);
+    v[6 + x] = T(0.5) * (y1 + z1);
+  }
+}
+// x_f += P x_c on the coarse cell number m (a thread's 8 fine nodes; a fine node on the
+// boundary is left alone)
+template <typename T>
+__device__ __forceinline__ void prolong_add_cell(const MGLevelT<T>& f, const MGLevelT<T>& c, const T* xc,
+                                                 T* xf, unsigned m) {
+  const unsigned cx = (unsigned)c.Nx - 1u, cy = (unsigned)c.Ny - 1u;
+  const unsigned t = m / cx, i = m - t * cx, k = t / cy, j = t - k * cy;
+  T v[8];
+  prolong_cell(c, xc, i + (unsigned)c.Nx * (j + (unsigned)c.Ny * k), v);
+  const unsigned n0 = 2u * i + (unsigned)f.Nx * (2u * j + (unsigned)f.Ny * 2u * k);
+#pragma unroll
+  for (int h = 0; h < 8; ++h) {
+    if ((!(h & 1) && i == 0) || (!(h & 2) && j == 0) || (!(h & 4) && k == 0)) continue;
+    const unsigned n = n0 + (h & 1) + (unsigned)f.Nx * (((h >> 1) & 1) + (unsigned)f.Ny * (h >> 2));
+    xf[n] += v[h];
+  }
 }
 template <typename T>
-__global__ void k_prolong_add(MGLevelT<T> f, MGLevelT<T> c, const T* __restrict__ xc,
-                              T* __restrict__ xf) {
-  const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (n < f.nodes) prolong_add_at(f, c, xc, xf, n);
+HM_HD unsigned coarse_cells(const MGLevelT<T>& c) {
+  return (unsigned)(c.Nx - 1) * (unsigned)(c.Ny - 1) * (unsigned)(c.Nz - 1);
+}
+template <typename T>
+__global__ void __launch_bounds__(256) k_prolong_add(MGLevelT<T> f, MGLevelT<T> c, const T* __restrict__ xc,
+                                                     T* __restrict__ xf) {
+  const unsigned m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m < coarse_cells(c)) prolong_add_cell(f, c, xc, xf, m);
 }
 
 // Chebyshev-Jacobi (idiag: the reciprocal of the Jacobi diagonal): start (r = b - t, or
@@ -330,12 +417,13 @@ __global__ void __launch_bounds__(256) k_coarse_factor(MGLevel lv) {
   __shared__ double A[kCoarseDirectMax][kCoarseDirectMax + 1];
   const int n = interior_count(lv);
   const int tid = threadIdx.x, nt = blockDim.x;
+  const Q1Entries<double> K(lv);
   for (int64_t i = tid; i < lv.nodes; i += nt) lv.t[i] = 0.0;
   __syncthreads();
   for (int j = 0; j < n; ++j) {
     if (tid == 0) lv.t[interior_node(lv, j)] = 1.0;
     __syncthreads();
-    for (int i = tid; i < n; i += nt) A[i][j] = q1_apply_at(lv, lv.t, interior_node(lv, i));
+    for (int i = tid; i < n; i += nt) A[i][j] = q1_row(lv, K, lv.t, (unsigned)interior_node(lv, i));
     __syncthreads();
     if (tid == 0) lv.t[interior_node(lv, j)] = 0.0;
     __syncthreads();
@@ -377,84 +465,323 @@ __global__ void __launch_bounds__(256) k_coarse_solve(MGLevelT<T> lv, const T* _
   coarse_direct(lv, b, x);
 }
 
-// ---- the small levels of a cycle in one CTA
-// The Q1 levels from the first with at most kTailNodes nodes down to the coarsest hold a
-// few thousand nodes together; launched level by level they cost ~14 launches per level
-// and 2 per step of the coarse solve, each mostly launch latency.  One CTA runs that
-// whole part of the V-cycle (the same smoothing, restriction and prolongation, node for
-// node, with block barriers where the launches were).
+// ---- the coarse levels of a cycle in one cluster
+// Launched level by level, a coarse level costs four launches (eight at degree 2) of a few
+// microseconds each, almost all latency.  One cluster of CTAs runs the whole part of the
+// V-cycle from the restriction into its first level to that level's result, the same
+// arithmetic node for node.  Its vectors live in the CTAs' shared memory: a level's node
+// planes are dealt out in slabs, a CTA computes its own planes and reads its neighbours'
+// through the cluster's shared memory, and a cluster barrier stands where the launches
+// were; coefficients and reciprocal diagonals are copied in at the start.  The levels of at
+// most kSoloNodes nodes lie in the first CTA alone, between block barriers.  Measured
+// (FP64, degree 1): 28 us for the levels 17^3, 9^3, 5^3, 3^3 of 32^3 and 64^3, 19 us for
+// 13^3, 7^3, 4^3, against ~47 and ~39 us as launches with one CTA from 1000 nodes down.  A
+// 33^3 level in the cluster takes 44 us more and ~16 us as launches: kTailNodes lies
+// between the two.  A level of 9^3 in one CTA takes 3 us more than in the cluster.
 constexpr int kTailMax = 8;
-constexpr int64_t kTailNodes = 1000;
+constexpr int64_t kTailNodes = 5000;
+constexpr int64_t kSoloNodes = 150, kTailMost = 1 << 20;
 constexpr int kTailThreads = 512;
+constexpr int kTailBytes = 216 * 1024;       // shared memory of a CTA at most
+enum TailVec { TV_B = 0, TV_X = 1, TV_R = 2, TV_D = 3, TV_E = 4 };   // D, E: degree > 1
+template <typename T>
+struct TailLevel {
+  int nx, ny, Nx, Ny, Nz;
+  int A, ppc;            // nodes of a plane, planes per CTA
+  int tab;               // first entry of the level in the plane table
+  int off, vs;           // the first vector's place in the pool, from one vector to the next
+  int idiag_at, coef_at; // places of the reciprocal diagonal and the coefficients
+  int degree;
+  T entries[8];          // Q1Entries
+  const T* coef;
+  const T* idiag;
+  const T* cinv;
+  const double* cheb;
+};
 template <typename T>
 struct MGTail {
-  MGLevelT<T> lv[kTailMax];
-  int count;
+  MGLevelT<T> fine;      // the level above: its r is restricted
+  TailLevel<T> lv[kTailMax];
+  T* out;                // the first level's result
+  int count, solo;           // levels, the first of those in one CTA alone
+  int planes, pool;          // entries of the plane table, reals of the pool
 };
-// Chebyshev smoothing of level lv inside the CTA (as smooth() launches it)
+// the layout for clusters of `ctas`; false: it does not fit
 template <typename T>
-__device__ void tail_smooth(const MGLevelT<T>& lv, bool zero_x, bool want_r, int degree) {
-  const int64_t n = lv.nodes;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const T* __restrict__ b = lv.b;
-  T* __restrict__ x = lv.x;
-  T* __restrict__ r = lv.r;
-  T* __restrict__ d = lv.d;
-  T* __restrict__ t = lv.t;
-  const T* __restrict__ idiag = lv.idiag;
-  const T inv_theta = T(1.0 / lv.cheb[0]);
-  if (!zero_x) {
-    for (int64_t i = tid; i < n; i += nt) t[i] = q1_apply_at(lv, x, i);
-    __syncthreads();
+bool plan_tail(const MGLevelT<T>* lvs, int first, int nlev, int ctas, MGTail<T>* t) {
+  t->count = nlev - first;
+  if (t->count < 1 || t->count > kTailMax) return false;
+  t->planes = t->pool = 0;
+  t->solo = t->count;
+  auto take = [&](int n) { const int at = t->pool; t->pool += n; return at; };
+  for (int q = 0; q < t->count; ++q) {
+    const MGLevelT<T>& l = lvs[first + q];
+    TailLevel<T>& v = t->lv[q];
+    if (l.nodes > kTailMost) return false;
+    if (l.nodes <= kSoloNodes && t->solo == t->count) t->solo = q;
+    v.nx = l.nx; v.ny = l.ny; v.Nx = l.Nx; v.Ny = l.Ny; v.Nz = l.Nz;
+    const Q1Entries<T> K(l);
+    for (int o = 0; o < 8; ++o) v.entries[o] = K.k[o];
+    v.A = l.Nx * l.Ny;
+    v.ppc = q >= t->solo ? l.Nz : (l.Nz + ctas - 1) / ctas;
+    v.tab = t->planes;
+    t->planes += l.Nz;
+    v.vs = v.ppc * v.A;
+    // degree 1 needs three vectors, more and a Chebyshev coarse solve five
+    v.off = take(v.vs * (l.degree == 1 ? 3 : 5));
+    v.idiag_at = take(v.vs);
+    v.coef_at = take((v.ppc + 1) * l.nx * l.ny);
+    v.degree = l.degree;
+    v.coef = l.coef; v.idiag = l.idiag; v.cinv = l.cinv; v.cheb = l.cheb;
   }
-  for (int64_t i = tid; i < n; i += nt) {
-    const T ri = zero_x ? b[i] : b[i] - t[i];
-    r[i] = ri;
-    d[i] = inv_theta * ri * idiag[i];
-    if (zero_x) x[i] = T(0);
+  return 8 * (int64_t)t->planes + (int64_t)sizeof(T) * t->pool <= kTailBytes;
+}
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// this CTA's shared memory address p, in CTA `rank` of the cluster (generic addresses)
+template <typename T>
+__device__ __forceinline__ T* in_cta(T* p, unsigned rank) {
+  uint64_t q;
+  asm("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"(reinterpret_cast<uint64_t>(p)), "r"(rank));
+  return reinterpret_cast<T*>(q);
+}
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+
+template <typename T>
+struct TailView {
+  const TailLevel<T>& l;
+  T* const* planes;      // the level's plane table
+  const T* idiag;        // of the own planes
+  const T* coef;         // of the element planes from k0 - 1 on
+  int k0, k1;            // own planes
+  Q1Entries<T> K;
+  const T* cheb;         // 1 / theta, then c1, c2 of step q at [2 q - 1], [2 q]
+  __device__ __forceinline__ TailView(const TailLevel<T>& lev, T* const* tab, T* pool, unsigned rank, const T* ch)
+      : l(lev), planes(tab + lev.tab), idiag(pool + lev.idiag_at), coef(pool + lev.coef_at),
+        k0(min((int)rank * lev.ppc, lev.Nz)), k1(min(((int)rank + 1) * lev.ppc, lev.Nz)), K(lev.entries), cheb(ch) {}
+  __device__ __forceinline__ T* plane(int v, int k) const { return planes[k] + v * l.vs; }
+  __device__ __forceinline__ void sync() const {
+    if (l.ppc == l.Nz) __syncthreads();
+    else cluster_sync();
   }
-  __syncthreads();
-  for (int k = 1; k <= degree; ++k) {
-    const bool last = k == degree;
-    if (last && !want_r) {
-      for (int64_t i = tid; i < n; i += nt) x[i] += d[i];
-      __syncthreads();
-      break;
+  // f(k, i, j, o, s): every own node, o its place in its plane, s in the own planes
+  template <typename F>
+  __device__ __forceinline__ void each(F f) const {
+    const unsigned n = (unsigned)(max(0, k1 - k0) * l.A);
+    for (unsigned s = threadIdx.x; s < n; s += blockDim.x) {
+      const unsigned kl = s / (unsigned)l.A, o = s - kl * (unsigned)l.A, j = o / (unsigned)l.Nx;
+      f(k0 + (int)kl, (int)(o - j * (unsigned)l.Nx), (int)j, (int)o, (int)s);
     }
-    for (int64_t i = tid; i < n; i += nt) t[i] = q1_apply_at(lv, d, i);
-    __syncthreads();
-    const T c1 = T(lv.cheb[1 + k]), c2 = T(lv.cheb[1 + kChebMax + k]);
-    for (int64_t i = tid; i < n; i += nt) {
-      const T di = d[i];
-      x[i] += di;
-      const T ri = r[i] - t[i];
-      r[i] = ri;
-      if (!last) d[i] = fma(c1, di, c2 * ri * idiag[i]);
-    }
-    __syncthreads();
+  }
+  __device__ __forceinline__ bool boundary(int i, int j, int k) const {
+    return on_boundary(i, j, k, l.Nx, l.Ny, l.Nz);
+  }
+  // (A x) at a node, x the vector v
+  __device__ __forceinline__ T row(int v, int k, int i, int j, int o) const {
+    const T* const p = plane(v, k);
+    if (boundary(i, j, k)) return p[o];
+    const T* const c0 = coef + ((i - 1) + l.nx * ((j - 1) + l.ny * (k - k0)));   // element plane k - 1
+    T c[2][2][2];
+#pragma unroll
+    for (int z = 0; z < 2; ++z)
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int w = 0; w < 2; ++w) c[z][y][w] = c0[w + l.nx * (y + l.ny * z)];
+    const T* const pl[3] = {plane(v, k - 1) + o, p + o, plane(v, k + 1) + o};
+    T xs[3][3][3];
+#pragma unroll
+    for (int z = 0; z < 3; ++z)
+#pragma unroll
+      for (int y = 0; y < 3; ++y)
+#pragma unroll
+        for (int w = 0; w < 3; ++w) xs[z][y][w] = pl[z][(w - 1) + l.Nx * (y - 1)];
+    return q1_stencil(K, c, xs);
+  }
+};
+
+// Chebyshev smoothing from zero: B and the first direction (X at degree 1, else D) given;
+// the result in X, with want_r its residual in R
+template <typename T>
+__device__ void tail_smooth_zero(const TailView<T>& V, bool want_r, int degree) {
+  if (degree == 1 && V.l.degree == 1) {
+    if (!want_r) return;
+    V.each([&](int k, int i, int j, int o, int) {
+      V.plane(TV_R, k)[o] = V.plane(TV_B, k)[o] - V.row(TV_X, k, i, j, o);
+    });
+    V.sync();
+    return;
+  }
+  int in = TV_D, out = TV_E;
+  for (int q = 1; q <= degree; ++q) {
+    const bool last = q == degree, first = q == 1;
+    const T c1 = V.cheb[2 * q - 1], c2 = V.cheb[2 * q];
+    V.each([&](int k, int i, int j, int o, int s) {
+      const T di = V.plane(in, k)[o];
+      T* const x = V.plane(TV_X, k) + o;
+      *x = first ? di : *x + di;
+      if (last && !want_r) return;
+      const T ri = (first ? V.plane(TV_B, k)[o] : V.plane(TV_R, k)[o]) - V.row(in, k, i, j, o);
+      V.plane(TV_R, k)[o] = ri;
+      if (!last) V.plane(out, k)[o] = fma(c1, di, c2 * ri * V.idiag[s]);
+    });
+    V.sync();
+    const int t = in; in = out; out = t;
   }
 }
-// the V-cycle from T.lv[0] (right-hand side in its b, result in its x) to the coarsest
+// the same from X; the result in R at degree 1, else in X, or in out (global memory)
+template <typename T>
+__device__ void tail_smooth_x(const TailView<T>& V, T* gout) {
+  const T inv_theta = V.cheb[0];
+  const int degree = V.l.degree;
+  if (degree == 1) {
+    V.each([&](int k, int i, int j, int o, int s) {
+      const T xn = V.plane(TV_X, k)[o] +
+                   mul_rn(inv_theta * (V.plane(TV_B, k)[o] - V.row(TV_X, k, i, j, o)), V.idiag[s]);
+      if (gout != nullptr) gout[(unsigned)k * (unsigned)V.l.A + (unsigned)o] = xn;
+      else V.plane(TV_R, k)[o] = xn;
+    });
+    V.sync();
+    return;
+  }
+  V.each([&](int k, int i, int j, int o, int s) {
+    const T ri = V.plane(TV_B, k)[o] - V.row(TV_X, k, i, j, o);
+    V.plane(TV_R, k)[o] = ri;
+    V.plane(TV_D, k)[o] = inv_theta * ri * V.idiag[s];
+  });
+  V.sync();
+  int in = TV_D, out = TV_E;
+  for (int q = 1; q < degree; ++q) {
+    const T c1 = V.cheb[2 * q - 1], c2 = V.cheb[2 * q];
+    const bool last = q + 1 == degree;
+    V.each([&](int k, int i, int j, int o, int s) {
+      const T di = V.plane(in, k)[o];
+      const T ri = V.plane(TV_R, k)[o] - V.row(in, k, i, j, o);
+      T* const x = V.plane(TV_X, k) + o;
+      const T dn = fma(c1, di, c2 * ri * V.idiag[s]);
+      const T xi = last ? (*x + di) + dn : *x + di;
+      V.plane(TV_R, k)[o] = ri;
+      V.plane(out, k)[o] = dn;
+      if (last && gout != nullptr) gout[(unsigned)k * (unsigned)V.l.A + (unsigned)o] = xi;
+      else *x = xi;
+    });
+    V.sync();
+    const int t = in; in = out; out = t;
+  }
+}
+
 template <typename R>
 __global__ void __launch_bounds__(kTailThreads) k_mg_tail(const __grid_constant__ MGTail<R> T) {
-  __shared__ MGLevelT<R> L[kTailMax];
-  if (threadIdx.x < (unsigned)T.count) L[threadIdx.x] = T.lv[threadIdx.x];
-  __syncthreads();
-  const int nl = T.count;
-  for (int l = 0; l + 1 < nl; ++l) {
-    tail_smooth(L[l], true, true, L[l].degree);
-    for (int64_t i = threadIdx.x; i < L[l + 1].nodes; i += blockDim.x)
-      L[l + 1].b[i] = restrict_at(L[l], L[l + 1], L[l].r, i);
-    __syncthreads();
+  extern __shared__ __align__(16) unsigned char tail_smem[];
+  __shared__ R coeffs[kTailMax][2 * kChebMax];
+  R** const tab = reinterpret_cast<R**>(tail_smem);
+  R* const pool = reinterpret_cast<R*>(tail_smem + 8 * T.planes);
+  const unsigned rank = cluster_rank();
+  // the plane table, coefficients and reciprocal diagonals
+  for (int q = 0; q < T.count; ++q) {
+    const TailLevel<R>& l = T.lv[q];
+    for (int k = threadIdx.x; k < l.Nz; k += blockDim.x) {
+      const unsigned owner = (unsigned)k / (unsigned)l.ppc;
+      R* const p = pool + l.off + (k - (int)owner * l.ppc) * l.A;
+      tab[l.tab + k] = owner == rank ? p : in_cta(p, owner);
+    }
+    for (int i = threadIdx.x; i <= 2 * l.degree; i += blockDim.x)
+      coeffs[q][i] = i == 0 ? R(1.0 / l.cheb[0]) : R(l.cheb[(i & 1) ? 1 + (i + 1) / 2 : 1 + kChebMax + i / 2]);
+    const int k0 = min((int)rank * l.ppc, l.Nz), k1 = min(((int)rank + 1) * l.ppc, l.Nz);
+    for (int i = threadIdx.x; i < (k1 - k0) * l.A; i += blockDim.x)
+      pool[l.idiag_at + i] = l.idiag[(unsigned)k0 * (unsigned)l.A + (unsigned)i];
+    const int ea = l.nx * l.ny;
+    const int e0 = max(k0 - 1, 0), e1 = min(k1, l.Nz - 1);       // element planes
+    for (int i = threadIdx.x; i < (e1 - e0) * ea; i += blockDim.x)
+      pool[l.coef_at + (e0 - (k0 - 1)) * ea + i] = l.coef[(unsigned)e0 * (unsigned)ea + (unsigned)i];
   }
-  if (L[nl - 1].cinv) coarse_direct(L[nl - 1], L[nl - 1].b, L[nl - 1].x);
-  else tail_smooth(L[nl - 1], true, false, L[nl - 1].degree);
-  for (int l = nl - 2; l >= 0; --l) {
-    for (int64_t i = threadIdx.x; i < L[l].nodes; i += blockDim.x)
-      prolong_add_at(L[l], L[l + 1], L[l + 1].x, L[l].x, i);
-    __syncthreads();
-    tail_smooth(L[l], false, false, L[l].degree);
+  cluster_sync();
+  auto down = [&](int q) {   // restriction (from global memory, then from R), smoothing
+    const TailView<R> V(T.lv[q], tab, pool, rank, coeffs[q]);
+    const R inv_theta = V.cheb[0];
+    const bool coarsest = q + 1 == T.count;
+    const int first = V.l.degree == 1 ? TV_X : TV_D;
+    const TailLevel<R>& fl = T.lv[q > 0 ? q - 1 : 0];
+    V.each([&](int k, int i, int j, int o, int s) {
+      R b = R(0);
+      if (!V.boundary(i, j, k)) {
+        const int fx = q == 0 ? T.fine.Nx : fl.Nx, fa = q == 0 ? fx * T.fine.Ny : fl.A;
+        const int f0 = (2 * i - 1) + fx * (2 * j - 1);
+#pragma unroll
+        for (int dk = 0; dk < 3; ++dk) {
+          const int fk = 2 * k - 1 + dk;
+          const R* const rp = (q == 0 ? T.fine.r + (size_t)fk * fa : tab[fl.tab + fk] + TV_R * fl.vs) + f0;
+#pragma unroll
+          for (int dj = 0; dj < 3; ++dj) {
+            const R* const r = rp + fx * dj;
+            b = fma(R((dj == 1 ? 1.0 : 0.5) * (dk == 1 ? 1.0 : 0.5)), fma(R(0.5), r[0] + r[2], r[1]), b);
+          }
+        }
+      }
+      V.plane(TV_B, k)[o] = b;
+      if (coarsest && V.l.cinv != nullptr) V.plane(TV_X, k)[o] = R(0);
+      else V.plane(first, k)[o] = mul_rn(inv_theta * b, V.idiag[s]);
+    });
+    V.sync();
+    if (!coarsest) {
+      tail_smooth_zero(V, true, V.l.degree);
+    } else if (V.l.cinv == nullptr) {
+      tail_smooth_zero(V, false, V.l.degree);
+    } else {
+      // the exact solve: a warp per row of the inverse, by the first CTA
+      const int ax = V.l.Nx - 2, ay = V.l.Ny - 2, n = ax * ay * (V.l.Nz - 2);
+      auto at = [&](int v, int m) -> R* {
+        return V.plane(v, 1 + m / (ax * ay)) + (1 + m % ax) + V.l.Nx * (1 + (m / ax) % ay);
+      };
+      if (rank == 0)
+        for (int i = threadIdx.x >> 5; i < n; i += blockDim.x >> 5) {
+          R acc = R(0);
+          for (int c = threadIdx.x & 31; c < n; c += 32) acc = fma(V.l.cinv[i * n + c], *at(TV_B, c), acc);
+#pragma unroll
+          for (int m = 16; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+          if ((threadIdx.x & 31) == 0) *at(TV_X, i) = acc;
+        }
+      V.sync();
+    }
+    if (coarsest && q == 0)
+      V.each([&](int k, int, int, int o, int) {
+        T.out[(unsigned)k * (unsigned)V.l.A + (unsigned)o] = V.plane(TV_X, k)[o];
+      });
+  };
+  auto up = [&](int q) {     // prolongation, smoothing
+    const TailView<R> V(T.lv[q], tab, pool, rank, coeffs[q]);
+    const TailLevel<R>& c = T.lv[q + 1];
+    const int cv = q + 2 == T.count || c.degree != 1 ? TV_X : TV_R;
+    V.each([&](int k, int i, int j, int o, int) {
+      if (V.boundary(i, j, k)) return;
+      R v[2];
+#pragma unroll
+      for (int z = 0; z < 2; ++z) {
+        const R* const p = tab[c.tab + ((k + z) >> 1)] + cv * c.vs;
+        const R* const p0 = p + c.Nx * (j >> 1);
+        const R* const p1 = p + c.Nx * ((j + 1) >> 1);
+        const int a0 = i >> 1, a1 = (i + 1) >> 1;
+        v[z] = R(0.5) * (R(0.5) * (p0[a0] + p0[a1]) + R(0.5) * (p1[a0] + p1[a1]));
+      }
+      V.plane(TV_X, k)[o] += R(0.5) * (v[0] + v[1]);
+    });
+    V.sync();
+    tail_smooth_x(V, q == 0 ? T.out : nullptr);
+  };
+  for (int q = 0; q < T.solo; ++q) down(q);
+  if (rank == 0) {
+    for (int q = T.solo; q < T.count; ++q) down(q);
+    for (int q = T.count - 2; q >= T.solo; --q) up(q);
   }
+  if (T.solo > 0) cluster_sync();
+  for (int q = min(T.solo, T.count - 1) - 1; q >= 0; --q) up(q);
+  cluster_sync();        // no CTA leaves while another reads its shared memory
 }
 
 // set-up: a deterministic pseudo-random start vector (0 on the boundary), partial sums of
@@ -569,7 +896,7 @@ int apply_level(hm_mg* mg, int l, const T* x, T* y, bool clean, cudaStream_t s) 
     }
   }
   const MGLevelT<T>& lv = levels_of<T>(mg)[l];
-  k_q1_apply<T><<<blocks_for(lv.nodes), 256, 0, s>>>(lv, x, y);
+  k_q1_apply<T><<<blocks_for(lv.nodes), 256, 0, s>>>(lv, Q1Entries<T>(lv), x, y);
   return HM_OK;
 }
 
@@ -599,61 +926,210 @@ int smooth(hm_mg* mg, int l, const T* b, T* x, bool zero_x, bool want_r, int deg
   return HM_OK;
 }
 
+// CTAs of a tail cluster on the current device (found once): 16 where the device holds such
+// a cluster, else the portable 8
+template <typename T>
+int tail_ctas() {
+  static std::atomic<int> most[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = most[dev].load();
+  if (n == 0) {
+    if (cudaFuncSetAttribute(k_mg_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailBytes) != cudaSuccess)
+      return 0;
+    n = 8;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 16; at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(kTailThreads);
+    cfg.dynamicSmemBytes = kTailBytes;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int active = 0;
+    if (cudaFuncSetAttribute(k_mg_tail<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&active, k_mg_tail<T>, &cfg) == cudaSuccess && active >= 1)
+      n = 16;
+    (void)cudaGetLastError();
+    most[dev].store(n);
+  }
+  return n;
+}
+// the tail from level mg->tail_first, the residual of the level above restricted first;
+// the result in that level's x
+template <typename T>
+int launch_tail(hm_mg* mg, cudaStream_t s) {
+  MGLevelT<T>* lvs = levels_of<T>(mg);
+  const int l = mg->tail_first, n = tail_ctas<T>();
+  MGTail<T> TL{};
+  if (n == 0 || !plan_tail<T>(lvs, l, mg->nlev, n, &TL)) return HM_ERR_CUDA;
+  TL.fine = lvs[l - 1];
+  TL.out = lvs[l].x;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = n; at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  if (TL.solo == 0) at.val.clusterDim.x = 1;
+  cfg.gridDim = dim3(at.val.clusterDim.x);
+  cfg.blockDim = dim3(kTailThreads);
+  cfg.dynamicSmemBytes = 8 * (size_t)TL.planes + sizeof(T) * (size_t)TL.pool;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_mg_tail<T>, TL) == cudaSuccess ? HM_OK : HM_ERR_CUDA;
+}
+
+template <typename T>
+int vcycle(hm_mg* mg, int l, const T* b, T* x, bool clean, cudaStream_t s, T** out);
+// the coarse correction of level l: its residual lv.r restricted and the cycle of level
+// l + 1; *xc: where its result lies
+template <typename T>
+int coarse_cycle(hm_mg* mg, int l, bool clean, cudaStream_t s, T** xc) {
+  MGLevelT<T>* lvs = levels_of<T>(mg);
+  MGLevelT<T>& cv = lvs[l + 1];
+  if (l + 1 == mg->tail_first) {
+    *xc = cv.x;
+    return launch_tail<T>(mg, s);
+  }
+  // with fused smoothing the first direction is formed here (at degree 1 into the iterate)
+  T* const d = !mg->fused || cv.cinv ? nullptr : cv.degree == 1 ? cv.x : cv.d;
+  k_restrict<T><<<blocks_for(cv.nodes), 256, 0, s>>>(lvs[l], cv, lvs[l].r, cv.b, d);
+  return vcycle<T>(mg, l + 1, cv.b, cv.x, clean, s, xc);
+}
+
+// fused smoothing of a Q1 level from zero, its first direction given (coarse_cycle): the
+// result in x, with want_r its residual in r
+template <typename T>
+void q1_smooth_zero(const MGLevelT<T>& lv, bool want_r, cudaStream_t s) {
+  const Q1Entries<T> K(lv);
+  const int g = blocks_for(lv.nodes), degree = lv.degree;
+  if (degree == 1) {
+    if (want_r)
+      k_q1_cheb<T, CH_RESIDUAL><<<g, 256, 0, s>>>(lv, K, lv.b, lv.x, nullptr, lv.r, nullptr, nullptr, 0, 0, 0);
+    return;
+  }
+  T* in = lv.d;
+  T* out = lv.t;
+  const int steps = want_r ? degree : degree - 1;
+  for (int k = 1; k <= steps; ++k) {
+    k_q1_cheb<T, CH_NEXT><<<g, 256, 0, s>>>(lv, K, lv.b, in, lv.x, lv.r, out, lv.x, k, k == 1,
+                                            k < steps ? 0 : want_r ? 1 : 2);
+    T* const t = in; in = out; out = t;
+  }
+}
+// fused smoothing from x; returns where the result lies
+template <typename T>
+T* q1_smooth_x(const MGLevelT<T>& lv, cudaStream_t s) {
+  const Q1Entries<T> K(lv);
+  const int g = blocks_for(lv.nodes), degree = lv.degree;
+  if (degree == 1) {
+    k_q1_cheb<T, CH_STEP1><<<g, 256, 0, s>>>(lv, K, lv.b, lv.x, nullptr, nullptr, nullptr, lv.t, 0, 0, 0);
+    return lv.t;
+  }
+  k_q1_cheb<T, CH_START><<<g, 256, 0, s>>>(lv, K, lv.b, lv.x, nullptr, lv.r, lv.d, nullptr, 0, 0, 0);
+  T* in = lv.d;
+  T* out = lv.t;
+  for (int k = 1; k < degree; ++k) {
+    k_q1_cheb<T, CH_NEXT><<<g, 256, 0, s>>>(lv, K, lv.b, in, lv.x, lv.r, out, lv.x, k, 0, k + 1 < degree ? 0 : 2);
+    T* const t = in; in = out; out = t;
+  }
+  return lv.x;
+}
+
 // The V-cycle from level l for A_l x = b.  *out: where the result lies -- x, except
-// for a Q1 level whose fused post-smoothing writes it to the level's lv.t.  In FP32 the
-// fused level-0 steps are taken by vcycle_single (they read and write FP64 vectors).
+// for a Q1 level whose fused post-smoothing writes it to the level's lv.t.  The fused
+// passes of level 0 are level0_cycle's.
 template <typename T>
 int vcycle(hm_mg* mg, int l, const T* b, T* x, bool clean, cudaStream_t s, T** out) {
   int rc;
   *out = x;
   MGLevelT<T>* lvs = levels_of<T>(mg);
-  if (l == mg->tail_first && b == lvs[l].b && x == lvs[l].x) {
-    MGTail<T> TL{};
-    TL.count = mg->nlev - l;
-    for (int q = 0; q < TL.count; ++q) TL.lv[q] = lvs[l + q];
-    k_mg_tail<T><<<1, kTailThreads, 0, s>>>(TL);
-    return HM_OK;
-  }
+  MGLevelT<T>& lv = lvs[l];
+  const bool fuse = mg->fused && l > 0;
   if (l == mg->nlev - 1) {
-    if (lvs[l].cinv) {
-      k_coarse_solve<T><<<1, 256, 0, s>>>(lvs[l], b, x);
+    if (lv.cinv) {
+      k_coarse_solve<T><<<1, 256, 0, s>>>(lv, b, x);
+      return HM_OK;
+    }
+    if (fuse && lv.degree > 1) {
+      q1_smooth_zero(lv, false, s);
       return HM_OK;
     }
     return smooth<T>(mg, l, b, x, true, false, mg->coarse_degree, clean, s);
   }
-  MGLevelT<T>& lv = lvs[l];
   MGLevelT<T>& cv = lvs[l + 1];
-  // degree 1 fused with the operator: on level 0 when every vector is zero on the
-  // Dirichlet nodes (inside the solves), on a Q1 level when its own buffers carry it
-  constexpr bool kFP64 = std::is_same<T, double>::value;
-  const bool fuse = mg->fused && mg->degree == 1 &&
-                    (l == 0 ? kFP64 && clean : (b == lv.b && x == lv.x));
-  // level 0 fused: the first direction, formed with the right-hand side (hm_mg_first_dir),
-  // is lv.t, which holds the iterate until the post-smoothing step writes to x
-  T* const xl = fuse && l == 0 ? lv.t : x;
-  if (fuse && l == 0) {
-    if constexpr (kFP64) {
-      if ((rc = hm_launch_residual(mg->L, mg->jac, mg->ess, b, xl, lv.r, (void*)s))) return rc;
-    }
-  } else if (fuse) {
-    k_q1_cheb1_from_zero<T><<<blocks_for(lv.nodes), 256, 0, s>>>(lv, b);
-  } else if ((rc = smooth<T>(mg, l, b, x, true, true, mg->degree, clean, s))) {
-    return rc;
-  }
-  k_restrict<T><<<blocks_for(cv.nodes), 256, 0, s>>>(lv, cv, lv.r, cv.b);
+  if (fuse) q1_smooth_zero(lv, true, s);
+  else if ((rc = smooth<T>(mg, l, b, x, true, true, mg->degree, clean, s))) return rc;
   T* xc = nullptr;
-  if ((rc = vcycle<T>(mg, l + 1, cv.b, cv.x, clean, s, &xc))) return rc;
-  k_prolong_add<T><<<blocks_for(lv.nodes), 256, 0, s>>>(lv, cv, xc, xl);
-  if (fuse && l == 0) {
-    if constexpr (kFP64)
-      return hm_launch_cheb1_step(mg->L, mg->jac, mg->ess, b, lv.idiag, lv.cheb, xl, x, (void*)s);
-  }
+  if ((rc = coarse_cycle<T>(mg, l, clean, s, &xc))) return rc;
+  k_prolong_add<T><<<blocks_for(coarse_cells(cv)), 256, 0, s>>>(lv, cv, xc, x);
   if (fuse) {
-    k_q1_cheb1_from_x<T><<<blocks_for(lv.nodes), 256, 0, s>>>(lv, b, x, lv.t);
-    *out = lv.t;
+    *out = q1_smooth_x(lv, s);
     return HM_OK;
   }
   return smooth<T>(mg, l, b, x, false, false, mg->degree, clean, s);
+}
+
+// z = V(r) inside the solves (every vector zero on the Dirichlet nodes) with the level-0
+// smoothing fused into its operator passes: the first direction is given (hm_mg_first_dir),
+// the passes read r and write z themselves, in FP32 too
+bool level0_fused(const hm_mg* mg) { return mg->fused && mg->nlev > 1; }
+template <typename T>
+int level0_cycle(hm_mg* mg, const double* r, double* z, cudaStream_t s, HmBeta* beta) {
+  MGLevelT<T>& lv = levels_of<T>(mg)[0];
+  const MGLevel& l0 = mg->lv[0];
+  constexpr bool kFP64 = std::is_same<T, double>::value;
+  const int degree = mg->degree;
+  void* const jac = kFP64 ? mg->jac : (void*)mg->jac32;
+  HmCheb<T> c{};
+  c.b = r; c.idiag = l0.idiag; c.cheb = l0.cheb;
+  c.r = lv.r;
+  // the iterate: at degree 1 beside z (the last pass reads its neighbours), FP64 at higher
+  // degrees z itself
+  T* d = lv.t;
+  T* e = lv.d;
+  if constexpr (kFP64) c.x = degree == 1 ? lv.t : z;
+  else c.x = degree == 1 ? (d = lv.x) : lv.x;
+  int rc;
+  if (degree == 1) {
+    c.mode = CH_RESIDUAL;
+    c.in = c.x;
+    if ((rc = hm_launch_cheb<T>(mg->L, jac, mg->ess, c, (void*)s))) return rc;
+  } else {
+    c.mode = CH_NEXT;
+    for (int k = 1; k <= degree; ++k) {
+      c.k = k; c.first = k == 1; c.last = k == degree ? 1 : 0;
+      c.in = d; c.dout = e;
+      if ((rc = hm_launch_cheb<T>(mg->L, jac, mg->ess, c, (void*)s))) return rc;
+      T* const t = d; d = e; e = t;
+    }
+  }
+  T* xc = nullptr;
+  if ((rc = coarse_cycle<T>(mg, 0, true, s, &xc))) return rc;
+  MGLevelT<T>& cv = levels_of<T>(mg)[1];
+  k_prolong_add<T><<<blocks_for(coarse_cells(cv)), 256, 0, s>>>(lv, cv, xc, c.x);
+  c.first = 0;
+  c.in = c.x;
+  c.z = z;
+  c.beta = beta;
+  if (degree == 1) {
+    c.mode = CH_STEP1;
+    return hm_launch_cheb<T>(mg->L, jac, mg->ess, c, (void*)s);
+  }
+  d = lv.t;
+  e = lv.d;
+  c.mode = CH_START;
+  c.dout = d;
+  if ((rc = hm_launch_cheb<T>(mg->L, jac, mg->ess, c, (void*)s))) return rc;
+  c.mode = CH_NEXT;
+  for (int k = 1; k < degree; ++k) {
+    c.k = k; c.last = k + 1 == degree ? 2 : 0;
+    c.in = d; c.dout = e;
+    if ((rc = hm_launch_cheb<T>(mg->L, jac, mg->ess, c, (void*)s))) return rc;
+    T* const t = d; d = e; e = t;
+  }
+  return HM_OK;
 }
 
 __global__ void k_to_float(int64_t n, const double* __restrict__ a, float* __restrict__ b) {
@@ -674,36 +1150,27 @@ __global__ void k_to_double(int64_t n, const float* __restrict__ a, double* __re
     b[i] = (double)a[i];
 }
 
-// z = V(r) with the cycle in FP32: r and z FP64.  With degree-1 fused smoothing inside
-// the solves (clean) the first direction is already in level 0's x (hm_mg_first_dir) and
-// the level-0 passes read r and write z themselves; otherwise r is rounded to FP32 first
-// and the result widened at the end.
+// z = V(r) with the cycle in FP32, step by step on level 0: r rounded to FP32 first, the
+// result widened at the end
 int vcycle_single(hm_mg* mg, const double* r, double* z, bool clean, cudaStream_t s) {
   MGLevelT<float>* lv = mg->lv32;
-  int rc;
-  if (mg->fused && mg->degree == 1 && clean && mg->nlev > 1) {
-    const MGLevel& l0 = mg->lv[0];
-    if ((rc = hm_launch_residual32(mg->L, mg->jac32, mg->ess, r, lv[0].x, lv[0].r, (void*)s)))
-      return rc;
-    k_restrict<float><<<blocks_for(lv[1].nodes), 256, 0, s>>>(lv[0], lv[1], lv[0].r, lv[1].b);
-    float* xc = nullptr;
-    if ((rc = vcycle<float>(mg, 1, lv[1].b, lv[1].x, clean, s, &xc))) return rc;
-    k_prolong_add<float><<<blocks_for(lv[0].nodes), 256, 0, s>>>(lv[0], lv[1], xc, lv[0].x);
-    return hm_launch_cheb1_step32(mg->L, mg->jac32, mg->ess, r, l0.idiag, l0.cheb, lv[0].x, z,
-                                  (void*)s);
-  }
   k_to_float<<<kMGBlocks, 256, 0, s>>>(lv[0].nodes, r, lv[0].b);
   float* out = nullptr;
-  if ((rc = vcycle<float>(mg, 0, lv[0].b, lv[0].x, clean, s, &out))) return rc;
+  const int rc = vcycle<float>(mg, 0, lv[0].b, lv[0].x, clean, s, &out);
+  if (rc) return rc;
   k_to_double<<<kMGBlocks, 256, 0, s>>>(lv[0].nodes, out, z);
   return HM_OK;
 }
 
-// the one-CTA tail: the Q1 levels (l >= 1) of at most max_nodes nodes, at most kTailMax
-// of them (max_nodes = 0: none)
+// the tail: the Q1 levels (l >= 1) of at most max_nodes nodes that fit a cluster's shared
+// memory (in FP64), at most kTailMax of them (max_nodes = 0: none)
 void set_tail(hm_mg* mg, int64_t max_nodes) {
+  mg->tail_nodes = max_nodes;
   mg->tail_first = mg->nlev;
-  for (int l = mg->nlev - 1; l >= 1 && mg->lv[l].nodes <= max_nodes && mg->nlev - l <= kTailMax; --l)
+  const int n = tail_ctas<double>();
+  if (n == 0 || tail_ctas<float>() != n) return;
+  MGTail<double> t;
+  for (int l = mg->nlev - 1; l >= 1 && mg->lv[l].nodes <= max_nodes && plan_tail(mg->lv, l, mg->nlev, n, &t); --l)
     mg->tail_first = l;
 }
 
@@ -808,19 +1275,22 @@ __global__ void k_count_mismatch(Lattice L, const uint8_t* __restrict__ ess, uns
 }  // namespace
 
 // inside the MG-PCG, whose residuals are zero on the Dirichlet nodes
-int hm_mg_vcycle(hm_mg* mg, const double* r, double* z, void* stream) {
-  if (mg->single) return vcycle_single(mg, r, z, true, S_(stream));
+int hm_mg_vcycle(hm_mg* mg, const double* r, double* z, void* stream, HmBeta* beta) {
+  cudaStream_t s = S_(stream);
+  if (level0_fused(mg))
+    return mg->single ? level0_cycle<float>(mg, r, z, s, beta) : level0_cycle<double>(mg, r, z, s, beta);
+  if (mg->single) return vcycle_single(mg, r, z, true, s);
   double* out = nullptr;
-  return vcycle<double>(mg, 0, r, z, true, S_(stream), &out);
+  return vcycle<double>(mg, 0, r, z, true, s, &out);
 }
 // the buffer and operands of the level-0 smoother's first direction, where the cycle inside
 // the solves takes it ready made
 HmFirstDir hm_mg_first_dir(const hm_mg* mg) {
   HmFirstDir f{};
-  if (!mg->fused || mg->degree != 1 || mg->nlev < 2) return f;
+  if (!level0_fused(mg)) return f;
   f.idiag = mg->lv[0].idiag;
   f.cheb = mg->lv[0].cheb;
-  if (mg->single) f.d32 = mg->lv32[0].x;
+  if (mg->single) f.d32 = mg->degree == 1 ? mg->lv32[0].x : mg->lv32[0].t;
   else f.d64 = mg->lv[0].t;
   return f;
 }
@@ -853,7 +1323,7 @@ extern "C" int hm_mg_create(const hm_lattice* h, void* work, int degree, int coa
   mg->degree = degree;
   mg->coarse_degree = coarse_degree;
   mg->nlev = plan_levels(*L, mg->lv, 16);
-  set_tail(mg, kTailNodes);
+  for (int l = 0; l < mg->nlev; ++l) mg->lv[l].degree = l == mg->nlev - 1 ? coarse_degree : degree;
   mg->fused = 1;
   mg->single = 0;
   mg->jac32 = nullptr;
@@ -879,6 +1349,7 @@ extern "C" int hm_mg_create(const hm_lattice* h, void* work, int degree, int coa
   // an exact coarse solve when the coarsest Q1 level has few interior nodes
   if (exact_coarsest(mg, mg->nlev - 1))
     mg->lv[mg->nlev - 1].cinv = take(kCoarseDirectMax * kCoarseDirectMax);
+  set_tail(mg, kTailNodes);
   *out = mg;
   return HM_OK;
 }
@@ -939,7 +1410,6 @@ extern "C" int hm_mg_setup(hm_mg* mg, void* jac, const uint8_t* ess, const doubl
       k_mg_scale_div<<<kMGBlocks, 256, 0, s>>>(lv.nodes, w, lv.diag, eig, v);
     }
     const bool coarsest = l == mg->nlev - 1;
-    lv.degree = coarsest ? mg->coarse_degree : mg->degree;
     k_mg_cheb_coeffs<<<1, 32, 0, s>>>(eig, coarsest ? 64.0 : 4.0, lv.degree, lv.cheb);
     if (coarsest && lv.cinv) k_coarse_factor<<<1, 256, 0, s>>>(lv);
   }

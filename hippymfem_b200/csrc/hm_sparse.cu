@@ -133,25 +133,6 @@ __global__ void k_pcg_alpha(const double* __restrict__ part, int64_t nparts, dou
   }
 }
 
-// beta = ((r.z)_new - rzc) / (r.z)_old, the convergence test and the iteration count
-// (thread 0).  rzc = 0: Fletcher-Reeves; rzc = r_new . z_old: a Polak-Ribiere-type step
-// for a preconditioner that is symmetric only to rounding.  The textbook flexible step
-// (Golub and Ye 1999) takes z_new . r_old instead; for a symmetric preconditioner the
-// two cross terms are equal, and both vanish in exact arithmetic.  With the FP32 V-cycle
-// at high contrast the textbook step stalled on fields where this one converged.
-__device__ __forceinline__ void beta_step(double rz, double rr, double* sc, double rzc = 0.0) {
-  const bool was = sc[SC_CONV] >= 0.0;
-  if (!was) {
-    const double it = sc[SC_IT] + 1.0;
-    sc[SC_IT] = it;
-    sc[SC_RR] = rr;
-    if (rr <= sc[SC_TOL2] * sc[SC_BB]) sc[SC_CONV] = it;
-    const double beta = sc[SC_RZ] == 0.0 ? 0.0 : (rz - rzc) / sc[SC_RZ];
-    sc[SC_BETA] = isfinite(beta) ? beta : 0.0;
-    sc[SC_RZ] = rz;
-  }
-}
-
 // x += alpha p, r -= alpha q, z = r / diag; partials of r.z and r.r; with counter, the
 // last block to finish takes the step's beta (else k_pcg_beta does)
 template <typename T>
@@ -245,35 +226,6 @@ __global__ void __launch_bounds__(kReduceThreads)
   if (zold != nullptr) {
     rzc = block_sum(rzc, sh);
     if (threadIdx.x == 0) part[2 * kReduceBlocks + blockIdx.x] = rzc;
-  }
-}
-
-// partials of r.z; the last block takes beta from them and the r.r partials (flex: and
-// the r.zold partials of k_pcg_update_rr, the flexible step)
-__global__ void __launch_bounds__(kReduceThreads)
-    k_pcg_rz_beta(int64_t n, const double* __restrict__ r, const double* __restrict__ z,
-                  double* __restrict__ part, unsigned* __restrict__ counter,
-                  double* __restrict__ sc, int flex = 0) {
-  __shared__ double sh[32];
-  double rz = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    rz = fma(r[i], z[i], rz);
-  rz = block_sum(rz, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = rz;
-  if (last_block(counter)) {
-    double v0 = 0.0, v1 = 0.0, v2 = 0.0;
-    for (int b = threadIdx.x; b < kReduceBlocks; b += blockDim.x) {
-      v0 += __ldcg(part + b);
-      v1 += __ldcg(part + kReduceBlocks + b);
-      if (flex) v2 += __ldcg(part + 2 * kReduceBlocks + b);
-    }
-    v0 = block_sum(v0, sh);
-    v1 = block_sum(v1, sh);
-    if (flex) v2 = block_sum(v2, sh);
-    if (threadIdx.x == 0) {
-      beta_step(v0, v1, sc, v2);
-      *counter = 0u;
-    }
   }
 }
 
@@ -620,7 +572,6 @@ extern "C" int hm_pcg_impl(int64_t n, const int32_t* indptr, const int32_t* indi
                          relres, stream);
 }
 
-int hm_mg_vcycle(hm_mg* mg, const double* r, double* z, void* stream);
 // the V-cycle is symmetric only to rounding (FP32): its CG takes the flexible step
 bool hm_mg_flexible(const hm_mg* mg);
 const double* hm_mg_level0_diag(const hm_mg* mg);
@@ -691,8 +642,10 @@ int pcg_mg_run(hm_mg* mg, const double* b, double* x, double rtol, int maxiter, 
         if (!fused) k_pcg_alpha<<<1, 1024, 0, s>>>(pq_part, np, sc);
         k_pcg_update_rr<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, sc, x, r, p, q, part, fd,
                                                                  flex ? z : nullptr);
-        if ((e = hm_mg_vcycle(mg, r, z, (void*)s))) return e;
-        k_pcg_rz_beta<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, r, z, part, cnt + 1, sc, flex);
+        // the cycle's last operator pass takes r.z and the step's beta where it can
+        HmBeta be{pq_part, part + kReduceBlocks, kReduceBlocks, flex, sc, cnt + 1, 0};
+        if ((e = hm_mg_vcycle(mg, r, z, (void*)s, &be))) return e;
+        if (!be.done && (e = hm_launch_beta(*L, r, z, be, (void*)s))) return e;
         k_pcg_pupdate<double><<<kReduceBlocks, kReduceThreads, 0, s>>>(n, sc, z, p);
       }
       return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
@@ -1022,8 +975,9 @@ int group_batch(hm_pcg_plan* pl, int count, cudaStream_t s) {
     k_pcg_update_rr<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, B.sc, pl->x, B.r, B.p, B.q, B.part,
                                                              hm_mg_first_dir(pl->mg),
                                                              flex ? B.z : nullptr);
-    if ((e = hm_mg_vcycle(pl->mg, B.r, B.z, (void*)s))) return e;
-    k_pcg_rz_beta<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, B.r, B.z, B.part, B.cnt + 1, B.sc, flex);
+    HmBeta be{B.pq_part, B.part + kReduceBlocks, kReduceBlocks, flex, B.sc, B.cnt + 1, 0};
+    if ((e = hm_mg_vcycle(pl->mg, B.r, B.z, (void*)s, &be))) return e;
+    if (!be.done && (e = hm_launch_beta(pl->L, B.r, B.z, be, (void*)s))) return e;
     k_pcg_pupdate<double><<<kReduceBlocks, kReduceThreads, 0, s>>>(n, B.sc, B.z, B.p);
   }
   return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;

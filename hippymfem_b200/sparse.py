@@ -348,12 +348,12 @@ class SolveGroup:
 
 
 def default_smoothing_degree(mesh):
-    """Chebyshev degree of the smoother when the caller gives none: 1 from a million dofs
-    up, 2 below.  Measured on a B200 (FP64 multigrid-PCG to rtol 1e-12): at 64^3 degree 1
-    takes 12 iterations and 7.3 ms against 8 and 7.9 ms (45 against 58 iterations, 33.5
-    against 42.3 ms at sigma 1); at 32^3, where a cycle's launches dominate, degree 2 is
-    faster (2.1 against 2.6 ms)."""
-    return 1 if mesh.ndof >= 1_000_000 else 2
+    """Chebyshev degree of the smoother when the caller gives none: 1.  Measured on a B200
+    (FP64 multigrid-PCG to rtol 1e-12, every pass fused with its operator; degree 1 against
+    2 and 3): at 64^3 12 iterations and 3.5 ms against 8-9 and 4.5, 7 and 4.6; at 32^3 3.0
+    against 3.8 and 4.5 ms; at 16^3 2.1 against 2.5 and 2.7; at 12^3 2.1 against 2.2 and
+    2.5; only on a mesh that does not coarsen (37 x 50 x 23) degree 2 is 5 % faster."""
+    return 1
 
 
 MG_PRECISIONS = ("fp64", "fp32")
