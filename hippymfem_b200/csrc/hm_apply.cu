@@ -47,9 +47,10 @@ constexpr int kRing = 6;             // node planes: a layer's two upper ones, f
 // what the input vector stands for: the vector itself (zero on the Dirichlet nodes), or the
 // vector with the Dirichlet nodes zeroed on the fly
 enum ApplyIn { IN_CLEAN = 0, IN_ESS = 1 };
-// what is done with a node's product: y = A x (x itself on the Dirichlet nodes), or a pass
-// of the smoother (HmChebMode)
-enum ApplyOut { OUT_Y = 0, OUT_R = 1, OUT_STEP1 = 2, OUT_START = 3, OUT_NEXT = 4 };
+// what is done with a node's product: y = A x (x itself on the Dirichlet nodes), a pass of
+// the smoother (HmChebMode), or an assembled vector, y = A x - f int phi (0 on the Dirichlet
+// nodes)
+enum ApplyOut { OUT_Y = 0, OUT_R = 1, OUT_STEP1 = 2, OUT_START = 3, OUT_NEXT = 4, OUT_VEC = 5 };
 
 // the constant of HmCheb's kChebMax (cheb[1 + k]: c1_k, cheb[1 + kChebMax + k]: c2_k)
 constexpr int kChebMax = 40;
@@ -68,6 +69,7 @@ struct ApplyArgs {
   int flex;
   uint32_t* status;        // the library's status word (a bounded wait that gave up)
   int tma, pitch;          // D by TMA; its row pitch
+  double f;                // OUT_VEC
 };
 
 // ------------------------------------------------------------- 1D transforms
@@ -106,6 +108,12 @@ __device__ __forceinline__ void add_from_derivs(T f0, T f1, T f2, T w, T w4, T& 
   r0 = fma(-w, fma(T(2), m, t), r0);
   r1 = fma(w4, m, r1);
   r2 = fma(w, fma(T(-2), m, t), r2);
+}
+
+// int phi over its elements of a node's 1D basis function, on an axis of n elements of
+// size h
+__device__ __forceinline__ double phi_1d(int i, int n, double h) {
+  return (i & 1) ? h * (2.0 / 3.0) : (i == 0 || i == 2 * n) ? h / 6.0 : h / 3.0;
 }
 
 // a node plane at the element to its 9 points: x its first node, rows rs apart
@@ -186,10 +194,10 @@ struct ApplySmem {
   }
 };
 
+// the work of one CTA, tile bt (D by the map at `map`)
 template <typename real, typename src, typename vec, int IN, int OUT>
-__global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlocks : 4)
-    k_apply_tile(const __grid_constant__ CUtensorMap map, const Lattice L, const real* __restrict__ Dq,
-                 const ApplyArgs<src, vec> a) {
+__device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice& L, const real* __restrict__ Dq,
+                                           const ApplyArgs<src, vec>& a, const int bt) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ unsigned long long mbar[2];           // D of the even and the odd layers
   const ApplySmem<real> at(L.ap);
@@ -199,8 +207,7 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlock
   real* const exch = reinterpret_cast<real*>(smem_raw + at.exch);
   const int RS = 2 * T1 + 1, P = RS * (2 * T2 + 1), TB = box_columns<real>(T1);
   const int tid = threadIdx.x;
-  // this CTA's first cells (a later tile's first column, row and layer are the halo)
-  const int bt = blockIdx.x;
+  // the tile's first cells (a later tile's first column, row and layer are the halo)
   const int i1 = bt % L.ap.t1, i2 = (bt / L.ap.t1) % L.ap.t2, i3 = bt / (L.ap.t1 * L.ap.t2);
   const int c1 = i1 * (T1 - 1), c2 = i2 * (T2 - 1), c3 = i3 * (L.ap.T3 - 1);
   const int layers = min(L.ap.T3, L.nz + 1 - c3);
@@ -214,7 +221,7 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlock
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
         " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(smem_raw + (l & 1) * at.dbuf)),
-        "l"(reinterpret_cast<uint64_t>(&map)), "r"(c1 & ~(A - 1)), "r"(c2), "r"(c3 + l), "r"(0),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(c1 & ~(A - 1)), "r"(c2), "r"(c3 + l), "r"(0),
         "r"(smem_u32(&mbar[l & 1]))
         : "memory");
   };
@@ -342,7 +349,13 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlock
       if (!a.tma) {                        // storage without a 16-byte pitch: this thread's own
         const real* const Dg = Dq + (size_t)cx + (size_t)a.pitch * ((size_t)cy + (size_t)L.ny * (size_t)cz);
 #pragma unroll 1
-        for (int q = 0; q < 27; ++q) Dl[q * ds] = __ldg(Dg + (size_t)q * a.pitch * L.ny * L.nz);
+        for (int q = 0; q < 27; q += 9) {
+          real v[9];
+#pragma unroll
+          for (int i = 0; i < 9; ++i) v[i] = __ldg(Dg + (size_t)(q + i) * a.pitch * L.ny * L.nz);
+#pragma unroll
+          for (int i = 0; i < 9; ++i) Dl[(q + i) * ds] = v[i];
+        }
       }
       real v1[9], v2[9];
       plane_to_points(p1, RS, v1);
@@ -381,7 +394,7 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlock
     }
     // the input at the own nodes, the smoother's operands
     real xc[8];
-    double bn[OUT == OUT_Y ? 1 : 8], gn[OUT == OUT_Y || OUT == OUT_R ? 1 : 8], xn[OUT == OUT_NEXT ? 8 : 1];
+    double bn[OUT == OUT_Y || OUT == OUT_VEC ? 1 : 8], gn[OUT == OUT_Y || OUT == OUT_R || OUT == OUT_VEC ? 1 : 8], xn[OUT == OUT_NEXT ? 8 : 1];
     unsigned fixed = 0;
 #pragma unroll
     for (int h = 0; h < 8; ++h) {
@@ -390,10 +403,10 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlock
       if constexpr (OUT == OUT_NEXT) {
         bn[h] = !on ? 0.0 : a.c.first ? __ldg(a.c.b + node) : (double)a.c.r[node];
         xn[h] = !on || a.c.first ? 0.0 : (double)a.c.x[node];
-      } else if constexpr (OUT != OUT_Y) {
+      } else if constexpr (OUT != OUT_Y && OUT != OUT_VEC) {
         bn[h] = on ? __ldg(a.c.b + node) : 0.0;
       }
-      if constexpr (OUT != OUT_Y && OUT != OUT_R) gn[h] = on ? __ldg(a.c.idiag + node) : 0.0;
+      if constexpr (OUT != OUT_Y && OUT != OUT_R && OUT != OUT_VEC) gn[h] = on ? __ldg(a.c.idiag + node) : 0.0;
       const int o = ((h >> 1) & 1) * RS + (h & 1);
       if (h < 4) {
         xc[h] = xlow[h];
@@ -439,6 +452,12 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlock
             const double yv = fx ? xv : acc;
             a.y[node] = (vec)yv;
             dot = fma(xv, yv, dot);
+          } else if constexpr (OUT == OUT_VEC) {
+            double v = acc;
+            if (a.f != 0.0)
+              v -= a.f * (phi_1d(2 * cx + (k & 1), L.nx, L.hx) * phi_1d(2 * cy + (k >> 1), L.ny, L.hy) *
+                          phi_1d(2 * cz + a3, L.nz, L.hz));
+            a.y[node] = (vec)(fx ? 0.0 : v);
           } else {
             const double in = (double)xc[h];
             const double ri = bn[h] - (fx ? in : acc);
@@ -471,7 +490,7 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlock
     }
   }
   copy_wait<0>();
-  if (OUT != OUT_R && OUT != OUT_START && a.part != nullptr) {
+  if (OUT != OUT_R && OUT != OUT_START && OUT != OUT_VEC && a.part != nullptr) {
     __shared__ double sh[32];
     const double t = block_sum(dot, sh);
     if (tid == 0) a.part[blockIdx.x] = t;
@@ -481,6 +500,333 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlock
       else finish_beta(a.part, gridDim.x, a.rr, a.nrr, a.flex, a.sc, a.counter, sh);
     }
   }
+}
+
+template <typename real, typename src, typename vec, int IN, int OUT>
+__global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlocks : 4)
+    k_apply_tile(const __grid_constant__ CUtensorMap map, const Lattice L, const real* __restrict__ Dq,
+                 const ApplyArgs<src, vec> a) {
+  apply_tile<real, src, vec, IN, OUT>(&map, L, Dq, a, (int)blockIdx.x);
+}
+
+// ------------------------------------------------------------ assembled vectors
+// dR/dp (ADJOINT, with the source) is A(D) u, dR/du (STATE) is A(D) p, both without
+// elimination: apply_tile.  dR/dm (PARAMETER) integrates W = D grad u . grad p against the
+// basis: grad_tile.  With mhat, D = w|J| e^m mhat and these are the second-order products
+// along mhat.  Bound: FP64 arithmetic (27 exponentials, then ~680 operations an element and
+// vector), D through memory once between the two launches.  Measured at 64^3: three vectors
+// 158 us (D 28), the gradient alone 78; at 32^3 46 and 20, at 16^3 15 and 12, at 8^3 13 and
+// 12, against 489 and 382, 70 and 55, 20 and 13, 14 and 7 us for an element pass whose
+// stages all went through shared memory and a node gather per vector.
+
+// D at the points of every element (a thread each), and the check that every pointwise value
+// the vectors are made of (E = D grad u, F = D grad p, W) is finite: by bounds on the nodes'
+// values, and only where those do not settle it by the values themselves.
+__global__ void __launch_bounds__(128)
+    k_points_D(const Lattice L, int pitch, const double* __restrict__ u, const double* __restrict__ m,
+               const double* __restrict__ p, const double* __restrict__ mhat, double* __restrict__ D,
+               uint32_t* __restrict__ status, const uint32_t* __restrict__ skip) {
+  if (skip != nullptr && *skip != 0u) return;
+  const unsigned e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= (unsigned)L.ne) return;
+  const unsigned row = e / (unsigned)L.nx, ex = e - row * (unsigned)L.nx;
+  const unsigned ez = row / (unsigned)L.ny, ey = row - ez * (unsigned)L.ny;
+  const unsigned nsy = (unsigned)L.Nx, nsz = nsy * (unsigned)L.Ny;
+  const unsigned n0 = 2u * ex + nsy * 2u * ey + nsz * 2u * ez;
+  auto load = [&](const double* x, double (&v)[27]) {
+#pragma unroll
+    for (int i = 0; i < 27; ++i) v[i] = __ldg(x + n0 + (unsigned)(i % 3) + nsy * (unsigned)((i / 3) % 3) + nsz * (unsigned)(i / 9));
+  };
+  auto points = [&](double (&v)[27]) {       // node values to point values, in place
+#pragma unroll
+    for (int i = 0; i < 9; ++i) to_points(v[3 * i], v[3 * i + 1], v[3 * i + 2], v[3 * i], v[3 * i + 1], v[3 * i + 2]);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+      const int o = (i / 3) * 9 + i % 3;
+      to_points(v[o], v[o + 3], v[o + 6], v[o], v[o + 3], v[o + 6]);
+    }
+#pragma unroll
+    for (int i = 0; i < 9; ++i) to_points(v[i], v[9 + i], v[18 + i], v[i], v[9 + i], v[18 + i]);
+  };
+  double d[27];
+  load(m, d);
+  points(d);
+  const double vol = L.hx * L.hy * L.hz;
+#pragma unroll
+  for (int q = 0; q < 27; ++q) d[q] = wq(q % 3) * wq((q / 3) % 3) * wq(q / 9) * vol * exp(d[q]);
+  if (mhat != nullptr) {
+    double h[27];
+    load(mhat, h);
+    points(h);
+#pragma unroll
+    for (int q = 0; q < 27; ++q) d[q] *= h[q];
+  }
+  double* const out = D + ex + (size_t)pitch * row;
+  const size_t dq = (size_t)pitch * L.ny * L.nz;
+  double dmax = 0.0;
+  bool bad = false;
+#pragma unroll
+  for (int q = 0; q < 27; ++q) {
+    out[q * dq] = d[q];
+    bad |= !(fabs(d[q]) < 1e290);
+    dmax = fmax(dmax, fabs(d[q]));
+  }
+  double umax = 0.0, pmax = 0.0, v[27];
+  load(u, v);
+#pragma unroll
+  for (int i = 0; i < 27; ++i) { bad |= !(fabs(v[i]) < 1e290); umax = fmax(umax, fabs(v[i])); }
+  load(p, v);
+#pragma unroll
+  for (int i = 0; i < 27; ++i) { bad |= !(fabs(v[i]) < 1e290); pmax = fmax(pmax, fabs(v[i])); }
+  // |grad| <= c max|.| per component: the derivative's absolute row sum is at most 8 / h, the
+  // values' at most 1.6 on either other axis
+  const double c = 24.0 * fmax(1.0 / L.hx, fmax(1.0 / L.hy, 1.0 / L.hz));
+  const double gu = c * umax, gp = c * pmax;
+  if (!bad && dmax * gu < 1e290 && dmax * gp < 1e290 && gu * gp < 1e290 && dmax * (3.0 * gu * gp) < 1e290) return;
+  // the values themselves
+#pragma unroll 1
+  for (int q = 0; q < 27; ++q) {
+    const int q1 = q % 3, q2 = (q / 3) % 3, q3 = q / 9;
+    double gr[2][3] = {{0, 0, 0}, {0, 0, 0}};
+#pragma unroll 1
+    for (int i = 0; i < 27; ++i) {
+      const unsigned n = n0 + (unsigned)(i % 3) + nsy * (unsigned)((i / 3) % 3) + nsz * (unsigned)(i / 9);
+      const double b1 = bq(q1, i % 3), b2 = bq(q2, (i / 3) % 3), b3 = bq(q3, i / 9);
+      const double x = dbq(q1, i % 3) * b2 * b3, y = b1 * dbq(q2, (i / 3) % 3) * b3, z = b1 * b2 * dbq(q3, i / 9);
+      for (int k = 0; k < 2; ++k) {
+        const double val = k == 0 ? u[n] : p[n];
+        gr[k][0] = fma(x, val, gr[k][0]); gr[k][1] = fma(y, val, gr[k][1]); gr[k][2] = fma(z, val, gr[k][2]);
+      }
+    }
+    const double dv = out[q * dq];
+    double dot = 0.0;
+    bool fine = true;
+    for (int k = 0; k < 3; ++k) {
+      const double h = k == 0 ? L.hx : k == 1 ? L.hy : L.hz;
+      const double a = gr[0][k] / h, b = gr[1][k] / h;
+      fine = fine && isfinite(dv * a) && isfinite(dv * b);
+      dot += a * b;
+    }
+    if (!(fine && isfinite(dv * dot))) {
+      atomicOr(status, HM_STATUS_NONFINITE);
+      return;
+    }
+  }
+}
+
+// dR/dm: a tile of columns marching up z as in apply_tile, for two vectors.  The in-plane
+// values of a layer's lower node plane are formed again from the ring (both vectors' would
+// be 36 registers more); D is needed only at the end of a layer's arithmetic and has one
+// buffer.
+constexpr int kGradRing = 5;         // a layer's three planes, two arriving
+struct GradSmem {
+  int ring, exch, bytes;
+  HM_HD GradSmem(const ApplyPlan& p) {
+    ring = (27 * p.T2 * box_columns<double>(p.T1) * 8 + 127) / 128 * 128;
+    exch = ring + 2 * kGradRing * (2 * p.T1 + 1) * (2 * p.T2 + 1) * 8;
+    bytes = exch + 20 * p.threads * 8;
+  }
+};
+__device__ __forceinline__ void grad_tile(const CUtensorMap* map, const Lattice& L, const double* __restrict__ Dq,
+                                          int tma, int pitch, const double* __restrict__ u,
+                                          const double* __restrict__ p, double* __restrict__ yout,
+                                          uint32_t* __restrict__ status, const int bt) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ unsigned long long mbar;
+  const GradSmem at(L.ap);
+  const int T1 = L.ap.T1, T2 = L.ap.T2, nt = blockDim.x;
+  double* const ring = reinterpret_cast<double*>(smem_raw + at.ring);
+  double* const exch = reinterpret_cast<double*>(smem_raw + at.exch);
+  const int RS = 2 * T1 + 1, P = RS * (2 * T2 + 1), TB = box_columns<double>(T1);
+  const int tid = threadIdx.x;
+  const int i1 = bt % L.ap.t1, i2 = (bt / L.ap.t1) % L.ap.t2, i3 = bt / (L.ap.t1 * L.ap.t2);
+  const int c1 = i1 * (T1 - 1), c2 = i2 * (T2 - 1), c3 = i3 * (L.ap.T3 - 1);
+  const int layers = min(L.ap.T3, L.nz + 1 - c3);
+  const unsigned nsy = (unsigned)L.Nx, nsz = (unsigned)L.Nx * (unsigned)L.Ny;
+  auto request_D = [&](int l) {
+    if (tid != 0 || !tma || l >= layers || c3 + l >= L.nz) return;
+    fence_proxy_async();                   // the buffer's readers are done (block barrier)
+    mbar_expect(&mbar, 27u * (uint32_t)(T2 * TB) * 8u);
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(smem_raw)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(c1 & ~1), "r"(c2), "r"(c3 + l), "r"(0),
+        "r"(smem_u32(&mbar))
+        : "memory");
+  };
+  if (tid == 0) {
+    mbar_init(&mbar, 1);
+    fence_mbar_init();
+  }
+  request_D(0);
+  unsigned off[kApplyItems];               // as in apply_tile
+  {
+    const int step_r = nt / RS, step_c = nt - step_r * RS;
+    int r = tid / RS, c = tid - r * RS;
+#pragma unroll
+    for (int k = 0; k < kApplyItems; ++k) {
+      const int gx = 2 * c1 + c, gy = 2 * c2 + r;
+      off[k] = tid + k * nt < P && gx < L.Nx && gy < L.Ny ? (unsigned)gx + nsy * (unsigned)gy : ~0u;
+      r += step_r;
+      c += step_c;
+      if (c >= RS) { c -= RS; ++r; }
+    }
+  }
+  auto request = [&](int j) {
+    if (2 * c3 + j < L.Nz && j <= 2 * layers) {
+      double* const pu = ring + j % kGradRing * P + tid;
+      const size_t z0 = (size_t)nsz * (2 * c3 + j);
+#pragma unroll
+      for (int k = 0; k < kApplyItems; ++k)
+        if (off[k] != ~0u) {
+          copy_async(pu + k * nt, u + z0 + off[k]);
+          copy_async(pu + kGradRing * P + k * nt, p + z0 + off[k]);
+        }
+    }
+  };
+  for (int j = 0; j < 3; ++j) request(j);
+  copy_commit();
+  const int ty = tid / T1, tx = tid - ty * T1;
+  const int cx = c1 + tx, cy = c2 + ty;
+  const bool column = ty < T2;
+  const bool element = column && cx < L.nx && cy < L.ny;
+  const bool own = column && cx <= L.nx && cy <= L.ny && (tx > 0 || i1 == 0) && (ty > 0 || i2 == 0);
+  const double sx = 1.0 / (0.6 * L.hx * L.hx);
+  const double ry = (L.hx * L.hx) / (L.hy * L.hy), rz = (L.hx * L.hx) / (L.hz * L.hz);
+  const int base = 2 * ty * RS + 2 * tx, ds = T2 * TB;
+  double carry[9];
+#pragma unroll
+  for (int i = 0; i < 9; ++i) carry[i] = 0.0;
+  copy_wait<0>();
+  __syncthreads();
+#pragma unroll 1
+  for (int l = 0; l < layers; ++l) {
+    const int cz = c3 + l;
+    const double* const p0 = ring + (2 * l) % kGradRing * P + base;
+    const double* const p1 = ring + (2 * l + 1) % kGradRing * P + base;
+    const double* const p2 = ring + (2 * l + 2) % kGradRing * P + base;
+    request(2 * l + 3);
+    request(2 * l + 4);
+    copy_commit();
+    if (l > 0) request_D(l);
+    const bool layer = cz < L.nz;
+    bool ok = true;
+    double y[18];
+    if (element && layer) {
+      double* const Dl = reinterpret_cast<double*>(smem_raw) + ty * TB + tx + (c1 & 1);
+      if (!tma) {
+        const double* const Dg = Dq + (size_t)cx + (size_t)pitch * ((size_t)cy + (size_t)L.ny * (size_t)cz);
+#pragma unroll 1
+        for (int q = 0; q < 27; q += 9) {
+          double v[9];
+#pragma unroll
+          for (int i = 0; i < 9; ++i) v[i] = __ldg(Dg + (size_t)(q + i) * pitch * L.ny * L.nz);
+#pragma unroll
+          for (int i = 0; i < 9; ++i) Dl[(q + i) * ds] = v[i];
+        }
+      }
+      double U[27], Q[27], W[27];
+      auto values = [&](int o, double (&V)[27]) {
+        double v0[9], v1[9], v2[9];
+        plane_to_points(p0 + o, RS, v0);
+        plane_to_points(p1 + o, RS, v1);
+        plane_to_points(p2 + o, RS, v2);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) to_points(v0[i], v1[i], v2[i], V[i], V[9 + i], V[18 + i]);
+      };
+      values(0, U);
+      values(kGradRing * P, Q);
+      auto line = [&](int a, int b, int c, double w, bool first) {
+        double g0, g1, g2, h0, h1, h2;
+        derivs(U[a], U[b], U[c], g0, g1, g2);
+        derivs(Q[a], Q[b], Q[c], h0, h1, h2);
+        h0 *= w; h1 *= w; h2 *= w;
+        W[a] = first ? g0 * h0 : fma(g0, h0, W[a]);
+        W[b] = first ? g1 * h1 : fma(g1, h1, W[b]);
+        W[c] = first ? g2 * h2 : fma(g2, h2, W[c]);
+      };
+#pragma unroll
+      for (int i = 0; i < 9; ++i) line(i, 9 + i, 18 + i, rz, true);
+#pragma unroll
+      for (int i = 0; i < 9; ++i) line((i / 3) * 9 + i % 3, (i / 3) * 9 + i % 3 + 3, (i / 3) * 9 + i % 3 + 6, ry, false);
+#pragma unroll
+      for (int i = 0; i < 9; ++i) line(3 * i, 3 * i + 1, 3 * i + 2, 1.0, false);
+      ok = !tma || mbar_wait(&mbar, (uint32_t)l & 1u);
+#pragma unroll
+      for (int q = 0; q < 27; ++q) W[q] *= Dl[q * ds];
+      double m0[9], m1[9];
+#pragma unroll
+      for (int i = 0; i < 9; ++i) {
+        double m2;
+        from_points(W[i], W[9 + i], W[18 + i], m0[i], m1[i], m2);
+        m0[i] += carry[i];
+        carry[i] = m2;
+      }
+      plane_from_points(m0);
+      plane_from_points(m1);
+#pragma unroll
+      for (int i = 0; i < 9; ++i) { y[i] = m0[i]; y[9 + i] = m1[i]; }
+    } else {
+      // every thread sees the layer's copy land before its buffer is requested again
+      ok = !tma || !layer || mbar_wait(&mbar, (uint32_t)l & 1u);
+      plane_from_points(carry);
+#pragma unroll
+      for (int i = 0; i < 9; ++i) { y[i] = carry[i]; y[9 + i] = carry[i] = 0.0; }
+    }
+    double* const ex = exch + (l & 1) * 10 * nt;
+#pragma unroll
+    for (int a3 = 0; a3 < 2; ++a3) {
+      double* const e = ex + a3 * 5 * nt + tid;
+      e[0] = y[9 * a3 + 2];
+      e[nt] = y[9 * a3 + 5];
+      e[2 * nt] = y[9 * a3 + 8];
+      e[3 * nt] = y[9 * a3 + 6];
+      e[4 * nt] = y[9 * a3 + 7];
+    }
+    copy_wait<0>();                        // the next layer's planes
+    if (__syncthreads_or(!ok)) {
+      if (tid == 0 && status != nullptr) atomicOr(status, HM_STATUS_TIMEOUT);
+      break;
+    }
+    if (own && (l > 0 || i3 == 0)) {
+      const bool left = tx > 0, front = ty > 0;
+      const unsigned n0 = (unsigned)(2 * cx) + nsy * (unsigned)(2 * cy) + nsz * (unsigned)(2 * cz);
+#pragma unroll
+      for (int a3 = 0; a3 < 2; ++a3) {
+        if (a3 == 1 && !layer) break;
+        const double* const e = ex + a3 * 5 * nt + tid;
+        double n[4];
+        n[0] = y[9 * a3]; n[1] = y[9 * a3 + 1]; n[2] = y[9 * a3 + 3]; n[3] = y[9 * a3 + 4];
+        if (left) { n[0] += e[-1]; n[2] += e[nt - 1]; }
+        if (front) { n[0] += e[3 * nt - T1]; n[1] += e[4 * nt - T1]; }
+        if (left && front) n[0] += e[2 * nt - T1 - 1];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (!((k & 1) && cx >= L.nx) && !((k & 2) && cy >= L.ny))
+            yout[n0 + (k & 1) + ((k & 2) ? nsy : 0u) + (a3 ? nsz : 0u)] = sx * n[k];
+      }
+    }
+  }
+  copy_wait<0>();
+}
+
+// The requested vectors in one launch: `count` CTAs in a row take one tile's vectors, so
+// that its D comes from memory once.
+struct VecArgs {
+  ApplyArgs<double, double> a[2];      // ADJOINT, STATE
+  const double* u;
+  const double* p;
+  double* grad;                        // PARAMETER
+  int which[3], count;                 // 0, 1: a[which]; 2: grad
+  const uint32_t* skip;                // nonzero there: the whole launch stands down
+};
+__global__ void __launch_bounds__(kApplyThreads, 2)
+    k_vectors(const __grid_constant__ CUtensorMap map, const Lattice L, const double* __restrict__ D,
+              const __grid_constant__ VecArgs v) {
+  if (v.skip != nullptr && *v.skip != 0u) return;
+  const int bt = (int)blockIdx.x / v.count, w = v.which[(int)blockIdx.x - bt * v.count];
+  if (w == 2) grad_tile(&map, L, D, v.a[0].tma, v.a[0].pitch, v.u, v.p, v.grad, v.a[0].status, bt);
+  else apply_tile<double, double, double, IN_CLEAN, OUT_VEC>(&map, L, D, v.a[w], bt);
 }
 
 // b . z and the CG step's beta on their own, after a cycle that ends in another kernel: the
@@ -568,42 +914,55 @@ int hm_jac_pitch(const Lattice& L, int precision) {
 }
 
 namespace {
-template <typename real, typename src, typename vec, int IN, int OUT>
-int launch(const Lattice& L, const void* jac, ApplyArgs<src, vec> a, void* stream) {
-  auto kern = k_apply_tile<real, src, vec, IN, OUT>;
-  const size_t smem = (size_t)ApplySmem<real>(L.ap).bytes;
-  a.pitch = hm_jac_pitch(L, sizeof(real) == 8 ? HM_FP64 : HM_FP32);
-  CUtensorMap map{};
-  a.tma = (reinterpret_cast<uintptr_t>(jac) & 15u) == 0 && a.pitch * sizeof(real) % 16 == 0;
-  if (a.tma) {
-    auto encode = hm_tensor_map_encoder();
-    if (encode == nullptr) return HM_ERR_CUDA;
-    const cuuint64_t row = (cuuint64_t)a.pitch * sizeof(real);
-    const cuuint64_t dims[4] = {(cuuint64_t)L.nx, (cuuint64_t)L.ny, (cuuint64_t)L.nz, 27};
-    const cuuint64_t strides[3] = {row, row * L.ny, row * L.ny * L.nz};
-    const cuuint32_t box[4] = {(cuuint32_t)box_columns<real>(L.ap.T1), (cuuint32_t)L.ap.T2, 1, 27};
-    const cuuint32_t one[4] = {1, 1, 1, 1};
-    if (encode(&map, sizeof(real) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
-               const_cast<void*>(jac), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+// raises a kernel's dynamic shared memory limit, once per device
+template <typename K>
+int raise_smem(K kern, std::atomic<uint64_t>& done) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return HM_ERR_CUDA;
+  if (dev < 0 || dev >= 64) return HM_ERR_UNSUPPORTED;
+  if (!((done.load() >> dev) & 1u)) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
       return HM_ERR_CUDA;
+    done.fetch_or(1ull << dev);
   }
+  return HM_OK;
+}
+// the map of D [q][ez][ey][ex] with rows `pitch` apart; *tma = 0 where its storage has no
+// 16-byte base or pitch
+template <typename real>
+int map_D(const Lattice& L, const void* D, int pitch, CUtensorMap* map, int* tma) {
+  *tma = (reinterpret_cast<uintptr_t>(D) & 15u) == 0 && pitch * sizeof(real) % 16 == 0;
+  if (!*tma) return HM_OK;
+  auto encode = hm_tensor_map_encoder();
+  if (encode == nullptr) return HM_ERR_CUDA;
+  const cuuint64_t row = (cuuint64_t)pitch * sizeof(real);
+  const cuuint64_t dims[4] = {(cuuint64_t)L.nx, (cuuint64_t)L.ny, (cuuint64_t)L.nz, 27};
+  const cuuint64_t strides[3] = {row, row * L.ny, row * L.ny * L.nz};
+  const cuuint32_t box[4] = {(cuuint32_t)box_columns<real>(L.ap.T1), (cuuint32_t)L.ap.T2, 1, 27};
+  const cuuint32_t one[4] = {1, 1, 1, 1};
+  return encode(map, sizeof(real) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
+                const_cast<void*>(D), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
+             ? HM_OK : HM_ERR_CUDA;
+}
+template <typename real, typename src, typename vec, int IN, int OUT>
+int launch(const Lattice& L, const void* jac, int pitch, ApplyArgs<src, vec> a, void* stream) {
+  auto kern = k_apply_tile<real, src, vec, IN, OUT>;
+  static std::atomic<uint64_t> done{0};
+  int rc = raise_smem(kern, done);
+  if (rc) return rc;
+  a.pitch = pitch;
   a.status = hm_status_word();
-  if (smem > 40 * 1024) {                     // with the static part above 48 KB
-    static std::atomic<uint64_t> done{0};     // devices on which the limit is raised
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return HM_ERR_CUDA;
-    if (dev < 0 || dev >= 64) return HM_ERR_UNSUPPORTED;
-    if (!((done.load() >> dev) & 1u)) {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
-        return HM_ERR_CUDA;
-      done.fetch_or(1ull << dev);
-    }
-  }
-  kern<<<L.ap.t1 * L.ap.t2 * L.ap.t3, L.ap.threads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
-      map, L, static_cast<const real*>(jac), a);
+  CUtensorMap map{};
+  if ((rc = map_D<real>(L, jac, pitch, &map, &a.tma))) return rc;
+  kern<<<L.ap.t1 * L.ap.t2 * L.ap.t3, L.ap.threads, (size_t)ApplySmem<real>(L.ap).bytes,
+         reinterpret_cast<cudaStream_t>(stream)>>>(map, L, static_cast<const real*>(jac), a);
   return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
+}
+template <typename real, typename src, typename vec, int IN, int OUT>
+int launch(const Lattice& L, const void* jac, const ApplyArgs<src, vec>& a, void* stream) {
+  return launch<real, src, vec, IN, OUT>(L, jac, hm_jac_pitch(L, sizeof(real) == 8 ? HM_FP64 : HM_FP32), a, stream);
 }
 template <typename real, typename T>
 int apply_y(const Lattice& L, const void* jac, const uint8_t* ess, const T* x, T* y, bool clean,
@@ -675,5 +1034,38 @@ template int hm_launch_cheb<double>(const Lattice&, void*, const uint8_t*, const
 template int hm_launch_cheb<float>(const Lattice&, void*, const uint8_t*, const HmCheb<float>&, void*);
 int hm_launch_beta(const Lattice& L, const double* b, const double* z, const HmBeta& be, void* stream) {
   k_tile_beta<<<L.ap.t1 * L.ap.t2 * L.ap.t3, L.ap.threads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(L, b, z, be);
+  return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
+}
+
+// The assembled vectors from the fields.  D: storage of at least 27 ne doubles (54 ne for
+// its 16-byte pitch where nx is odd), work_reals of them; outs: ADJOINT, STATE, PARAMETER
+// (NULL: skip).  With skip nonzero on the device nothing is done.
+int hm_launch_vectors(const Lattice& L, const double* u, const double* m, const double* p,
+                      const double* mhat, double f, const uint8_t* zero_ess, double* const outs[3],
+                      double* D, int64_t work_reals, uint32_t* status, const uint32_t* skip, void* stream) {
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  int pitch = hm_jac_pitch(L, HM_FP64);
+  if (27 * (int64_t)pitch * L.ny * L.nz > work_reals) pitch = L.nx;
+  k_points_D<<<(int)((L.ne + 127) / 128), 128, 0, s>>>(L, pitch, u, m, p, mhat, D, status, skip);
+  static std::atomic<uint64_t> done{0};
+  int rc = raise_smem(k_vectors, done);
+  if (rc) return rc;
+  CUtensorMap map{};
+  VecArgs v{};
+  v.u = u; v.p = p; v.grad = outs[2]; v.skip = skip;
+  for (int i = 0; i < 2; ++i) {
+    ApplyArgs<double, double>& a = v.a[i];
+    a.ess = zero_ess; a.x = i == 0 ? u : p; a.y = outs[i];
+    a.f = i == 0 && mhat == nullptr ? f : 0.0;
+    a.pitch = pitch;
+    a.status = hm_status_word();
+    if ((rc = map_D<double>(L, D, pitch, &map, &a.tma))) return rc;
+  }
+  for (int i = 0; i < 3; ++i)
+    if (outs[i]) v.which[v.count++] = i;
+  const int bytes = ApplySmem<double>(L.ap).bytes, grad = GradSmem(L.ap).bytes;
+  const bool applies = outs[0] || outs[1];
+  k_vectors<<<L.ap.t1 * L.ap.t2 * L.ap.t3 * v.count, L.ap.threads,
+              (size_t)(!outs[2] || (applies && bytes > grad) ? bytes : grad), s>>>(map, L, D, v);
   return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
 }
