@@ -976,9 +976,6 @@ int apply_y(const Lattice& L, const void* jac, const uint8_t* ess, const T* x, T
 }
 }  // namespace
 
-// number of partial sums of the fused inner product
-int64_t hm_apply_dot_parts(const Lattice& L) { return (int64_t)L.ap.t1 * L.ap.t2 * L.ap.t3; }
-
 int hm_launch_apply_A(const Lattice& L, void* jac, int precision, const uint8_t* ess,
                       const double* x, double* y, void* stream) {
   if (precision == HM_FP32) return apply_y<float>(L, jac, ess, x, y, false, nullptr, nullptr, nullptr, stream);

@@ -1,13 +1,14 @@
 // CSR products, deterministic reductions and the Jacobi-PCG of the incremental solves.
 //
-// Every reduction is two-pass over a fixed grid (kReduceBlocks blocks, grid-stride),
+// Every reduction is two-pass over a grid fixed by n (reduce_blocks, grid-stride),
 // so its summation order depends on n alone: repeated solves are bit-identical.
 // The PCG keeps alpha, beta and the residual norms on the device; the host only
 // launches and, every check_every iterations, reads one flag.  After convergence the
 // step length is frozen at zero, so the result is that of the exact iteration count
 // whatever check_every is.
-#include <new>
+#include <algorithm>
 #include <cmath>
+#include <new>
 #include <type_traits>
 #include <vector>
 
@@ -16,30 +17,78 @@
 
 namespace hm {
 
-constexpr int kReduceBlocks = 1184;  // 8 x 148 SMs
+constexpr int kReduceBlocks = 1184;  // 8 x 148 SMs, at most
 constexpr int kReduceThreads = 256;
+// blocks of the vector kernels on n entries (a block with nothing to do still costs its share
+// of the reduction: 9.7 against 5 us for the update of 118 k entries)
+inline int reduce_blocks(int64_t n) {
+  const int64_t b = (n + kReduceThreads - 1) / kReduceThreads;
+  return (int)(b < 1 ? 1 : b < kReduceBlocks ? b : kReduceBlocks);
+}
 
 // ------------------------------------------------------------------------ SpMV
 // G lanes per row (G = 8): a warp covers 4 consecutive rows, which are contiguous in
-// the CSR arrays; each group reduces its row with shuffles in a fixed order.
-template <int G, bool TRANS>
-__global__ void __launch_bounds__(256)
+// the CSR arrays; each group reduces its row with shuffles in a fixed order.  A block takes
+// every gridDim.x-th set of 32 rows.  With DOT (a square matrix), also the partial sums of
+// x.y, one a block, from which the last block takes the CG step's alpha.
+//
+// Bound: the values and indices, 12 bytes an entry, once the gathers' latency is hidden: a
+// lane has U entries in flight (index, value, then x).  On a 64^3-element lattice (1.6 GB)
+// U = 1 took 357 us, 2 379, 4 344, 8 336; on 45 x 52 x 39 125, 118, 107, 104; 32^3 51, 49,
+// 45, 45; 24^3 23, 26, 23, 23.  The grid is one wave of resident blocks: with DOT a block's
+// reduction then comes once (CG iteration at 24^3, five launches before: 49 -> 41 us, 45 x
+// 52 x 39 166 -> 147, 64^3 424 -> 406; with three waves the product alone lost 3 us, with
+// one block per 32 rows 4 at 24^3 and 130 at 64^3).
+// The transposed product reads its values through tpos, 16 bytes an entry, at scattered
+// places; rows that run at the same time have to stay close for the values' lines to be
+// shared in L2: one block per 32 rows, 570 us at 64^3 (U = 4; 595 with U = 1, 627 with 8),
+// against 690 with 9472 blocks and 876 with 888.
+constexpr int kSpmvRows = 32;                          // rows a block covers at a time (256 / G)
+constexpr int kSpmvBlocks = 6, kSpmvDotBlocks = 5;     // resident blocks on an SM
+template <int G, bool TRANS, bool DOT, int U>
+__global__ void __launch_bounds__(256, DOT ? kSpmvDotBlocks : kSpmvBlocks)
     k_spmv(int64_t nrow, const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
            const int32_t* __restrict__ tpos, const double* __restrict__ vals,
-           const double* __restrict__ x, double* __restrict__ y, double alpha, double beta) {
-  const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
+           const double* __restrict__ x, double* __restrict__ y, double alpha, double beta,
+           double* __restrict__ part, double* __restrict__ sc, unsigned* __restrict__ counter) {
+  __shared__ double sh[32];
   const int lane = threadIdx.x % G;
-  double acc = 0.0;
-  if (row < nrow) {
-    const int b = indptr[row], e = indptr[row + 1];
-    for (int s = b + lane; s < e; s += G) {
-      const double v = TRANS ? vals[tpos[s]] : vals[s];
-      acc = fma(v, __ldg(x + indices[s]), acc);
+  double dot = 0.0;
+  for (int64_t r0 = blockIdx.x * (int64_t)(blockDim.x / G); r0 < nrow; r0 += gridDim.x * (int64_t)(blockDim.x / G)) {
+    const int64_t row = r0 + threadIdx.x / G;
+    double acc = 0.0;
+    if (row < nrow) {
+      const int b = __ldg(indptr + row), e = __ldg(indptr + row + 1);
+      int64_t s = (int64_t)b + lane;
+      for (int left = e - b - lane; left > 0; left -= G * U, s += G * U) {
+        int col[U];
+        double v[U], w[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const bool on = left > u * G;
+          col[u] = on ? __ldg(indices + s + u * G) : 0;
+          if constexpr (TRANS) v[u] = on ? __ldg(vals + __ldg(tpos + s + u * G)) : 0.0;
+          else v[u] = on ? __ldg(vals + s + u * G) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) w[u] = left > u * G ? __ldg(x + col[u]) : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) acc = fma(v[u], w[u], acc);
+      }
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, G);
+    if (row < nrow && lane == 0) {
+      const double yn = beta == 0.0 ? alpha * acc : fma(beta, y[row], alpha * acc);
+      y[row] = yn;
+      if constexpr (DOT) dot = fma(__ldg(x + row), yn, dot);
     }
   }
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, G);
-  if (row < nrow && lane == 0) y[row] = beta == 0.0 ? alpha * acc : fma(beta, y[row], alpha * acc);
+  if constexpr (DOT) {
+    const double t = block_sum(dot, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = t;
+    if (last_block(counter)) finish_alpha(part, gridDim.x, sc, counter, sh);
+  }
 }
 
 __global__ void k_csr_diag(int64_t nrow, const int32_t* __restrict__ indptr,
@@ -60,12 +109,12 @@ __global__ void __launch_bounds__(kReduceThreads)
   if (threadIdx.x == 0) part[blockIdx.x] = v;
 }
 
-// sum of nq interleaved partial arrays part[q * kReduceBlocks + b] -> out[q]
-__global__ void k_reduce_final(const double* __restrict__ part, int nq, double* __restrict__ out) {
+// sum of nq partial arrays part[q * nb + b] -> out[q]
+__global__ void k_reduce_final(const double* __restrict__ part, int nb, int nq, double* __restrict__ out) {
   __shared__ double sh[32];
   for (int q = 0; q < nq; ++q) {
     double v = 0.0;
-    for (int b = threadIdx.x; b < kReduceBlocks; b += blockDim.x) v += part[q * kReduceBlocks + b];
+    for (int b = threadIdx.x; b < nb; b += blockDim.x) v += part[q * nb + b];
     v = block_sum(v, sh);
     if (threadIdx.x == 0) out[q] = v;
   }
@@ -98,17 +147,17 @@ __global__ void __launch_bounds__(kReduceThreads)
   bb = block_sum(bb, sh);
   if (threadIdx.x == 0) {
     part[blockIdx.x] = rz;
-    part[kReduceBlocks + blockIdx.x] = rr;
-    part[2 * kReduceBlocks + blockIdx.x] = bb;
+    part[gridDim.x + blockIdx.x] = rr;
+    part[2 * gridDim.x + blockIdx.x] = bb;
   }
 }
 
-__global__ void k_pcg_init_final(const double* __restrict__ part, double* __restrict__ sc, double rtol) {
+__global__ void k_pcg_init_final(const double* __restrict__ part, int nb, double* __restrict__ sc, double rtol) {
   __shared__ double sh[32];
   double v[3];
   for (int q = 0; q < 3; ++q) {
     double t = 0.0;
-    for (int b = threadIdx.x; b < kReduceBlocks; b += blockDim.x) t += part[q * kReduceBlocks + b];
+    for (int b = threadIdx.x; b < nb; b += blockDim.x) t += part[q * nb + b];
     v[q] = block_sum(t, sh);
   }
   if (threadIdx.x == 0) {
@@ -121,20 +170,9 @@ __global__ void k_pcg_init_final(const double* __restrict__ part, double* __rest
   }
 }
 
-__global__ void k_pcg_alpha(const double* __restrict__ part, int64_t nparts, double* __restrict__ sc) {
-  __shared__ double sh[32];
-  double t = 0.0;
-  for (int64_t b = threadIdx.x; b < nparts; b += blockDim.x) t += part[b];
-  t = block_sum(t, sh);
-  if (threadIdx.x == 0) {
-    sc[SC_PQ] = t;
-    const double a = sc[SC_RZ] / t;
-    sc[SC_ALPHA] = (sc[SC_CONV] >= 0.0 || t == 0.0 || !isfinite(a)) ? 0.0 : a;
-  }
-}
-
-// x += alpha p, r -= alpha q, z = r / diag; partials of r.z and r.r; with counter, the
-// last block to finish takes the step's beta (else k_pcg_beta does)
+// x += alpha p, r -= alpha q, z = r / diag; partials of r.z and r.r; the last
+// block to finish takes the step's beta (the iteration count lives on the device, so that
+// every batch of iterations launches the same kernels with the same arguments)
 template <typename T>
 __global__ void __launch_bounds__(kReduceThreads)
     k_pcg_update(int64_t n, double* __restrict__ sc, T* __restrict__ x, T* __restrict__ r,
@@ -156,13 +194,13 @@ __global__ void __launch_bounds__(kReduceThreads)
   rr = block_sum(rr, sh);
   if (threadIdx.x == 0) {
     part[blockIdx.x] = rz;
-    part[kReduceBlocks + blockIdx.x] = rr;
+    part[gridDim.x + blockIdx.x] = rr;
   }
-  if (counter != nullptr && last_block(counter)) {
+  if (last_block(counter)) {
     double v0 = 0.0, v1 = 0.0;
-    for (int b = threadIdx.x; b < kReduceBlocks; b += blockDim.x) {
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
       v0 += __ldcg(part + b);
-      v1 += __ldcg(part + kReduceBlocks + b);
+      v1 += __ldcg(part + gridDim.x + b);
     }
     v0 = block_sum(v0, sh);
     v1 = block_sum(v1, sh);
@@ -171,19 +209,6 @@ __global__ void __launch_bounds__(kReduceThreads)
       *counter = 0u;
     }
   }
-}
-
-// the iteration count lives on the device (sc[SC_IT]), so that every batch of
-// iterations launches the same kernels with the same arguments (a graph replays it)
-__global__ void k_pcg_beta(const double* __restrict__ part, double* __restrict__ sc) {
-  __shared__ double sh[32];
-  double v[2];
-  for (int q = 0; q < 2; ++q) {
-    double t = 0.0;
-    for (int b = threadIdx.x; b < kReduceBlocks; b += blockDim.x) t += part[q * kReduceBlocks + b];
-    v[q] = block_sum(t, sh);
-  }
-  if (threadIdx.x == 0) beta_step(v[0], v[1], sc);
 }
 
 template <typename T>
@@ -222,10 +247,10 @@ __global__ void __launch_bounds__(kReduceThreads)
     if (zold != nullptr) rzc = fma(ri, zold[i], rzc);
   }
   rr = block_sum(rr, sh);
-  if (threadIdx.x == 0) part[kReduceBlocks + blockIdx.x] = rr;
+  if (threadIdx.x == 0) part[gridDim.x + blockIdx.x] = rr;
   if (zold != nullptr) {
     rzc = block_sum(rzc, sh);
-    if (threadIdx.x == 0) part[2 * kReduceBlocks + blockIdx.x] = rzc;
+    if (threadIdx.x == 0) part[2 * gridDim.x + blockIdx.x] = rzc;
   }
 }
 
@@ -246,8 +271,8 @@ __global__ void __launch_bounds__(kReduceThreads)
   rr = block_sum(rr, sh);
   bb = block_sum(bb, sh);
   if (threadIdx.x == 0) {
-    part[kReduceBlocks + blockIdx.x] = rr;
-    part[2 * kReduceBlocks + blockIdx.x] = bb;
+    part[gridDim.x + blockIdx.x] = rr;
+    part[2 * gridDim.x + blockIdx.x] = bb;
   }
 }
 
@@ -292,10 +317,10 @@ __global__ void __launch_bounds__(kReduceThreads)
 }
 
 // the true residual's r.r; the new scale
-__global__ void k_mx_scale(const double* __restrict__ part, double* __restrict__ sc) {
+__global__ void k_mx_scale(const double* __restrict__ part, int nb, double* __restrict__ sc) {
   __shared__ double sh[32];
   double t = 0.0;
-  for (int b = threadIdx.x; b < kReduceBlocks; b += blockDim.x) t += part[b];
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) t += part[b];
   t = block_sum(t, sh);
   if (threadIdx.x == 0) {
     sc[SC_TRUE] = t;
@@ -325,18 +350,18 @@ __global__ void __launch_bounds__(kReduceThreads)
   rr = block_sum(rr, sh);
   if (threadIdx.x == 0) {
     part[blockIdx.x] = rz;
-    part[kReduceBlocks + blockIdx.x] = rr;
+    part[gridDim.x + blockIdx.x] = rr;
   }
 }
 
 // scalars of the recurrence after an anchor; bb and tol2 are in the scaled units
-__global__ void k_mx_anchor_final(const double* __restrict__ part, double* __restrict__ sc,
+__global__ void k_mx_anchor_final(const double* __restrict__ part, int nb, double* __restrict__ sc,
                                   const double* __restrict__ bbp, double rtol) {
   __shared__ double sh[32];
   double v[2];
   for (int q = 0; q < 2; ++q) {
     double t = 0.0;
-    for (int b = threadIdx.x; b < kReduceBlocks; b += blockDim.x) t += part[q * kReduceBlocks + b];
+    for (int b = threadIdx.x; b < nb; b += blockDim.x) t += part[q * nb + b];
     v[q] = block_sum(t, sh);
   }
   if (threadIdx.x == 0) {
@@ -356,6 +381,9 @@ using namespace hm;
 namespace {
 inline cudaStream_t S_(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 inline int grid1(int64_t n, int block) { return (int)((n + block - 1) / block); }
+inline int spmv_blocks(int64_t nrow, int per_sm) {
+  return (int)std::min<int64_t>((nrow + kSpmvRows - 1) / kSpmvRows, 148 * per_sm);
+}
 inline int ok_or_cuda() { return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA; }
 }  // namespace
 
@@ -364,7 +392,7 @@ extern "C" int hm_csr_spmv(int64_t nrow, const int32_t* indptr, const int32_t* i
                            double beta, void* stream) {
   if (nrow < 0 || (nrow > 0 && (!indptr || !indices || !vals || !x || !y))) return HM_ERR_ARG;
   if (nrow == 0) return HM_OK;
-  k_spmv<8, false><<<grid1(nrow * 8, 256), 256, 0, S_(stream)>>>(nrow, indptr, indices, nullptr, vals, x, y, alpha, beta);
+  k_spmv<8, false, false, 8><<<spmv_blocks(nrow, kSpmvBlocks), 256, 0, S_(stream)>>>(nrow, indptr, indices, nullptr, vals, x, y, alpha, beta, nullptr, nullptr, nullptr);
   return ok_or_cuda();
 }
 
@@ -373,7 +401,7 @@ extern "C" int hm_csr_spmv_t(int64_t nrow, const int32_t* indptr, const int32_t*
                              double alpha, double beta, void* stream) {
   if (nrow < 0 || (nrow > 0 && (!indptr || !indices || !tpos || !vals || !x || !y))) return HM_ERR_ARG;
   if (nrow == 0) return HM_OK;
-  k_spmv<8, true><<<grid1(nrow * 8, 256), 256, 0, S_(stream)>>>(nrow, indptr, indices, tpos, vals, x, y, alpha, beta);
+  k_spmv<8, true, false, 4><<<grid1(nrow, kSpmvRows), 256, 0, S_(stream)>>>(nrow, indptr, indices, tpos, vals, x, y, alpha, beta, nullptr, nullptr, nullptr);
   return ok_or_cuda();
 }
 
@@ -394,13 +422,13 @@ extern "C" int hm_dot(int64_t n, const double* x, const double* y, double* out, 
                       void* stream) {
   if (n < 0 || !out || !work || (n > 0 && (!x || !y))) return HM_ERR_ARG;
   double* part = static_cast<double*>(work);
-  k_dot_partial<<<kReduceBlocks, kReduceThreads, 0, S_(stream)>>>(n, x, y, part);
-  k_reduce_final<<<1, 1024, 0, S_(stream)>>>(part, 1, out);
+  k_dot_partial<<<reduce_blocks(n), kReduceThreads, 0, S_(stream)>>>(n, x, y, part);
+  k_reduce_final<<<1, 1024, 0, S_(stream)>>>(part, reduce_blocks(n), 1, out);
   return ok_or_cuda();
 }
 
-// slots for the partial sums of p.q: one per block of the lattice operator's gather
-// (at most n), or the fixed reduction grid after a CSR product
+// slots for the partial sums of p.q: one per block of the operator (at most n, or
+// kReduceBlocks of the CSR product)
 inline int64_t pq_slots(int64_t n) { return n > kReduceBlocks ? n : (int64_t)kReduceBlocks; }
 
 extern "C" int64_t hm_pcg_workspace_bytes(int64_t n) {
@@ -408,15 +436,14 @@ extern "C" int64_t hm_pcg_workspace_bytes(int64_t n) {
   return (int64_t)sizeof(double) * (4 * n + pq_slots(n) + SC_N + 3 * (int64_t)kReduceBlocks + 8);
 }
 
-int64_t hm_apply_dot_parts(const hm::Lattice& L);
 int hm_pcg_operator(int64_t n, const int32_t* indptr, const int32_t* indices, const double* vals,
                     const hm::Lattice* L, const void* quad, int precision, const uint8_t* ess,
                     const double* x, double* y, void* stream);
 
 namespace {
 
-// The operator of one PCG: y = A x, and, when part is given, the partial sums of x.y
-// (returns their count through *nparts).
+// The operator of one PCG: y = A x; with part (and sc, counter) a CG step's product, whose
+// last block also takes the step's alpha from the partial sums of x.y.
 struct PcgOp {
   int64_t n;
   const int32_t* indptr;
@@ -428,48 +455,34 @@ struct PcgOp {
   const uint8_t* ess;
 };
 
-// With sc and counter, the lattice operator's last block also takes the step's alpha
-// (*fused = true); the CSR product leaves it to k_pcg_alpha.
-int op_apply(const PcgOp& o, const double* x, double* y, double* part, int64_t* nparts, void* stream,
-             double* sc = nullptr, unsigned* counter = nullptr, bool* fused = nullptr) {
-  if (fused) *fused = false;
-  if (o.L != nullptr) {
-    if (part) {
-      *nparts = hm_apply_dot_parts(*o.L);
-      if (fused) *fused = sc != nullptr;
-      return hm_launch_apply_A_dot(*o.L, o.jac, o.precision, o.ess, x, y, part, stream, sc, counter);
-    }
-    return hm_pcg_operator(o.n, nullptr, nullptr, nullptr, o.L, o.jac, o.precision, o.ess, x, y, stream);
-  }
-  int rc = hm_pcg_operator(o.n, o.indptr, o.indices, o.vals, nullptr, nullptr, HM_FP64, o.ess, x, y, stream);
-  if (rc || !part) return rc;
-  *nparts = kReduceBlocks;
-  k_dot_partial_t<double><<<kReduceBlocks, kReduceThreads, 0, S_(stream)>>>(o.n, x, y, part);
+int op_apply(const PcgOp& o, const double* x, double* y, void* stream, double* part = nullptr,
+             double* sc = nullptr, unsigned* counter = nullptr) {
+  if (part == nullptr)
+    return hm_pcg_operator(o.n, o.indptr, o.indices, o.vals, o.L, o.jac, o.L ? o.precision : HM_FP64, o.ess, x, y,
+                           stream);
+  if (o.L != nullptr) return hm_launch_apply_A_dot(*o.L, o.jac, o.precision, o.ess, x, y, part, stream, sc, counter);
+  k_spmv<8, false, true, 8><<<spmv_blocks(o.n, kSpmvDotBlocks), 256, 0, S_(stream)>>>(o.n, o.indptr, o.indices, nullptr, o.vals, x, y,
+                                                                     1.0, 0.0, part, sc, counter);
   return ok_or_cuda();
 }
 
-int op_apply(const PcgOp& o, const float* x, float* y, double* part, int64_t* nparts, void* stream,
-             double* sc = nullptr, unsigned* counter = nullptr, bool* fused = nullptr) {
-  if (part) *nparts = hm_apply_dot_parts(*o.L);
-  if (fused) *fused = part != nullptr && sc != nullptr;
+int op_apply(const PcgOp& o, const float* x, float* y, void* stream, double* part = nullptr,
+             double* sc = nullptr, unsigned* counter = nullptr) {
   return hm_launch_apply_A32_dot(*o.L, o.jac, o.ess, x, y, part, stream, sc, counter);
 }
 
-// `count` PCG iterations (operator + fused p.q, alpha, update with r.z and r.r, beta,
+// `count` PCG iterations (operator with p.q and alpha, update with r.z and r.r, beta,
 // direction); nothing in it synchronises with the host
 // cnt: two counters (zero between uses) for the reductions the producing kernels finish
 template <typename T>
 int pcg_batch(const PcgOp& o, const double* diag, T* x, T* r, T* z, T* p, T* q, double* pq_part,
               double* sc, double* part, unsigned* cnt, int count, cudaStream_t s) {
-  int64_t np = 0;
   for (int j = 0; j < count; ++j) {
-    bool fused = false;
-    const int rc = op_apply(o, p, q, pq_part, &np, (void*)s, sc, cnt, &fused);
+    const int rc = op_apply(o, p, q, (void*)s, pq_part, sc, cnt);
     if (rc) return rc;
-    if (!fused) k_pcg_alpha<<<1, 1024, 0, s>>>(pq_part, np, sc);
-    k_pcg_update<T><<<kReduceBlocks, kReduceThreads, 0, s>>>(o.n, sc, x, r, z, p, q, diag, part,
+    k_pcg_update<T><<<reduce_blocks(o.n), kReduceThreads, 0, s>>>(o.n, sc, x, r, z, p, q, diag, part,
                                                                cnt + 1);
-    k_pcg_pupdate<T><<<kReduceBlocks, kReduceThreads, 0, s>>>(o.n, sc, z, p);
+    k_pcg_pupdate<T><<<reduce_blocks(o.n), kReduceThreads, 0, s>>>(o.n, sc, z, p);
   }
   return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
 }
@@ -534,11 +547,10 @@ int pcg_run(const PcgOp& o, const double* diag, const T* b, T* x, double rtol, i
   // the lattice operator's direction products rely on
   if constexpr (std::is_same<T, double>::value)
     if (o.L && (rc = hm_launch_ess_take_b(*o.L, o.ess, b, x, stream))) return rc;
-  int64_t nparts = 0;
-  rc = op_apply(o, x, q, nullptr, &nparts, stream);
+  rc = op_apply(o, x, q, stream);
   if (rc) return rc;
-  k_pcg_init<T><<<kReduceBlocks, kReduceThreads, 0, s>>>(n, b, q, diag, r, z, p, part);
-  k_pcg_init_final<<<1, 1024, 0, s>>>(part, sc, rtol);
+  k_pcg_init<T><<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, b, q, diag, r, z, p, part);
+  k_pcg_init_final<<<1, 1024, 0, s>>>(part, reduce_blocks(n), sc, rtol);
   double host[SC_N];
   int it = 0;
   for (;;) {
@@ -602,14 +614,13 @@ int pcg_mg_run(hm_mg* mg, const double* b, double* x, double rtol, int maxiter, 
   if (cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned), s) != cudaSuccess) return HM_ERR_CUDA;
   int rc = hm_launch_ess_take_b(*L, o.ess, b, x, stream);   // as in pcg_run
   if (rc) return rc;
-  int64_t np = 0;
-  rc = op_apply(o, x, q, nullptr, &np, stream);
+  rc = op_apply(o, x, q, stream);
   if (rc) return rc;
   const HmFirstDir fd = hm_mg_first_dir(mg);
-  k_pcg_mg_init<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, b, q, r, part, fd);
+  k_pcg_mg_init<<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, b, q, r, part, fd);
   if ((rc = hm_mg_vcycle(mg, r, z, stream))) return rc;
-  k_dot_partial_t<double><<<kReduceBlocks, kReduceThreads, 0, s>>>(n, r, z, part);
-  k_pcg_init_final<<<1, 1024, 0, s>>>(part, sc, rtol);
+  k_dot_partial_t<double><<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, r, z, part);
+  k_pcg_init_final<<<1, 1024, 0, s>>>(part, reduce_blocks(n), sc, rtol);
   if (cudaMemcpyAsync(p, z, sizeof(double) * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
     return HM_ERR_CUDA;
   double host[SC_N];
@@ -636,17 +647,15 @@ int pcg_mg_run(hm_mg* mg, const double* b, double* x, double rtol, int maxiter, 
     const int count = it + check_every < maxiter ? check_every : maxiter - it;
     rc = run_batch(graph, count == check_every, s, [&]() -> int {
       for (int j = 0; j < count; ++j) {
-        bool fused = false;
-        int e = op_apply(o, p, q, pq_part, &np, (void*)s, sc, cnt, &fused);
+        int e = op_apply(o, p, q, (void*)s, pq_part, sc, cnt);
         if (e) return e;
-        if (!fused) k_pcg_alpha<<<1, 1024, 0, s>>>(pq_part, np, sc);
-        k_pcg_update_rr<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, sc, x, r, p, q, part, fd,
+        k_pcg_update_rr<<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, sc, x, r, p, q, part, fd,
                                                                  flex ? z : nullptr);
         // the cycle's last operator pass takes r.z and the step's beta where it can
-        HmBeta be{pq_part, part + kReduceBlocks, kReduceBlocks, flex, sc, cnt + 1, 0};
+        HmBeta be{pq_part, part + reduce_blocks(n), (unsigned)reduce_blocks(n), flex, sc, cnt + 1, 0};
         if ((e = hm_mg_vcycle(mg, r, z, (void*)s, &be))) return e;
         if (!be.done && (e = hm_launch_beta(*L, r, z, be, (void*)s))) return e;
-        k_pcg_pupdate<double><<<kReduceBlocks, kReduceThreads, 0, s>>>(n, sc, z, p);
+        k_pcg_pupdate<double><<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, sc, z, p);
       }
       return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
     });
@@ -719,21 +728,20 @@ int pcg_mixed_run(const hm::Lattice* L, void* jac64, void* jac32, const uint8_t*
   // the anchor: [x += s x32; t = A64 x]; r = b - t; new scale; FP32 r, z, p from r (p
   // restarted as z on the first anchor and on a restart)
   auto anchor = [&](bool first, bool restart) -> int {
-    int64_t np = 0;
     if (!first) {
-      k_mx_accum<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, sc, x32, x);
-      const int rc = op_apply(o64, x, t64, nullptr, &np, stream);
+      k_mx_accum<<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, sc, x32, x);
+      const int rc = op_apply(o64, x, t64, stream);
       if (rc) return rc;
     }
     // first: x is b on the Dirichlet nodes and 0 elsewhere, so r = b off them, 0 on them
-    k_residual64<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, b, first ? nullptr : t64,
+    k_residual64<<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, b, first ? nullptr : t64,
                                                           first ? ess : nullptr, r64, part);
-    k_mx_scale<<<1, 1024, 0, s>>>(part, sc);
+    k_mx_scale<<<1, 1024, 0, s>>>(part, reduce_blocks(n), sc);
     if (first && cudaMemcpyAsync(bbp, sc + SC_TRUE, sizeof(double), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
       return HM_ERR_CUDA;
-    k_mx_anchor<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, r64, diag, sc, (first || restart) ? 1 : 0,
+    k_mx_anchor<<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, r64, diag, sc, (first || restart) ? 1 : 0,
                                                          r32, z32, p32, part);
-    k_mx_anchor_final<<<1, 1024, 0, s>>>(part, sc, bbp, rtol);
+    k_mx_anchor_final<<<1, 1024, 0, s>>>(part, reduce_blocks(n), sc, bbp, rtol);
     if (cudaGetLastError() != cudaSuccess) return HM_ERR_CUDA;
     return read();
   };
@@ -939,20 +947,19 @@ int group_init(hm_pcg_plan* pl, double rtol, cudaStream_t s) {
     return HM_ERR_CUDA;
   int rc = hm_launch_ess_take_b(pl->L, o.ess, pl->b, pl->x, (void*)s);
   if (rc) return rc;
-  int64_t np = 0;
-  if ((rc = op_apply(o, pl->x, B.q, nullptr, &np, (void*)s))) return rc;
+  if ((rc = op_apply(o, pl->x, B.q, (void*)s))) return rc;
   if (pl->mg != nullptr) {
-    k_pcg_mg_init<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, pl->b, B.q, B.r, B.part,
+    k_pcg_mg_init<<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, pl->b, B.q, B.r, B.part,
                                                            hm_mg_first_dir(pl->mg));
     if ((rc = hm_mg_vcycle(pl->mg, B.r, B.z, (void*)s))) return rc;
-    k_dot_partial_t<double><<<kReduceBlocks, kReduceThreads, 0, s>>>(n, B.r, B.z, B.part);
-    k_pcg_init_final<<<1, 1024, 0, s>>>(B.part, B.sc, rtol);
+    k_dot_partial_t<double><<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, B.r, B.z, B.part);
+    k_pcg_init_final<<<1, 1024, 0, s>>>(B.part, reduce_blocks(n), B.sc, rtol);
     if (cudaMemcpyAsync(B.p, B.z, sizeof(double) * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
       return HM_ERR_CUDA;
   } else {
-    k_pcg_init<double><<<kReduceBlocks, kReduceThreads, 0, s>>>(n, pl->b, B.q, pl->diag, B.r, B.z,
+    k_pcg_init<double><<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, pl->b, B.q, pl->diag, B.r, B.z,
                                                                B.p, B.part);
-    k_pcg_init_final<<<1, 1024, 0, s>>>(B.part, B.sc, rtol);
+    k_pcg_init_final<<<1, 1024, 0, s>>>(B.part, reduce_blocks(n), B.sc, rtol);
   }
   return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
 }
@@ -965,20 +972,17 @@ int group_batch(hm_pcg_plan* pl, int count, cudaStream_t s) {
   if (pl->mg == nullptr)
     return pcg_batch<double>(o, pl->diag, pl->x, B.r, B.z, B.p, B.q, B.pq_part, B.sc, B.part,
                              B.cnt, count, s);
-  int64_t np = 0;
   for (int j = 0; j < count; ++j) {
-    bool fused = false;
-    int e = op_apply(o, B.p, B.q, B.pq_part, &np, (void*)s, B.sc, B.cnt, &fused);
+    int e = op_apply(o, B.p, B.q, (void*)s, B.pq_part, B.sc, B.cnt);
     if (e) return e;
-    if (!fused) k_pcg_alpha<<<1, 1024, 0, s>>>(B.pq_part, np, B.sc);
     const int flex = hm_mg_flexible(pl->mg) ? 1 : 0;
-    k_pcg_update_rr<<<kReduceBlocks, kReduceThreads, 0, s>>>(n, B.sc, pl->x, B.r, B.p, B.q, B.part,
+    k_pcg_update_rr<<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, B.sc, pl->x, B.r, B.p, B.q, B.part,
                                                              hm_mg_first_dir(pl->mg),
                                                              flex ? B.z : nullptr);
-    HmBeta be{B.pq_part, B.part + kReduceBlocks, kReduceBlocks, flex, B.sc, B.cnt + 1, 0};
+    HmBeta be{B.pq_part, B.part + reduce_blocks(n), (unsigned)reduce_blocks(n), flex, B.sc, B.cnt + 1, 0};
     if ((e = hm_mg_vcycle(pl->mg, B.r, B.z, (void*)s, &be))) return e;
     if (!be.done && (e = hm_launch_beta(pl->L, B.r, B.z, be, (void*)s))) return e;
-    k_pcg_pupdate<double><<<kReduceBlocks, kReduceThreads, 0, s>>>(n, B.sc, B.z, B.p);
+    k_pcg_pupdate<double><<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, B.sc, B.z, B.p);
   }
   return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
 }
