@@ -98,100 +98,145 @@ __global__ void k_pattern_tpos(Lattice L, const int32_t* __restrict__ indptr,
 }
 
 // ============================================================ quadrature data
-// One thread per (element, Gauss point), 8 elements per 216-thread block.  Layout:
-// quad[e][c][q], c = 0 D, 1-3 E, 4-6 F, 7 W (each element's 216 values contiguous).
+// Layout: quad[e][c][q], c = 0 D, 1-3 E, 4-6 F, 7 W (each element's 216 values contiguous).
 // With mhat, D = w|J| e^m mhat: the data of the directional derivative along mhat
 // (the second-order products of the assembled vectors, with f = 0).
+//
+// Nine threads an element and field, each the three points of a line along x: the
+// contractions along y and z are taken once for the three, 39 multiply-adds and 9 shared
+// loads a field and point where a thread a point takes 93 and 27.  The points' products and
+// the stores follow with a thread a point.
+// Bound: the stores, 1728 bytes an element (68 us at 64^3 elements at the copy rate), with
+// the FP64 pipe close behind (65), in three phases that only other blocks overlap.  64^3
+// elements: 342 us with a thread a point, 186 here; 45 x 52 x 39 120 and 66, 32^3 46 and 25,
+// 4^3 3.5 and 2.9.  One set of nine threads for the three fields takes 171 at 64^3 but 4.5
+// at 4^3 (the longer chain); 16 elements a block 238, six blocks an SM (spills) 237.
+constexpr int kQuadElems = 8;
+constexpr int kQuadThreads = 27 * kQuadElems;
+constexpr int kQuadBlocks = 5;
+// the 1D derivative tables by point and node, divided by the element's edge
 template <typename real>
-__global__ void __launch_bounds__(216) k_quad(Lattice L, const double* __restrict__ u,
-                                              const double* __restrict__ m,
-                                              const double* __restrict__ p,
-                                              const double* __restrict__ mhat,
-                                              real* __restrict__ quad,
-                                              uint32_t* __restrict__ status) {
-  __shared__ real sv[8][4][27];
-  const int le = threadIdx.x / 27, q = threadIdx.x % 27;
-  const int64_t e = blockIdx.x * 8LL + le;
-  const bool live = e < L.ne;
-  if (live) {
-    const int ex = (int)(e % L.nx), ey = (int)((e / L.nx) % L.ny), ez = (int)(e / ((int64_t)L.nx * L.ny));
-    const int a = q;
+struct QuadTab {
+  real d[3][3][3];
+};
+
+// The contractions of a field's nodal values x along y and z at a line's (q2, q3): values,
+// and with GRAD derivatives along y and along z, at the three nodes along x.
+template <bool GRAD, typename real>
+__device__ __forceinline__ void quad_line(const real* x, const real (&b2)[3], const real (&d2)[3],
+                                          const real (&b3)[3], const real (&d3)[3], real (&bb)[3],
+                                          real (&bd)[3], real (&dz)[3]) {
+#pragma unroll
+  for (int a1 = 0; a1 < 3; ++a1) bb[a1] = bd[a1] = dz[a1] = real(0);
+#pragma unroll
+  for (int a3 = 0; a3 < 3; ++a3)
+#pragma unroll
+    for (int a1 = 0; a1 < 3; ++a1) {
+      real sb = 0, sd = 0;
+#pragma unroll
+      for (int a2 = 0; a2 < 3; ++a2) {
+        const real v = x[a1 + 3 * a2 + 9 * a3];
+        sb = fma(b2[a2], v, sb);
+        if constexpr (GRAD) sd = fma(d2[a2], v, sd);
+      }
+      bb[a1] = fma(b3[a3], sb, bb[a1]);
+      if constexpr (GRAD) {
+        bd[a1] = fma(b3[a3], sd, bd[a1]);
+        dz[a1] = fma(d3[a3], sb, dz[a1]);
+      }
+    }
+}
+
+template <typename real, bool MHAT>
+__global__ void __launch_bounds__(kQuadThreads, kQuadBlocks)
+    k_quad(Lattice L, const __grid_constant__ QuadTab<real> tab, const double* __restrict__ u,
+           const double* __restrict__ m, const double* __restrict__ p, const double* __restrict__ mhat,
+           real* __restrict__ quad, uint32_t* __restrict__ status) {
+  constexpr int NF = MHAT ? 4 : 3;
+  __shared__ real sx[NF][kQuadElems][27];                // m, u, p, mhat
+  __shared__ real sg[7][kQuadElems][27];                 // D, grad u, grad p at the points
+  __shared__ real sb[3][3], sd[2][3][3];
+  const int tid = threadIdx.x;
+  const int64_t e0 = blockIdx.x * (int64_t)kQuadElems;
+  const int count = (int)min((int64_t)kQuadElems, L.ne - e0);
+  if (tid < 9) {
+    sb[tid / 3][tid % 3] = (real)bq(tid / 3, tid % 3);
+    sd[0][tid / 3][tid % 3] = tab.d[1][tid / 3][tid % 3];
+    sd[1][tid / 3][tid % 3] = tab.d[2][tid / 3][tid % 3];
+  }
+  const int pe = tid / 27, a = tid - pe * 27;            // the thread's element as a node or a point
+  if (pe < count) {
+    const unsigned e = (unsigned)e0 + pe, row = e / (unsigned)L.nx;
+    const int ex = (int)(e - row * L.nx), ez = (int)(row / (unsigned)L.ny), ey = (int)(row - (unsigned)ez * L.ny);
     const int64_t node = (2 * ex + a % 3) + (int64_t)L.Nx * ((2 * ey + (a / 3) % 3) + (int64_t)L.Ny * (2 * ez + a / 9));
-    sv[le][0][a] = (real)u[node];
-    sv[le][1][a] = (real)m[node];
-    sv[le][2][a] = (real)p[node];
-    if (mhat) sv[le][3][a] = (real)mhat[node];
+    sx[0][pe][a] = (real)__ldg(m + node);
+    sx[1][pe][a] = (real)__ldg(u + node);
+    sx[2][pe][a] = (real)__ldg(p + node);
+    if constexpr (MHAT) sx[3][pe][a] = (real)__ldg(mhat + node);
   }
   __syncthreads();
-  if (!live) return;
-  const int q1 = q % 3, q2 = (q / 3) % 3, q3 = q / 9;
-  real b1[3], b2[3], b3[3], d1[3], d2[3], d3[3];
+  // a third of the threads a field
+  const int f = tid / (9 * kQuadElems), t = tid - f * 9 * kQuadElems;
+  const int le = t / 9, line = t - le * 9, q2 = line % 3, q3 = line / 3;
+  if (le < count) {
+    real b2[3], d2[3], b3[3], d3[3], bb[3], bd[3], dz[3];
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    b1[a] = (real)bq(q1, a); b2[a] = (real)bq(q2, a); b3[a] = (real)bq(q3, a);
-    d1[a] = (real)dbq(q1, a); d2[a] = (real)dbq(q2, a); d3[a] = (real)dbq(q3, a);
-  }
-  real val[3], gx[3], gy[3], gz[3];
+    for (int k = 0; k < 3; ++k) {
+      b2[k] = sb[q2][k]; b3[k] = sb[q3][k];
+      d2[k] = sd[0][q2][k]; d3[k] = sd[1][q3][k];
+    }
+    if (f == 0) {
+      const double w23 = (q2 == 1 ? wq(1) : wq(0)) * (q3 == 1 ? wq(1) : wq(0)) * L.hx * L.hy * L.hz;
+      quad_line<false>(sx[0][le], b2, d2, b3, d3, bb, bd, dz);
+      if constexpr (MHAT) quad_line<false>(sx[3][le], b2, d2, b3, d3, dz, bd, d3);
 #pragma unroll
-  for (int f = 0; f < 3; ++f) {
-    const real* x = sv[le][f];
-    real vb = 0, vx = 0, vy = 0, vz = 0;
+      for (int q = 0; q < 3; ++q) {
+        real v = 0, vh = 0;
 #pragma unroll
-    for (int a3 = 0; a3 < 3; ++a3) {
-      real sbb = 0, sdb = 0, sbd = 0;
-#pragma unroll
-      for (int a2 = 0; a2 < 3; ++a2) {
-        real xb = 0, xd = 0;
-#pragma unroll
-        for (int a1 = 0; a1 < 3; ++a1) {
-          xb = fma(b1[a1], x[a1 + 3 * a2 + 9 * a3], xb);
-          xd = fma(d1[a1], x[a1 + 3 * a2 + 9 * a3], xd);
+        for (int k = 0; k < 3; ++k) {
+          v = fma((real)bq(q, k), bb[k], v);
+          if constexpr (MHAT) vh = fma((real)bq(q, k), dz[k], vh);
         }
-        sbb = fma(b2[a2], xb, sbb);
-        sdb = fma(b2[a2], xd, sdb);
-        sbd = fma(d2[a2], xb, sbd);
+        real D = (real)(wq(q) * w23) * exp(v);
+        if constexpr (MHAT) D *= vh;
+        sg[0][le][3 * line + q] = D;
       }
-      vb = fma(b3[a3], sbb, vb);
-      vx = fma(b3[a3], sdb, vx);
-      vy = fma(b3[a3], sbd, vy);
-      vz = fma(d3[a3], sbb, vz);
-    }
-    val[f] = vb;
-    gx[f] = vx / (real)L.hx;
-    gy[f] = vy / (real)L.hy;
-    gz[f] = vz / (real)L.hz;
-  }
-  const real wdet = (real)(wq(q1) * wq(q2) * wq(q3) * L.hx * L.hy * L.hz);
-  real D = wdet * exp(val[1]);
-  if (mhat) {
-    // mhat at the point (value only)
-    const real* x = sv[le][3];
-    real vb = 0;
+    } else {
+      quad_line<true>(sx[f][le], b2, d2, b3, d3, bb, bd, dz);
 #pragma unroll
-    for (int a3 = 0; a3 < 3; ++a3) {
-      real sbb = 0;
+      for (int q = 0; q < 3; ++q) {
+        real gx = 0, gy = 0, gz = 0;
 #pragma unroll
-      for (int a2 = 0; a2 < 3; ++a2) {
-        real xb = 0;
-#pragma unroll
-        for (int a1 = 0; a1 < 3; ++a1) xb = fma(b1[a1], x[a1 + 3 * a2 + 9 * a3], xb);
-        sbb = fma(b2[a2], xb, sbb);
+        for (int k = 0; k < 3; ++k) {
+          gx = fma(tab.d[0][q][k], bb[k], gx);
+          gy = fma((real)bq(q, k), bd[k], gy);
+          gz = fma((real)bq(q, k), dz[k], gz);
+        }
+        sg[3 * f - 2][le][3 * line + q] = gx;
+        sg[3 * f - 1][le][3 * line + q] = gy;
+        sg[3 * f][le][3 * line + q] = gz;
       }
-      vb = fma(b3[a3], sbb, vb);
     }
-    D *= vb;
   }
-  const real E[3] = {D * gx[0], D * gy[0], D * gz[0]};
-  const real F[3] = {D * gx[2], D * gy[2], D * gz[2]};
-  const real W = D * (gx[0] * gx[2] + gy[0] * gy[2] + gz[0] * gz[2]);
-  real* out = quad + e * 216;
-  out[q] = D;
-  out[27 + q] = E[0]; out[54 + q] = E[1]; out[81 + q] = E[2];
-  out[108 + q] = F[0]; out[135 + q] = F[1]; out[162 + q] = F[2];
-  out[189 + q] = W;
-  const bool finite = isfinite(D) && isfinite(E[0]) && isfinite(E[1]) && isfinite(E[2]) &&
-                      isfinite(F[0]) && isfinite(F[1]) && isfinite(F[2]) && isfinite(W);
-  if (!finite) atomicOr(status, HM_STATUS_NONFINITE);
+  __syncthreads();
+  if (pe >= count) return;
+  const real D = sg[0][pe][a];
+  real* const out = quad + (e0 + pe) * 216 + a;
+  real W = 0;
+  bool finite = isfinite(D);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const real gu = sg[1 + c][pe][a], gp = sg[4 + c][pe][a];
+    const real E = D * gu, F = D * gp;
+    W = c == 0 ? gu * gp : W + gu * gp;
+    finite = finite && isfinite(E) && isfinite(F);
+    out[27 * (1 + c)] = E;
+    out[27 * (4 + c)] = F;
+  }
+  W *= D;
+  out[0] = D;
+  out[189] = W;
+  if (!finite || !isfinite(W)) atomicOr(status, HM_STATUS_NONFINITE);
 }
 
 // =============================================== data of the matrix-free Jacobian apply
@@ -207,53 +252,109 @@ __global__ void k_extract_D(Lattice L, int pitch, const src* __restrict__ quad, 
   Dq[((int64_t)q * L.ny * L.nz + row) * pitch + (e - row * L.nx)] = (real)quad[e * 216 + q];
 }
 
-// diagonal of A(D): sum_g D(g) sum_d (d_d phi_n)^2, one thread per node
+// Diagonal of A(D): sum_g D(g) sum_d (d_d phi_n)^2.  A block owns the nodes of a tile of
+// 8 x 4 x 4 elements (and reads one more layer below it): a thread takes one element's 27
+// contributions by contractions along x, y and z (567 multiply-adds; 27 x 27 products of
+// three factors and three directions node by node), then the nodes sum those of the elements
+// that touch them in a fixed order.  Bound: the latency of the loads, 216 of every 1728
+// bytes.  64^3 elements: 328 us node by node, 95 here; 45 x 52 x 39 117 and 34; 16^3 11 and
+// 14 (few blocks, each a longer chain).
+constexpr int kDiagX = 8, kDiagY = 4, kDiagZ = 4;
+constexpr int kDiagElems = (kDiagX + 1) * (kDiagY + 1) * (kDiagZ + 1);
+// squared derivatives by axis, point and node, divided by the squared edge
+struct DiagTab {
+  double d2[3][3][3];
+};
 template <typename real>
-__global__ void k_diag_A(Lattice L, const real* __restrict__ quad, const uint8_t* __restrict__ ess,
-                         double* __restrict__ diag) {
-  const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (n >= L.ndof) return;
-  const int i = (int)(n % L.Nx), j = (int)((n / L.Nx) % L.Ny), k = (int)(n / ((int64_t)L.Nx * L.Ny));
-  if (ess != nullptr && ess[n]) { diag[n] = 1.0; return; }
-  const int gi[3] = {i, j, k};
-  const int ne[3] = {L.nx, L.ny, L.nz};
-  const double h2[3] = {1.0 / (L.hx * L.hx), 1.0 / (L.hy * L.hy), 1.0 / (L.hz * L.hz)};
-  // elements touching the node along each axis
-  int el0[3], nel[3];
-  for (int d = 0; d < 3; ++d) {
-    if (gi[d] & 1) { el0[d] = gi[d] / 2; nel[d] = 1; }
-    else {
-      el0[d] = gi[d] / 2 - 1; nel[d] = 2;
-      if (el0[d] < 0) { el0[d] = 0; nel[d] = 1; }
-      else if (el0[d] + 1 >= ne[d]) nel[d] = 1;
+__global__ void __launch_bounds__(256, 2)
+    k_diag_A(Lattice L, const __grid_constant__ DiagTab tab, const real* __restrict__ quad,
+             const uint8_t* __restrict__ ess, double* __restrict__ diag) {
+  __shared__ double sD[kDiagElems * 27];
+  const int tx = (L.nx + kDiagX - 1) / kDiagX, ty = (L.ny + kDiagY - 1) / kDiagY;
+  const int bx = blockIdx.x % tx, by = (blockIdx.x / tx) % ty, bz = blockIdx.x / (tx * ty);
+  // the first element of the tile with its lower layer (-1 in the first tile of an axis)
+  const int ex0 = bx * kDiagX - 1, ey0 = by * kDiagY - 1, ez0 = bz * kDiagZ - 1;
+  // eight loads in flight a thread
+  constexpr int kLoads = (kDiagElems * 27 + 255) / 256;
+#pragma unroll 1
+  for (int r = 0; r < kLoads; r += 8) {
+    double v[8];
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+      const int t = threadIdx.x + 256 * (r + g), le = t / 27, q = t - le * 27;
+      const int ex = ex0 + le % (kDiagX + 1), ey = ey0 + (le / (kDiagX + 1)) % (kDiagY + 1),
+                ez = ez0 + le / ((kDiagX + 1) * (kDiagY + 1));
+      const bool on = t < kDiagElems * 27 && ex >= 0 && ey >= 0 && ez >= 0 && ex < L.nx && ey < L.ny && ez < L.nz;
+      v[g] = on ? (double)__ldg(quad + (ex + (int64_t)L.nx * (ey + (int64_t)L.ny * ez)) * 216 + q) : 0.0;
     }
+#pragma unroll
+    for (int g = 0; g < 8; ++g)
+      if (const int t = threadIdx.x + 256 * (r + g); t < kDiagElems * 27) sD[t] = v[g];
   }
-  double acc = 0.0;
-  for (int c3 = 0; c3 < nel[2]; ++c3)
-    for (int c2 = 0; c2 < nel[1]; ++c2)
-      for (int c1 = 0; c1 < nel[0]; ++c1) {
-        const int e1 = el0[0] + c1, e2 = el0[1] + c2, e3 = el0[2] + c3;
-        const int a1 = i - 2 * e1, a2 = j - 2 * e2, a3 = k - 2 * e3;
-        const real* Dq = quad + (e1 + (int64_t)L.nx * (e2 + (int64_t)L.ny * e3)) * 216;
-        // the node's 1D values and derivatives at the three points of each axis, once
-        // per element (the products below keep their order)
-        double b[3][3], d[3][3];
+  __syncthreads();
+  if (threadIdx.x < kDiagElems) {
+    double* const D = sD + threadIdx.x * 27;
+    double C[3][3][3];
 #pragma unroll
-        for (int t = 0; t < 3; ++t) {
-          b[0][t] = bq(t, a1); b[1][t] = bq(t, a2); b[2][t] = bq(t, a3);
-          d[0][t] = dbq(t, a1); d[1][t] = dbq(t, a2); d[2][t] = dbq(t, a3);
+    for (int a = 0; a < 27; ++a) C[a / 9][(a / 3) % 3][a % 3] = 0.0;
+#pragma unroll
+    for (int q3 = 0; q3 < 3; ++q3) {
+      double R[3][3], S[3][3];                 // derivatives along x or y, none
+#pragma unroll
+      for (int a = 0; a < 9; ++a) R[a / 3][a % 3] = S[a / 3][a % 3] = 0.0;
+#pragma unroll
+      for (int q2 = 0; q2 < 3; ++q2) {
+        double P[3] = {0.0, 0.0, 0.0}, Q[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int q1 = 0; q1 < 3; ++q1) {
+          const double v = D[q1 + 3 * q2 + 9 * q3];
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            P[a] = fma(bq(q1, a) * bq(q1, a), v, P[a]);
+            Q[a] = fma(tab.d2[0][q1][a], v, Q[a]);
+          }
         }
 #pragma unroll
-        for (int q = 0; q < 27; ++q) {
-          const int q1 = q % 3, q2 = (q / 3) % 3, q3 = q / 9;
-          const double b1 = b[0][q1], b2 = b[1][q2], b3 = b[2][q3];
-          const double d1 = d[0][q1], d2 = d[1][q2], d3 = d[2][q3];
-          const double s = d1 * d1 * b2 * b2 * b3 * b3 * h2[0] + b1 * b1 * d2 * d2 * b3 * b3 * h2[1] +
-                           b1 * b1 * b2 * b2 * d3 * d3 * h2[2];
-          acc += (double)Dq[q] * s;
-        }
+        for (int a2 = 0; a2 < 3; ++a2)
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            R[a2][a] = fma(bq(q2, a2) * bq(q2, a2), Q[a], fma(tab.d2[1][q2][a2], P[a], R[a2][a]));
+            S[a2][a] = fma(bq(q2, a2) * bq(q2, a2), P[a], S[a2][a]);
+          }
       }
-  diag[n] = acc;
+#pragma unroll
+      for (int a3 = 0; a3 < 3; ++a3)
+#pragma unroll
+        for (int a = 0; a < 9; ++a)
+          C[a3][a / 3][a % 3] = fma(bq(q3, a3) * bq(q3, a3), R[a / 3][a % 3],
+                                    fma(tab.d2[2][q3][a3], S[a / 3][a % 3], C[a3][a / 3][a % 3]));
+    }
+#pragma unroll
+    for (int a = 0; a < 27; ++a) D[a] = C[a / 9][(a / 3) % 3][a % 3];
+  }
+  __syncthreads();
+  const int i0 = 2 * (ex0 + 1), j0 = 2 * (ey0 + 1), k0 = 2 * (ez0 + 1);
+  // the tile's nodes; the last tile of an axis has the mesh's last node plane as well
+  const int ni = i0 + 2 * kDiagX < L.Nx - 1 ? 2 * kDiagX : L.Nx - i0;
+  const int nj = j0 + 2 * kDiagY < L.Ny - 1 ? 2 * kDiagY : L.Ny - j0;
+  const int nk = k0 + 2 * kDiagZ < L.Nz - 1 ? 2 * kDiagZ : L.Nz - k0;
+  for (int t = threadIdx.x; t < ni * nj * nk; t += 256) {
+    const int li = t % ni, lj = (t / ni) % nj, lk = t / (ni * nj);
+    const int i = i0 + li, j = j0 + lj, k = k0 + lk;
+    const int64_t n = i + (int64_t)L.Nx * (j + (int64_t)L.Ny * k);
+    // along each axis the element that holds the node as 1, or as 2 and (the next) as 0;
+    // elements outside the mesh have zeros
+    double acc = 0.0;
+    for (int c3 = lk & 1; c3 < 2; ++c3)
+      for (int c2 = lj & 1; c2 < 2; ++c2)
+        for (int c1 = li & 1; c1 < 2; ++c1) {
+          const int e1 = li / 2 + c1, e2 = lj / 2 + c2, e3 = lk / 2 + c3;
+          if (e1 > kDiagX || e2 > kDiagY || e3 > kDiagZ) continue;       // past the mesh
+          const int a = (li - 2 * (e1 - 1)) + 3 * (lj - 2 * (e2 - 1)) + 9 * (lk - 2 * (e3 - 1));
+          acc += sD[(e1 + (kDiagX + 1) * (e2 + (kDiagY + 1) * e3)) * 27 + a];
+        }
+    diag[n] = ess != nullptr && ess[n] ? 1.0 : acc;
+  }
 }
 
 }  // namespace hm
@@ -279,14 +380,30 @@ int hm_launch_tpos(const Lattice& L, const int32_t* indptr, int32_t* tpos, void*
   return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
 }
 
+namespace {
+template <typename real, bool MHAT>
+int launch_quad_as(const Lattice& L, const double* u, const double* m, const double* p, const double* mhat,
+                   real* quad, uint32_t* status, cudaStream_t s) {
+  QuadTab<real> tab;
+  const double h[3] = {L.hx, L.hy, L.hz};
+  for (int d = 0; d < 3; ++d)
+    for (int q = 0; q < 3; ++q)
+      for (int a = 0; a < 3; ++a) tab.d[d][q][a] = (real)(dbq(q, a) / h[d]);
+  k_quad<real, MHAT><<<grid1(L.ne, kQuadElems), kQuadThreads, 0, s>>>(L, tab, u, m, p, mhat, quad, status);
+  return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
+}
+template <typename real>
+int launch_quad(const Lattice& L, const double* u, const double* m, const double* p, const double* mhat,
+                real* quad, uint32_t* status, cudaStream_t s) {
+  return mhat ? launch_quad_as<real, true>(L, u, m, p, mhat, quad, status, s)
+              : launch_quad_as<real, false>(L, u, m, p, nullptr, quad, status, s);
+}
+}  // namespace
+
 int hm_launch_quad(const Lattice& L, const double* u, const double* m, const double* p,
                    int precision, void* quad, uint32_t* status, void* stream, const double* mhat) {
-  const int blocks = grid1(L.ne, 8);
-  if (precision == HM_FP32)
-    k_quad<float><<<blocks, 216, 0, S_(stream)>>>(L, u, m, p, mhat, (float*)quad, status);
-  else
-    k_quad<double><<<blocks, 216, 0, S_(stream)>>>(L, u, m, p, mhat, (double*)quad, status);
-  return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
+  if (precision == HM_FP32) return launch_quad<float>(L, u, m, p, mhat, static_cast<float*>(quad), status, S_(stream));
+  return launch_quad<double>(L, u, m, p, mhat, static_cast<double*>(quad), status, S_(stream));
 }
 
 int hm_launch_jacobian_prepare(const Lattice& L, const void* quad, int quad_precision, void* jac,
@@ -319,10 +436,16 @@ int hm_launch_ess_take_b(const Lattice& L, const uint8_t* ess, const double* b, 
 
 int hm_launch_diag_A(const Lattice& L, const void* quad, int precision, const uint8_t* ess,
                      double* diag, void* stream) {
+  DiagTab tab;
+  const double h[3] = {L.hx, L.hy, L.hz};
+  for (int d = 0; d < 3; ++d)
+    for (int q = 0; q < 3; ++q)
+      for (int a = 0; a < 3; ++a) tab.d2[d][q][a] = dbq(q, a) * dbq(q, a) / (h[d] * h[d]);
+  const int blocks = ((L.nx + kDiagX - 1) / kDiagX) * ((L.ny + kDiagY - 1) / kDiagY) * ((L.nz + kDiagZ - 1) / kDiagZ);
   if (precision == HM_FP32)
-    k_diag_A<float><<<grid1(L.ndof, 256), 256, 0, S_(stream)>>>(L, (const float*)quad, ess, diag);
+    k_diag_A<float><<<blocks, 256, 0, S_(stream)>>>(L, tab, (const float*)quad, ess, diag);
   else
-    k_diag_A<double><<<grid1(L.ndof, 256), 256, 0, S_(stream)>>>(L, (const double*)quad, ess, diag);
+    k_diag_A<double><<<blocks, 256, 0, S_(stream)>>>(L, tab, (const double*)quad, ess, diag);
   return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
 }
 
