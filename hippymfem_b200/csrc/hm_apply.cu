@@ -50,7 +50,7 @@ enum ApplyIn { IN_CLEAN = 0, IN_ESS = 1 };
 // what is done with a node's product: y = A x (x itself on the Dirichlet nodes), a pass of
 // the smoother (HmChebMode), or an assembled vector, y = A x - f int phi (0 on the Dirichlet
 // nodes)
-enum ApplyOut { OUT_Y = 0, OUT_R = 1, OUT_STEP1 = 2, OUT_START = 3, OUT_NEXT = 4, OUT_VEC = 5 };
+enum ApplyOut { OUT_Y = 0, OUT_R = 1, OUT_STEP1 = 2, OUT_START = 3, OUT_NEXT = 4, OUT_VEC = 5, OUT_POWER = 6 };
 
 // the constant of HmCheb's kChebMax (cheb[1 + k]: c1_k, cheb[1 + kChebMax + k]: c2_k)
 constexpr int kChebMax = 40;
@@ -394,7 +394,7 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
     }
     // the input at the own nodes, the smoother's operands
     real xc[8];
-    double bn[OUT == OUT_Y || OUT == OUT_VEC ? 1 : 8], gn[OUT == OUT_Y || OUT == OUT_R || OUT == OUT_VEC ? 1 : 8], xn[OUT == OUT_NEXT ? 8 : 1];
+    double bn[OUT == OUT_Y || OUT == OUT_VEC || OUT == OUT_POWER ? 1 : 8], gn[OUT == OUT_Y || OUT == OUT_R || OUT == OUT_VEC ? 1 : 8], xn[OUT == OUT_NEXT ? 8 : 1];
     unsigned fixed = 0;
 #pragma unroll
     for (int h = 0; h < 8; ++h) {
@@ -403,7 +403,7 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
       if constexpr (OUT == OUT_NEXT) {
         bn[h] = !on ? 0.0 : a.c.first ? __ldg(a.c.b + node) : (double)a.c.r[node];
         xn[h] = !on || a.c.first ? 0.0 : (double)a.c.x[node];
-      } else if constexpr (OUT != OUT_Y && OUT != OUT_VEC) {
+      } else if constexpr (OUT != OUT_Y && OUT != OUT_VEC && OUT != OUT_POWER) {
         bn[h] = on ? __ldg(a.c.b + node) : 0.0;
       }
       if constexpr (OUT != OUT_Y && OUT != OUT_R && OUT != OUT_VEC) gn[h] = on ? __ldg(a.c.idiag + node) : 0.0;
@@ -458,6 +458,8 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
               v -= a.f * (phi_1d(2 * cx + (k & 1), L.nx, L.hx) * phi_1d(2 * cy + (k >> 1), L.ny, L.hy) *
                           phi_1d(2 * cz + a3, L.nz, L.hz));
             a.y[node] = (vec)(fx ? 0.0 : v);
+          } else if constexpr (OUT == OUT_POWER) {
+            a.y[node] = (vec)(fx ? 0.0 : acc * gn[h]);
           } else {
             const double in = (double)xc[h];
             const double ri = bn[h] - (fx ? in : acc);
@@ -490,7 +492,7 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
     }
   }
   copy_wait<0>();
-  if (OUT != OUT_R && OUT != OUT_START && OUT != OUT_VEC && a.part != nullptr) {
+  if (OUT != OUT_R && OUT != OUT_START && OUT != OUT_VEC && OUT != OUT_POWER && a.part != nullptr) {
     __shared__ double sh[32];
     const double t = block_sum(dot, sh);
     if (tid == 0) a.part[blockIdx.x] = t;
@@ -994,6 +996,14 @@ int hm_launch_apply_A_dot(const Lattice& L, void* jac, int precision, const uint
 int hm_launch_apply_A_clean(const Lattice& L, void* jac, const uint8_t* ess, const double* x,
                             double* y, void* stream) {
   return apply_y<double>(L, jac, ess, x, y, true, nullptr, nullptr, nullptr, stream);
+}
+
+// y = D^-1 A x, x zero on the Dirichlet nodes: a step of the power iteration
+int hm_launch_power(const Lattice& L, void* jac, const uint8_t* ess, const double* idiag, const double* x,
+                    double* y, void* stream) {
+  ApplyArgs<double, double> a{};
+  a.ess = ess; a.x = x; a.y = y; a.c.idiag = idiag;
+  return launch<double, double, double, IN_CLEAN, OUT_POWER>(L, jac, a, stream);
 }
 
 int hm_launch_apply_A32(const Lattice& L, void* jac32, const uint8_t* ess, const float* x,

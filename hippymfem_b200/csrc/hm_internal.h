@@ -96,6 +96,9 @@ struct HmCheb {
 };
 template <typename T>
 int hm_launch_cheb(const hm::Lattice& L, void* jac, const uint8_t* ess, const HmCheb<T>& c, void* stream);
+// y = D^-1 A x, x zero on the Dirichlet nodes (a step of the set-up's power iteration)
+int hm_launch_power(const hm::Lattice& L, void* jac, const uint8_t* ess, const double* idiag, const double* x,
+                    double* y, void* stream);
 // Inside the MG-PCG: where the level-0 smoother's first direction d = r idiag / theta is
 // wanted (d64 or d32; both null: nowhere), formed by the kernel that forms r
 struct HmFirstDir {

@@ -19,10 +19,12 @@
 // written in FP64, the CG around it unchanged).  Deterministic, and free of host
 // synchronisation after set-up, so a CG iteration with its V-cycle can be captured as a
 // CUDA graph.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <new>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "hm_common.cuh"
@@ -784,8 +786,7 @@ __global__ void __launch_bounds__(kTailThreads) k_mg_tail(const __grid_constant_
   cluster_sync();        // no CTA leaves while another reads its shared memory
 }
 
-// set-up: a deterministic pseudo-random start vector (0 on the boundary), partial sums of
-// a.b, and v = w / (s * diag)
+// set-up: a deterministic pseudo-random start vector (0 on the boundary)
 __global__ void k_mg_seed(MGLevel lv, double* __restrict__ v) {
   const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= lv.nodes) return;
@@ -796,69 +797,45 @@ __global__ void k_mg_seed(MGLevel lv, double* __restrict__ v) {
   h ^= h >> 31; h *= 0xBF58476D1CE4E5B9ull; h ^= h >> 29;
   v[n] = on_boundary(i, j, k, lv.Nx, lv.Ny, lv.Nz) ? 0.0 : (double)(h >> 11) * 0x1.0p-53 - 0.5;
 }
-__global__ void __launch_bounds__(256) k_mg_dot(int64_t n, const double* __restrict__ a,
-                                                const double* __restrict__ b,
-                                                const double* __restrict__ w,
-                                                double* __restrict__ part) {
-  __shared__ double sh[32];
-  double s = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    s = fma(a[i] * (w ? w[i] : 1.0), b[i], s);
-  s = block_sum(s, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+// A step of the power iteration on a Q1 level, y = D^-1 A x (0 on the boundary)
+__global__ void __launch_bounds__(256) k_q1_power(MGLevel lv, Q1Entries<double> K, const double* __restrict__ x,
+                                                  double* __restrict__ y) {
+  const unsigned n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n < (unsigned)lv.nodes) y[n] = q1_row(lv, K, x, n) * lv.idiag[n];
 }
-// partials of v.w, v.diag.v and w.w (slots 0, 1, 2)
-__global__ void __launch_bounds__(256) k_mg_dot3(int64_t n, const double* __restrict__ v,
-                                                 const double* __restrict__ w,
-                                                 const double* __restrict__ diag,
-                                                 double* __restrict__ part) {
+// The Rayleigh quotient lambda = v.w / v.diag.v of w = A v, and from it the Chebyshev
+// coefficients of the interval [hi / lo_div, hi], hi = 1.1 lambda (the last block; lambda
+// is 0 where the quotient is not defined).  part holds two sums a block.
+__global__ void __launch_bounds__(256) k_mg_interval(int64_t n, const double* __restrict__ v,
+                                                     const double* __restrict__ w,
+                                                     const double* __restrict__ diag, double* __restrict__ part,
+                                                     unsigned* __restrict__ counter, double lo_div, int degree,
+                                                     double* __restrict__ cheb) {
   __shared__ double sh[32];
-  double a = 0.0, b = 0.0, c = 0.0;
+  double a = 0.0, b = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double vi = v[i], wi = w[i];
-    a = fma(vi, wi, a);
+    const double vi = v[i];
+    a = fma(vi, w[i], a);
     b = fma(vi * diag[i], vi, b);
-    c = fma(wi, wi, c);
   }
   a = block_sum(a, sh);
   b = block_sum(b, sh);
-  c = block_sum(c, sh);
   if (threadIdx.x == 0) {
     part[blockIdx.x] = a;
-    part[kMGBlocks + blockIdx.x] = b;
-    part[2 * kMGBlocks + blockIdx.x] = c;
+    part[gridDim.x + blockIdx.x] = b;
   }
-}
-// eig[0] = v.Av / v.Dv (kept while the iteration is defined), eig[1] = 1 / |w|
-__global__ void k_mg_eig_step(const double* __restrict__ part, double* __restrict__ eig) {
-  __shared__ double sh[32];
-  double v[3];
-  for (int q = 0; q < 3; ++q) {
-    double t = 0.0;
-    for (int b = threadIdx.x; b < kMGBlocks; b += blockDim.x) t += part[q * kMGBlocks + b];
-    v[q] = block_sum(t, sh);
+  if (!last_block(counter)) return;
+  a = b = 0.0;
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
+    a += __ldcg(part + i);
+    b += __ldcg(part + gridDim.x + i);
   }
-  if (threadIdx.x == 0) {
-    if (v[1] > 0.0 && v[2] > 0.0 && isfinite(v[0] / v[1])) {
-      eig[0] = v[0] / v[1];
-      eig[1] = 1.0 / sqrt(v[2]);
-    } else {
-      eig[1] = 0.0;
-    }
-  }
-}
-__global__ void k_mg_scale_div(int64_t n, const double* __restrict__ w, const double* __restrict__ diag,
-                               const double* __restrict__ eig, double* __restrict__ v) {
-  const double s = eig[1];
-  if (s == 0.0) return;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    v[i] = s * w[i] / diag[i];
-}
-// the Chebyshev coefficients of the interval [hi / lo_div, hi], hi = 1.1 lambda
-__global__ void k_mg_cheb_coeffs(const double* __restrict__ eig, double lo_div, int degree,
-                                 double* __restrict__ cheb) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const double hi = 1.1 * eig[0], lo = hi / lo_div;
+  a = block_sum(a, sh);
+  b = block_sum(b, sh);
+  if (threadIdx.x != 0) return;
+  *counter = 0u;
+  const double lambda = b > 0.0 && isfinite(a / b) ? a / b : 0.0;
+  const double hi = 1.1 * lambda, lo = hi / lo_div;
   const double theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo), sigma = theta / delta;
   double rho_old = 1.0 / sigma;
   cheb[0] = theta;
@@ -1391,26 +1368,34 @@ extern "C" int hm_mg_setup(hm_mg* mg, void* jac, const uint8_t* ess, const doubl
   for (int l = 0; l < mg->nlev; ++l)
     k_recip<<<blocks_for(mg->lv[l].nodes), 256, 0, s>>>(mg->lv[l].nodes, mg->lv[l].diag,
                                                         mg->lv[l].idiag);
-  // largest eigenvalue of D^{-1} A per level, on the device: power iteration with the
-  // Rayleigh quotient v.Av / v.Dv (10 steps from a fixed start); smoothing interval
-  // [hi/4, hi], the coarsest level's solve on [hi/64, hi]
+  // largest eigenvalue of D^{-1} A per level, on the device: nine steps of the power
+  // iteration from a fixed start, unscaled (a step grows the vector by the eigenvalue at
+  // most, and that is below 27, the most nodes an element couples), each one launch, then
+  // the Rayleigh quotient v.Av / v.Dv; smoothing interval [hi/4, hi], the coarsest level's
+  // solve on [hi/64, hi].  (With the scaling, and a quotient at each of ten steps, a step
+  // took four launches: 2.3 ms of 16.3 of the two forward solves on 64^3 elements.)
   double* part = mg->scratch;
-  double* eig = mg->scratch + 3 * kMGBlocks;
+  unsigned* counter = reinterpret_cast<unsigned*>(mg->scratch + 3 * kMGBlocks);
+  if (cudaMemsetAsync(counter, 0, sizeof(unsigned), s) != cudaSuccess) return HM_ERR_CUDA;
   for (int l = 0; l < mg->nlev; ++l) {
     MGLevel& lv = mg->lv[l];
     double* v = lv.d;
     double* w = lv.t;
     k_mg_seed<<<blocks_for(lv.nodes), 256, 0, s>>>(lv, v);
-    if (cudaMemsetAsync(eig, 0, 2 * sizeof(double), s) != cudaSuccess) return HM_ERR_CUDA;
-    for (int it = 0; it < 10; ++it) {
-      const int rc = apply_level(mg, l, v, w, true, s);   // v is zero on the boundary
-      if (rc) return rc;
-      k_mg_dot3<<<kMGBlocks, 256, 0, s>>>(lv.nodes, v, w, lv.diag, part);
-      k_mg_eig_step<<<1, 256, 0, s>>>(part, eig);
-      k_mg_scale_div<<<kMGBlocks, 256, 0, s>>>(lv.nodes, w, lv.diag, eig, v);
+    for (int it = 0; it < 9; ++it) {                    // v is zero on the boundary
+      if (l == 0) {
+        const int rc = hm_launch_power(L, jac, ess, lv.idiag, v, w, stream);
+        if (rc) return rc;
+      } else {
+        k_q1_power<<<blocks_for(lv.nodes), 256, 0, s>>>(lv, Q1Entries<double>(lv), v, w);
+      }
+      std::swap(v, w);
     }
+    const int rc = apply_level(mg, l, v, w, true, s);
+    if (rc) return rc;
     const bool coarsest = l == mg->nlev - 1;
-    k_mg_cheb_coeffs<<<1, 32, 0, s>>>(eig, coarsest ? 64.0 : 4.0, lv.degree, lv.cheb);
+    k_mg_interval<<<std::min<int64_t>(blocks_for(lv.nodes), kMGBlocks), 256, 0, s>>>(
+        lv.nodes, v, w, lv.diag, part, counter, coarsest ? 64.0 : 4.0, lv.degree, lv.cheb);
     if (coarsest && lv.cinv) k_coarse_factor<<<1, 256, 0, s>>>(lv);
   }
   if (mg->single) refresh_single(mg, s);
