@@ -108,17 +108,12 @@ __global__ void k_pattern_tpos(Lattice L, const int32_t* __restrict__ indptr,
 // the stores follow with a thread a point.
 // Bound: the stores, 1728 bytes an element (68 us at 64^3 elements at the copy rate), with
 // the FP64 pipe close behind (65), in three phases that only other blocks overlap.  64^3
-// elements: 342 us with a thread a point, 186 here; 45 x 52 x 39 120 and 66, 32^3 46 and 25,
-// 4^3 3.5 and 2.9.  One set of nine threads for the three fields takes 171 at 64^3 but 4.5
+// elements: 342 us with a thread a point, 189 here; 45 x 52 x 39 120 and 67, 32^3 46 and 26,
+// 4^3 3.5 and 3.2.  One set of nine threads for the three fields takes 171 at 64^3 but 4.5
 // at 4^3 (the longer chain); 16 elements a block 238, six blocks an SM (spills) 237.
 constexpr int kQuadElems = 8;
 constexpr int kQuadThreads = 27 * kQuadElems;
 constexpr int kQuadBlocks = 5;
-// the 1D derivative tables by point and node, divided by the element's edge
-template <typename real>
-struct QuadTab {
-  real d[3][3][3];
-};
 
 // The contractions of a field's nodal values x along y and z at a line's (q2, q3): values,
 // and with GRAD derivatives along y and along z, at the three nodes along x.
@@ -149,20 +144,19 @@ __device__ __forceinline__ void quad_line(const real* x, const real (&b2)[3], co
 
 template <typename real, bool MHAT>
 __global__ void __launch_bounds__(kQuadThreads, kQuadBlocks)
-    k_quad(Lattice L, const __grid_constant__ QuadTab<real> tab, const double* __restrict__ u,
+    k_quad(Lattice L, const double* __restrict__ u,
            const double* __restrict__ m, const double* __restrict__ p, const double* __restrict__ mhat,
            real* __restrict__ quad, uint32_t* __restrict__ status) {
   constexpr int NF = MHAT ? 4 : 3;
   __shared__ real sx[NF][kQuadElems][27];                // m, u, p, mhat
   __shared__ real sg[7][kQuadElems][27];                 // D, grad u, grad p at the points
-  __shared__ real sb[3][3], sd[2][3][3];
+  __shared__ real sb[3][3], sd[3][3];
   const int tid = threadIdx.x;
   const int64_t e0 = blockIdx.x * (int64_t)kQuadElems;
   const int count = (int)min((int64_t)kQuadElems, L.ne - e0);
   if (tid < 9) {
     sb[tid / 3][tid % 3] = (real)bq(tid / 3, tid % 3);
-    sd[0][tid / 3][tid % 3] = tab.d[1][tid / 3][tid % 3];
-    sd[1][tid / 3][tid % 3] = tab.d[2][tid / 3][tid % 3];
+    sd[tid / 3][tid % 3] = (real)dbq(tid / 3, tid % 3);
   }
   const int pe = tid / 27, a = tid - pe * 27;            // the thread's element as a node or a point
   if (pe < count) {
@@ -183,7 +177,7 @@ __global__ void __launch_bounds__(kQuadThreads, kQuadBlocks)
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       b2[k] = sb[q2][k]; b3[k] = sb[q3][k];
-      d2[k] = sd[0][q2][k]; d3[k] = sd[1][q3][k];
+      d2[k] = sd[q2][k]; d3[k] = sd[q3][k];
     }
     if (f == 0) {
       const double w23 = (q2 == 1 ? wq(1) : wq(0)) * (q3 == 1 ? wq(1) : wq(0)) * L.hx * L.hy * L.hz;
@@ -203,18 +197,21 @@ __global__ void __launch_bounds__(kQuadThreads, kQuadBlocks)
       }
     } else {
       quad_line<true>(sx[f][le], b2, d2, b3, d3, bb, bd, dz);
+      // scaled after the contractions: a derivative table's entries cancel exactly on a
+      // constant field, divided by the edge they would not
+      const real ihx = (real)(1.0 / L.hx), ihy = (real)(1.0 / L.hy), ihz = (real)(1.0 / L.hz);
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         real gx = 0, gy = 0, gz = 0;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          gx = fma(tab.d[0][q][k], bb[k], gx);
+          gx = fma((real)dbq(q, k), bb[k], gx);
           gy = fma((real)bq(q, k), bd[k], gy);
           gz = fma((real)bq(q, k), dz[k], gz);
         }
-        sg[3 * f - 2][le][3 * line + q] = gx;
-        sg[3 * f - 1][le][3 * line + q] = gy;
-        sg[3 * f][le][3 * line + q] = gz;
+        sg[3 * f - 2][le][3 * line + q] = gx * ihx;
+        sg[3 * f - 1][le][3 * line + q] = gy * ihy;
+        sg[3 * f][le][3 * line + q] = gz * ihz;
       }
     }
   }
@@ -381,22 +378,13 @@ int hm_launch_tpos(const Lattice& L, const int32_t* indptr, int32_t* tpos, void*
 }
 
 namespace {
-template <typename real, bool MHAT>
-int launch_quad_as(const Lattice& L, const double* u, const double* m, const double* p, const double* mhat,
-                   real* quad, uint32_t* status, cudaStream_t s) {
-  QuadTab<real> tab;
-  const double h[3] = {L.hx, L.hy, L.hz};
-  for (int d = 0; d < 3; ++d)
-    for (int q = 0; q < 3; ++q)
-      for (int a = 0; a < 3; ++a) tab.d[d][q][a] = (real)(dbq(q, a) / h[d]);
-  k_quad<real, MHAT><<<grid1(L.ne, kQuadElems), kQuadThreads, 0, s>>>(L, tab, u, m, p, mhat, quad, status);
-  return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
-}
 template <typename real>
 int launch_quad(const Lattice& L, const double* u, const double* m, const double* p, const double* mhat,
                 real* quad, uint32_t* status, cudaStream_t s) {
-  return mhat ? launch_quad_as<real, true>(L, u, m, p, mhat, quad, status, s)
-              : launch_quad_as<real, false>(L, u, m, p, nullptr, quad, status, s);
+  const int blocks = grid1(L.ne, kQuadElems);
+  if (mhat) k_quad<real, true><<<blocks, kQuadThreads, 0, s>>>(L, u, m, p, mhat, quad, status);
+  else k_quad<real, false><<<blocks, kQuadThreads, 0, s>>>(L, u, m, p, nullptr, quad, status);
+  return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
 }
 }  // namespace
 
