@@ -61,7 +61,7 @@ struct hm_mg {
   void* jac;             // level-0 operator data (FP64, from hm_lattice_jacobian_prepare)
   const uint8_t* ess;
   int degree, coarse_degree;
-  double* scratch;       // partial sums of the set-up's inner products, eigenvalue state
+  double* scratch;       // partial sums of the set-up's inner products, their counter
   const uint8_t* checked_ess;   // the markers last found to be the whole boundary
   int tail_first;        // first level of the one-launch tail (nlev: none)
   int64_t tail_nodes;    // its levels' nodes at most
@@ -860,8 +860,8 @@ template <typename T> MGLevelT<T>* levels_of(hm_mg* mg);
 template <> MGLevelT<double>* levels_of<double>(hm_mg* mg) { return mg->lv; }
 template <> MGLevelT<float>* levels_of<float>(hm_mg* mg) { return mg->lv32; }
 
-// clean: x is zero on the Dirichlet nodes (the level-0 element pass then skips the
-// markers); every vector of a cycle is when its right-hand side is
+// clean: x is zero on the Dirichlet nodes (the level-0 operator pass then skips
+// the markers); every vector of a cycle is when its right-hand side is
 template <typename T>
 int apply_level(hm_mg* mg, int l, const T* x, T* y, bool clean, cudaStream_t s) {
   if (l == 0) {

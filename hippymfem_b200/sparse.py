@@ -68,8 +68,7 @@ class CSRBlock:
 class MatrixFreeJacobian:
     """The Jacobian ``A(m)`` applied from the quadrature data of a point, with its
     elimination (``apply_ij_at`` for the (ADJOINT, STATE) pair).  Keeps the operator's
-    data (D of the point in the layout the operator streams, plus its scratch); applies
-    that share one instance must run in one stream."""
+    data (D of the point in the layout the operator streams), which applies only read."""
 
     def __init__(self, mesh, quad, ess_marker, precision=_lib.HM_FP64, stream=None,
                  quad_precision=None):
@@ -416,7 +415,7 @@ class Multigrid:
         return z
 
     def set_tail_nodes(self, max_nodes):
-        """Levels of at most ``max_nodes`` nodes run as one CTA-wide kernel (0: none)."""
+        """Levels of at most ``max_nodes`` nodes run in one cluster launch (0: none)."""
         check(lib.hm_mg_set_tail_nodes(self._mg, int(max_nodes)), "hm_mg_set_tail_nodes")
         return self
 

@@ -158,9 +158,9 @@ int hm_lattice_add_boundary_mass(const hm_lattice* h, double beta, double* d_val
  * (u, m, p), or with d_mhat != NULL the second-order products along mhat (D = w|J| e^m
  * mhat, no source: ADJOINT C mhat, STATE W_um mhat, PARAMETER W_mm mhat, rows not
  * eliminated) -- the vectors hm_lattice_quadrature(_dir) + hm_lattice_assemble give,
- * summed in another fixed order (equal to rounding; deterministic).  One pass evaluates
- * the fields at each element's 27 points and contracts its element vectors, a node
- * gather sums them; the replacement of element_vectors + assemble_vector
+ * summed in another fixed order (equal to rounding; deterministic).  One pass forms D at
+ * each element's 27 points, one launch of tile-marching passes the vectors; the
+ * replacement of element_vectors + assemble_vector
  * (hippymfem/fem/kernel.py:2070-2078, fem/pattern.py:1186-1233) and of the directional
  * products of apply_ij_at (modeling/PDEVariationalProblem.py:1672).  With
  * zero_ess_vectors the STATE and ADJOINT vectors are zeroed on d_ess.  d_work:
@@ -190,8 +190,8 @@ int hm_lattice_vectors_at(const hm_lattice* h, const double* d_u, const double* 
  * d_ess, y = x there): the product apply_ij_at gives for (ADJOINT, STATE)
  * (modeling/PDEVariationalProblem.py:1672).  Its data d_jac (hm_lattice_jacobian_bytes)
  * holds D of the point in a layout the operator streams, filled once per point by
- * hm_lattice_jacobian_prepare from the quadrature data, and the operator's own scratch:
- * two applies with the same d_jac must not overlap on the GPU. */
+ * hm_lattice_jacobian_prepare from the quadrature data and only read by an apply (a part
+ * of the array stays unused). */
 int64_t hm_lattice_jacobian_bytes(const hm_lattice* h, int precision);
 int hm_lattice_jacobian_prepare(const hm_lattice* h, const void* d_quad, int quad_precision,
                                 void* d_jac, int precision, void* stream);
@@ -390,24 +390,23 @@ int hm_mg_setup(hm_mg* mg, void* d_jac64, const uint8_t* d_ess, const double* d_
                 void* stream);
 int hm_mg_apply(hm_mg* mg, const double* d_r, double* d_z, void* stream);
 int hm_mg_levels(const hm_mg* mg);
-/* The Q1 levels with at most max_nodes nodes (1000 by default; 0: none) run as one
- * CTA-wide kernel per cycle instead of level by level (the same arithmetic, node for
- * node; one launch instead of ~14 per level).  Set it before a plan's first solve: a
- * plan's captured iteration batches keep the launches they were captured with. */
+/* The Q1 levels with at most max_nodes nodes (5000 by default; 0: none) run in one launch
+ * per cycle, a cluster of thread blocks with the levels' vectors in its shared memory,
+ * instead of level by level (the same arithmetic, node for node), as far as the levels fit.
+ * Set it before a plan's first solve: a plan's captured iteration batches keep the launches
+ * they were captured with. */
 int hm_mg_set_tail_nodes(hm_mg* mg, int64_t max_nodes);
-/* With smoothing degree 1 (the default from a million dofs up) each smoothing step runs
- * as one pass with its level's operator: on level 0 inside the solves (every vector
- * zero on the Dirichlet nodes) the Q2 operator's two kernels carry the Chebyshev update,
- * on the Q1 levels one kernel does both; the arithmetic is the step-by-step one, bit for
- * bit (fused = 1, the default).  fused = 0 launches the steps one by one.  Set it before
- * a plan's first solve, as the tail. */
+/* Each smoothing step runs as one pass with its level's operator, on level 0 inside the
+ * solves (every vector zero on the Dirichlet nodes) and on the Q1 levels; at degree 1 the
+ * arithmetic is the step-by-step one, bit for bit (fused = 1, the default).  fused = 0
+ * launches the steps one by one.  Set it before a plan's first solve, as the tail. */
 int hm_mg_set_fused(hm_mg* mg, int fused);
 /* The cycle in FP32 (d_work32 of hm_mg_single_workspace_bytes), or in FP64 again
  * (d_work32 = NULL, the default).  The set-up stays FP64; each set-up (and this call,
  * after one, on `stream`) rounds the point's D, the coarse coefficients, the reciprocal
  * diagonals and the coarse inverse to FP32 copies.  r and z of hm_mg_apply stay FP64;
- * with fused degree-1 smoothing inside the solves the level-0 passes read the FP64
- * residual and write the FP64 result themselves.  A preconditioner of the FP64 CG
+ * with fused smoothing inside the solves the level-0 passes read the FP64 residual and
+ * write the FP64 result themselves.  A preconditioner of the FP64 CG
  * (hm_pcg_mg, plans): the recurrence, its inner products and the stopping test are
  * unchanged, so a solve meets the same tolerance.  With it the CG takes a
  * Polak-Ribiere-type step (beta = r+.(z+ - z) / r.z), the cycle being symmetric only to
