@@ -1045,11 +1045,21 @@ int hm_launch_beta(const Lattice& L, const double* b, const double* z, const HmB
 }
 
 // The assembled vectors from the fields.  D: storage of at least 27 ne doubles (54 ne for
-// its 16-byte pitch where nx is odd), work_reals of them; outs: ADJOINT, STATE, PARAMETER
-// (NULL: skip).  With skip nonzero on the device nothing is done.
+// its 16-byte pitch where nx is odd), work_reals of them, 27 ne a vector at least; outs:
+// ADJOINT, STATE, PARAMETER (NULL: skip).  With skip nonzero on the device nothing is done.
 int hm_launch_vectors(const Lattice& L, const double* u, const double* m, const double* p,
                       const double* mhat, double f, const uint8_t* zero_ess, double* const outs[3],
                       double* D, int64_t work_reals, uint32_t* status, const uint32_t* skip, void* stream) {
+  // The passes write nodes while other tiles, and the other vectors' passes, still read u and
+  // p: an output that overlaps either takes the element route.
+  auto overlaps = [&](const double* out, const double* x) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(out), b = reinterpret_cast<uintptr_t>(x);
+    const uintptr_t bytes = sizeof(double) * (uintptr_t)L.ndof;
+    return a < b + bytes && b < a + bytes;
+  };
+  for (int i = 0; i < 3; ++i)
+    if (outs[i] && (overlaps(outs[i], u) || overlaps(outs[i], p)))
+      return hm_launch_elem_vectors(L, u, m, p, mhat, f, zero_ess, outs, D, status, skip, stream);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   int pitch = hm_jac_pitch(L, HM_FP64);
   if (27 * (int64_t)pitch * L.ny * L.nz > work_reals) pitch = L.nx;

@@ -47,6 +47,10 @@ int hm_launch_apply_A_clean(const hm::Lattice& L, void* jac, const uint8_t* ess,
 int hm_launch_vectors(const hm::Lattice& L, const double* u, const double* m, const double* p,
                       const double* mhat, double f, const uint8_t* zero_ess, double* const outs[3],
                       double* D, int64_t work_reals, uint32_t* status, const uint32_t* skip, void* stream);
+// the same by the element route, whose outputs may overlap the fields (hm_lattice.cu)
+int hm_launch_elem_vectors(const hm::Lattice& L, const double* u, const double* m, const double* p,
+                           const double* mhat, double f, const uint8_t* zero_ess, double* const outs[3],
+                           double* work, uint32_t* status, const uint32_t* skip, void* stream);
 // x = b on the Dirichlet nodes
 int hm_launch_ess_take_b(const hm::Lattice& L, const uint8_t* ess, const double* b, double* x,
                          void* stream);

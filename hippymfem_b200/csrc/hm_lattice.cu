@@ -4,6 +4,8 @@
 //                   transpose map of a Q2 x Q2 block, arithmetically
 //   k_quad          pointwise data D, E = D grad u, F = D grad p, W = D grad u.grad p
 //   k_extract_D     the matrix-free Jacobian's data (its apply is in hm_apply.cu)
+//   k_elem_vectors, the assembled vectors by element results and a gather, for outputs that
+//   k_node_gather   overlap the fields (the others are in hm_apply.cu)
 // (the fused assembly k_tile_assemble is in hm_tile.cu)
 #include <cstdio>
 
@@ -496,8 +498,229 @@ extern "C" int hm_lattice_residual_noalloc(const hm_lattice* h, const double* d_
 // dR/dp (ADJOINT, with the source -f w|J| phi), dR/du (STATE) and dR/dm (PARAMETER) of the
 // point (u, m, p) -- or, with mhat, the second-order products along mhat (D = w|J| e^m
 // mhat, f = 0) -- without the pointwise-data array: D at the points, then a pass per vector
-// (hm_apply.cu).
+// (hm_apply.cu); or the element route below, which reads every field before it writes any
+// vector: one pass evaluates the fields at the element's 27 points and contracts the
+// element vectors (written as Ye[a][e] into the workspace), the node gather sums them per
+// node in a fixed order.
 namespace hm {
+// Element vectors Ye[a][e] to nodes.  One thread per pair of x-neighbours (2m, 2m+1) of a
+// node row (the row's last node, 2n, alone), so that every lane of a warp runs the same
+// loop: node 2m takes element m-1 (local a1 = 2) and m (a1 = 0), node 2m+1 element m
+// (a1 = 1); consecutive lanes read consecutive elements of each Ye plane.  Per node the
+// contributions are summed over (z, y, x) element pairs with the lower element first, a
+// fixed order.
+__device__ __forceinline__ void axis_elems(int i, int nel, int& e0, int& a0, int& cnt) {
+  if (i & 1) { e0 = i >> 1; a0 = 1; cnt = 1; }
+  else if (i == 0) { e0 = 0; a0 = 0; cnt = 1; }
+  else if ((i >> 1) >= nel) { e0 = (i >> 1) - 1; a0 = 2; cnt = 1; }
+  else { e0 = (i >> 1) - 1; a0 = 2; cnt = 2; }   // elements i/2-1 (a=2), i/2 (a=0)
+}
+
+__global__ void __launch_bounds__(256)
+    k_node_gather(Lattice L, const double* __restrict__ Ye, const uint8_t* __restrict__ zero,
+                  double* __restrict__ yout, const uint32_t* __restrict__ skip) {
+  if (skip != nullptr && *skip != 0u) return;    // the whole launch stands down
+  const unsigned per_row = (unsigned)L.nx + 1u;                  // pairs + the last node
+  const unsigned rows = (unsigned)L.Ny * (unsigned)L.Nz;
+  const unsigned task = blockIdx.x * blockDim.x + threadIdx.x;
+  if (task >= rows * per_row) return;
+  const unsigned row = task / per_row;
+  const unsigned m = task - row * per_row;
+  const unsigned iz = row / (unsigned)L.Ny, iy = row - iz * (unsigned)L.Ny;
+  const bool last = m == (unsigned)L.nx;                          // node 2n alone
+  const unsigned n0 = row * (unsigned)L.Nx + 2u * m;              // node 2m
+  int ey0, ay0, cy, ez0, az0, cz;
+  axis_elems((int)iy, L.ny, ey0, ay0, cy);
+  axis_elems((int)iz, L.nz, ez0, az0, cz);
+  const unsigned ne = (unsigned)L.ne, nx = (unsigned)L.nx;
+  // every contribution is loaded before any is added (all twelve loads in flight at
+  // once), then summed in the fixed order (z, y element pairs, lower element first)
+  double v[4][3];
+#pragma unroll
+  for (int c3 = 0; c3 < 2; ++c3)
+#pragma unroll
+    for (int c2 = 0; c2 < 2; ++c2) {
+      const int c = 2 * c3 + c2;
+      const bool on = c3 < cz && c2 < cy;
+      const unsigned a23 = 3u * (unsigned)(c2 ? 0 : ay0) + 9u * (unsigned)(c3 ? 0 : az0);
+      const unsigned erow = nx * ((unsigned)(ey0 + c2) + (unsigned)L.ny * (unsigned)(ez0 + c3));
+      // node 2m: element m-1 (a1 = 2) then element m (a1 = 0); node 2m+1: element m
+      v[c][0] = (on && m > 0) ? Ye[(size_t)(2u + a23) * ne + erow + m - 1u] : 0.0;
+      v[c][1] = (on && !last) ? Ye[(size_t)a23 * ne + erow + m] : 0.0;
+      v[c][2] = (on && !last) ? Ye[(size_t)(1u + a23) * ne + erow + m] : 0.0;
+    }
+  double acc0 = 0, acc1 = 0;
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    if ((c >> 1) < cz && (c & 1) < cy) {
+      if (m > 0) acc0 += v[c][0];
+      if (!last) {
+        acc0 += v[c][1];
+        acc1 += v[c][2];
+      }
+    }
+  yout[n0] = zero != nullptr && zero[n0] ? 0.0 : acc0;
+  if (!last) yout[n0 + 1] = zero != nullptr && zero[n0 + 1] ? 0.0 : acc1;
+}
+
+template <int NV>
+struct VecOut { double* ye[3]; };   // element results: ADJOINT, STATE, PARAMETER (NULL: skip)
+
+// Sum factorisation on the element's 3 x 3 x 3 nodes and points: nodes -> points one
+// axis at a time (x, y, z), the pointwise data at the 27 points, then points -> nodes
+// (z, y, x) for the three element vectors.  One CTA holds 8 elements, a thread per
+// (element, index); every stage reads the previous one's arrays in shared memory.
+//   evaluation   X: B u, B' u, B p, B' p, B m, B mhat        (index q1 + 3 a2 + 9 a3)
+//                Y: u: BB, BB', B'B;  p: the same;  m, mhat: BB  (q1 + 3 q2 + 9 a3)
+//                Z: grad u, grad p, m, mhat at the point      (q1 + 3 q2 + 9 q3)
+//   integration  Z: E_x B, E_y B, E_z B' + s B | F_x B, F_y B, F_z B' | W B
+//                Y: (.) B, (.) B' + (.) B per vector        (q1 + 3 a2 + 9 a3)
+//                X: B' (.) + B (.)                          (a1 + 3 a2 + 9 a3)
+// with the 1/h of each derivative folded in at its z sums.
+__device__ __forceinline__ double b1d(int q, int a) { return bq(q, a); }
+__device__ __forceinline__ double d1d(int q, int a) { return dbq(q, a); }
+
+__global__ void __launch_bounds__(216, 4) k_elem_vectors(Lattice L, const double* __restrict__ u,
+                                                      const double* __restrict__ m,
+                                                      const double* __restrict__ p,
+                                                      const double* __restrict__ mhat, double f,
+                                                      VecOut<3> o, uint32_t* __restrict__ status,
+                                                      const uint32_t* __restrict__ skip) {
+  if (skip != nullptr && *skip != 0u) return;    // the whole launch stands down
+  // per element: arrays of 27, the element's block padded to 11 (mod 16) doubles, so
+  // that the two elements a warp spans fall on different banks
+  constexpr int kV = 4 * 27 + 15, kA = 7 * 27 + 14, kB = 8 * 27 + 3;
+  __shared__ double sv[8][kV];           // node values u, m, p, mhat
+  __shared__ double s1[8][kA];           // evaluation X / integration Z
+  __shared__ double s2[8][kB];           // evaluation Y / integration Y
+  __shared__ double sp[8][kB];           // E(3), F(3), W, source weight at the points
+  const int tid = threadIdx.x, le = tid / 27, i = tid % 27;
+  const int c1 = i % 3, c2 = (i / 3) % 3, c3 = i / 9;   // the thread's three indices
+  const double ihx = 1.0 / L.hx, ihy = 1.0 / L.hy, ihz = 1.0 / L.hz;
+  const double wdet = wq(c1) * wq(c2) * wq(c3) * L.hx * L.hy * L.hz;
+  for (int64_t g0 = blockIdx.x * 8LL; g0 < L.ne; g0 += (int64_t)gridDim.x * 8) {
+    const int64_t e = g0 + le;
+    const bool live = le < 8 && e < L.ne;
+    __syncthreads();                      // the previous group's arrays are consumed
+    if (live) {
+      const int ex = (int)(e % L.nx), ey = (int)((e / L.nx) % L.ny), ez = (int)(e / ((int64_t)L.nx * L.ny));
+      const int64_t node = (2 * ex + c1) + (int64_t)L.Nx * ((2 * ey + c2) + (int64_t)L.Ny * (2 * ez + c3));
+      sv[le][(0) * 27 + i] = u[node];
+      sv[le][(1) * 27 + i] = m[node];
+      sv[le][(2) * 27 + i] = p[node];
+      sv[le][(3) * 27 + i] = mhat ? mhat[node] : 0.0;
+    }
+    __syncthreads();
+    if (live) {   // X: index (q1 = c1, a2 = c2, a3 = c3), sums over a1
+      double r[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+      for (int a1 = 0; a1 < 3; ++a1) {
+        const int j = a1 + 3 * c2 + 9 * c3;
+        const double b = b1d(c1, a1), d = d1d(c1, a1);
+        const double vu = sv[le][(0) * 27 + j], vm = sv[le][(1) * 27 + j], vp = sv[le][(2) * 27 + j], vh = sv[le][(3) * 27 + j];
+        r[0] = fma(b, vu, r[0]); r[1] = fma(d, vu, r[1]);
+        r[2] = fma(b, vp, r[2]); r[3] = fma(d, vp, r[3]);
+        r[4] = fma(b, vm, r[4]); r[5] = fma(b, vh, r[5]);
+      }
+#pragma unroll
+      for (int k = 0; k < 6; ++k) s1[le][(k) * 27 + i] = r[k];
+    }
+    __syncthreads();
+    if (live) {   // Y: index (q1 = c1, q2 = c2, a3 = c3), sums over a2
+      double r[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+      for (int a2 = 0; a2 < 3; ++a2) {
+        const int j = c1 + 3 * a2 + 9 * c3;
+        const double b = b1d(c2, a2), d = d1d(c2, a2);
+        const double x0 = s1[le][(0) * 27 + j], x1 = s1[le][(1) * 27 + j], x2 = s1[le][(2) * 27 + j], x3 = s1[le][(3) * 27 + j];
+        r[0] = fma(b, x0, r[0]); r[1] = fma(b, x1, r[1]); r[2] = fma(d, x0, r[2]);
+        r[3] = fma(b, x2, r[3]); r[4] = fma(b, x3, r[4]); r[5] = fma(d, x2, r[5]);
+        r[6] = fma(b, s1[le][(4) * 27 + j], r[6]); r[7] = fma(b, s1[le][(5) * 27 + j], r[7]);
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) s2[le][(k) * 27 + i] = r[k];
+    }
+    __syncthreads();
+    if (live) {   // Z: the point (c1, c2, c3), sums over a3; then the pointwise data
+      double gu[3] = {0, 0, 0}, gp[3] = {0, 0, 0}, mv = 0.0, mh = 0.0;
+#pragma unroll
+      for (int a3 = 0; a3 < 3; ++a3) {
+        const int j = c1 + 3 * c2 + 9 * a3;
+        const double b = b1d(c3, a3), d = d1d(c3, a3);
+        gu[0] = fma(b, s2[le][(1) * 27 + j], gu[0]); gu[1] = fma(b, s2[le][(2) * 27 + j], gu[1]);
+        gu[2] = fma(d, s2[le][(0) * 27 + j], gu[2]);
+        gp[0] = fma(b, s2[le][(4) * 27 + j], gp[0]); gp[1] = fma(b, s2[le][(5) * 27 + j], gp[1]);
+        gp[2] = fma(d, s2[le][(3) * 27 + j], gp[2]);
+        mv = fma(b, s2[le][(6) * 27 + j], mv); mh = fma(b, s2[le][(7) * 27 + j], mh);
+      }
+      gu[0] *= ihx; gu[1] *= ihy; gu[2] *= ihz;
+      gp[0] *= ihx; gp[1] *= ihy; gp[2] *= ihz;
+      double D = wdet * exp(mv);
+      if (mhat) D *= mh;
+      const double E0 = D * gu[0], E1 = D * gu[1], E2 = D * gu[2];
+      const double F0 = D * gp[0], F1 = D * gp[1], F2 = D * gp[2];
+      const double W = D * (gu[0] * gp[0] + gu[1] * gp[1] + gu[2] * gp[2]);
+      sp[le][(0) * 27 + i] = E0; sp[le][(1) * 27 + i] = E1; sp[le][(2) * 27 + i] = E2;
+      sp[le][(3) * 27 + i] = F0; sp[le][(4) * 27 + i] = F1; sp[le][(5) * 27 + i] = F2;
+      sp[le][(6) * 27 + i] = W;
+      sp[le][(7) * 27 + i] = mhat ? 0.0 : -f * wdet;
+      if (!(isfinite(E0) && isfinite(E1) && isfinite(E2) && isfinite(F0) && isfinite(F1) &&
+            isfinite(F2) && isfinite(W)))
+        atomicOr(status, HM_STATUS_NONFINITE);
+    }
+    __syncthreads();
+    if (live) {   // integration Z: index (q1 = c1, q2 = c2, a3 = c3), sums over q3
+      double r[7] = {0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+      for (int q3 = 0; q3 < 3; ++q3) {
+        const int j = c1 + 3 * c2 + 9 * q3;
+        const double b = b1d(q3, c3), d = d1d(q3, c3);
+        r[0] = fma(b, sp[le][(0) * 27 + j], r[0]);
+        r[1] = fma(b, sp[le][(1) * 27 + j], r[1]);
+        r[2] = fma(d * ihz, sp[le][(2) * 27 + j], fma(b, sp[le][(7) * 27 + j], r[2]));
+        r[3] = fma(b, sp[le][(3) * 27 + j], r[3]);
+        r[4] = fma(b, sp[le][(4) * 27 + j], r[4]);
+        r[5] = fma(d, sp[le][(5) * 27 + j], r[5]);
+        r[6] = fma(b, sp[le][(6) * 27 + j], r[6]);
+      }
+      s1[le][(0) * 27 + i] = r[0] * ihx; s1[le][(1) * 27 + i] = r[1] * ihy; s1[le][(2) * 27 + i] = r[2];
+      s1[le][(3) * 27 + i] = r[3] * ihx; s1[le][(4) * 27 + i] = r[4] * ihy; s1[le][(5) * 27 + i] = r[5] * ihz;
+      s1[le][(6) * 27 + i] = r[6];
+    }
+    __syncthreads();
+    if (live) {   // integration Y: index (q1 = c1, a2 = c2, a3 = c3), sums over q2
+      double r[5] = {0, 0, 0, 0, 0};
+#pragma unroll
+      for (int q2 = 0; q2 < 3; ++q2) {
+        const int j = c1 + 3 * q2 + 9 * c3;
+        const double b = b1d(q2, c2), d = d1d(q2, c2);
+        r[0] = fma(b, s1[le][(0) * 27 + j], r[0]);
+        r[1] = fma(d, s1[le][(1) * 27 + j], fma(b, s1[le][(2) * 27 + j], r[1]));
+        r[2] = fma(b, s1[le][(3) * 27 + j], r[2]);
+        r[3] = fma(d, s1[le][(4) * 27 + j], fma(b, s1[le][(5) * 27 + j], r[3]));
+        r[4] = fma(b, s1[le][(6) * 27 + j], r[4]);
+      }
+#pragma unroll
+      for (int k = 0; k < 5; ++k) s2[le][(k) * 27 + i] = r[k];
+    }
+    __syncthreads();
+    if (live) {   // integration X: the node (a1 = c1, a2 = c2, a3 = c3), sums over q1
+      double ra = 0.0, rs = 0.0, rp = 0.0;
+#pragma unroll
+      for (int q1 = 0; q1 < 3; ++q1) {
+        const int j = q1 + 3 * c2 + 9 * c3;
+        const double b = b1d(q1, c1), d = d1d(q1, c1);
+        ra = fma(d, s2[le][(0) * 27 + j], fma(b, s2[le][(1) * 27 + j], ra));
+        rs = fma(d, s2[le][(2) * 27 + j], fma(b, s2[le][(3) * 27 + j], rs));
+        rp = fma(b, s2[le][(4) * 27 + j], rp);
+      }
+      if (o.ye[0]) o.ye[0][(int64_t)i * L.ne + e] = ra;
+      if (o.ye[1]) o.ye[1][(int64_t)i * L.ne + e] = rs;
+      if (o.ye[2]) o.ye[2][(int64_t)i * L.ne + e] = rp;
+    }
+  }
+}
+
 // *same = 0 where (u, m, p) differs from (u0, m0, p0) in any entry (compared as values:
 // NaN differs from itself); *same was set nonzero before
 __global__ void k_points_compare(int64_t n, const double* __restrict__ u, const double* __restrict__ u0,
@@ -519,6 +742,32 @@ __global__ void k_copy_if_same(int64_t n, const uint32_t* __restrict__ same,
     out[i] = kept[i];
 }
 }  // namespace hm
+
+namespace {
+// the blocks of the gather: one thread per x-pair of every node row
+inline int gather_blocks(const Lattice& L) {
+  return grid1((int64_t)L.Ny * L.Nz * (L.nx + 1), 256);
+}
+}  // namespace
+
+// The vectors by the element route: work of 27 ne doubles a vector; outs ADJOINT, STATE,
+// PARAMETER (NULL: skip), which may be or overlap any of the fields.  With skip nonzero on
+// the device no vector is written.
+int hm_launch_elem_vectors(const Lattice& L, const double* u, const double* m, const double* p,
+                           const double* mhat, double f, const uint8_t* zero_ess, double* const outs[3],
+                           double* work, uint32_t* status, const uint32_t* skip, void* stream) {
+  cudaStream_t s = S_(stream);
+  VecOut<3> o{};
+  int k = 0;
+  for (int i = 0; i < 3; ++i)
+    if (outs[i]) o.ye[i] = work + (int64_t)(k++) * 27 * L.ne;
+  const int64_t groups = (L.ne + 7) / 8;
+  k_elem_vectors<<<(int)(groups < 148 * 16 ? groups : 148 * 16), 216, 0, s>>>(L, u, m, p, mhat, f, o, status, skip);
+  for (int i = 0; i < 3; ++i)
+    if (outs[i])
+      k_node_gather<<<gather_blocks(L), 256, 0, s>>>(L, o.ye[i], i != 2 ? zero_ess : nullptr, outs[i], skip);
+  return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
+}
 
 extern "C" int64_t hm_lattice_vectors_workspace_bytes(const hm_lattice* h, int nvectors) {
   if (!h || nvectors < 1 || nvectors > 3) return 0;

@@ -164,7 +164,9 @@ int hm_lattice_add_boundary_mass(const hm_lattice* h, double beta, double* d_val
  * (hippymfem/fem/kernel.py:2070-2078, fem/pattern.py:1186-1233) and of the directional
  * products of apply_ij_at (modeling/PDEVariationalProblem.py:1672).  With
  * zero_ess_vectors the STATE and ADJOINT vectors are zeroed on d_ess.  d_work:
- * hm_lattice_vectors_workspace_bytes(h, number of vectors asked for).  Non-finite
+ * hm_lattice_vectors_workspace_bytes(h, number of vectors asked for).  A vector may
+ * overwrite a field it is made of (d_vec_* equal to d_u, d_m, d_p or d_mhat): every field is
+ * then read before any vector is written, by an element pass and a node gather.  Non-finite
  * pointwise values set HM_STATUS_NONFINITE in *d_status. */
 int64_t hm_lattice_vectors_workspace_bytes(const hm_lattice* h, int nvectors);
 int hm_lattice_vectors(const hm_lattice* h, const double* d_u, const double* d_m,
