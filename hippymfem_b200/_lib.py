@@ -15,7 +15,7 @@ LIBPATH = os.path.join(HERE, "libhippymfem_b200.so")
 
 HM_OK, HM_ERR_ARG, HM_ERR_CUDA, HM_ERR_NONFINITE = 0, 1, 2, 3
 HM_ERR_NOMEM, HM_ERR_NOCONV, HM_ERR_RANGE, HM_ERR_UNSUPPORTED = 4, 5, 6, 7
-HM_STATUS_NONFINITE, HM_STATUS_RANGE = 1, 2
+HM_STATUS_NONFINITE, HM_STATUS_RANGE, HM_STATUS_TIMEOUT = 1, 2, 4
 HM_FP64, HM_FP32 = 0, 1
 
 
@@ -69,6 +69,7 @@ SIGNATURES = {
     "hm_pcg_mixed": (_i32, [_p, _p, _p, _p, _p, _p, _p, _d, _d, _i32, _i32, _i32, _p, _p, _p, _p,
                             _p]),
     "hm_device_status": (_i32, [_p, _i32]),
+    "hm_lattice_fail_waits": (_i32, [_p, _i32]),
     "hm_pcg_plan_create": (_i32, [_p, _p, _p, _p, _p, _p, _p, _p, _i32, _p]),
     "hm_pcg_plan_solve": (_i32, [_p, _d, _d, _i32, _i32, _p, _p, _p, _p]),
     "hm_pcg_plan_destroy": (_i32, [_p]),

@@ -52,6 +52,12 @@ extern "C" int hm_lattice_create(int nx, int ny, int nz, double Lx, double Ly, d
   return HM_OK;
 }
 
+extern "C" int hm_lattice_fail_waits(hm_lattice* h, int on) {
+  if (!h) return HM_ERR_ARG;
+  h->L.give_up = on != 0;
+  return HM_OK;
+}
+
 extern "C" int hm_lattice_destroy(hm_lattice* h) {
   delete h;
   return HM_OK;
@@ -142,8 +148,8 @@ extern "C" int hm_lattice_diag_A(const hm_lattice* h, const void* quad, int prec
 // the operator of a PCG: a CSR block or the lattice's matrix-free Jacobian
 int hm_pcg_operator(int64_t n, const int32_t* indptr, const int32_t* indices, const double* vals,
                     const hm::Lattice* L, const void* quad, int precision, const uint8_t* ess,
-                    const double* x, double* y, void* stream) {
-  if (L) return hm_launch_apply_A(*L, const_cast<void*>(quad), precision, ess, x, y, stream);
+                    const double* x, double* y, void* stream, double* fail) {
+  if (L) return hm_launch_apply_A(*L, const_cast<void*>(quad), precision, ess, x, y, stream, fail);
   return hm_csr_spmv(n, indptr, indices, vals, x, y, 1.0, 0.0, stream);
 }
 

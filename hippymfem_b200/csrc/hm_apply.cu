@@ -68,6 +68,8 @@ struct ApplyArgs {
   unsigned nrr;
   int flex;
   uint32_t* status;        // the library's status word (a bounded wait that gave up)
+  uint32_t* caller;        // the caller's (NULL: none)
+  double* fail;            // the solve's SC_FAIL (NULL: none)
   int tma, pitch;          // D by TMA; its row pitch
   double f;                // OUT_VEC
 };
@@ -419,10 +421,13 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
     copy_wait<1>();                        // the next layer's planes
     finish(2 * l + 3);
     finish(2 * l + 4);
-    if (__syncthreads_or(!ok)) {           // a copy never landed: flagged, nothing more written
+    if (__syncthreads_or(!ok || L.give_up)) {   // a copy never landed: flagged, nothing more written
       if (tid == 0) {
         if (a.status != nullptr) atomicOr(a.status, HM_STATUS_TIMEOUT);
-        // the other buffer's copy, before the CTA leaves
+        if (a.caller != nullptr) atomicOr(a.caller, HM_STATUS_TIMEOUT);
+        if (a.fail != nullptr) *a.fail = 1.0;
+        // both buffers' copies, before the CTA leaves
+        (void)mbar_wait(&mbar[l & 1], (uint32_t)(l >> 1) & 1u);
         if (l + 1 < layers && cz + 1 < L.nz) (void)mbar_wait(&mbar[(l + 1) & 1], (uint32_t)((l + 1) >> 1) & 1u);
       }
       break;
@@ -632,7 +637,7 @@ struct GradSmem {
 __device__ __forceinline__ void grad_tile(const CUtensorMap* map, const Lattice& L, const double* __restrict__ Dq,
                                           int tma, int pitch, const double* __restrict__ u,
                                           const double* __restrict__ p, double* __restrict__ yout,
-                                          uint32_t* __restrict__ status, const int bt) {
+                                          uint32_t* status, uint32_t* caller, const int bt) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ unsigned long long mbar;
   const GradSmem at(L.ap);
@@ -786,8 +791,12 @@ __device__ __forceinline__ void grad_tile(const CUtensorMap* map, const Lattice&
       e[4 * nt] = y[9 * a3 + 7];
     }
     copy_wait<0>();                        // the next layer's planes
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0 && status != nullptr) atomicOr(status, HM_STATUS_TIMEOUT);
+    if (__syncthreads_or(!ok || L.give_up)) {
+      if (tid == 0) {
+        if (status != nullptr) atomicOr(status, HM_STATUS_TIMEOUT);
+        atomicOr(caller, HM_STATUS_TIMEOUT);
+        (void)mbar_wait(&mbar, (uint32_t)l & 1u);        // the copy, before the CTA leaves
+      }
       break;
     }
     if (own && (l > 0 || i3 == 0)) {
@@ -827,7 +836,7 @@ __global__ void __launch_bounds__(kApplyThreads, 2)
               const __grid_constant__ VecArgs v) {
   if (v.skip != nullptr && *v.skip != 0u) return;
   const int bt = (int)blockIdx.x / v.count, w = v.which[(int)blockIdx.x - bt * v.count];
-  if (w == 2) grad_tile(&map, L, D, v.a[0].tma, v.a[0].pitch, v.u, v.p, v.grad, v.a[0].status, bt);
+  if (w == 2) grad_tile(&map, L, D, v.a[0].tma, v.a[0].pitch, v.u, v.p, v.grad, v.a[0].status, v.a[0].caller, bt);
   else apply_tile<double, double, double, IN_CLEAN, OUT_VEC>(&map, L, D, v.a[w], bt);
 }
 
@@ -968,9 +977,9 @@ int launch(const Lattice& L, const void* jac, const ApplyArgs<src, vec>& a, void
 }
 template <typename real, typename T>
 int apply_y(const Lattice& L, const void* jac, const uint8_t* ess, const T* x, T* y, bool clean,
-            double* part, double* sc, unsigned* counter, void* stream) {
+            double* part, double* sc, unsigned* counter, double* fail, void* stream) {
   ApplyArgs<T, T> a{};
-  a.ess = ess; a.x = x; a.y = y; a.part = part;
+  a.ess = ess; a.x = x; a.y = y; a.part = part; a.fail = fail;
   a.sc = part != nullptr ? sc : nullptr;
   a.counter = counter;
   if (clean) return launch<real, T, T, IN_CLEAN, OUT_Y>(L, jac, a, stream);
@@ -979,9 +988,9 @@ int apply_y(const Lattice& L, const void* jac, const uint8_t* ess, const T* x, T
 }  // namespace
 
 int hm_launch_apply_A(const Lattice& L, void* jac, int precision, const uint8_t* ess,
-                      const double* x, double* y, void* stream) {
-  if (precision == HM_FP32) return apply_y<float>(L, jac, ess, x, y, false, nullptr, nullptr, nullptr, stream);
-  return apply_y<double>(L, jac, ess, x, y, false, nullptr, nullptr, nullptr, stream);
+                      const double* x, double* y, void* stream, double* fail) {
+  if (precision == HM_FP32) return apply_y<float>(L, jac, ess, x, y, false, nullptr, nullptr, nullptr, fail, stream);
+  return apply_y<double>(L, jac, ess, x, y, false, nullptr, nullptr, nullptr, fail, stream);
 }
 
 // with sc and counter the last block also takes the CG step's alpha; x must be zero on
@@ -989,13 +998,14 @@ int hm_launch_apply_A(const Lattice& L, void* jac, int precision, const uint8_t*
 int hm_launch_apply_A_dot(const Lattice& L, void* jac, int precision, const uint8_t* ess,
                           const double* x, double* y, double* part, void* stream, double* sc,
                           unsigned* counter) {
-  if (precision == HM_FP32) return apply_y<float>(L, jac, ess, x, y, true, part, sc, counter, stream);
-  return apply_y<double>(L, jac, ess, x, y, true, part, sc, counter, stream);
+  double* const fail = sc != nullptr ? sc + SC_FAIL : nullptr;
+  if (precision == HM_FP32) return apply_y<float>(L, jac, ess, x, y, true, part, sc, counter, fail, stream);
+  return apply_y<double>(L, jac, ess, x, y, true, part, sc, counter, fail, stream);
 }
 
 int hm_launch_apply_A_clean(const Lattice& L, void* jac, const uint8_t* ess, const double* x,
                             double* y, void* stream) {
-  return apply_y<double>(L, jac, ess, x, y, true, nullptr, nullptr, nullptr, stream);
+  return apply_y<double>(L, jac, ess, x, y, true, nullptr, nullptr, nullptr, nullptr, stream);
 }
 
 // y = D^-1 A x, x zero on the Dirichlet nodes: a step of the power iteration
@@ -1008,14 +1018,14 @@ int hm_launch_power(const Lattice& L, void* jac, const uint8_t* ess, const doubl
 
 int hm_launch_apply_A32(const Lattice& L, void* jac32, const uint8_t* ess, const float* x,
                         float* y, bool clean, void* stream) {
-  return apply_y<float>(L, jac32, ess, x, y, clean, nullptr, nullptr, nullptr, stream);
+  return apply_y<float>(L, jac32, ess, x, y, clean, nullptr, nullptr, nullptr, nullptr, stream);
 }
 
 // the FP32 operator on FP32 vectors (the inner solves of the mixed-precision PCG), x zero
 // on the Dirichlet nodes
 int hm_launch_apply_A32_dot(const Lattice& L, void* jac32, const uint8_t* ess, const float* x,
                             float* y, double* part, void* stream, double* sc, unsigned* counter) {
-  return apply_y<float>(L, jac32, ess, x, y, true, part, sc, counter, stream);
+  return apply_y<float>(L, jac32, ess, x, y, true, part, sc, counter, sc != nullptr ? sc + SC_FAIL : nullptr, stream);
 }
 
 // A pass of the multigrid smoother: the arithmetic of its start / step / finish kernels.
@@ -1023,7 +1033,7 @@ int hm_launch_apply_A32_dot(const Lattice& L, void* jac32, const uint8_t* ess, c
 template <typename T>
 int hm_launch_cheb(const Lattice& L, void* jac, const uint8_t* ess, const HmCheb<T>& c, void* stream) {
   ApplyArgs<T, T> a{};
-  a.ess = ess; a.x = c.in; a.c = c;
+  a.ess = ess; a.x = c.in; a.c = c; a.fail = c.fail;
   a.c.beta = nullptr;                      // a host address
   if (c.beta != nullptr && (c.mode == CH_STEP1 || (c.mode == CH_NEXT && c.last == 2))) {
     a.part = c.beta->rz; a.sc = c.beta->sc; a.counter = c.beta->counter;
@@ -1076,6 +1086,7 @@ int hm_launch_vectors(const Lattice& L, const double* u, const double* m, const 
     a.f = i == 0 && mhat == nullptr ? f : 0.0;
     a.pitch = pitch;
     a.status = hm_status_word();
+    a.caller = status;
     if ((rc = map_D<double>(L, D, pitch, &map, &a.tma))) return rc;
   }
   for (int i = 0; i < 3; ++i)

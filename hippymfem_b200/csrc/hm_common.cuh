@@ -97,6 +97,7 @@ struct Lattice {
   double hx, hy, hz;   // element sizes
   int64_t ne, ndof;
   ApplyPlan ap;        // hm_plan_apply
+  int give_up = 0;     // the tile-marching passes' waits count as run out (hm_lattice_fail_waits)
 };
 
 // 1D stencil of node i on an axis of N nodes: [lo, lo + n)
@@ -125,9 +126,10 @@ HM_HD int64_t row_start(const Lattice& L, int i, int j, int k) {
 }
 
 // ------------------------------------------------------------ PCG device scalars
-// (shared by the solver and the operator kernels that finish a CG step's reductions)
+// (shared by the solver and the operator kernels that finish a CG step's reductions).
+// SC_FAIL: nonzero once a pass of the solve has given up a wait, its outputs invalid
 enum { SC_RZ = 0, SC_PQ, SC_ALPHA, SC_BETA, SC_RR, SC_BB, SC_TOL2, SC_CONV, SC_TMP0, SC_TMP1,
-       SC_TMP2, SC_IT, SC_N };
+       SC_TMP2, SC_IT, SC_FAIL, SC_N };
 
 #ifdef __CUDACC__
 // sum over the block (valid in thread 0); every thread of the block must call it

@@ -31,7 +31,7 @@ int hm_launch_assemble(const hm::Lattice& L, const void* quad, int precision,
 int hm_launch_jacobian_prepare(const hm::Lattice& L, const void* quad, int quad_precision,
                                void* jac, int precision, void* stream);
 int hm_launch_apply_A(const hm::Lattice& L, void* jac, int precision, const uint8_t* ess,
-                      const double* x, double* y, void* stream);
+                      const double* x, double* y, void* stream, double* fail = nullptr);
 int hm_launch_diag_A(const hm::Lattice& L, const void* quad, int precision,
                      const uint8_t* ess, double* diag, void* stream);
 int hm_launch_apply_A_dot(const hm::Lattice& L, void* jac, int precision, const uint8_t* ess,
@@ -73,7 +73,8 @@ struct HmBeta {
 };
 // the same on its own
 int hm_launch_beta(const hm::Lattice& L, const double* b, const double* z, const HmBeta& be, void* stream);
-int hm_mg_vcycle(hm_mg* mg, const double* r, double* z, void* stream, HmBeta* beta = nullptr);
+// fail: the solve's SC_FAIL, set where a fused level-0 pass gives up a wait
+int hm_mg_vcycle(hm_mg* mg, const double* r, double* z, void* stream, double* fail, HmBeta* beta = nullptr);
 // One operator pass of the level-0 Chebyshev-Jacobi smoother (hm_apply.cu), every vector
 // zero on the Dirichlet nodes, T the cycle's precision:
 //   CH_RESIDUAL  r = b - A in                     (degree 1: in = x = the first direction)
@@ -97,6 +98,7 @@ struct HmCheb {
   T* dout;
   double* z;
   HmBeta* beta;
+  double* fail;
 };
 template <typename T>
 int hm_launch_cheb(const hm::Lattice& L, void* jac, const uint8_t* ess, const HmCheb<T>& c, void* stream);

@@ -1053,14 +1053,14 @@ int vcycle(hm_mg* mg, int l, const T* b, T* x, bool clean, cudaStream_t s, T** o
 // the passes read r and write z themselves, in FP32 too
 bool level0_fused(const hm_mg* mg) { return mg->fused && mg->nlev > 1; }
 template <typename T>
-int level0_cycle(hm_mg* mg, const double* r, double* z, cudaStream_t s, HmBeta* beta) {
+int level0_cycle(hm_mg* mg, const double* r, double* z, cudaStream_t s, double* fail, HmBeta* beta) {
   MGLevelT<T>& lv = levels_of<T>(mg)[0];
   const MGLevel& l0 = mg->lv[0];
   constexpr bool kFP64 = std::is_same<T, double>::value;
   const int degree = mg->degree;
   void* const jac = kFP64 ? mg->jac : (void*)mg->jac32;
   HmCheb<T> c{};
-  c.b = r; c.idiag = l0.idiag; c.cheb = l0.cheb;
+  c.b = r; c.idiag = l0.idiag; c.cheb = l0.cheb; c.fail = fail;
   c.r = lv.r;
   // the iterate: at degree 1 beside z (the last pass reads its neighbours), FP64 at higher
   // degrees z itself
@@ -1252,10 +1252,10 @@ __global__ void k_count_mismatch(Lattice L, const uint8_t* __restrict__ ess, uns
 }  // namespace
 
 // inside the MG-PCG, whose residuals are zero on the Dirichlet nodes
-int hm_mg_vcycle(hm_mg* mg, const double* r, double* z, void* stream, HmBeta* beta) {
+int hm_mg_vcycle(hm_mg* mg, const double* r, double* z, void* stream, double* fail, HmBeta* beta) {
   cudaStream_t s = S_(stream);
   if (level0_fused(mg))
-    return mg->single ? level0_cycle<float>(mg, r, z, s, beta) : level0_cycle<double>(mg, r, z, s, beta);
+    return mg->single ? level0_cycle<float>(mg, r, z, s, fail, beta) : level0_cycle<double>(mg, r, z, s, fail, beta);
   if (mg->single) return vcycle_single(mg, r, z, true, s);
   double* out = nullptr;
   return vcycle<double>(mg, 0, r, z, true, s, &out);

@@ -438,12 +438,13 @@ extern "C" int64_t hm_pcg_workspace_bytes(int64_t n) {
 
 int hm_pcg_operator(int64_t n, const int32_t* indptr, const int32_t* indices, const double* vals,
                     const hm::Lattice* L, const void* quad, int precision, const uint8_t* ess,
-                    const double* x, double* y, void* stream);
+                    const double* x, double* y, void* stream, double* fail);
 
 namespace {
 
-// The operator of one PCG: y = A x; with part (and sc, counter) a CG step's product, whose
-// last block also takes the step's alpha from the partial sums of x.y.
+// The operator of one PCG: y = A x; with part (and counter) a CG step's product, whose
+// last block also takes the step's alpha from the partial sums of x.y.  sc[SC_FAIL] is set
+// where the matrix-free operator gives up a wait.
 struct PcgOp {
   int64_t n;
   const int32_t* indptr;
@@ -455,20 +456,27 @@ struct PcgOp {
   const uint8_t* ess;
 };
 
-int op_apply(const PcgOp& o, const double* x, double* y, void* stream, double* part = nullptr,
-             double* sc = nullptr, unsigned* counter = nullptr) {
+int op_apply(const PcgOp& o, const double* x, double* y, void* stream, double* sc, double* part = nullptr,
+             unsigned* counter = nullptr) {
   if (part == nullptr)
     return hm_pcg_operator(o.n, o.indptr, o.indices, o.vals, o.L, o.jac, o.L ? o.precision : HM_FP64, o.ess, x, y,
-                           stream);
+                           stream, sc + SC_FAIL);
   if (o.L != nullptr) return hm_launch_apply_A_dot(*o.L, o.jac, o.precision, o.ess, x, y, part, stream, sc, counter);
   k_spmv<8, false, true, 8><<<spmv_blocks(o.n, kSpmvDotBlocks), 256, 0, S_(stream)>>>(o.n, o.indptr, o.indices, nullptr, o.vals, x, y,
                                                                      1.0, 0.0, part, sc, counter);
   return ok_or_cuda();
 }
 
-int op_apply(const PcgOp& o, const float* x, float* y, void* stream, double* part = nullptr,
-             double* sc = nullptr, unsigned* counter = nullptr) {
+int op_apply(const PcgOp& o, const float* x, float* y, void* stream, double* sc, double* part = nullptr,
+             unsigned* counter = nullptr) {
   return hm_launch_apply_A32_dot(*o.L, o.jac, o.ess, x, y, part, stream, sc, counter);
+}
+
+// at a solve's start: the two counters of pcg_batch, and no pass has failed
+int reset_counters(double* sc, unsigned* cnt, cudaStream_t s) {
+  return cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned), s) == cudaSuccess &&
+                 cudaMemsetAsync(sc + SC_FAIL, 0, sizeof(double), s) == cudaSuccess
+             ? HM_OK : HM_ERR_CUDA;
 }
 
 // `count` PCG iterations (operator with p.q and alpha, update with r.z and r.r, beta,
@@ -478,7 +486,7 @@ template <typename T>
 int pcg_batch(const PcgOp& o, const double* diag, T* x, T* r, T* z, T* p, T* q, double* pq_part,
               double* sc, double* part, unsigned* cnt, int count, cudaStream_t s) {
   for (int j = 0; j < count; ++j) {
-    const int rc = op_apply(o, p, q, (void*)s, pq_part, sc, cnt);
+    const int rc = op_apply(o, p, q, (void*)s, sc, pq_part, cnt);
     if (rc) return rc;
     k_pcg_update<T><<<reduce_blocks(o.n), kReduceThreads, 0, s>>>(o.n, sc, x, r, z, p, q, diag, part,
                                                                cnt + 1);
@@ -541,13 +549,13 @@ int pcg_run(const PcgOp& o, const double* diag, const T* b, T* x, double rtol, i
   double* part = sc + SC_N;
   unsigned* cnt = reinterpret_cast<unsigned*>(part + 3 * kReduceBlocks);
   if (check_every <= 0) check_every = 1;
-  if (cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned), S_(stream)) != cudaSuccess) return HM_ERR_CUDA;
+  if (reset_counters(sc, cnt, s) != HM_OK) return HM_ERR_CUDA;
   int rc;
   // x = b on the Dirichlet nodes: every residual and direction is then zero there, which
   // the lattice operator's direction products rely on
   if constexpr (std::is_same<T, double>::value)
     if (o.L && (rc = hm_launch_ess_take_b(*o.L, o.ess, b, x, stream))) return rc;
-  rc = op_apply(o, x, q, stream);
+  rc = op_apply(o, x, q, stream, sc);
   if (rc) return rc;
   k_pcg_init<T><<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, b, q, diag, r, z, p, part);
   k_pcg_init_final<<<1, 1024, 0, s>>>(part, reduce_blocks(n), sc, rtol);
@@ -555,7 +563,7 @@ int pcg_run(const PcgOp& o, const double* diag, const T* b, T* x, double rtol, i
   int it = 0;
   for (;;) {
     if (cudaMemcpyAsync(host, sc, sizeof(host), cudaMemcpyDeviceToHost, s) != cudaSuccess) return HM_ERR_CUDA;
-    if (cudaStreamSynchronize(s) != cudaSuccess) return HM_ERR_CUDA;
+    if (cudaStreamSynchronize(s) != cudaSuccess || host[SC_FAIL] != 0.0) return HM_ERR_CUDA;
     if (host[SC_CONV] >= 0.0 || it >= maxiter) break;
     const int count = it + check_every < maxiter ? check_every : maxiter - it;
     rc = run_batch(graph, count == check_every, s, [&] {
@@ -611,14 +619,14 @@ int pcg_mg_run(hm_mg* mg, const double* b, double* x, double rtol, int maxiter, 
   double* part = sc + SC_N;
   unsigned* cnt = reinterpret_cast<unsigned*>(part + 3 * kReduceBlocks);
   if (check_every <= 0) check_every = 1;
-  if (cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned), s) != cudaSuccess) return HM_ERR_CUDA;
+  if (reset_counters(sc, cnt, s) != HM_OK) return HM_ERR_CUDA;
   int rc = hm_launch_ess_take_b(*L, o.ess, b, x, stream);   // as in pcg_run
   if (rc) return rc;
-  rc = op_apply(o, x, q, stream);
+  rc = op_apply(o, x, q, stream, sc);
   if (rc) return rc;
   const HmFirstDir fd = hm_mg_first_dir(mg);
   k_pcg_mg_init<<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, b, q, r, part, fd);
-  if ((rc = hm_mg_vcycle(mg, r, z, stream))) return rc;
+  if ((rc = hm_mg_vcycle(mg, r, z, stream, sc + SC_FAIL))) return rc;
   k_dot_partial_t<double><<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, r, z, part);
   k_pcg_init_final<<<1, 1024, 0, s>>>(part, reduce_blocks(n), sc, rtol);
   if (cudaMemcpyAsync(p, z, sizeof(double) * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
@@ -634,7 +642,7 @@ int pcg_mg_run(hm_mg* mg, const double* b, double* x, double rtol, int maxiter, 
   bool stalled = false;
   for (;;) {
     if (cudaMemcpyAsync(host, sc, sizeof(host), cudaMemcpyDeviceToHost, s) != cudaSuccess) return HM_ERR_CUDA;
-    if (cudaStreamSynchronize(s) != cudaSuccess) return HM_ERR_CUDA;
+    if (cudaStreamSynchronize(s) != cudaSuccess || host[SC_FAIL] != 0.0) return HM_ERR_CUDA;
     if (host[SC_CONV] >= 0.0 || it >= maxiter) break;
     if (flex) {
       hist.push_back(host[SC_RR]);
@@ -647,13 +655,13 @@ int pcg_mg_run(hm_mg* mg, const double* b, double* x, double rtol, int maxiter, 
     const int count = it + check_every < maxiter ? check_every : maxiter - it;
     rc = run_batch(graph, count == check_every, s, [&]() -> int {
       for (int j = 0; j < count; ++j) {
-        int e = op_apply(o, p, q, (void*)s, pq_part, sc, cnt);
+        int e = op_apply(o, p, q, (void*)s, sc, pq_part, cnt);
         if (e) return e;
         k_pcg_update_rr<<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, sc, x, r, p, q, part, fd,
                                                                  flex ? z : nullptr);
         // the cycle's last operator pass takes r.z and the step's beta where it can
         HmBeta be{pq_part, part + reduce_blocks(n), (unsigned)reduce_blocks(n), flex, sc, cnt + 1, 0};
-        if ((e = hm_mg_vcycle(mg, r, z, (void*)s, &be))) return e;
+        if ((e = hm_mg_vcycle(mg, r, z, (void*)s, sc + SC_FAIL, &be))) return e;
         if (!be.done && (e = hm_launch_beta(*L, r, z, be, (void*)s))) return e;
         k_pcg_pupdate<double><<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, sc, z, p);
       }
@@ -723,14 +731,14 @@ int pcg_mixed_run(const hm::Lattice* L, void* jac64, void* jac32, const uint8_t*
   double h[SC_N];
   auto read = [&]() -> int {
     if (cudaMemcpyAsync(h, sc, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess) return HM_ERR_CUDA;
-    return cudaStreamSynchronize(s) == cudaSuccess ? HM_OK : HM_ERR_CUDA;
+    return cudaStreamSynchronize(s) == cudaSuccess && h[SC_FAIL] == 0.0 ? HM_OK : HM_ERR_CUDA;
   };
   // the anchor: [x += s x32; t = A64 x]; r = b - t; new scale; FP32 r, z, p from r (p
   // restarted as z on the first anchor and on a restart)
   auto anchor = [&](bool first, bool restart) -> int {
     if (!first) {
       k_mx_accum<<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, sc, x32, x);
-      const int rc = op_apply(o64, x, t64, stream);
+      const int rc = op_apply(o64, x, t64, stream, sc);
       if (rc) return rc;
     }
     // first: x is b on the Dirichlet nodes and 0 elsewhere, so r = b off them, 0 on them
@@ -942,16 +950,15 @@ int group_init(hm_pcg_plan* pl, double rtol, cudaStream_t s) {
   const int64_t n = pl->L.ndof;
   const PlanBufs B = plan_bufs(pl);
   PcgOp o{n, nullptr, nullptr, nullptr, &pl->L, pl->jac64, HM_FP64, pl->ess};
-  if (cudaMemsetAsync(pl->x, 0, sizeof(double) * n, s) != cudaSuccess ||
-      cudaMemsetAsync(B.cnt, 0, 2 * sizeof(unsigned), s) != cudaSuccess)
+  if (cudaMemsetAsync(pl->x, 0, sizeof(double) * n, s) != cudaSuccess || reset_counters(B.sc, B.cnt, s) != HM_OK)
     return HM_ERR_CUDA;
   int rc = hm_launch_ess_take_b(pl->L, o.ess, pl->b, pl->x, (void*)s);
   if (rc) return rc;
-  if ((rc = op_apply(o, pl->x, B.q, (void*)s))) return rc;
+  if ((rc = op_apply(o, pl->x, B.q, (void*)s, B.sc))) return rc;
   if (pl->mg != nullptr) {
     k_pcg_mg_init<<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, pl->b, B.q, B.r, B.part,
                                                            hm_mg_first_dir(pl->mg));
-    if ((rc = hm_mg_vcycle(pl->mg, B.r, B.z, (void*)s))) return rc;
+    if ((rc = hm_mg_vcycle(pl->mg, B.r, B.z, (void*)s, B.sc + SC_FAIL))) return rc;
     k_dot_partial_t<double><<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, B.r, B.z, B.part);
     k_pcg_init_final<<<1, 1024, 0, s>>>(B.part, reduce_blocks(n), B.sc, rtol);
     if (cudaMemcpyAsync(B.p, B.z, sizeof(double) * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
@@ -973,14 +980,14 @@ int group_batch(hm_pcg_plan* pl, int count, cudaStream_t s) {
     return pcg_batch<double>(o, pl->diag, pl->x, B.r, B.z, B.p, B.q, B.pq_part, B.sc, B.part,
                              B.cnt, count, s);
   for (int j = 0; j < count; ++j) {
-    int e = op_apply(o, B.p, B.q, (void*)s, B.pq_part, B.sc, B.cnt);
+    int e = op_apply(o, B.p, B.q, (void*)s, B.sc, B.pq_part, B.cnt);
     if (e) return e;
     const int flex = hm_mg_flexible(pl->mg) ? 1 : 0;
     k_pcg_update_rr<<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, B.sc, pl->x, B.r, B.p, B.q, B.part,
                                                              hm_mg_first_dir(pl->mg),
                                                              flex ? B.z : nullptr);
     HmBeta be{B.pq_part, B.part + reduce_blocks(n), (unsigned)reduce_blocks(n), flex, B.sc, B.cnt + 1, 0};
-    if ((e = hm_mg_vcycle(pl->mg, B.r, B.z, (void*)s, &be))) return e;
+    if ((e = hm_mg_vcycle(pl->mg, B.r, B.z, (void*)s, B.sc + SC_FAIL, &be))) return e;
     if (!be.done && (e = hm_launch_beta(pl->L, B.r, B.z, be, (void*)s))) return e;
     k_pcg_pupdate<double><<<reduce_blocks(n), kReduceThreads, 0, s>>>(n, B.sc, B.z, B.p);
   }
@@ -1044,6 +1051,8 @@ extern "C" int hm_pcg_group_solve(hm_pcg_group* g, double rtol, int maxiter, int
                           cudaMemcpyDeviceToHost, s) != cudaSuccess)
         return HM_ERR_CUDA;
     if (cudaStreamSynchronize(s) != cudaSuccess) return HM_ERR_CUDA;
+    for (int i = 0; i < k; ++i)
+      if (host[(size_t)i * SC_N + SC_FAIL] != 0.0) return HM_ERR_CUDA;
     all = true;
     for (int i = 0; i < k; ++i) all = all && host[(size_t)i * SC_N + SC_CONV] >= 0.0;
     if (all || it >= maxiter) break;

@@ -193,7 +193,12 @@ class PDEVariationalProblem:
         return vecs
 
     def _require_finite(self, what):
-        if self.check_finite and int(self._status.item()) & _lib.HM_STATUS_NONFINITE:
+        if not self.check_finite:
+            return
+        status = int(self._status.item())
+        if status & _lib.HM_STATUS_TIMEOUT:
+            raise RuntimeError("a kernel gave up waiting for its data in %s" % what)
+        if status & _lib.HM_STATUS_NONFINITE:
             raise RuntimeError("non-finite values in %s" % what)
 
     def _assemble(self, quad, blocks=(), vectors=(), zero_ess_vectors=False, f=None):

@@ -49,9 +49,13 @@ const char* hm_error_string(int code);
 int hm_version(void);
 
 /* The library's own device status word on the current device: bits (HM_STATUS_*) that
- * kernels without a d_status argument set -- HM_STATUS_TIMEOUT when the assembly's
- * wait for its staged data gave up.  Synchronises the device; with clear != 0 the word
- * is reset.  No counterpart in the reference (its host kernels cannot time out). */
+ * kernels set here, with or without a d_status argument -- HM_STATUS_TIMEOUT when a
+ * kernel's bounded wait for its staged data gave up: the assembly's, or that of a
+ * tile-marching pass (the matrix-free operator, the multigrid smoother on level 0, the
+ * assembled vectors).  hm_lattice_vectors(_at) set the bit in *d_status too, and a solve
+ * one of whose operator passes gave up returns HM_ERR_CUDA at its next convergence check.
+ * Synchronises the device; with clear != 0 the word is reset.  No counterpart in the
+ * reference (its host kernels cannot time out). */
 int hm_device_status(uint32_t* out, int clear);
 
 /* ------------------------------------------------------------------ sparsity pattern
@@ -82,6 +86,10 @@ typedef struct hm_lattice hm_lattice;
 int hm_lattice_create(int nx, int ny, int nz, double Lx, double Ly, double Lz,
                       hm_lattice** out);
 int hm_lattice_destroy(hm_lattice* h);
+/* With on != 0 the tile-marching passes treat their first bounded wait as run out
+ * (HM_STATUS_TIMEOUT), to exercise the handling of that error; plans and multigrid handles
+ * keep the setting the lattice had when they were made. */
+int hm_lattice_fail_waits(hm_lattice* h, int on);
 /* ne, ndof, nnz of a Q2 x Q2 block, and the bytes of the quadrature workspace of
  * hm_lattice_quadrature at the given precision */
 int hm_lattice_sizes(const hm_lattice* h, int precision, int64_t* ne, int64_t* ndof,
@@ -167,7 +175,8 @@ int hm_lattice_add_boundary_mass(const hm_lattice* h, double beta, double* d_val
  * hm_lattice_vectors_workspace_bytes(h, number of vectors asked for).  A vector may
  * overwrite a field it is made of (d_vec_* equal to d_u, d_m, d_p or d_mhat): every field is
  * then read before any vector is written, by an element pass and a node gather.  Non-finite
- * pointwise values set HM_STATUS_NONFINITE in *d_status. */
+ * pointwise values set HM_STATUS_NONFINITE in *d_status, a bounded wait that gave up
+ * HM_STATUS_TIMEOUT. */
 int64_t hm_lattice_vectors_workspace_bytes(const hm_lattice* h, int nvectors);
 int hm_lattice_vectors(const hm_lattice* h, const double* d_u, const double* d_m,
                        const double* d_p, const double* d_mhat, double f, const uint8_t* d_ess,
