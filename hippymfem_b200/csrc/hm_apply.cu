@@ -10,7 +10,9 @@
 // two new node planes to the 3 x 3 in-plane Gauss points, the three planes to the 27
 // points, takes the derivatives *at the Gauss points* (three points carry a quadratic, so
 // a 1D derivative is the 3 x 3 matrix (-3 4 -1; -1 0 1; 1 -4 3) / (2 sqrt(0.15))), and goes
-// back the same way.  The upper plane's in-plane values, and its sums before they return
+// back the same way; every plane enters less its middle node's value, and the three meet
+// less the middle plane's, so that the rounding follows the field's variation over the
+// element and not its value.  The upper plane's in-plane values, and its sums before they return
 // to nodes, stay in the thread for the next layer.  The ten results that other columns'
 // nodes need (the element's upper x and y faces on the two lower planes) go through a
 // double-buffered exchange, one block barrier a layer, and each thread writes its own 8
@@ -19,7 +21,7 @@
 // front, corner), whatever the tiling: results do not depend on the tile sizes or on how
 // a mesh is cut into slabs.
 //
-// Bound: FP64 arithmetic (~680 operations an element) and its latency.  At 64^3 that is
+// Bound: FP64 arithmetic (~720 operations an element) and its latency.  At 64^3 that is
 // 10 us at the full FP64 rate; the 91 MB of traffic take 14 us at the measured copy rate.
 // Measured with the product's inner product (CG's A p): 41 us at 64^3, 20 at 48^3, 14 at
 // 32^3, 9 at 16^3, against 80, 37, 16 and 10 us for an element pass (three threads an
@@ -118,13 +120,14 @@ __device__ __forceinline__ double phi_1d(int i, int n, double h) {
   return (i & 1) ? h * (2.0 / 3.0) : (i == 0 || i == 2 * n) ? h / 6.0 : h / 3.0;
 }
 
-// a node plane at the element to its 9 points: x its first node, rows rs apart
+// a node plane at the element, less the value c, to its 9 points: x its first node, rows rs
+// apart
 template <typename T>
-__device__ __forceinline__ void plane_to_points(const T* x, int rs, T (&v)[9]) {
+__device__ __forceinline__ void plane_to_points(const T* x, int rs, T c, T (&v)[9]) {
   T r[9];
 #pragma unroll
   for (int a2 = 0; a2 < 3; ++a2)
-    to_points(x[a2 * rs], x[a2 * rs + 1], x[a2 * rs + 2], r[3 * a2], r[3 * a2 + 1], r[3 * a2 + 2]);
+    to_points(x[a2 * rs] - c, x[a2 * rs + 1] - c, x[a2 * rs + 2] - c, r[3 * a2], r[3 * a2 + 1], r[3 * a2 + 2]);
 #pragma unroll
   for (int q1 = 0; q1 < 3; ++q1)
     to_points(r[q1], r[3 + q1], r[6 + q1], v[q1], v[3 + q1], v[6 + q1]);
@@ -309,12 +312,17 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
   const real sx = (real)(1.0 / (0.6 * L.hx * L.hx));
   const real ry = (real)((L.hx * L.hx) / (L.hy * L.hy)), rz = (real)((L.hx * L.hx) / (L.hz * L.hz));
   const int base = 2 * ty * RS + 2 * tx;  // the element's first node in a plane
-  // in-plane values of the lower node plane, sums of the lower layer on it, the input at
-  // the own nodes there
-  real low[9], carry[9], xlow[4];
+  // in-plane values of the lower node plane less its middle node's, that value, sums of the
+  // lower layer on it, the input at the own nodes there.  (The operator annihilates
+  // constants: values at the points that carried the field's own would give every
+  // derivative the field's rounding over h.)
+  real low[9], clow = real(0), carry[9], xlow[4];
 #pragma unroll
   for (int i = 0; i < 9; ++i) low[i] = carry[i] = real(0);
-  if (element) plane_to_points(ring + base, RS, low);
+  if (element) {
+    clow = ring[base + RS + 1];
+    plane_to_points(ring + base, RS, clow, low);
+  }
 #pragma unroll
   for (int k = 0; k < 4; ++k) xlow[k] = own ? ring[base + (k >> 1) * RS + (k & 1)] : real(0);
   __syncthreads();                        // plane 0's slot is plane 6's, requested next
@@ -360,11 +368,19 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
         }
       }
       real v1[9], v2[9];
-      plane_to_points(p1, RS, v1);
-      plane_to_points(p2, RS, v2);
+      const real c1v = p1[RS + 1], c2v = p2[RS + 1];
+      plane_to_points(p1, RS, c1v, v1);
+      plane_to_points(p2, RS, c2v, v2);
       real up[9];
+      // the three planes less the middle one's value
+      const real d0 = clow - c1v, d2 = c2v - c1v;
+      clow = c2v;
 #pragma unroll
-      for (int i = 0; i < 9; ++i) up[i] = v2[i];
+      for (int i = 0; i < 9; ++i) {
+        up[i] = v2[i];
+        low[i] += d0;
+        v2[i] += d2;
+      }
       element_points(low, v1, v2, [&](int q) { return Dl[q * ds]; }, ry, rz);
 #pragma unroll
       for (int i = 0; i < 9; ++i) {
@@ -735,9 +751,10 @@ __device__ __forceinline__ void grad_tile(const CUtensorMap* map, const Lattice&
       double U[27], Q[27], W[27];
       auto values = [&](int o, double (&V)[27]) {
         double v0[9], v1[9], v2[9];
-        plane_to_points(p0 + o, RS, v0);
-        plane_to_points(p1 + o, RS, v1);
-        plane_to_points(p2 + o, RS, v2);
+        const double c = p1[o + RS + 1];       // the element's middle node (as in apply_tile)
+        plane_to_points(p0 + o, RS, c, v0);
+        plane_to_points(p1 + o, RS, c, v1);
+        plane_to_points(p2 + o, RS, c, v2);
 #pragma unroll
         for (int i = 0; i < 9; ++i) to_points(v0[i], v1[i], v2[i], V[i], V[9 + i], V[18 + i]);
       };

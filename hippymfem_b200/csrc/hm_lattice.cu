@@ -605,9 +605,12 @@ __global__ void __launch_bounds__(216, 4) k_elem_vectors(Lattice L, const double
     if (live) {
       const int ex = (int)(e % L.nx), ey = (int)((e / L.nx) % L.ny), ez = (int)(e / ((int64_t)L.nx * L.ny));
       const int64_t node = (2 * ex + c1) + (int64_t)L.Nx * ((2 * ey + c2) + (int64_t)L.Ny * (2 * ez + c3));
-      sv[le][(0) * 27 + i] = u[node];
+      // u and p less their value at the element's middle node: only their derivatives
+      // are wanted, and the value's rounding over h would be in each
+      const int64_t mid = (2 * ex + 1) + (int64_t)L.Nx * ((2 * ey + 1) + (int64_t)L.Ny * (2 * ez + 1));
+      sv[le][(0) * 27 + i] = u[node] - u[mid];
       sv[le][(1) * 27 + i] = m[node];
-      sv[le][(2) * 27 + i] = p[node];
+      sv[le][(2) * 27 + i] = p[node] - p[mid];
       sv[le][(3) * 27 + i] = mhat ? mhat[node] : 0.0;
     }
     __syncthreads();
