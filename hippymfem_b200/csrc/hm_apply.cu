@@ -21,7 +21,7 @@
 // front, corner), whatever the tiling: results do not depend on the tile sizes or on how
 // a mesh is cut into slabs.
 //
-// Bound: FP64 arithmetic (~720 operations an element) and its latency.  At 64^3 that is
+// Bound: FP64 arithmetic (~700 operations an element) and its latency.  At 64^3 that is
 // 10 us at the full FP64 rate; the 91 MB of traffic take 14 us at the measured copy rate.
 // Measured with the product's inner product (CG's A p): 41 us at 64^3, 20 at 48^3, 14 at
 // 32^3, 9 at 16^3, against 80, 37, 16 and 10 us for an element pass (three threads an
@@ -43,6 +43,7 @@ namespace hm {
 
 constexpr int kApplyThreads = 128;   // columns of a tile at most
 constexpr int kApplyBlocks = 2;      // CTAs per SM in FP64 (8 warps, up to 255 registers)
+constexpr int kApplyBlocks32 = 3;    // in FP32 (12 warps, up to 168; at four, 128, it spills: 38.5 against 33.1 us at 64^3)
 constexpr int kApplyItems = 5;       // entries of a node plane per thread at most
 constexpr int kRing = 6;             // node planes: a layer's two upper ones, four arriving
 
@@ -120,17 +121,36 @@ __device__ __forceinline__ double phi_1d(int i, int n, double h) {
   return (i & 1) ? h * (2.0 / 3.0) : (i == 0 || i == 2 * n) ? h / 6.0 : h / 3.0;
 }
 
-// a node plane at the element, less the value c, to its 9 points: x its first node, rows rs
-// apart
-template <typename T>
-__device__ __forceinline__ void plane_to_points(const T* x, int rs, T c, T (&v)[9]) {
+// A node plane at the element to its 9 points, less its middle node's value (x its first
+// node, rows rs apart): each row less its own middle node first, whose value relative to the
+// plane's goes in with the row's sum -- four operations more than the values themselves.
+// Differences in the nodes' type, the rest in the arithmetic's.
+template <typename T, typename src>
+__device__ __forceinline__ void plane_to_points(const src* x, int rs, T (&v)[9]) {
+  const src c = x[rs + 1];
   T r[9];
 #pragma unroll
-  for (int a2 = 0; a2 < 3; ++a2)
-    to_points(x[a2 * rs] - c, x[a2 * rs + 1] - c, x[a2 * rs + 2] - c, r[3 * a2], r[3 * a2 + 1], r[3 * a2 + 2]);
+  for (int a2 = 0; a2 < 3; ++a2) {
+    const src m = x[a2 * rs + 1];
+    const T a = (T)(x[a2 * rs] - m), b = (T)(x[a2 * rs + 2] - m), w = a2 == 1 ? T(0) : (T)(m - c);
+    const T d = b - a, t = fma(T(0.3), a + b, w);
+    r[3 * a2] = fma(T(-kS), d, t);
+    r[3 * a2 + 1] = w;
+    r[3 * a2 + 2] = fma(T(kS), d, t);
+  }
 #pragma unroll
   for (int q1 = 0; q1 < 3; ++q1)
     to_points(r[q1], r[3 + q1], r[6 + q1], v[q1], v[3 + q1], v[6 + q1]);
+}
+// three planes' values along z, each less its own plane's reference r0, r1, r2, to the points
+// less r1: k = 0.3 ((r0 - r1) + (r2 - r1)), g = r2 - r0
+template <typename T>
+__device__ __forceinline__ void to_points_z(T x0, T x1, T x2, T k, T g, T& v0, T& v1, T& v2) {
+  const T d = (x2 - x0) + g;
+  const T e = fma(T(0.4), x1, fma(T(0.3), x0 + x2, k));
+  v0 = fma(T(-kS), d, e);
+  v1 = x1;
+  v2 = fma(T(kS), d, e);
 }
 template <typename T>
 __device__ __forceinline__ void plane_from_points(T (&v)[9]) {
@@ -140,13 +160,14 @@ __device__ __forceinline__ void plane_from_points(T (&v)[9]) {
   for (int a2 = 0; a2 < 3; ++a2)
     from_points(v[3 * a2], v[3 * a2 + 1], v[3 * a2 + 2], v[3 * a2], v[3 * a2 + 1], v[3 * a2 + 2]);
 }
-// One element at its 27 points: v0, v1, v2 the in-plane values of its three node planes,
+// One element at its 27 points: v0, v1, v2 the in-plane values of its three node planes (k, g:
+// of to_points_z),
 // D(q) the weights; on return the in-plane sums of the three planes
 template <typename T, typename LDD>
-__device__ __forceinline__ void element_points(T (&v0)[9], T (&v1)[9], T (&v2)[9], LDD D, T ry, T rz) {
+__device__ __forceinline__ void element_points(T (&v0)[9], T (&v1)[9], T (&v2)[9], T k, T g, LDD D, T ry, T rz) {
   T V[27], R[27];          // [q1 + 3 q2 + 9 q3]
 #pragma unroll
-  for (int i = 0; i < 9; ++i) to_points(v0[i], v1[i], v2[i], V[i], V[9 + i], V[18 + i]);
+  for (int i = 0; i < 9; ++i) to_points_z(v0[i], v1[i], v2[i], k, g, V[i], V[9 + i], V[18 + i]);
 #pragma unroll
   for (int i = 0; i < 9; ++i) {          // z lines
     T g0, g1, g2;
@@ -179,6 +200,33 @@ __device__ __forceinline__ void element_points(T (&v0)[9], T (&v1)[9], T (&v2)[9
   for (int i = 0; i < 9; ++i) from_points(R[i], R[9 + i], R[18 + i], v0[i], v1[i], v2[i]);
 }
 
+// Loads where `on`, else 0, by a predicate and issued where they stand: with a branch around
+// each, as conditional expressions and statements compile to here, a layer's loads and copies
+// took 2,000 cycles to issue, with predicates 900 (16^3, y = A x alone: 9.8 -> 6.7 us in FP64,
+// 11.9 -> 6.3 in FP32; 64^3 49.8 -> 38.6 and 57.2 -> 33.8).
+__device__ __forceinline__ uint32_t load_mark(const uint8_t* p, bool on) {
+  uint32_t m;
+  asm volatile(
+      "{\n .reg .pred p;\n .reg .u16 t;\n setp.ne.u32 p, %2, 0;\n mov.u16 t, 0;\n"
+      " @p ld.global.nc.u8 t, [%1];\n cvt.u32.u16 %0, t;\n}"
+      : "=r"(m)
+      : "l"(p), "r"((uint32_t)on));
+  return m;
+}
+// (not .nc: r and x are the kernel's own outputs too, node by node)
+__device__ __forceinline__ double load_if(const double* p, bool on) {
+  double v;
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n mov.f64 %0, 0d0000000000000000;\n @p ld.global.f64 %0, [%1];\n}"
+               : "=d"(v) : "l"(p), "r"((uint32_t)on) : "memory");
+  return v;
+}
+__device__ __forceinline__ float load_if(const float* p, bool on) {
+  float v;
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n mov.f32 %0, 0f00000000;\n @p ld.global.f32 %0, [%1];\n}"
+               : "=f"(v) : "l"(p), "r"((uint32_t)on) : "memory");
+  return v;
+}
+
 // Dynamic shared memory: D of two layers [q][row][column] (one TMA box from the 16-byte
 // boundary at or before the tile's first column), the ring of node planes, the exchange.
 template <typename real> HM_HD constexpr int row_align() { return 16 / (int)sizeof(real); }
@@ -187,14 +235,14 @@ HM_HD int box_columns(int T1) {
   constexpr int A = row_align<real>();
   return (T1 + 2 * A - 2) / A * A;
 }
-template <typename real>
+template <typename real, typename src>
 struct ApplySmem {
   int dbuf, ring, exch, bytes;       // bytes of one D buffer, offsets in bytes
   HM_HD ApplySmem(const ApplyPlan& p) {
     const int s = (int)sizeof(real);
     dbuf = (27 * p.T2 * box_columns<real>(p.T1) * s + 127) / 128 * 128;
     ring = 2 * dbuf;
-    exch = ring + kRing * (2 * p.T1 + 1) * (2 * p.T2 + 1) * s;
+    exch = ring + kRing * (2 * p.T1 + 1) * (2 * p.T2 + 1) * (int)sizeof(src);
     bytes = exch + 20 * p.threads * s;
   }
 };
@@ -205,10 +253,10 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
                                            const ApplyArgs<src, vec>& a, const int bt) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ unsigned long long mbar[2];           // D of the even and the odd layers
-  const ApplySmem<real> at(L.ap);
+  const ApplySmem<real, src> at(L.ap);
   constexpr int A = row_align<real>();
   const int T1 = L.ap.T1, T2 = L.ap.T2, nt = blockDim.x;
-  real* const ring = reinterpret_cast<real*>(smem_raw + at.ring);
+  src* const ring = reinterpret_cast<src*>(smem_raw + at.ring);
   real* const exch = reinterpret_cast<real*>(smem_raw + at.exch);
   const int RS = 2 * T1 + 1, P = RS * (2 * T2 + 1), TB = box_columns<real>(T1);
   const int tid = threadIdx.x;
@@ -239,7 +287,6 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
   request_D(1);
   // ---- node planes: plane j (relative to 2 c3) into ring slot j % kRing, entry i of a
   // plane by thread i % nt, the same ones every time
-  constexpr bool kDirect = sizeof(src) == sizeof(real);        // copied as it is
   unsigned off[kApplyItems];               // the entries' nodes in the mesh's plane (~0: none)
   {
     const int step_r = nt / RS, step_c = nt - step_r * RS;
@@ -254,37 +301,37 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
     }
   }
   auto request = [&](int j) {
-    if constexpr (kDirect) {
-      if (2 * c3 + j < L.Nz && j <= 2 * layers) {
-        real* const plane = ring + j % kRing * P + tid;
-        const real* const x = reinterpret_cast<const real*>(a.x) + (size_t)nsz * (2 * c3 + j);
+    if (2 * c3 + j < L.Nz && j <= 2 * layers) {
+      src* const plane = ring + j % kRing * P + tid;
+      const src* const x = a.x + (size_t)nsz * (2 * c3 + j);
 #pragma unroll
-        for (int k = 0; k < kApplyItems; ++k)
-          if (off[k] != ~0u) copy_async(plane + k * nt, x + off[k]);
-      }
+      for (int k = 0; k < kApplyItems; ++k)
+        if constexpr (OUT == OUT_VEC) {    // (beside grad_tile's passes: 158 us against 163)
+          if (off[k] != ~0u) copy_async(plane + k * nt, x + off[k], true);
+        } else {
+          copy_async(plane + k * nt, x + off[k], off[k] != ~0u);
+        }
     }
   };
-  // after the copies of plane j, by the same threads: the Dirichlet nodes zeroed, operands of
-  // another type than the arithmetic's converted
-  auto finish = [&](int j) {
-    if constexpr (kDirect && IN == IN_CLEAN) return;
-    if (2 * c3 + j >= L.Nz || j > 2 * layers) return;
-    real* const plane = ring + j % kRing * P + tid;
-    const size_t z0 = (size_t)nsz * (2 * c3 + j);
-    src v[kApplyItems];
-    bool zero[kApplyItems];
+  // The Dirichlet markers of plane j are loaded a layer before finish() zeroes the marked
+  // entries, after the plane's copies and by the same threads (loaded there, their latency
+  // stood open twice a layer).
+  struct Marks { uint32_t m[IN == IN_ESS ? kApplyItems : 1]; };
+  auto load = [&](int j, Marks& e) {
+    if constexpr (IN == IN_ESS) {
+      const bool plane = a.ess != nullptr && 2 * c3 + j < L.Nz && j <= 2 * layers;
+      const uint8_t* const ess = a.ess + (size_t)nsz * (2 * c3 + j);
 #pragma unroll
-    for (int k = 0; k < kApplyItems; ++k) {
-      const bool on = off[k] != ~0u;
-      zero[k] = IN == IN_ESS && on && a.ess != nullptr && __ldg(a.ess + z0 + off[k]) != 0;
-      v[k] = !kDirect && on ? __ldg(a.x + z0 + off[k]) : src(0);
+      for (int k = 0; k < kApplyItems; ++k) e.m[k] = load_mark(ess + off[k], plane && off[k] != ~0u);
     }
+  };
+  auto finish = [&](int j, const Marks& e) {
+    if constexpr (IN == IN_ESS) {
+      src* const plane = ring + j % kRing * P + tid;
 #pragma unroll
-    for (int k = 0; k < kApplyItems; ++k)
-      if (off[k] != ~0u) {
-        if (zero[k]) plane[k * nt] = real(0);
-        else if constexpr (!kDirect) plane[k * nt] = (real)v[k];
-      }
+      for (int k = 0; k < kApplyItems; ++k)
+        if (e.m[k] != 0u) plane[k * nt] = src(0);
+    }
   };
   // D is requested a layer ahead, node planes two layers, a group of copies each
   for (int j = 0; j < 3; ++j) request(j);
@@ -304,38 +351,40 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
     w1 = __ldg(a.c.cheb + 1 + a.c.k);
     w2 = __ldg(a.c.cheb + 1 + kChebMax + a.c.k);
   }
-  copy_wait<1>();
-  for (int j = 0; j < 3; ++j) finish(j);
+  {
+    Marks e[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) load(j, e[j]);
+    copy_wait<1>();
+#pragma unroll
+    for (int j = 0; j < 3; ++j) finish(j, e[j]);
+  }
   __syncthreads();
 
   // the derivatives carry 2 sqrt(0.15) each: 1 / (4 * 0.15) in the product
-  const real sx = (real)(1.0 / (0.6 * L.hx * L.hx));
-  const real ry = (real)((L.hx * L.hx) / (L.hy * L.hy)), rz = (real)((L.hx * L.hx) / (L.hz * L.hz));
+  const real sx = (real)L.ap.sx, ry = (real)L.ap.ry, rz = (real)L.ap.rz;
   const int base = 2 * ty * RS + 2 * tx;  // the element's first node in a plane
   // in-plane values of the lower node plane less its middle node's, that value, sums of the
   // lower layer on it, the input at the own nodes there.  (The operator annihilates
   // constants: values at the points that carried the field's own would give every
   // derivative the field's rounding over h.)
-  real low[9], clow = real(0), carry[9], xlow[4];
+  real low[9], carry[9];
+  src clow = src(0), xlow[4];
 #pragma unroll
   for (int i = 0; i < 9; ++i) low[i] = carry[i] = real(0);
   if (element) {
     clow = ring[base + RS + 1];
-    plane_to_points(ring + base, RS, clow, low);
+    plane_to_points(ring + base, RS, low);
   }
 #pragma unroll
-  for (int k = 0; k < 4; ++k) xlow[k] = own ? ring[base + (k >> 1) * RS + (k & 1)] : real(0);
+  for (int k = 0; k < 4; ++k) xlow[k] = own ? ring[base + (k >> 1) * RS + (k & 1)] : src(0);
   __syncthreads();                        // plane 0's slot is plane 6's, requested next
   double dot = 0.0;
 #pragma unroll 1
   for (int l = 0; l < layers; ++l) {
     const int cz = c3 + l;
-    const real* const p1 = ring + (2 * l + 1) % kRing * P + base;
-    const real* const p2 = ring + (2 * l + 2) % kRing * P + base;
-    request(2 * l + 5);
-    request(2 * l + 6);
-    copy_commit();
-    if (l > 0) request_D(l + 1);
+    const src* const p1 = ring + (2 * l + 1) % kRing * P + base;
+    const src* const p2 = ring + (2 * l + 2) % kRing * P + base;
     // The own nodes h = (x, y, z parity bits): which of them exist, their markers
     // (requested here, used after the barrier)
     const bool out = own && (l > 0 || i3 == 0);
@@ -345,11 +394,22 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
     if (cy >= L.ny) have &= 0x33u;
     if (cz >= L.nz) have &= 0x0fu;
     uint32_t mark[8];
+    // (left to the compiler where the pass loads nothing else by predicate: CG's product at
+    // 64^3 40.2 us against 41.0, dR/du 68 against 70)
 #pragma unroll
-    for (int h = 0; h < 8; ++h)
-      mark[h] = a.ess != nullptr && ((have >> h) & 1u)
-                    ? __ldg(a.ess + n0 + (h & 1) + ((h & 2) ? nsy : 0u) + ((h & 4) ? nsz : 0u))
-                    : 0u;
+    for (int h = 0; h < 8; ++h) {
+      const unsigned node = n0 + (h & 1) + ((h & 2) ? nsy : 0u) + ((h & 4) ? nsz : 0u);
+      const bool on = a.ess != nullptr && ((have >> h) & 1u);
+      if constexpr (IN == IN_CLEAN && (OUT == OUT_Y || OUT == OUT_VEC)) mark[h] = on ? __ldg(a.ess + node) : 0u;
+      else mark[h] = load_mark(a.ess + node, on);
+    }
+    request(2 * l + 5);
+    request(2 * l + 6);
+    copy_commit();
+    if (l > 0) request_D(l + 1);
+    Marks next[2];
+    load(2 * l + 3, next[0]);
+    load(2 * l + 4, next[1]);
     real y[18];                            // the element's sums on its two lower planes
     const bool layer = cz < L.nz;          // not the virtual one
     const bool ok = !a.tma || !layer || mbar_wait(&mbar[l & 1], (uint32_t)(l >> 1) & 1u);
@@ -368,20 +428,15 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
         }
       }
       real v1[9], v2[9];
-      const real c1v = p1[RS + 1], c2v = p2[RS + 1];
-      plane_to_points(p1, RS, c1v, v1);
-      plane_to_points(p2, RS, c2v, v2);
+      plane_to_points(p1, RS, v1);
+      plane_to_points(p2, RS, v2);
       real up[9];
-      // the three planes less the middle one's value
-      const real d0 = clow - c1v, d2 = c2v - c1v;
-      clow = c2v;
 #pragma unroll
-      for (int i = 0; i < 9; ++i) {
-        up[i] = v2[i];
-        low[i] += d0;
-        v2[i] += d2;
-      }
-      element_points(low, v1, v2, [&](int q) { return Dl[q * ds]; }, ry, rz);
+      for (int i = 0; i < 9; ++i) up[i] = v2[i];
+      const src mid = p1[RS + 1], cup = p2[RS + 1];
+      const real k = real(0.3) * (real)((clow - mid) + (cup - mid)), g = (real)(cup - clow);
+      clow = cup;
+      element_points(low, v1, v2, k, g, [&](int q) { return Dl[q * ds]; }, ry, rz);
 #pragma unroll
       for (int i = 0; i < 9; ++i) {
         low[i] += carry[i];
@@ -410,8 +465,8 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
       e[3 * nt] = y[9 * a3 + 6];
       e[4 * nt] = y[9 * a3 + 7];
     }
-    // the input at the own nodes, the smoother's operands
-    real xc[8];
+    // the input at the own nodes (the zeroed ones' too), the smoother's operands
+    src xc[8];
     double bn[OUT == OUT_Y || OUT == OUT_VEC || OUT == OUT_POWER ? 1 : 8], gn[OUT == OUT_Y || OUT == OUT_R || OUT == OUT_VEC ? 1 : 8], xn[OUT == OUT_NEXT ? 8 : 1];
     unsigned fixed = 0;
 #pragma unroll
@@ -419,24 +474,27 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
       const bool on = (have >> h) & 1u;
       const unsigned node = n0 + (h & 1) + ((h & 2) ? nsy : 0u) + ((h & 4) ? nsz : 0u);
       if constexpr (OUT == OUT_NEXT) {
-        bn[h] = !on ? 0.0 : a.c.first ? __ldg(a.c.b + node) : (double)a.c.r[node];
-        xn[h] = !on || a.c.first ? 0.0 : (double)a.c.x[node];
+        if (a.c.first) bn[h] = load_if(a.c.b + node, on);
+        else bn[h] = (double)load_if(a.c.r + node, on);
+        xn[h] = (double)load_if(a.c.x + node, on && !a.c.first);
       } else if constexpr (OUT != OUT_Y && OUT != OUT_VEC && OUT != OUT_POWER) {
-        bn[h] = on ? __ldg(a.c.b + node) : 0.0;
+        bn[h] = load_if(a.c.b + node, on);
       }
-      if constexpr (OUT != OUT_Y && OUT != OUT_R && OUT != OUT_VEC) gn[h] = on ? __ldg(a.c.idiag + node) : 0.0;
+      if constexpr (OUT != OUT_Y && OUT != OUT_R && OUT != OUT_VEC) gn[h] = load_if(a.c.idiag + node, on);
       const int o = ((h >> 1) & 1) * RS + (h & 1);
       if (h < 4) {
         xc[h] = xlow[h];
-        xlow[h] = own ? p2[o] : real(0);
+        xlow[h] = own ? p2[o] : src(0);
       } else {
-        xc[h] = own ? p1[o] : real(0);
+        xc[h] = own ? p1[o] : src(0);
       }
       fixed |= (unsigned)(mark[h] != 0u) << h;
+      if constexpr (IN == IN_ESS)
+        if (on && mark[h] != 0u) xc[h] = __ldg(a.x + node);
     }
     copy_wait<1>();                        // the next layer's planes
-    finish(2 * l + 3);
-    finish(2 * l + 4);
+    finish(2 * l + 3, next[0]);
+    finish(2 * l + 4, next[1]);
     if (__syncthreads_or(!ok || L.give_up)) {   // a copy never landed: flagged, nothing more written
       if (tid == 0) {
         if (a.status != nullptr) atomicOr(a.status, HM_STATUS_TIMEOUT);
@@ -466,10 +524,7 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
           const bool fx = (fixed >> h) & 1u;
           const double acc = (double)(sx * n[k]);
           if constexpr (OUT == OUT_Y) {
-            // the ring's value is the input's own, but for zeroed or rounded entries
-            const double xv = (IN == IN_CLEAN && kDirect) ? (double)xc[h]
-                              : (fx || (a.part != nullptr && !kDirect)) ? (double)__ldg(a.x + node)
-                                                                        : (double)xc[h];
+            const double xv = (double)xc[h];
             const double yv = fx ? xv : acc;
             a.y[node] = (vec)yv;
             dot = fma(xv, yv, dot);
@@ -526,7 +581,7 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
 }
 
 template <typename real, typename src, typename vec, int IN, int OUT>
-__global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlocks : 4)
+__global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlocks : kApplyBlocks32)
     k_apply_tile(const __grid_constant__ CUtensorMap map, const Lattice L, const real* __restrict__ Dq,
                  const ApplyArgs<src, vec> a) {
   apply_tile<real, src, vec, IN, OUT>(&map, L, Dq, a, (int)blockIdx.x);
@@ -700,11 +755,10 @@ __device__ __forceinline__ void grad_tile(const CUtensorMap* map, const Lattice&
       double* const pu = ring + j % kGradRing * P + tid;
       const size_t z0 = (size_t)nsz * (2 * c3 + j);
 #pragma unroll
-      for (int k = 0; k < kApplyItems; ++k)
-        if (off[k] != ~0u) {
-          copy_async(pu + k * nt, u + z0 + off[k]);
-          copy_async(pu + kGradRing * P + k * nt, p + z0 + off[k]);
-        }
+      for (int k = 0; k < kApplyItems; ++k) {
+        copy_async(pu + k * nt, u + z0 + off[k], off[k] != ~0u);
+        copy_async(pu + kGradRing * P + k * nt, p + z0 + off[k], off[k] != ~0u);
+      }
     }
   };
   for (int j = 0; j < 3; ++j) request(j);
@@ -714,8 +768,7 @@ __device__ __forceinline__ void grad_tile(const CUtensorMap* map, const Lattice&
   const bool column = ty < T2;
   const bool element = column && cx < L.nx && cy < L.ny;
   const bool own = column && cx <= L.nx && cy <= L.ny && (tx > 0 || i1 == 0) && (ty > 0 || i2 == 0);
-  const double sx = 1.0 / (0.6 * L.hx * L.hx);
-  const double ry = (L.hx * L.hx) / (L.hy * L.hy), rz = (L.hx * L.hx) / (L.hz * L.hz);
+  const double sx = L.ap.sx, ry = L.ap.ry, rz = L.ap.rz;
   const int base = 2 * ty * RS + 2 * tx, ds = T2 * TB;
   double carry[9];
 #pragma unroll
@@ -751,12 +804,13 @@ __device__ __forceinline__ void grad_tile(const CUtensorMap* map, const Lattice&
       double U[27], Q[27], W[27];
       auto values = [&](int o, double (&V)[27]) {
         double v0[9], v1[9], v2[9];
-        const double c = p1[o + RS + 1];       // the element's middle node (as in apply_tile)
-        plane_to_points(p0 + o, RS, c, v0);
-        plane_to_points(p1 + o, RS, c, v1);
-        plane_to_points(p2 + o, RS, c, v2);
+        plane_to_points(p0 + o, RS, v0);
+        plane_to_points(p1 + o, RS, v1);
+        plane_to_points(p2 + o, RS, v2);
+        const double r0 = p0[o + RS + 1], r1 = p1[o + RS + 1], r2 = p2[o + RS + 1];
+        const double k = 0.3 * ((r0 - r1) + (r2 - r1)), g = r2 - r0;
 #pragma unroll
-        for (int i = 0; i < 9; ++i) to_points(v0[i], v1[i], v2[i], V[i], V[9 + i], V[18 + i]);
+        for (int i = 0; i < 9; ++i) to_points_z(v0[i], v1[i], v2[i], k, g, V[i], V[9 + i], V[18 + i]);
       };
       values(0, U);
       values(kGradRing * P, Q);
@@ -931,6 +985,9 @@ void hm_plan_apply(Lattice* L) {
       }
     }
   }
+  p.sx = 1.0 / (0.6 * L->hx * L->hx);
+  p.ry = (L->hx * L->hx) / (L->hy * L->hy);
+  p.rz = (L->hx * L->hx) / (L->hz * L->hz);
   L->ap = p;
 }
 
@@ -984,7 +1041,7 @@ int launch(const Lattice& L, const void* jac, int pitch, ApplyArgs<src, vec> a, 
   a.status = hm_status_word();
   CUtensorMap map{};
   if ((rc = map_D<real>(L, jac, pitch, &map, &a.tma))) return rc;
-  kern<<<L.ap.t1 * L.ap.t2 * L.ap.t3, L.ap.threads, (size_t)ApplySmem<real>(L.ap).bytes,
+  kern<<<L.ap.t1 * L.ap.t2 * L.ap.t3, L.ap.threads, (size_t)ApplySmem<real, src>(L.ap).bytes,
          reinterpret_cast<cudaStream_t>(stream)>>>(map, L, static_cast<const real*>(jac), a);
   return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
 }
@@ -1108,7 +1165,7 @@ int hm_launch_vectors(const Lattice& L, const double* u, const double* m, const 
   }
   for (int i = 0; i < 3; ++i)
     if (outs[i]) v.which[v.count++] = i;
-  const int bytes = ApplySmem<double>(L.ap).bytes, grad = GradSmem(L.ap).bytes;
+  const int bytes = ApplySmem<double, double>(L.ap).bytes, grad = GradSmem(L.ap).bytes;
   const bool applies = outs[0] || outs[1];
   k_vectors<<<L.ap.t1 * L.ap.t2 * L.ap.t3 * v.count, L.ap.threads,
               (size_t)(!outs[2] || (applies && bytes > grad) ? bytes : grad), s>>>(map, L, D, v);

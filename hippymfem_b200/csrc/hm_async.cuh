@@ -46,12 +46,14 @@ __device__ __forceinline__ void mbar_expect(unsigned long long* b, uint32_t byte
                : "memory");
 }
 
-// single elements, in groups that are waited for in order
-__device__ __forceinline__ void copy_async(void* dst, const double* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy_async(void* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+// single elements where `on` (a predicate, not a branch around the copy), in groups that are
+// waited for in order
+template <typename T>
+__device__ __forceinline__ void copy_async(void* dst, const T* src, bool on) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p cp.async.ca.shared.global [%0], [%1], %2;\n}" ::"r"(
+                   smem_u32(dst)),
+               "l"(src), "n"(sizeof(T)), "r"((uint32_t)on)
+               : "memory");
 }
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 // all but the newest N groups of this thread have landed

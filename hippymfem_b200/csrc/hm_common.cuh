@@ -88,8 +88,9 @@ HM_HD constexpr double vrow_coef(int tab, int r, int t) {
 
 // ------------------------------------------------------------------ lattice
 // tiling of the matrix-free apply: t1 x t2 x t3 tiles of T1 x T2 x T3 cells (the halo
-// included), `threads` per CTA
-struct ApplyPlan { int T1, T2, T3, t1, t2, t3, threads; };
+// included), `threads` per CTA; the scale of the product, the weights of the y and z
+// derivatives in it
+struct ApplyPlan { int T1, T2, T3, t1, t2, t3, threads; double sx, ry, rz; };
 struct Lattice {
   int nx, ny, nz;      // elements per axis
   int Nx, Ny, Nz;      // nodes per axis (2 n + 1)
