@@ -70,6 +70,7 @@ SIGNATURES = {
                             _p]),
     "hm_device_status": (_i32, [_p, _i32]),
     "hm_lattice_fail_waits": (_i32, [_p, _i32]),
+    "hm_lattice_set_slab": (_i32, [_p, _i32]),
     "hm_pcg_plan_create": (_i32, [_p, _p, _p, _p, _p, _p, _p, _p, _i32, _p]),
     "hm_pcg_plan_solve": (_i32, [_p, _d, _d, _i32, _i32, _p, _p, _p, _p]),
     "hm_pcg_plan_destroy": (_i32, [_p]),

@@ -52,6 +52,12 @@ extern "C" int hm_lattice_create(int nx, int ny, int nz, double Lx, double Ly, d
   return HM_OK;
 }
 
+extern "C" int hm_lattice_set_slab(hm_lattice* h, int on) {
+  if (!h) return HM_ERR_ARG;
+  h->L.slab = on != 0;
+  return HM_OK;
+}
+
 extern "C" int hm_lattice_fail_waits(hm_lattice* h, int on) {
   if (!h) return HM_ERR_ARG;
   h->L.give_up = on != 0;

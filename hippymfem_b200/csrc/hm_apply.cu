@@ -1141,9 +1141,16 @@ int hm_launch_vectors(const Lattice& L, const double* u, const double* m, const 
     const uintptr_t bytes = sizeof(double) * (uintptr_t)L.ndof;
     return a < b + bytes && b < a + bytes;
   };
+  // And one or two vectors on a small mesh, where the passes are latency -- k_points_D, then
+  // layers in series: 11 to 13 us whatever the size, against 7 to 10 for one vector by the
+  // element route up to 14^3 (10.1 against 11.1-12.5; 16^3 12.0 against 11.1-12.3, 20^3 17.0
+  // against 11.7-13) and 10 to 12 for two up to 12^3 (12.0 against 12.6; 14^3 13.5 against
+  // 12.9); three take 13.3 either way at 8^3.  Not on a slab: the routes sum in other orders.
+  const int count = (outs[0] != nullptr) + (outs[1] != nullptr) + (outs[2] != nullptr);
+  bool element = !L.slab && ((count == 1 && L.ne <= 2744) || (count == 2 && L.ne <= 1728));
   for (int i = 0; i < 3; ++i)
-    if (outs[i] && (overlaps(outs[i], u) || overlaps(outs[i], p)))
-      return hm_launch_elem_vectors(L, u, m, p, mhat, f, zero_ess, outs, D, status, skip, stream);
+    if (outs[i] && (overlaps(outs[i], u) || overlaps(outs[i], p))) element = true;
+  if (element) return hm_launch_elem_vectors(L, u, m, p, mhat, f, zero_ess, outs, D, status, skip, stream);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   int pitch = hm_jac_pitch(L, HM_FP64);
   if (27 * (int64_t)pitch * L.ny * L.nz > work_reals) pitch = L.nx;

@@ -98,6 +98,7 @@ struct Lattice {
   double hx, hy, hz;   // element sizes
   int64_t ne, ndof;
   ApplyPlan ap;        // hm_plan_apply
+  int slab = 0;        // part of a larger mesh (hm_lattice_set_slab)
   int give_up = 0;     // the tile-marching passes' waits count as run out (hm_lattice_fail_waits)
 };
 

@@ -4,8 +4,8 @@
 //                   transpose map of a Q2 x Q2 block, arithmetically
 //   k_quad          pointwise data D, E = D grad u, F = D grad p, W = D grad u.grad p
 //   k_extract_D     the matrix-free Jacobian's data (its apply is in hm_apply.cu)
-//   k_elem_vectors, the assembled vectors by element results and a gather, for outputs that
-//   k_node_gather   overlap the fields (the others are in hm_apply.cu)
+//   k_elem_vectors, the assembled vectors by element results and a gather, for small meshes
+//   k_node_gather   and outputs that overlap the fields (the others are in hm_apply.cu)
 // (the fused assembly k_tile_assemble is in hm_tile.cu)
 #include <cstdio>
 

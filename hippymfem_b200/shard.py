@@ -386,10 +386,13 @@ class DeviceSlabOps:
     the assembled vectors straight from the fields, the device observation operator)."""
 
     def __init__(self, part, rank, points, noise_variance, device):
+        from ._lib import check, lib
         from .mesh import BoxMesh
         from .modeling import device_observation_operator
         n, L = part.local_box(rank)
         self.mesh = BoxMesh(n, L, device=device)
+        # the vectors' sums in the order that does not depend on the slab's height
+        check(lib.hm_lattice_set_slab(self.mesh.handle, 1), "hm_lattice_set_slab")
         loc, _ = local_points(part, rank, points)
         self.nobs = len(loc)
         self.B = device_observation_operator(self.mesh, loc) if self.nobs else None

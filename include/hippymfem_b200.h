@@ -86,6 +86,10 @@ typedef struct hm_lattice hm_lattice;
 int hm_lattice_create(int nx, int ny, int nz, double Lx, double Ly, double Lz,
                       hm_lattice** out);
 int hm_lattice_destroy(hm_lattice* h);
+/* With on != 0 the lattice is a slab of a larger mesh: hm_lattice_vectors sums every node in
+ * the one order that no cut of the mesh changes, also where it would take another one for a
+ * lattice of this size. */
+int hm_lattice_set_slab(hm_lattice* h, int on);
 /* With on != 0 the tile-marching passes treat their first bounded wait as run out
  * (HM_STATUS_TIMEOUT), to exercise the handling of that error; plans and multigrid handles
  * keep the setting the lattice had when they were made. */
@@ -167,7 +171,8 @@ int hm_lattice_add_boundary_mass(const hm_lattice* h, double beta, double* d_val
  * mhat, no source: ADJOINT C mhat, STATE W_um mhat, PARAMETER W_mm mhat, rows not
  * eliminated) -- the vectors hm_lattice_quadrature(_dir) + hm_lattice_assemble give,
  * summed in another fixed order (equal to rounding; deterministic).  One pass forms D at
- * each element's 27 points, one launch of tile-marching passes the vectors; the
+ * each element's 27 points, one launch of tile-marching passes the vectors (one or two
+ * vectors on a small mesh: an element pass and a gather a vector); the
  * replacement of element_vectors + assemble_vector
  * (hippymfem/fem/kernel.py:2070-2078, fem/pattern.py:1186-1233) and of the directional
  * products of apply_ij_at (modeling/PDEVariationalProblem.py:1672).  With

@@ -62,6 +62,7 @@ def test_vectors_set_the_callers_status(cuda, n, slots):
     from hippymfem_b200._lib import check, lib, ptr, stream_ptr
 
     hm, mesh, V, bc, f = _setup(n)
+    check(lib.hm_lattice_set_slab(mesh.handle, 1))       # the tile-marching passes at every size
     nbytes = lib.hm_lattice_vectors_workspace_bytes(mesh.handle, 3)
     work = torch.empty(nbytes // 8, dtype=torch.float64, device=cuda)
     status = torch.zeros(1, dtype=torch.int32, device=cuda)
