@@ -347,12 +347,15 @@ class SolveGroup:
 
 
 def default_smoothing_degree(mesh):
-    """Chebyshev degree of the smoother when the caller gives none: 1.  Measured on a B200
-    (FP64 multigrid-PCG to rtol 1e-12, every pass fused with its operator; degree 1 against
-    2 and 3): at 64^3 12 iterations and 3.5 ms against 8-9 and 4.5, 7 and 4.6; at 32^3 3.0
-    against 3.8 and 4.5 ms; at 16^3 2.1 against 2.5 and 2.7; at 12^3 2.1 against 2.2 and
-    2.5; only on a mesh that does not coarsen (37 x 50 x 23) degree 2 is 5 % faster."""
-    return 1
+    """Chebyshev degree of the smoother when the caller gives none: 1 where the Q1 levels
+    coarsen, and from half a million dofs up; 2 on a smaller mesh that does not (an odd axis),
+    whose iterations each pay for a Chebyshev solve of a whole Q1 grid.  Measured on a B200
+    (FP64 multigrid-PCG to rtol 1e-12, degree 1 against 2): 64^3 3.5 against 4.5 ms, 32^3 2.1
+    and 2.5, 12^3 1.3 and 1.3, 48 x 32 x 40 4.8 and 5.6; without coarsening 5 x 7 x 9 2.5 and
+    1.9, 13 x 17 x 9 3.2 and 2.3, 21 x 27 x 15 6.1 and 4.4, 37 x 50 x 23 7.4 and 5.5, 33^3 3.8
+    and 3.4, but 41 x 43 x 45 6.5 and 8.3, 63 x 61 x 59 9.8 and 13.2."""
+    coarsens = all(v % 2 == 0 and v >= 4 for v in mesh.n)
+    return 1 if coarsens or mesh.ndof >= 500_000 else 2
 
 
 MG_PRECISIONS = ("fp64", "fp32")
