@@ -23,10 +23,10 @@
 //
 // Bound: FP64 arithmetic (~700 operations an element) and its latency.  At 64^3 that is
 // 10 us at the full FP64 rate; the 91 MB of traffic take 14 us at the measured copy rate.
-// Measured with the product's inner product (CG's A p): 41 us at 64^3, 20 at 48^3, 14 at
-// 32^3, 9 at 16^3, against 80, 37, 16 and 10 us for an element pass (three threads an
+// Measured with the product's inner product (CG's A p): 40-42 us at 64^3, 20.7 at 48^3, 13.8
+// at 32^3, 8.4 at 16^3, against 80, 37, 16 and 10 us for an element pass (three threads an
 // element, element results through memory) and a node gather.  A layer of two CTAs takes
-// ~4,800 cycles: ~2,000 the arithmetic (1,350 at the full rate), 1,000 the requests, 950
+// ~5,000 cycles: ~2,000 the arithmetic (1,400 at the full rate), 1,000 the requests, 950
 // the epilogue; 12 warps per SM at 168 registers spill and are slower (81 us).  D as one
 // TMA box: row by row as bulk copies, or per thread by 8-byte copies, the issue alone
 // costs 1,500-2,500 cycles a layer.
@@ -74,7 +74,8 @@ struct ApplyArgs {
   uint32_t* caller;        // the caller's (NULL: none)
   double* fail;            // the solve's SC_FAIL (NULL: none)
   int tma, pitch;          // D by TMA; its row pitch
-  double f;                // OUT_VEC
+  double f;                // OUT_VEC: the source, and int phi along each axis (phi_1d)
+  double phi[3][3];
 };
 
 // ------------------------------------------------------------- 1D transforms
@@ -115,10 +116,10 @@ __device__ __forceinline__ void add_from_derivs(T f0, T f1, T f2, T w, T w4, T& 
   r2 = fma(w, fma(T(-2), m, t), r2);
 }
 
-// int phi over its elements of a node's 1D basis function, on an axis of n elements of
-// size h
-__device__ __forceinline__ double phi_1d(int i, int n, double h) {
-  return (i & 1) ? h * (2.0 / 3.0) : (i == 0 || i == 2 * n) ? h / 6.0 : h / 3.0;
+// int phi over its elements of a node's 1D basis function, on an axis of n elements: w[0] a
+// middle node's, w[1] an end of the axis, w[2] between two elements
+__device__ __forceinline__ double phi_1d(int i, int n, const double (&w)[3]) {
+  return (i & 1) ? w[0] : (i == 0 || i == 2 * n) ? w[1] : w[2];
 }
 
 // A node plane at the element to its 9 points, less its middle node's value (x its first
@@ -531,8 +532,8 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
           } else if constexpr (OUT == OUT_VEC) {
             double v = acc;
             if (a.f != 0.0)
-              v -= a.f * (phi_1d(2 * cx + (k & 1), L.nx, L.hx) * phi_1d(2 * cy + (k >> 1), L.ny, L.hy) *
-                          phi_1d(2 * cz + a3, L.nz, L.hz));
+              v -= a.f * (phi_1d(2 * cx + (k & 1), L.nx, a.phi[0]) * phi_1d(2 * cy + (k >> 1), L.ny, a.phi[1]) *
+                          phi_1d(2 * cz + a3, L.nz, a.phi[2]));
             a.y[node] = (vec)(fx ? 0.0 : v);
           } else if constexpr (OUT == OUT_POWER) {
             a.y[node] = (vec)(fx ? 0.0 : acc * gn[h]);
@@ -593,9 +594,9 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlock
 // basis: grad_tile.  With mhat, D = w|J| e^m mhat and these are the second-order products
 // along mhat.  Bound: FP64 arithmetic (27 exponentials, then ~680 operations an element and
 // vector), D through memory once between the two launches.  Measured at 64^3: three vectors
-// 158 us (D 28), the gradient alone 78; at 32^3 46 and 20, at 16^3 15 and 12, at 8^3 13 and
-// 12, against 489 and 382, 70 and 55, 20 and 13, 14 and 7 us for an element pass whose
-// stages all went through shared memory and a node gather per vector.
+// 159 us (D 28; 173 with L2 flushed before), the gradient alone 73; at 32^3 45 and 19, at
+// 16^3 14 and 11, against 486 (499) and 381, 68 and 53, 19 and 12 us for an element pass
+// whose stages all go through shared memory and a node gather per vector.
 
 // D at the points of every element (a thread each), and the check that every pointwise value
 // the vectors are made of (E = D grad u, F = D grad p, W) is finite: by bounds on the nodes'
@@ -1165,6 +1166,10 @@ int hm_launch_vectors(const Lattice& L, const double* u, const double* m, const 
     ApplyArgs<double, double>& a = v.a[i];
     a.ess = zero_ess; a.x = i == 0 ? u : p; a.y = outs[i];
     a.f = i == 0 && mhat == nullptr ? f : 0.0;
+    const double h[3] = {L.hx, L.hy, L.hz};
+    for (int d = 0; d < 3; ++d) {
+      a.phi[d][0] = h[d] * (2.0 / 3.0); a.phi[d][1] = h[d] / 6.0; a.phi[d][2] = h[d] / 3.0;
+    }
     a.pitch = pitch;
     a.status = hm_status_word();
     a.caller = status;
