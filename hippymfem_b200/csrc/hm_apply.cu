@@ -34,6 +34,7 @@
 #include <cudaTypedefs.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "hm_async.cuh"
 #include "hm_common.cuh"
@@ -58,23 +59,34 @@ enum ApplyOut { OUT_Y = 0, OUT_R = 1, OUT_STEP1 = 2, OUT_START = 3, OUT_NEXT = 4
 // the constant of HmCheb's kChebMax (cheb[1 + k]: c1_k, cheb[1 + kChebMax + k]: c2_k)
 constexpr int kChebMax = 40;
 
+// (a launch pays for the bytes of its parameters, ~0.1 us for 90: each kind of pass has its own)
 template <typename src, typename vec>
 struct ApplyArgs {
   const uint8_t* ess;
   const src* x;            // the input vector
-  vec* y;                  // OUT_Y
-  HmCheb<vec> c;           // the smoother's operands
+  vec* y;                  // OUT_Y, OUT_VEC, OUT_POWER
   double* part;            // partial sums of x . y (OUT_Y) or b . z, one per CTA (NULL: none)
   double* sc;              // with part: the CG step's scalars (alpha or beta from the last block)
   unsigned* counter;
+  double* fail;            // the solve's SC_FAIL (NULL: none)
+  uint32_t* status;        // the library's status word (a bounded wait that gave up)
+  int tma, pitch;          // D by TMA; its row pitch
+  double sx, ry, rz;       // the product's scale, the weights of the y and z derivatives in it
+};
+// beside them for a pass of the smoother or of the power iteration
+template <typename src, typename vec>
+struct SmoothArgs : ApplyArgs<src, vec> {
+  HmCheb<vec> c;
   const double* rr;        // beta: the partials of r.r
   unsigned nrr;
   int flex;
-  uint32_t* status;        // the library's status word (a bounded wait that gave up)
-  uint32_t* caller;        // the caller's (NULL: none)
-  double* fail;            // the solve's SC_FAIL (NULL: none)
-  int tma, pitch;          // D by TMA; its row pitch
-  double f;                // OUT_VEC: the source, and int phi along each axis (phi_1d)
+};
+template <typename src, typename vec, int OUT>
+using PassArgs = std::conditional_t<OUT == OUT_Y, ApplyArgs<src, vec>, SmoothArgs<src, vec>>;
+// beside them for an assembled vector (OUT_VEC)
+struct VecPart : ApplyArgs<double, double> {
+  uint32_t* caller;        // the caller's status word
+  double f;                // the source, and int phi along each axis (phi_1d)
   double phi[3][3];
 };
 
@@ -249,9 +261,9 @@ struct ApplySmem {
 };
 
 // the work of one CTA, tile bt (D by the map at `map`)
-template <typename real, typename src, typename vec, int IN, int OUT>
+template <typename real, typename src, typename vec, int IN, int OUT, typename Args>
 __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice& L, const real* __restrict__ Dq,
-                                           const ApplyArgs<src, vec>& a, const int bt) {
+                                           const Args& a, const int bt) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ unsigned long long mbar[2];           // D of the even and the odd layers
   const ApplySmem<real, src> at(L.ap);
@@ -307,7 +319,7 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
       const src* const x = a.x + (size_t)nsz * (2 * c3 + j);
 #pragma unroll
       for (int k = 0; k < kApplyItems; ++k)
-        if constexpr (OUT == OUT_VEC) {    // (beside grad_tile's passes: 158 us against 163)
+        if constexpr (OUT == OUT_VEC) {    // (a branch is the faster here, beside grad_tile: 158 us against 163 for three)
           if (off[k] != ~0u) copy_async(plane + k * nt, x + off[k], true);
         } else {
           copy_async(plane + k * nt, x + off[k], off[k] != ~0u);
@@ -362,8 +374,7 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
   }
   __syncthreads();
 
-  // the derivatives carry 2 sqrt(0.15) each: 1 / (4 * 0.15) in the product
-  const real sx = (real)L.ap.sx, ry = (real)L.ap.ry, rz = (real)L.ap.rz;
+  const real sx = (real)a.sx, ry = (real)a.ry, rz = (real)a.rz;
   const int base = 2 * ty * RS + 2 * tx;  // the element's first node in a plane
   // in-plane values of the lower node plane less its middle node's, that value, sums of the
   // lower layer on it, the input at the own nodes there.  (The operator annihilates
@@ -499,8 +510,8 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
     if (__syncthreads_or(!ok || L.give_up)) {   // a copy never landed: flagged, nothing more written
       if (tid == 0) {
         if (a.status != nullptr) atomicOr(a.status, HM_STATUS_TIMEOUT);
-        if (a.caller != nullptr) atomicOr(a.caller, HM_STATUS_TIMEOUT);
-        if (a.fail != nullptr) *a.fail = 1.0;
+        if constexpr (OUT == OUT_VEC) atomicOr(a.caller, HM_STATUS_TIMEOUT);
+        else if (a.fail != nullptr) *a.fail = 1.0;
         // both buffers' copies, before the CTA leaves
         (void)mbar_wait(&mbar[l & 1], (uint32_t)(l >> 1) & 1u);
         if (l + 1 < layers && cz + 1 < L.nz) (void)mbar_wait(&mbar[(l + 1) & 1], (uint32_t)((l + 1) >> 1) & 1u);
@@ -569,14 +580,16 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
     }
   }
   copy_wait<0>();
-  if (OUT != OUT_R && OUT != OUT_START && OUT != OUT_VEC && OUT != OUT_POWER && a.part != nullptr) {
-    __shared__ double sh[32];
-    const double t = block_sum(dot, sh);
-    if (tid == 0) a.part[blockIdx.x] = t;
-    // a CG step: the last block takes alpha, or beta, from the partials
-    if (a.sc != nullptr && last_block(a.counter)) {
-      if constexpr (OUT == OUT_Y) finish_alpha(a.part, gridDim.x, a.sc, a.counter, sh);
-      else finish_beta(a.part, gridDim.x, a.rr, a.nrr, a.flex, a.sc, a.counter, sh);
+  if constexpr (OUT != OUT_R && OUT != OUT_START && OUT != OUT_VEC && OUT != OUT_POWER) {
+    if (a.part != nullptr) {
+      __shared__ double sh[32];
+      const double t = block_sum(dot, sh);
+      if (tid == 0) a.part[blockIdx.x] = t;
+      // a CG step: the last block takes alpha, or beta, from the partials
+      if (a.sc != nullptr && last_block(a.counter)) {
+        if constexpr (OUT == OUT_Y) finish_alpha(a.part, gridDim.x, a.sc, a.counter, sh);
+        else finish_beta(a.part, gridDim.x, a.rr, a.nrr, a.flex, a.sc, a.counter, sh);
+      }
     }
   }
 }
@@ -584,7 +597,7 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
 template <typename real, typename src, typename vec, int IN, int OUT>
 __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlocks : kApplyBlocks32)
     k_apply_tile(const __grid_constant__ CUtensorMap map, const Lattice L, const real* __restrict__ Dq,
-                 const ApplyArgs<src, vec> a) {
+                 const PassArgs<src, vec, OUT> a) {
   apply_tile<real, src, vec, IN, OUT>(&map, L, Dq, a, (int)blockIdx.x);
 }
 
@@ -594,7 +607,7 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(real) == 8 ? kApplyBlock
 // basis: grad_tile.  With mhat, D = w|J| e^m mhat and these are the second-order products
 // along mhat.  Bound: FP64 arithmetic (27 exponentials, then ~680 operations an element and
 // vector), D through memory once between the two launches.  Measured at 64^3: three vectors
-// 159 us (D 28; 173 with L2 flushed before), the gradient alone 73; at 32^3 45 and 19, at
+// 152 us (D 28; 163 with L2 flushed before), the gradient alone 73; at 32^3 44 and 19, at
 // 16^3 14 and 11, against 486 (499) and 381, 68 and 53, 19 and 12 us for an element pass
 // whose stages all go through shared memory and a node gather per vector.
 
@@ -709,7 +722,7 @@ struct GradSmem {
 __device__ __forceinline__ void grad_tile(const CUtensorMap* map, const Lattice& L, const double* __restrict__ Dq,
                                           int tma, int pitch, const double* __restrict__ u,
                                           const double* __restrict__ p, double* __restrict__ yout,
-                                          uint32_t* status, uint32_t* caller, const int bt) {
+                                          const VecPart& a, const int bt) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ unsigned long long mbar;
   const GradSmem at(L.ap);
@@ -769,7 +782,7 @@ __device__ __forceinline__ void grad_tile(const CUtensorMap* map, const Lattice&
   const bool column = ty < T2;
   const bool element = column && cx < L.nx && cy < L.ny;
   const bool own = column && cx <= L.nx && cy <= L.ny && (tx > 0 || i1 == 0) && (ty > 0 || i2 == 0);
-  const double sx = L.ap.sx, ry = L.ap.ry, rz = L.ap.rz;
+  const double sx = a.sx, ry = a.ry, rz = a.rz;
   const int base = 2 * ty * RS + 2 * tx, ds = T2 * TB;
   double carry[9];
 #pragma unroll
@@ -865,8 +878,8 @@ __device__ __forceinline__ void grad_tile(const CUtensorMap* map, const Lattice&
     copy_wait<0>();                        // the next layer's planes
     if (__syncthreads_or(!ok || L.give_up)) {
       if (tid == 0) {
-        if (status != nullptr) atomicOr(status, HM_STATUS_TIMEOUT);
-        atomicOr(caller, HM_STATUS_TIMEOUT);
+        if (a.status != nullptr) atomicOr(a.status, HM_STATUS_TIMEOUT);
+        atomicOr(a.caller, HM_STATUS_TIMEOUT);
         (void)mbar_wait(&mbar, (uint32_t)l & 1u);        // the copy, before the CTA leaves
       }
       break;
@@ -896,7 +909,7 @@ __device__ __forceinline__ void grad_tile(const CUtensorMap* map, const Lattice&
 // The requested vectors in one launch: `count` CTAs in a row take one tile's vectors, so
 // that its D comes from memory once.
 struct VecArgs {
-  ApplyArgs<double, double> a[2];      // ADJOINT, STATE
+  VecPart a[2];                        // ADJOINT, STATE
   const double* u;
   const double* p;
   double* grad;                        // PARAMETER
@@ -908,7 +921,7 @@ __global__ void __launch_bounds__(kApplyThreads, 2)
               const __grid_constant__ VecArgs v) {
   if (v.skip != nullptr && *v.skip != 0u) return;
   const int bt = (int)blockIdx.x / v.count, w = v.which[(int)blockIdx.x - bt * v.count];
-  if (w == 2) grad_tile(&map, L, D, v.a[0].tma, v.a[0].pitch, v.u, v.p, v.grad, v.a[0].status, v.a[0].caller, bt);
+  if (w == 2) grad_tile(&map, L, D, v.a[0].tma, v.a[0].pitch, v.u, v.p, v.grad, v.a[0], bt);
   else apply_tile<double, double, double, IN_CLEAN, OUT_VEC>(&map, L, D, v.a[w], bt);
 }
 
@@ -986,9 +999,6 @@ void hm_plan_apply(Lattice* L) {
       }
     }
   }
-  p.sx = 1.0 / (0.6 * L->hx * L->hx);
-  p.ry = (L->hx * L->hx) / (L->hy * L->hy);
-  p.rz = (L->hx * L->hx) / (L->hz * L->hz);
   L->ap = p;
 }
 
@@ -1013,6 +1023,14 @@ int raise_smem(K kern, std::atomic<uint64_t>& done) {
   }
   return HM_OK;
 }
+// what a pass takes from the lattice's edges (the derivatives carry 2 sqrt(0.15) each: 1 / 0.6
+// in the product)
+template <typename src, typename vec>
+void set_scales(const Lattice& L, ApplyArgs<src, vec>& a) {
+  a.sx = 1.0 / (0.6 * L.hx * L.hx);
+  a.ry = (L.hx * L.hx) / (L.hy * L.hy);
+  a.rz = (L.hx * L.hx) / (L.hz * L.hz);
+}
 // the map of D [q][ez][ey][ex] with rows `pitch` apart; *tma = 0 where its storage has no
 // 16-byte base or pitch
 template <typename real>
@@ -1033,13 +1051,14 @@ int map_D(const Lattice& L, const void* D, int pitch, CUtensorMap* map, int* tma
              ? HM_OK : HM_ERR_CUDA;
 }
 template <typename real, typename src, typename vec, int IN, int OUT>
-int launch(const Lattice& L, const void* jac, int pitch, ApplyArgs<src, vec> a, void* stream) {
+int launch(const Lattice& L, const void* jac, int pitch, PassArgs<src, vec, OUT> a, void* stream) {
   auto kern = k_apply_tile<real, src, vec, IN, OUT>;
   static std::atomic<uint64_t> done{0};
   int rc = raise_smem(kern, done);
   if (rc) return rc;
   a.pitch = pitch;
   a.status = hm_status_word();
+  set_scales(L, a);
   CUtensorMap map{};
   if ((rc = map_D<real>(L, jac, pitch, &map, &a.tma))) return rc;
   kern<<<L.ap.t1 * L.ap.t2 * L.ap.t3, L.ap.threads, (size_t)ApplySmem<real, src>(L.ap).bytes,
@@ -1047,7 +1066,7 @@ int launch(const Lattice& L, const void* jac, int pitch, ApplyArgs<src, vec> a, 
   return cudaGetLastError() == cudaSuccess ? HM_OK : HM_ERR_CUDA;
 }
 template <typename real, typename src, typename vec, int IN, int OUT>
-int launch(const Lattice& L, const void* jac, const ApplyArgs<src, vec>& a, void* stream) {
+int launch(const Lattice& L, const void* jac, const PassArgs<src, vec, OUT>& a, void* stream) {
   return launch<real, src, vec, IN, OUT>(L, jac, hm_jac_pitch(L, sizeof(real) == 8 ? HM_FP64 : HM_FP32), a, stream);
 }
 template <typename real, typename T>
@@ -1086,7 +1105,7 @@ int hm_launch_apply_A_clean(const Lattice& L, void* jac, const uint8_t* ess, con
 // y = D^-1 A x, x zero on the Dirichlet nodes: a step of the power iteration
 int hm_launch_power(const Lattice& L, void* jac, const uint8_t* ess, const double* idiag, const double* x,
                     double* y, void* stream) {
-  ApplyArgs<double, double> a{};
+  SmoothArgs<double, double> a{};
   a.ess = ess; a.x = x; a.y = y; a.c.idiag = idiag;
   return launch<double, double, double, IN_CLEAN, OUT_POWER>(L, jac, a, stream);
 }
@@ -1107,7 +1126,7 @@ int hm_launch_apply_A32_dot(const Lattice& L, void* jac32, const uint8_t* ess, c
 // In the FP32 cycle in, x, r and dout are FP32; b, the update and z stay FP64.
 template <typename T>
 int hm_launch_cheb(const Lattice& L, void* jac, const uint8_t* ess, const HmCheb<T>& c, void* stream) {
-  ApplyArgs<T, T> a{};
+  SmoothArgs<T, T> a{};
   a.ess = ess; a.x = c.in; a.c = c; a.fail = c.fail;
   a.c.beta = nullptr;                      // a host address
   if (c.beta != nullptr && (c.mode == CH_STEP1 || (c.mode == CH_NEXT && c.last == 2))) {
@@ -1163,7 +1182,7 @@ int hm_launch_vectors(const Lattice& L, const double* u, const double* m, const 
   VecArgs v{};
   v.u = u; v.p = p; v.grad = outs[2]; v.skip = skip;
   for (int i = 0; i < 2; ++i) {
-    ApplyArgs<double, double>& a = v.a[i];
+    VecPart& a = v.a[i];
     a.ess = zero_ess; a.x = i == 0 ? u : p; a.y = outs[i];
     a.f = i == 0 && mhat == nullptr ? f : 0.0;
     const double h[3] = {L.hx, L.hy, L.hz};
@@ -1173,6 +1192,7 @@ int hm_launch_vectors(const Lattice& L, const double* u, const double* m, const 
     a.pitch = pitch;
     a.status = hm_status_word();
     a.caller = status;
+    set_scales(L, a);
     if ((rc = map_D<double>(L, D, pitch, &map, &a.tma))) return rc;
   }
   for (int i = 0; i < 3; ++i)

@@ -88,9 +88,8 @@ HM_HD constexpr double vrow_coef(int tab, int r, int t) {
 
 // ------------------------------------------------------------------ lattice
 // tiling of the matrix-free apply: t1 x t2 x t3 tiles of T1 x T2 x T3 cells (the halo
-// included), `threads` per CTA; the scale of the product, the weights of the y and z
-// derivatives in it
-struct ApplyPlan { int T1, T2, T3, t1, t2, t3, threads; double sx, ry, rz; };
+// included), `threads` per CTA
+struct ApplyPlan { int T1, T2, T3, t1, t2, t3, threads; };
 struct Lattice {
   int nx, ny, nz;      // elements per axis
   int Nx, Ny, Nz;      // nodes per axis (2 n + 1)
@@ -98,8 +97,8 @@ struct Lattice {
   double hx, hy, hz;   // element sizes
   int64_t ne, ndof;
   ApplyPlan ap;        // hm_plan_apply
-  int slab = 0;        // part of a larger mesh (hm_lattice_set_slab)
-  int give_up = 0;     // the tile-marching passes' waits count as run out (hm_lattice_fail_waits)
+  uint8_t slab = 0;    // part of a larger mesh (hm_lattice_set_slab)
+  uint8_t give_up = 0; // the tile-marching passes' waits count as run out (hm_lattice_fail_waits)
 };
 
 // 1D stencil of node i on an axis of N nodes: [lo, lo + n)

@@ -98,7 +98,7 @@ struct HmCheb {
   T* dout;
   double* z;
   HmBeta* beta;
-  double* fail;
+  double* fail;             // the solve's SC_FAIL (NULL: none)
 };
 template <typename T>
 int hm_launch_cheb(const hm::Lattice& L, void* jac, const uint8_t* ess, const HmCheb<T>& c, void* stream);
