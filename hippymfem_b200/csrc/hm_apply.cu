@@ -215,8 +215,8 @@ __device__ __forceinline__ void element_points(T (&v0)[9], T (&v1)[9], T (&v2)[9
 
 // Loads where `on`, else 0, by a predicate and issued where they stand: with a branch around
 // each, as conditional expressions and statements compile to here, a layer's loads and copies
-// took 2,000 cycles to issue, with predicates 900 (16^3, y = A x alone: 9.8 -> 6.7 us in FP64,
-// 11.9 -> 6.3 in FP32; 64^3 49.8 -> 38.6 and 57.2 -> 33.8).
+// took 2,000 cycles to issue, with predicates 900 (16^3, y = A x alone: 9.8 -> 7.0 us in FP64,
+// 11.9 -> 6.8 in FP32; 64^3 49.8 -> 38.8 and 57.2 -> 33.5).
 __device__ __forceinline__ uint32_t load_mark(const uint8_t* p, bool on) {
   uint32_t m;
   asm volatile(

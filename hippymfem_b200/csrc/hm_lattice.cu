@@ -256,8 +256,8 @@ __global__ void k_extract_D(Lattice L, int pitch, const src* __restrict__ quad, 
 // contributions by contractions along x, y and z (567 multiply-adds; 27 x 27 products of
 // three factors and three directions node by node), then the nodes sum those of the elements
 // that touch them in a fixed order.  Bound: the latency of the loads, 216 of every 1728
-// bytes.  64^3 elements: 328 us node by node, 95 here; 45 x 52 x 39 117 and 34; 16^3 11 and
-// 14 (few blocks, each a longer chain).
+// bytes.  64^3 elements: 328 us node by node, 95 here; 45 x 52 x 39 117 and 34; 32^3 48 and
+// 13.5; 16^3 10.7 both, 8^3 10.1 and 10.5 (few blocks, each a longer chain; graph replays).
 constexpr int kDiagX = 8, kDiagY = 4, kDiagZ = 4;
 constexpr int kDiagElems = (kDiagX + 1) * (kDiagY + 1) * (kDiagZ + 1);
 // squared derivatives by axis, point and node, divided by the squared edge

@@ -68,7 +68,7 @@ struct hm_mg {
   int fused;             // smoothing steps fused with their operator pass
   // the FP32 cycle (single != 0): every level's vectors, coefficients, reciprocal
   // diagonal and coarse inverse in single precision, refreshed from the FP64 set-up; the
-  // level-0 operator data (the points' D, then the element results) in jac32
+  // level-0 operator data (the points' D) in jac32
   int single;
   hm::MGLevelT<float> lv32[16];
   float* jac32;
@@ -470,16 +470,19 @@ __global__ void __launch_bounds__(256) k_coarse_solve(MGLevelT<T> lv, const T* _
 // ---- the coarse levels of a cycle in one cluster
 // Launched level by level, a coarse level costs four launches (eight at degree 2) of a few
 // microseconds each, almost all latency.  One cluster of CTAs runs the whole part of the
-// V-cycle from the restriction into its first level to that level's result, the same
-// arithmetic node for node.  Its vectors live in the CTAs' shared memory: a level's node
+// V-cycle from the restriction into its first level to that level's result, node for node the
+// same arithmetic but for the exact coarse solve (a warp sums a row by shuffles).  Its vectors live in the CTAs' shared memory: a level's node
 // planes are dealt out in slabs, a CTA computes its own planes and reads its neighbours'
 // through the cluster's shared memory, and a cluster barrier stands where the launches
 // were; coefficients and reciprocal diagonals are copied in at the start.  The levels of at
 // most kSoloNodes nodes lie in the first CTA alone, between block barriers.  Measured
 // (FP64, degree 1): 28 us for the levels 17^3, 9^3, 5^3, 3^3 of 32^3 and 64^3, 19 us for
 // 13^3, 7^3, 4^3, against ~47 and ~39 us as launches with one CTA from 1000 nodes down.  A
-// 33^3 level in the cluster takes 44 us more and ~16 us as launches: kTailNodes lies
-// between the two.  A level of 9^3 in one CTA takes 3 us more than in the cluster.
+// 33^3 level in the cluster takes 44 us more and ~16 us as launches.  An iteration with the
+// cluster from the level named down, against from the level below it: 17^3 73.6 us and 82.4
+// (16^3 elements), 21^3 76.6 and 84.9, 25x17x21 134 and 143, 25^3 89 and 92 (48^3: 165 and
+// 175), 29^3 125 and 123, 31x27x23 225 and 223 -- kTailNodes could lie at 16,000; it was set
+// between 17^3 and 33^3.  A level of 9^3 in one CTA takes 3 us more than in the cluster.
 constexpr int kTailMax = 8;
 constexpr int64_t kTailNodes = 5000;
 constexpr int64_t kSoloNodes = 150, kTailMost = 1 << 20;

@@ -423,8 +423,8 @@ class Multigrid:
         return self
 
     def set_fused(self, fused):
-        """Degree-1 smoothing steps fused with their operator pass (the default), or
-        launched step by step; the same arithmetic either way."""
+        """Smoothing steps fused with their operator pass (the default), or launched step
+        by step: equal to rounding, and bit for bit at degree 1 of the FP64 cycle."""
         check(lib.hm_mg_set_fused(self._mg, int(bool(fused))), "hm_mg_set_fused")
         return self
 

@@ -207,7 +207,7 @@ int hm_lattice_vectors_at(const hm_lattice* h, const double* d_u, const double* 
  * (modeling/PDEVariationalProblem.py:1672).  Its data d_jac (hm_lattice_jacobian_bytes)
  * holds D of the point in a layout the operator streams, filled once per point by
  * hm_lattice_jacobian_prepare from the quadrature data and only read by an apply (a part
- * of the array stays unused). */
+ * of the array stays unused).  d_y must not overlap d_x. */
 int64_t hm_lattice_jacobian_bytes(const hm_lattice* h, int precision);
 int hm_lattice_jacobian_prepare(const hm_lattice* h, const void* d_quad, int quad_precision,
                                 void* d_jac, int precision, void* stream);
@@ -408,14 +408,16 @@ int hm_mg_apply(hm_mg* mg, const double* d_r, double* d_z, void* stream);
 int hm_mg_levels(const hm_mg* mg);
 /* The Q1 levels with at most max_nodes nodes (5000 by default; 0: none) run in one launch
  * per cycle, a cluster of thread blocks with the levels' vectors in its shared memory,
- * instead of level by level (the same arithmetic, node for node), as far as the levels fit.
+ * instead of level by level (node for node the same arithmetic but for the exact coarse
+ * solve, whose sums are in another order), as far as the levels fit.
  * Set it before a plan's first solve: a plan's captured iteration batches keep the launches
  * they were captured with. */
 int hm_mg_set_tail_nodes(hm_mg* mg, int64_t max_nodes);
 /* Each smoothing step runs as one pass with its level's operator, on level 0 inside the
- * solves (every vector zero on the Dirichlet nodes) and on the Q1 levels; at degree 1 the
- * arithmetic is the step-by-step one, bit for bit (fused = 1, the default).  fused = 0
- * launches the steps one by one.  Set it before a plan's first solve, as the tail. */
+ * solves (every vector zero on the Dirichlet nodes) and on the Q1 levels; at degree 1 of the
+ * FP64 cycle the arithmetic is the step-by-step one, bit for bit (the FP32 cycle's level-0
+ * passes read and write FP64, the step-by-step one rounds the residual first).  fused = 1 is
+ * the default, 0 launches the steps one by one.  Set it before a plan's first solve, as the tail. */
 int hm_mg_set_fused(hm_mg* mg, int fused);
 /* The cycle in FP32 (d_work32 of hm_mg_single_workspace_bytes), or in FP64 again
  * (d_work32 = NULL, the default).  The set-up stays FP64; each set-up (and this call,
