@@ -71,12 +71,16 @@ struct ApplyArgs {
   double* fail;            // the solve's SC_FAIL (NULL: none)
   uint32_t* status;        // the library's status word (a bounded wait that gave up)
   int tma, pitch;          // D by TMA; its row pitch
-  double sx, ry, rz;       // the product's scale, the weights of the y and z derivatives in it
 };
 // beside them for a pass of the smoother or of the power iteration
 template <typename src, typename vec>
 struct SmoothArgs : ApplyArgs<src, vec> {
-  HmCheb<vec> c;
+  struct {                 // of HmCheb
+    int k, first, last;
+    const double *b, *idiag, *cheb;
+    vec *x, *r, *dout;
+    double* z;
+  } c;
   const double* rr;        // beta: the partials of r.r
   unsigned nrr;
   int flex;
@@ -85,6 +89,8 @@ template <typename src, typename vec, int OUT>
 using PassArgs = std::conditional_t<OUT == OUT_Y, ApplyArgs<src, vec>, SmoothArgs<src, vec>>;
 // beside them for an assembled vector (OUT_VEC)
 struct VecPart : ApplyArgs<double, double> {
+  double sx, ry, rz;       // apply_tile's (computed there they take 2 us of 158 at 64^3; a small
+                           // product is faster without the 24 bytes, 9.05 against 9.25 us at 12^3)
   uint32_t* caller;        // the caller's status word
   double f;                // the source, and int phi along each axis (phi_1d)
   double phi[3][3];
@@ -374,7 +380,16 @@ __device__ __forceinline__ void apply_tile(const CUtensorMap* map, const Lattice
   }
   __syncthreads();
 
-  const real sx = (real)a.sx, ry = (real)a.ry, rz = (real)a.rz;
+  // the product's scale (the derivatives carry 2 sqrt(0.15) each: 1 / (4 * 0.15) in the product),
+  // the weights of the y and z derivatives in it
+  real sx, ry, rz;
+  if constexpr (OUT == OUT_VEC) {
+    sx = a.sx; ry = a.ry; rz = a.rz;
+  } else {
+    sx = (real)(1.0 / (0.6 * L.hx * L.hx));
+    ry = (real)((L.hx * L.hx) / (L.hy * L.hy));
+    rz = (real)((L.hx * L.hx) / (L.hz * L.hz));
+  }
   const int base = 2 * ty * RS + 2 * tx;  // the element's first node in a plane
   // in-plane values of the lower node plane less its middle node's, that value, sums of the
   // lower layer on it, the input at the own nodes there.  (The operator annihilates
@@ -1023,14 +1038,6 @@ int raise_smem(K kern, std::atomic<uint64_t>& done) {
   }
   return HM_OK;
 }
-// what a pass takes from the lattice's edges (the derivatives carry 2 sqrt(0.15) each: 1 / 0.6
-// in the product)
-template <typename src, typename vec>
-void set_scales(const Lattice& L, ApplyArgs<src, vec>& a) {
-  a.sx = 1.0 / (0.6 * L.hx * L.hx);
-  a.ry = (L.hx * L.hx) / (L.hy * L.hy);
-  a.rz = (L.hx * L.hx) / (L.hz * L.hz);
-}
 // the map of D [q][ez][ey][ex] with rows `pitch` apart; *tma = 0 where its storage has no
 // 16-byte base or pitch
 template <typename real>
@@ -1058,7 +1065,6 @@ int launch(const Lattice& L, const void* jac, int pitch, PassArgs<src, vec, OUT>
   if (rc) return rc;
   a.pitch = pitch;
   a.status = hm_status_word();
-  set_scales(L, a);
   CUtensorMap map{};
   if ((rc = map_D<real>(L, jac, pitch, &map, &a.tma))) return rc;
   kern<<<L.ap.t1 * L.ap.t2 * L.ap.t3, L.ap.threads, (size_t)ApplySmem<real, src>(L.ap).bytes,
@@ -1127,8 +1133,8 @@ int hm_launch_apply_A32_dot(const Lattice& L, void* jac32, const uint8_t* ess, c
 template <typename T>
 int hm_launch_cheb(const Lattice& L, void* jac, const uint8_t* ess, const HmCheb<T>& c, void* stream) {
   SmoothArgs<T, T> a{};
-  a.ess = ess; a.x = c.in; a.c = c; a.fail = c.fail;
-  a.c.beta = nullptr;                      // a host address
+  a.ess = ess; a.x = c.in; a.fail = c.fail;
+  a.c = {c.k, c.first, c.last, c.b, c.idiag, c.cheb, c.x, c.r, c.dout, c.z};
   if (c.beta != nullptr && (c.mode == CH_STEP1 || (c.mode == CH_NEXT && c.last == 2))) {
     a.part = c.beta->rz; a.sc = c.beta->sc; a.counter = c.beta->counter;
     a.rr = c.beta->rr; a.nrr = c.beta->n; a.flex = c.beta->flex;
@@ -1192,7 +1198,9 @@ int hm_launch_vectors(const Lattice& L, const double* u, const double* m, const 
     a.pitch = pitch;
     a.status = hm_status_word();
     a.caller = status;
-    set_scales(L, a);
+    a.sx = 1.0 / (0.6 * L.hx * L.hx);
+    a.ry = (L.hx * L.hx) / (L.hy * L.hy);
+    a.rz = (L.hx * L.hx) / (L.hz * L.hz);
     if ((rc = map_D<double>(L, D, pitch, &map, &a.tma))) return rc;
   }
   for (int i = 0; i < 3; ++i)

@@ -128,9 +128,10 @@ HM_HD int64_t row_start(const Lattice& L, int i, int j, int k) {
 
 // ------------------------------------------------------------ PCG device scalars
 // (shared by the solver and the operator kernels that finish a CG step's reductions).
-// SC_FAIL: nonzero once a pass of the solve has given up a wait, its outputs invalid
+// SC_FAIL: nonzero once a pass of the solve has given up a wait, its outputs invalid;
+// SC_CNT: two counters (unsigned) of the reductions that their kernels finish
 enum { SC_RZ = 0, SC_PQ, SC_ALPHA, SC_BETA, SC_RR, SC_BB, SC_TOL2, SC_CONV, SC_TMP0, SC_TMP1,
-       SC_TMP2, SC_IT, SC_FAIL, SC_N };
+       SC_TMP2, SC_IT, SC_FAIL, SC_CNT, SC_N };
 
 #ifdef __CUDACC__
 // sum over the block (valid in thread 0); every thread of the block must call it

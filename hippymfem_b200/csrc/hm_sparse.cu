@@ -472,11 +472,12 @@ int op_apply(const PcgOp& o, const float* x, float* y, void* stream, double* sc,
   return hm_launch_apply_A32_dot(*o.L, o.jac, o.ess, x, y, part, stream, sc, counter);
 }
 
-// at a solve's start: the two counters of pcg_batch, and no pass has failed
-int reset_counters(double* sc, unsigned* cnt, cudaStream_t s) {
-  return cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned), s) == cudaSuccess &&
-                 cudaMemsetAsync(sc + SC_FAIL, 0, sizeof(double), s) == cudaSuccess
-             ? HM_OK : HM_ERR_CUDA;
+// the two counters of a solve (pcg_batch), zero between uses
+inline unsigned* solve_counters(double* sc) { return reinterpret_cast<unsigned*>(sc + SC_CNT); }
+// at a solve's start: the counters, and no pass has failed
+int reset_counters(double* sc, cudaStream_t s) {
+  static_assert(SC_CNT == SC_FAIL + 1 && sizeof(double) == 2 * sizeof(unsigned), "one fill");
+  return cudaMemsetAsync(sc + SC_FAIL, 0, 2 * sizeof(double), s) == cudaSuccess ? HM_OK : HM_ERR_CUDA;
 }
 
 // `count` PCG iterations (operator with p.q and alpha, update with r.z and r.r, beta,
@@ -547,9 +548,9 @@ int pcg_run(const PcgOp& o, const double* diag, const T* b, T* x, double rtol, i
   double* pq_part = wd;
   double* sc = wd + pq_slots(n);
   double* part = sc + SC_N;
-  unsigned* cnt = reinterpret_cast<unsigned*>(part + 3 * kReduceBlocks);
+  unsigned* cnt = solve_counters(sc);
   if (check_every <= 0) check_every = 1;
-  if (reset_counters(sc, cnt, s) != HM_OK) return HM_ERR_CUDA;
+  if (reset_counters(sc, s) != HM_OK) return HM_ERR_CUDA;
   int rc;
   // x = b on the Dirichlet nodes: every residual and direction is then zero there, which
   // the lattice operator's direction products rely on
@@ -617,9 +618,9 @@ int pcg_mg_run(hm_mg* mg, const double* b, double* x, double rtol, int maxiter, 
   double* pq_part = w + 4 * n;
   double* sc = pq_part + pq_slots(n);
   double* part = sc + SC_N;
-  unsigned* cnt = reinterpret_cast<unsigned*>(part + 3 * kReduceBlocks);
+  unsigned* cnt = solve_counters(sc);
   if (check_every <= 0) check_every = 1;
-  if (reset_counters(sc, cnt, s) != HM_OK) return HM_ERR_CUDA;
+  if (reset_counters(sc, s) != HM_OK) return HM_ERR_CUDA;
   int rc = hm_launch_ess_take_b(*L, o.ess, b, x, stream);   // as in pcg_run
   if (rc) return rc;
   rc = op_apply(o, x, q, stream, sc);
@@ -718,7 +719,7 @@ int pcg_mixed_run(const hm::Lattice* L, void* jac64, void* jac32, const uint8_t*
   double* sc = pq_part + pq_slots(n);
   double* part = sc + SC_N;
   double* bbp = part + 3 * kReduceBlocks;
-  unsigned* cnt = reinterpret_cast<unsigned*>(bbp + 1);
+  unsigned* cnt = solve_counters(sc);
   float* f32 = reinterpret_cast<float*>(bbp + 8);
   float* x32 = f32;
   float* r32 = f32 + n;
@@ -754,7 +755,6 @@ int pcg_mixed_run(const hm::Lattice* L, void* jac64, void* jac32, const uint8_t*
     return read();
   };
   if (cudaMemsetAsync(sc, 0, sizeof(double) * SC_N, s) != cudaSuccess ||
-      cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned), s) != cudaSuccess ||
       cudaMemsetAsync(x, 0, sizeof(double) * n, s) != cudaSuccess ||
       cudaMemsetAsync(x32, 0, sizeof(float) * n, s) != cudaSuccess)
     return HM_ERR_CUDA;
@@ -941,7 +941,7 @@ PlanBufs plan_bufs(const hm_pcg_plan* pl) {
   b.pq_part = w + 4 * n;
   b.sc = b.pq_part + pq_slots(n);
   b.part = b.sc + SC_N;
-  b.cnt = reinterpret_cast<unsigned*>(b.part + 3 * kReduceBlocks);
+  b.cnt = solve_counters(b.sc);
   return b;
 }
 
@@ -950,7 +950,7 @@ int group_init(hm_pcg_plan* pl, double rtol, cudaStream_t s) {
   const int64_t n = pl->L.ndof;
   const PlanBufs B = plan_bufs(pl);
   PcgOp o{n, nullptr, nullptr, nullptr, &pl->L, pl->jac64, HM_FP64, pl->ess};
-  if (cudaMemsetAsync(pl->x, 0, sizeof(double) * n, s) != cudaSuccess || reset_counters(B.sc, B.cnt, s) != HM_OK)
+  if (cudaMemsetAsync(pl->x, 0, sizeof(double) * n, s) != cudaSuccess || reset_counters(B.sc, s) != HM_OK)
     return HM_ERR_CUDA;
   int rc = hm_launch_ess_take_b(pl->L, o.ess, pl->b, pl->x, (void*)s);
   if (rc) return rc;
